@@ -142,7 +142,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const int nsub = 2 * nkv;                         // 64-key half blocks
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = true;
             mbar_expect_tx(q_full, TILE_BYTES);
             tma_load_3d(sQ, &tmQ, q_full, 0, q0, bh);
@@ -158,7 +158,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 11); }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // Half blocks of 64 keys, software-pipelined: the scores of half block i+2 are issued as soon
             // as the softmax warps have drained buffer i&1, so the tensor core works on Q K^T (i+1, i+2)
             // and P V (i-1) while the softmax of i runs -- no step waits for a full round trip.
@@ -532,7 +532,7 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     const uint32_t tS = tmem_base, tdP = tmem_base + 128, tdV = tmem_base + 256, tdK = tmem_base + 320;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = true;
             mbar_expect_tx(kv_full, 2 * TILE_BYTES);
             tma_load_3d(sK, &tmK, kv_full, 0, k0, bh);
@@ -549,7 +549,7 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 21); }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t id_s = umma_idesc(1u, 0u, 0u, 128, 128);      // Q K^T, dO V^T
             const uint64_t dKk = kmajor_tile(smem_u32(sK)), dVk = kmajor_tile(smem_u32(sV));
             const uint64_t dQk0 = kmajor_tile(smem_u32(sQ)), ddOk0 = kmajor_tile(smem_u32(sdO));
@@ -575,7 +575,7 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
         }
     } else if (warp == 10) {
         // second issuer: dV += P^T dO and dK += dS^T Q once the compute warps have written P and dS
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t id_t = umma_idesc(1u, 1u, 1u, 128, 64);       // both operands MN-major
             const uint64_t dPm = mnmajor_tile(smem_u32(sP), TILE_BYTES), ddSm0 = mnmajor_tile(smem_u32(sdS), TILE_BYTES);
             const long long nblk = (long long)p.nq * (p.nq + 1) / 2;
@@ -775,7 +775,7 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     pdl_wait();                 // everything above is independent of earlier kernels' results
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = true;
             const long long nblk = (long long)p.nq * (p.nq + 1) / 2;
             const uint8_t* src = reinterpret_cast<const uint8_t*>(p.ds) +
@@ -792,7 +792,7 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 31); }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t id_q = umma_idesc(1u, 0u, 1u, 128, 64);       // dS (K-major) x K block (MN-major)
             bool ok = true;
             for (int it = 0; it < niter && ok; ++it) {

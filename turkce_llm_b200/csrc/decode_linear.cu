@@ -177,7 +177,7 @@ decode_linear_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
     }
     __syncthreads();
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---- producer: the activations (when they arrive as bf16) and the rest of the slab
         bool ok = true;
         if (!p.norm) {
@@ -194,7 +194,7 @@ decode_linear_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_const
         }
         pdl_launch_dependents_now();
         if (!ok) { *abort_flag = 1; atomicExch(p.err, 51); }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---- MMA issuer: D[128 columns, 64 sequences] += W_slab^T (MN-major) . X^T (K-major)
         const uint32_t idesc = umma_idesc(1u, 1u, 0u, DL_COLS, DL_SEQ);
         bool ok = p.norm ? true : mbar_wait(x_bar, 0u, abort_flag);

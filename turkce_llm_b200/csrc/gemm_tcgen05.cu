@@ -230,7 +230,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             int stage = 0; uint32_t phase = 0;
             bool ok = true;
             for (int t = worker; t < total_tiles && ok; t += nworkers) {
@@ -284,7 +284,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
     } else if (warp == 1) {
         // -------------------------------------------------------------- MMA issuer (PAIR: rank 0 for both CTAs)
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             constexpr int UMMA_N = BN == 384 ? 128 : BN;       // columns per tensor-core instruction
             constexpr int NSUB = BN / UMMA_N;
             const uint32_t idesc = umma_idesc(TF32 ? 2u : 1u, (uint32_t)p.a_mn, (uint32_t)p.b_mn, TILE_M, UMMA_N);

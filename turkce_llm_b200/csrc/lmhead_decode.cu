@@ -95,7 +95,7 @@ lmhead_argmax_kernel(const __grid_constant__ CUtensorMap tmE, const __grid_const
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();                 // the hidden states come from the previous kernel of the stream
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         mbar_expect_tx(x_bar, (uint32_t)(p.kblocks * LH_XK_BYTES));
         for (int kb = 0; kb < p.kblocks; ++kb) tma_load_3d(sX + kb * LH_XK_BYTES, &tmX, x_bar, kb * LH_BK, 0, 0);
         if (!p.early_table) {
@@ -105,7 +105,7 @@ lmhead_argmax_kernel(const __grid_constant__ CUtensorMap tmE, const __grid_const
             }
         }
         pdl_launch_dependents_now();
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         const uint32_t idesc = umma_idesc(1u, 0u, 0u, 128, LH_SEQ);
         bool ok = mbar_wait(x_bar, 0u, abort_flag);
         for (int kb = 0; kb < p.kblocks && ok; ++kb) {

@@ -15,6 +15,10 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// One lane of a converged warp.  The roles that issue TMA copies and UMMAs are entered through this and not through
+// `lane == 0`: the operands of those instructions sit in uniform registers, and only behind elect.sync does the compiler
+// know that one lane is active -- otherwise every such instruction is wrapped in code that works that out.  Measured for
+// 96 UMMAs of 128 x 16 x 16 from one thread: 69 clocks each behind `lane == 0`, 40 behind elect.sync.
 __device__ __forceinline__ uint32_t elect_one() {
     uint32_t pred = 0;
     asm volatile(
