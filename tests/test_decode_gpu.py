@@ -371,3 +371,31 @@ def test_one_kernel_decode_step_matches_launch_per_kernel_step(tb, oracle, monke
     srt = np.sort(outs[1], axis=1)
     clear = (srt[:, -1] - srt[:, -2]) > 2e-2 * np.abs(outs[1]).max()
     assert np.array_equal(toks[0][same_so_far & clear, -1], toks[1][same_so_far & clear, -1])
+
+
+@pytest.mark.parametrize("dims", [(97, 32, 2, 2, 48, 3, 5, 4),          # head dim 16, K shorter than one 64-column block
+                                  (211, 96, 3, 2, 80, 17, 62, 5),       # columns that do not fill the CTAs; cache across a 64-row block
+                                  (300, 192, 3, 1, 1024, 9, 127, 3),    # three slices of K; more than eight sequences in a cluster
+                                  (300, 768, 12, 1, 1008, 7, 64, 3),    # two tiles for the QKV columns
+                                  (300, 64, 2, 2, 128, 1, 1, 70),       # one sequence from a one-token prompt
+                                  (97, 128, 2, 1, 256, 100, 9, 3)])     # more sequences than the clusters hold at once
+def test_one_kernel_decode_step_at_the_edges_of_its_tiles(tb, oracle, monkeypatch, dims):
+    """The cluster kernel against the launch-per-kernel step where its tiles, slices and row groups end."""
+    from turkce_llm_b200.decode import Decoder
+    V, D, H, L, F, S, prompt_len, n_new = dims
+    p = make_params(oracle, (V, D, H, L, F, 1, 1, 1e-5), 5)
+    prompts = np.random.default_rng(6).integers(0, V, (S, prompt_len)).astype(np.uint32)
+    outs, toks = [], []
+    for off in (False, True):
+        if off:
+            monkeypatch.setenv("TB_DECODE_NO_MEGA", "1")
+        dec = Decoder(V, D, H, L, F, S, prompt_len + n_new + 2)
+        dec.upload(p)
+        dec.prefill(prompts)
+        dec.generate(n_new - 1)
+        outs.append(dec.logits())
+        toks.append(dec.tokens(n_new))
+        dec.destroy()
+    same_so_far = (toks[0][:, :-1] == toks[1][:, :-1]).all(axis=1)
+    assert same_so_far.mean() >= 0.6, same_so_far.mean()
+    assert rel_to_maxabs(outs[0][same_so_far], outs[1][same_so_far]) <= 1e-2

@@ -44,7 +44,7 @@ struct TbDecoder {
     bf16 *n = nullptr, *att = nullptr, *h = nullptr, *Q = nullptr;
     uint32_t *ids = nullptr, *tok = nullptr, *out = nullptr;
     int* pos = nullptr;
-    DecodeMega* mega = nullptr;                // decode step of all layers as one cooperative kernel (default when the shape fits)
+    DecodeCluster* cluster = nullptr;          // decode step of all layers in one kernel (default when the shape fits)
     bool lean_step = false;                    // decode step on decode_linear_kernel (norm / SwiGLU / residual fused)
     bool fused_head = false;                   // LM head with the greedy choice fused (no logits in HBM)
     unsigned long long* head_best = nullptr;   // packed per-sequence maxima of the fused head (zero between launches)
@@ -114,10 +114,9 @@ int head_logits(TbDecoder* g, int rows) {
     return launch_gemm_bf16_ws(g->ctx, a, g->splitk_ws, g->splitk_floats, g->stream);
 }
 
-// final norm of `rows` rows of src, tied LM head, greedy choice
-int head(TbDecoder* g, const float* src, int rows, int advance_pos) {
+// tied LM head on the normalised rows in g->n, greedy or sampled choice
+int choose(TbDecoder* g, int rows, int advance_pos) {
     DeviceCtx* c = g->ctx; cudaStream_t st = g->stream;
-    TB_TRY(launch_rmsnorm_fwd(c, src, P32(g, pidx(g->L, 0)), g->n, g->r, rows, g->D, g->eps, st));
     g->head_rows = rows;
     if (g->temperature > 0.f) {
         TB_TRY(head_logits(g, rows));
@@ -131,14 +130,20 @@ int head(TbDecoder* g, const float* src, int rows, int advance_pos) {
     return launch_argmax_rows(c, g->logits, g->tok, g->out, g->pos, rows, g->V, g->Vp, g->cap, advance_pos, st);
 }
 
+// final norm of `rows` rows of src, then the choice
+int head(TbDecoder* g, const float* src, int rows, int advance_pos) {
+    TB_TRY(launch_rmsnorm_fwd(g->ctx, src, P32(g, pidx(g->L, 0)), g->n, g->r, rows, g->D, g->eps, g->stream));
+    return choose(g, rows, advance_pos);
+}
+
 int decode_step_body(TbDecoder* g) {
     DeviceCtx* c = g->ctx; cudaStream_t st = g->stream;
     const int S = g->S, D = g->D, H = g->H, hd = g->hd;
     const bool split_rope = getenv("TB_DECODE_SPLIT_ROPE") != nullptr;    // the two-kernel form, for comparison
-    if (g->mega) {
-        // all layers in one cooperative kernel (embedding gather included), then the head as usual
-        TB_TRY(launch_decode_mega(c, g->mega, g->tok, g->pos, g->cos_t, g->sin_t, g->x, g->x2, g->qkv, g->att, g->h, st));
-        return head(g, g->x, S, 1);
+    if (g->cluster) {
+        // embedding gather, all layers and the final norm in one kernel
+        TB_TRY(launch_decode_cluster(c, g->cluster, g->tok, g->pos, g->cos_t, g->sin_t, g->n, st));
+        return choose(g, S, 1);
     }
     TB_TRY(launch_embed_fwd(c, P32(g, 0), g->tok, g->x, S, D, st));
     for (int l = 0; l < g->L; ++l) {
@@ -215,10 +220,9 @@ int tb_decoder_create(TbDecoder** out, int V, int D, int H, int L, int F, int ma
     g->lean_step = getenv("TB_DECODE_LEAN") != nullptr && getenv("TB_DECODE_SPLIT_ROPE") == nullptr &&
                    decode_linear_supported((int)S, 3 * D, D, false) && decode_linear_supported((int)S, D, D, false) &&
                    decode_linear_supported((int)S, 2 * F, D, true) && decode_linear_supported((int)S, D, F, false) && D % 4 == 0;
-    // One cooperative kernel for the layers of a decode step (TB_DECODE_NO_MEGA=1: the launch-per-kernel path)
-    if (L > 0 && getenv("TB_DECODE_NO_MEGA") == nullptr && !g->lean_step &&
-        decode_mega_supported(g->ctx, (int)S, D, H, F, max_len))
-        TB_TRY(decode_mega_create(g->ctx, &g->mega, (int)S, D, H, F, L, max_len, eps, g->scale));
+    // One kernel for the layers of a decode step (TB_DECODE_NO_MEGA=1: the launch-per-kernel path)
+    if (getenv("TB_DECODE_NO_MEGA") == nullptr && !g->lean_step)
+        TB_TRY(decode_cluster_create(g->ctx, &g->cluster, (int)S, D, H, F, L, max_len, eps, g->scale));
     if (g->fused_head) {
         TB_TRY(dalloc(g, &g->head_best, 64)); TB_CUDA(cudaMemset(g->head_best, 0, 64 * sizeof(unsigned long long)));
         TB_TRY(dalloc(g, &g->head_ticket, 1)); TB_CUDA(cudaMemset(g->head_ticket, 0, sizeof(unsigned int)));
@@ -253,7 +257,7 @@ int tb_decoder_destroy(TbDecoder* g) {
     cudaDeviceSynchronize();
     if (g->step_graph) cudaGraphExecDestroy(g->step_graph);
     for (void* p : g->allocs) cudaFree(p);
-    decode_mega_destroy(g->mega);
+    decode_cluster_destroy(g->cluster);
     cudaFreeHost(g->h_pinned);
     delete g;
     return 0;
@@ -266,9 +270,9 @@ int tb_decoder_upload(TbDecoder* g, const float* h_flat) {
     TB_H2D_SYNC(g->params, h_flat, (size_t)g->total * 4);
     TB_CHECK(g->total < (1LL << 31), "model too large for the single-row pack");
     TB_TRY(launch_pack_bf16(g->ctx, g->params, g->params16, 1, (int)g->total, g->total, g->total, 1, 0, 0, g->stream));
-    if (g->mega)
-        TB_TRY(decode_mega_set_weights(g->ctx, g->mega, g->params, g->params16, g->offsets.data(), g->Kc.data(), g->Vc.data(),
-                                       g->stream));
+    if (g->cluster)
+        TB_TRY(decode_cluster_set_weights(g->ctx, g->cluster, g->params, g->params16, g->offsets.data(), g->Kc.data(), g->Vc.data(),
+                                          g->stream));
     TB_CUDA(cudaStreamSynchronize(g->stream));
     return 0;
 }
@@ -330,8 +334,8 @@ int tb_decoder_generate(TbDecoder* g, int n) {
     TB_CUDA(cudaSetDevice(g->device));
     TB_CHECK(g->generated >= 1, "tb_decoder_generate: call tb_decoder_prefill first");
     TB_CHECK(g->prompt_len + g->generated + n <= g->cap + 1, "cache capacity %d exceeded", g->cap);
-    // (with the one-kernel step there are three launches per token: nothing for a graph to save)
-    const bool use_graph = getenv("TB_NO_GRAPH") == nullptr && !g->ctx->prof_on && g->mega == nullptr;
+    // (with the one-kernel step there are two or three launches per token: nothing for a graph to save)
+    const bool use_graph = getenv("TB_NO_GRAPH") == nullptr && !g->ctx->prof_on && g->cluster == nullptr;
     for (int i = 0; i < n; ++i) {
         if (!use_graph || g->step_state == 0) {
             TB_TRY(decode_step_body(g));
