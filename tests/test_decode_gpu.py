@@ -399,3 +399,26 @@ def test_one_kernel_decode_step_at_the_edges_of_its_tiles(tb, oracle, monkeypatc
     same_so_far = (toks[0][:, :-1] == toks[1][:, :-1]).all(axis=1)
     assert same_so_far.mean() >= 0.6, same_so_far.mean()
     assert rel_to_maxabs(outs[0][same_so_far], outs[1][same_so_far]) <= 1e-2
+
+
+@pytest.mark.parametrize("V", [1, 2, 4095, 4096 * 3 + 1, 470_000])
+def test_sampling_over_small_and_large_vocabularies(tb, oracle, V):
+    """A vocabulary smaller than the sampler's threads, one that ends inside a thread's share, one too large to be staged."""
+    from turkce_llm_b200.decode import Decoder, pcg_uniform
+    D, H, L, F, S, prompt_len, n_new = 32, 2, 1, 48, 3, 4, 5
+    p = make_params(oracle, (V, D, H, L, F, 1, 1, 1e-5), 11)
+    dec = Decoder(V, D, H, L, F, S, prompt_len + n_new + 2)
+    dec.upload(p)
+    dec.set_sampling(0.85, 99, 7)
+    dec.prefill(np.random.default_rng(8).integers(0, V, (S, prompt_len)).astype(np.uint32))
+    u = np.stack([pcg_uniform(99, 7 + s, n_new) for s in range(S)])
+    for step in range(n_new):
+        if step > 0:
+            dec.generate(1)
+        logits, tok = dec.logits(), dec.tokens(step + 1)[:, step]
+        for s in range(S):
+            want, c = sample_next(logits[s], 0.85, u[s, step])
+            if tok[s] != want:
+                r = u[s, step] * c[-1]
+                assert abs(int(tok[s]) - want) == 1 and abs(c[min(tok[s], want)] - r) <= 1e-6 * c[-1], (step, s)
+    dec.destroy()

@@ -208,6 +208,7 @@ int launch_split3_f32(DeviceCtx* ctx, const float* src, float* dst, int rows, in
 // earlier work of the stream, so its loads may start before that work has finished.
 // Also stores the token as out[s, state[1]] and advances state = {position, generated} like launch_argmax_rows
 // (out and state may be NULL).  logits (optional, [S, ld_logits] float32) receives the full products.
+// tok NULL: the logits are all that is wanted.
 bool lmhead_argmax_supported(const DeviceCtx* ctx, int S, int V, int K);
 int lmhead_argmax_ctas(const DeviceCtx* ctx, int S, int V, int K);
 int launch_lmhead_argmax(DeviceCtx* ctx, const bf16* X, const bf16* E, int S, int V, int K, bool table_is_stable,

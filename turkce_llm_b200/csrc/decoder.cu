@@ -119,9 +119,14 @@ int choose(TbDecoder* g, int rows, int advance_pos) {
     DeviceCtx* c = g->ctx; cudaStream_t st = g->stream;
     g->head_rows = rows;
     if (g->temperature > 0.f) {
-        TB_TRY(head_logits(g, rows));
-        return launch_sample_rows(c, g->logits, g->sample_u, g->temperature, g->tok, g->out, g->pos, rows, g->V, g->Vp,
-                                  g->cap, advance_pos, st);
+        // (the fused head without its choice: it streams the table while the step before it still runs)
+        if (g->fused_head)
+            TB_TRY(launch_lmhead_argmax(c, g->n, P16(g, 0), rows, g->V, g->D, true, g->head_best, g->head_ticket, nullptr, nullptr,
+                                        nullptr, 0, 0, g->logits, g->Vp, st));
+        else
+            TB_TRY(head_logits(g, rows));
+        return launch_sample_rows(c, g->logits, g->sample_u, g->temperature, g->tok, g->out, g->pos, g->head_ticket, rows, g->V,
+                                  g->Vp, g->cap, advance_pos, st);
     }
     if (g->fused_head)
         return launch_lmhead_argmax(c, g->n, P16(g, 0), rows, g->V, g->D, true, g->head_best, g->head_ticket,
@@ -223,10 +228,8 @@ int tb_decoder_create(TbDecoder** out, int V, int D, int H, int L, int F, int ma
     // One kernel for the layers of a decode step (TB_DECODE_NO_MEGA=1: the launch-per-kernel path)
     if (getenv("TB_DECODE_NO_MEGA") == nullptr && !g->lean_step)
         TB_TRY(decode_cluster_create(g->ctx, &g->cluster, (int)S, D, H, F, L, max_len, eps, g->scale));
-    if (g->fused_head) {
-        TB_TRY(dalloc(g, &g->head_best, 64)); TB_CUDA(cudaMemset(g->head_best, 0, 64 * sizeof(unsigned long long)));
-        TB_TRY(dalloc(g, &g->head_ticket, 1)); TB_CUDA(cudaMemset(g->head_ticket, 0, sizeof(unsigned int)));
-    }
+    TB_TRY(dalloc(g, &g->head_best, 64)); TB_CUDA(cudaMemset(g->head_best, 0, 64 * sizeof(unsigned long long)));
+    TB_TRY(dalloc(g, &g->head_ticket, 1)); TB_CUDA(cudaMemset(g->head_ticket, 0, sizeof(unsigned int)));
     TB_TRY(dalloc(g, &g->n, N * D)); TB_TRY(dalloc(g, &g->att, N * D)); TB_TRY(dalloc(g, &g->h, N * F));
     TB_TRY(dalloc(g, &g->Q, N * D));
     TB_TRY(dalloc(g, &g->ids, N)); TB_TRY(dalloc(g, &g->tok, S)); TB_TRY(dalloc(g, &g->out, N));

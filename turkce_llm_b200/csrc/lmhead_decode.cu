@@ -36,7 +36,7 @@ struct LmHeadParams {
     int early_table;          // the table is not written by earlier kernels of the stream: load it before the fence
     unsigned long long* best; // [64] packed (value key, ~index) maxima over the CTAs; zero between launches
     unsigned int* ticket;     // zero between launches
-    uint32_t* tok;            // [S]
+    uint32_t* tok;            // [S]; NULL: the logits alone, no choice
     uint32_t* out;            // optional [S, out_ld]: generated tokens
     int* state;               // optional {position of the next token, tokens generated}
     int out_ld, advance_pos;
@@ -150,6 +150,13 @@ lmhead_argmax_kernel(const __grid_constant__ CUtensorMap tmE, const __grid_const
     const int all_done = __syncthreads_and(done ? 1 : 0);
     if (warp == 1) tmem_dealloc(tmem_base, 128);
 
+    if (p.tok == nullptr) {
+        if (all_done)
+            for (int s = 0; s < p.S; ++s)
+                for (int rr = threadIdx.x; rr < rows_here; rr += LH_THREADS)
+                    p.logits[(long long)s * p.ld_logits + row0 + rr] = stage[s * LH_STAGE_LD + rr];
+        return;
+    }
     if (all_done) {
     // ---- per sequence: 4 threads scan a quarter of the rows each, four rows per load, in four
     // independent chains (row mod 4); every comparison prefers the lower row on equal values

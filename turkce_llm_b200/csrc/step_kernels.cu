@@ -838,36 +838,64 @@ int launch_argmax_rows(DeviceCtx* ctx, const float* logits, uint32_t* tok, uint3
 
 // Temperature sampling, sample_next of the reference's generator (training/generate.c:57-73):
 // e_j = exp((z_j - max z) / temperature) in float32, r = u * sum_j e_j, the token is the first j whose running
-// sum (float64, ascending j) reaches r; the last index if none does.  One block per sequence; thread t owns the
-// contiguous columns [t * per, (t + 1) * per), so that the running sum is formed in ascending order: per-thread
-// sums in column order, an exclusive scan over the threads in thread order.  u[state[1] * S + s] is the uniform
-// draw of sequence s for generated token number state[1].
-__global__ void __launch_bounds__(1024, 1)
+// sum (float64, ascending j) reaches r; the last index if none does.  u[state[1] * S + s] is the uniform draw of
+// sequence s for generated token number state[1].
+//
+// A cluster of eight CTAs per sequence: a row is ~32,000 exponentials and divisions, which took one CTA 37 us (it also read
+// the row twice with 32 cache lines per load); eight take ~5.  Thread t of CTA c owns `per` adjacent columns (an odd number,
+// so that the threads' walks through shared memory meet no bank conflicts): sums per thread, scanned over the threads,
+// the warps and the CTAs in column order.  The bounds of a thread's share of the running sum are formed so that they tile
+// [0, total] exactly, so just one thread holds r; it walks its columns and writes the token.  The writer of the last
+// sequence (a ticket) advances the state, which everybody has read before the cluster's first meeting.
+constexpr int kSampleCtas = 8, kSampleThreads = 512;
+
+__global__ void __launch_bounds__(kSampleThreads, 1)
 sample_rows_kernel(const float* __restrict__ logits, const double* __restrict__ u, float temperature,
-                   uint32_t* __restrict__ tok, uint32_t* __restrict__ out, const int* __restrict__ state, int S, int V,
-                   long long ld, int out_ld) {
+                   uint32_t* __restrict__ tok, uint32_t* __restrict__ out, int* __restrict__ state, unsigned int* __restrict__ ticket,
+                   int S, int V, int per, int staged, long long ld, int out_ld, int advance_pos) {
+    extern __shared__ float e_sh[];                       // [kSampleThreads * per] this CTA's columns, when they fit
+    __shared__ float wmax[kSampleThreads / 32], cmax[kSampleCtas];
+    __shared__ double wsum[kSampleThreads / 32], csum[kSampleCtas];
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ float wmax[32];
-    __shared__ double wsum[32];
-    __shared__ int wfirst[32];
-    const int sq = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const float* z = logits + (long long)sq * ld;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = (int)(blockIdx.x % kSampleCtas), sq = blockIdx.x / kSampleCtas;
+    const int first = rank * kSampleThreads * per, n = max(0, min(kSampleThreads * per, V - first));
+    const float* z = logits + (long long)sq * ld + first;
+    const int generated = state[1];
+    const double draw = u[(long long)generated * S + sq];
     float mx = -3.0e38f;
-    for (int j = tid; j < V; j += blockDim.x) mx = fmaxf(mx, z[j]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+#pragma unroll 8
+    for (int j = tid; j < n; j += kSampleThreads) {
+        const float v = z[j];
+        if (staged) e_sh[j] = v;
+        mx = fmaxf(mx, v);
+    }
+    mx = warp_max(mx);
     if (lane == 0) wmax[warp] = mx;
     __syncthreads();
-    mx = wmax[0];
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) mx = fmaxf(mx, wmax[w]);
+    mx = wmax[lane & (kSampleThreads / 32 - 1)];
+    mx = warp_max(mx);
+    auto to_cta = [](const void* p, int cta) {            // the same shared variable in CTA `cta` of the cluster
+        uint32_t a;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(cta));
+        return a;
+    };
+    auto meet = []() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); };
+    if (tid < kSampleCtas) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to_cta(cmax + rank, tid)), "f"(mx) : "memory");
+    meet();
+    mx = cmax[0];
+#pragma unroll
+    for (int c = 1; c < kSampleCtas; ++c) mx = fmaxf(mx, cmax[c]);
 
-    const int per = (V + (int)blockDim.x - 1) / (int)blockDim.x;
-    const int j0 = min(tid * per, V), j1 = min(j0 + per, V);
+    const int j0 = min(tid * per, n), j1 = min(j0 + per, n);
     double local = 0.0;
-    for (int j = j0; j < j1; ++j) local += (double)expf((z[j] - mx) / temperature);
-    // inclusive scan inside the warp, then the warps' totals in warp order
-    double incl = local;
+    for (int j = j0; j < j1; ++j) {
+        const float e = expf(((staged ? e_sh[j] : z[j]) - mx) / temperature);
+        if (staged) e_sh[j] = e;
+        local += (double)e;
+    }
+    double incl = local;                                  // inclusive scan inside the warp
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const double v = __shfl_up_sync(0xffffffffu, incl, o);
@@ -875,41 +903,62 @@ sample_rows_kernel(const float* __restrict__ logits, const double* __restrict__ 
     }
     if (lane == 31) wsum[warp] = incl;
     __syncthreads();
-    double before = 0.0, total = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-        if (w < warp) before += wsum[w];
-        total += wsum[w];
+    double wbefore = 0.0, ctotal = 0.0;
+#pragma unroll
+    for (int w = 0; w < kSampleThreads / 32; ++w) {
+        if (w == warp) wbefore = ctotal;
+        ctotal += wsum[w];
     }
-    const double r = u[(long long)state[1] * S + sq] * total;
-    double c = before + (incl - local);
-    int first = 0x7fffffff;
-    if (c + local >= r || j1 == V) {          // the crossing can only lie in a chunk whose end reaches r
+    if (tid < kSampleCtas) asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to_cta(csum + rank, tid)), "d"(ctotal) : "memory");
+    meet();
+    double cbefore = 0.0, cend = 0.0, total = 0.0;
+#pragma unroll
+    for (int c = 0; c < kSampleCtas; ++c) {
+        if (c == rank) cbefore = total;
+        total += csum[c];
+        if (c == rank) cend = total;
+    }
+    const double r = draw * total;
+    const double below = __shfl_up_sync(0xffffffffu, incl, 1);
+    const double lo = cbefore + (lane == 0 ? wbefore : wbefore + below);
+    const double hi = tid == kSampleThreads - 1 ? cend : cbefore + (lane == 31 ? wbefore + wsum[warp] : wbefore + incl);
+    const bool none = !(r <= total);                      // not a number: the last index, as the running sum never reaches it
+    int pick = -1;
+    if (none) {
+        if (n > 0 && first + n == V && tid == 0) pick = V - 1;
+    } else if ((lo < r || (rank == 0 && tid == 0)) && r <= hi) {
+        double c = lo;
+        pick = first + max(j1 - 1, 0);
         for (int j = j0; j < j1; ++j) {
-            c += (double)expf((z[j] - mx) / temperature);
-            if (c >= r) { first = j; break; }
+            c += (double)(staged ? e_sh[j] : expf((z[j] - mx) / temperature));
+            if (c >= r) { pick = first + j; break; }
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
-    if (lane == 0) wfirst[warp] = first;
-    __syncthreads();
-    if (tid == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) first = min(first, wfirst[w]);
-        if (first == 0x7fffffff) first = V - 1;
-        tok[sq] = (uint32_t)first;
-        if (out) out[(long long)sq * out_ld + state[1]] = (uint32_t)first;
+    if (pick >= 0) {
+        tok[sq] = (uint32_t)pick;
+        if (out) out[(long long)sq * out_ld + generated] = (uint32_t)pick;
+        __threadfence();
+        if (atomicAdd(ticket, 1u) == (unsigned int)S - 1u) {
+            *ticket = 0u;
+            state[1] = generated + 1;
+            if (advance_pos) state[0] += 1;
+        }
     }
 }
 
+// (ticket: a word that is zero between launches)
 int launch_sample_rows(DeviceCtx* ctx, const float* logits, const double* u, float temperature, uint32_t* tok,
-                       uint32_t* out, int* state, int S, int V, long long ld, int out_ld, int advance_pos,
+                       uint32_t* out, int* state, unsigned int* ticket, int S, int V, long long ld, int out_ld, int advance_pos,
                        cudaStream_t st) {
+    const int per = (V + kSampleCtas * kSampleThreads - 1) / (kSampleCtas * kSampleThreads) | 1;
+    const size_t row = (size_t)kSampleThreads * per * sizeof(float);
+    const int staged = row <= 224 * 1024 ? 1 : 0;         // (vocabularies beyond ~450,000 tokens are read from memory again)
+    const size_t smem = staged ? row : 0;
+    if (smem > 48 * 1024)
+        TB_CUDA(cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
     prof_mark(ctx, "sample_rows", 0.0, 0.0, st);
-    TB_CUDA(launch_kernel(sample_rows_kernel, dim3(S), dim3(1024), 0, st, logits, u, temperature, tok, out,
-                          (const int*)state, S, V, ld, out_ld));
-    TB_LAUNCHED(ctx);
-    prof_mark(ctx, "advance_state", 0.0, 0.0, st);
-    TB_CUDA(launch_kernel(advance_state_kernel, dim3(1), dim3(32), 0, st, state, advance_pos));
+    TB_CUDA(launch_kernel_cluster(sample_rows_kernel, dim3(S * kSampleCtas), dim3(kSampleThreads), smem, st, kSampleCtas, logits, u,
+                                  temperature, tok, out, state, ticket, S, V, per, staged, ld, out_ld, advance_pos));
     TB_LAUNCHED(ctx);
     return 0;
 }

@@ -36,7 +36,8 @@ int launch_gather_last_rows(DeviceCtx*, const float* in, float* out, int S, int 
 int launch_rope_attn_decode(DeviceCtx*, const float* qkv, const float* cos_t, const float* sin_t, bf16* Kc, bf16* Vc,
                             bf16* att, const int* pos, int S, int H, int hd, int cap, float scale, cudaStream_t);
 int launch_sample_rows(DeviceCtx*, const float* logits, const double* u, float temperature, uint32_t* tok,
-                       uint32_t* out, int* state, int S, int V, long long ld, int out_ld, int advance_pos, cudaStream_t);
+                       uint32_t* out, int* state, unsigned int* ticket, int S, int V, long long ld, int out_ld, int advance_pos,
+                       cudaStream_t);
 int launch_argmax_rows(DeviceCtx*, const float* logits, uint32_t* tok, uint32_t* out, int* state, int S, int V,
                        long long ld, int out_ld, int advance_pos, cudaStream_t);
 int launch_rope_merge_bwd(DeviceCtx*, const float* dQ, const float* dK, const float* dV, const float* cos_t,
