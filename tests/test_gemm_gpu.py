@@ -424,3 +424,22 @@ def test_matmul_host_from_several_threads(tb, oracle):
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("precision", ["bf16", "tf32", "fp32"])
+@pytest.mark.parametrize("shape", [(255, 1031, 900), (257, 2000, 1025), (1030, 701, 777), (128, 300, 20000), (2049, 513, 1)])
+def test_matmul_host_in_row_blocks(tb, oracle, shape, precision):
+    """Host products around the sizes where they are cut into row blocks and the copies go through several threads: short
+    last blocks, one block only, a result of one column."""
+    M, K, N = shape
+    rng = np.random.default_rng(5)
+    A = rng.standard_normal((M, K)).astype(np.float32)
+    B = (rng.standard_normal((K, N)) * 0.05).astype(np.float32)
+    want = A.astype(np.float64) @ B.astype(np.float64)
+    out = np.full((M, N), np.nan, np.float32)
+    prec = {"bf16": tb.PREC_BF16, "tf32": tb.PREC_TF32, "fp32": tb.PREC_FP32}[precision]
+    for _ in range(2):                       # (the second call finds the first one's buffers and packed operands)
+        tb.matmul_host(A, B, out, M, K, N, prec)
+        assert rel_to_maxabs(out, want) <= {"bf16": 2e-2, "tf32": 5e-3, "fp32": 1e-5}[precision]
+        A *= -1.0
+        want *= -1.0

@@ -2,6 +2,7 @@
 #include "../../include/turkce_b200.h"
 #include "common.h"
 
+#include <algorithm>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -46,7 +47,7 @@ int tb_shutdown(void) {
     if (ctx->scratch) TB_CUDA(cudaFree(ctx->scratch));
     ctx->scratch = nullptr;
     ctx->scratch_bytes = 0;
-    return 0;
+    return copy_give_back();
 }
 
 int tb_profile_begin(void) {
@@ -234,7 +235,8 @@ static inline bool tma_ok_f32(const float* p, long long ld, int batch, long long
 static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int M, int N, int K,
                          long long lda, long long ldb, long long ldc, int batch, long long sA, long long sB,
                          long long sC, float alpha, float beta, const float* bias, const float* residual,
-                         int precision, cudaStream_t stream) {
+                         int precision, cudaStream_t stream, bool same_b = false) {
+    // (same_b: B is what the call before it on this stream had, and is still packed in the scratch memory)
     DeviceCtx* ctx;
     TB_TRY(get_ctx(&ctx));
     TB_CHECK(kind >= 0 && kind <= 2, "unknown GEMM kind %d", kind);
@@ -261,12 +263,13 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
         const int splits = residual ? 1 : choose_splits(ctx, g, (N <= 64) ? 64 : 128);
         g.splits = splits;
         const size_t ws_floats = splits > 1 ? (size_t)splits * batch * M * N : 0;
+        if (a_bytes + b_bytes + ws_floats * sizeof(float) > ctx->scratch_bytes) same_b = false;      // the scratch memory moves
         TB_TRY(ensure_scratch(ctx, a_bytes + b_bytes + ws_floats * sizeof(float)));
-        bf16* pa = static_cast<bf16*>(ctx->scratch);
-        bf16* pb = reinterpret_cast<bf16*>(static_cast<char*>(ctx->scratch) + a_bytes);
+        bf16* pb = static_cast<bf16*>(ctx->scratch);
+        bf16* pa = reinterpret_cast<bf16*>(static_cast<char*>(ctx->scratch) + b_bytes);
         float* ws = reinterpret_cast<float*>(static_cast<char*>(ctx->scratch) + a_bytes + b_bytes);
         TB_TRY(launch_pack_bf16(ctx, A, pa, a_rows, a_cols, lda, a_ld, batch, sA, a_stride, stream));
-        TB_TRY(launch_pack_bf16(ctx, B, pb, b_rows, b_cols, ldb, b_ld, batch, sB, b_stride, stream));
+        if (!same_b) TB_TRY(launch_pack_bf16(ctx, B, pb, b_rows, b_cols, ldb, b_ld, batch, sB, b_stride, stream));
         g.A = pa; g.B = pb;
         return launch_gemm_bf16_ws(ctx, g, ws, ws_floats, stream);
     }
@@ -290,16 +293,17 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
     const int splits = residual ? 1 : choose_splits(ctx, g, (N <= 64) ? 64 : 128);
     g.splits = splits;
     const size_t ws_floats = splits > 1 ? (size_t)splits * batch * M * N : 0;
+    if (a_bytes + b_bytes + ws_floats * sizeof(float) > ctx->scratch_bytes) same_b = false;      // the scratch memory moves
     TB_TRY(ensure_scratch(ctx, a_bytes + b_bytes + ws_floats * sizeof(float)));
-    float* pa = static_cast<float*>(ctx->scratch);
-    float* pb = reinterpret_cast<float*>(static_cast<char*>(ctx->scratch) + a_bytes);
+    float* pb = static_cast<float*>(ctx->scratch);
+    float* pa = reinterpret_cast<float*>(static_cast<char*>(ctx->scratch) + b_bytes);
     float* ws = reinterpret_cast<float*>(static_cast<char*>(ctx->scratch) + a_bytes + b_bytes);
     if (split3) {
         TB_TRY(launch_split3_f32(ctx, A, pa, a_rows, a_cols, lda, a_ld, a_cat_cols ? 1 : 0, 0, batch, sA, a_stride, stream));
-        TB_TRY(launch_split3_f32(ctx, B, pb, b_rows, b_cols, ldb, b_ld, b_cat_cols ? 1 : 0, 1, batch, sB, b_stride, stream));
+        if (!same_b) TB_TRY(launch_split3_f32(ctx, B, pb, b_rows, b_cols, ldb, b_ld, b_cat_cols ? 1 : 0, 1, batch, sB, b_stride, stream));
     } else {
         if (!a_inplace) TB_TRY(launch_copy_f32(ctx, A, pa, a_rows, a_cols, lda, a_ld, batch, sA, a_stride, stream));
-        if (!b_inplace) TB_TRY(launch_copy_f32(ctx, B, pb, b_rows, b_cols, ldb, b_ld, batch, sB, b_stride, stream));
+        if (!b_inplace && !same_b) TB_TRY(launch_copy_f32(ctx, B, pb, b_rows, b_cols, ldb, b_ld, batch, sB, b_stride, stream));
     }
     g.A = a_inplace ? static_cast<const void*>(A) : pa;
     g.B = b_inplace ? static_cast<const void*>(B) : pb;
@@ -326,17 +330,32 @@ int tb_gemm_bias_f32(const float* d_A, const float* d_B, const float* d_bias, co
 // grow on demand and live until the thread ends, so the steady state allocates nothing, and threads never share a
 // slot (no lock on the data path, as the reference's worker slots).
 namespace {
+constexpr int kMatmulBlocks = 4;
 struct MatmulSlot {
     int device = -1;
     float *dA = nullptr, *dB = nullptr, *dC = nullptr;
     size_t capA = 0, capB = 0, capC = 0;
+    cudaStream_t in = nullptr, out = nullptr;            // the copies of a product in blocks
+    cudaEvent_t arrived[kMatmulBlocks + 1] = {}, done[kMatmulBlocks] = {};
     ~MatmulSlot() {
         if (device < 0) return;
         int cur = -1;
         if (cudaGetDevice(&cur) != cudaSuccess) return;      // the runtime is already shutting down
         cudaSetDevice(device);
         cudaFree(dA); cudaFree(dB); cudaFree(dC);
+        if (in) cudaStreamDestroy(in);
+        if (out) cudaStreamDestroy(out);
+        for (cudaEvent_t e : arrived) if (e) cudaEventDestroy(e);
+        for (cudaEvent_t e : done) if (e) cudaEventDestroy(e);
         cudaSetDevice(cur);
+    }
+    int streams() {
+        if (done[kMatmulBlocks - 1]) return 0;
+        TB_CUDA(cudaStreamCreateWithFlags(&in, cudaStreamNonBlocking));
+        TB_CUDA(cudaStreamCreateWithFlags(&out, cudaStreamNonBlocking));
+        for (cudaEvent_t& e : arrived) TB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        for (cudaEvent_t& e : done) TB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        return 0;
     }
 };
 thread_local MatmulSlot t_slots[8];
@@ -365,16 +384,54 @@ int tb_matmul_host(const float* h_A, const float* h_B, float* h_C, int M, int K,
     TB_TRY(grow(&slot->dA, &slot->capA, na));
     TB_TRY(grow(&slot->dB, &slot->capB, nb));
     TB_TRY(grow(&slot->dC, &slot->capC, nc));
-    TB_H2D_SYNC(slot->dA, h_A, na * 4);
-    TB_H2D_SYNC(slot->dB, h_B, nb * 4);
     // the library scratch (operand packing, split-K partials) is one per device: calls of different threads take turns
     static std::mutex gemm_mutex;
+    auto product = [&](size_t row0, size_t rows, bool same_b) {
+        return gemm_f32_impl(TB_GEMM_NN, slot->dA + row0 * K, slot->dB, slot->dC + row0 * N, (int)rows, N, K, K, N, N, 1, 0, 0, 0, 1.0f, 0.0f,
+                             nullptr, nullptr, precision, nullptr, same_b);
+    };
+    // A large product goes by row blocks: block i is multiplied and on its way back while block i + 1 comes in, so that the
+    // two directions of the bus and the product overlap (1024 x 1024 x 1024: the copies in, 8 MB, are ~170 us at the bus
+    // rate, the copy back ~85).  From 2 MB of A and C, in blocks of at least 1 MB and 128 rows.
+    const size_t moved = (na + nc) * 4;
+    const int blocks = (int)std::min<size_t>({(size_t)kMatmulBlocks, moved >> 20, (size_t)M / 128});
+    if (blocks < 2) {
+        const CopySpan in[2] = {{slot->dB, const_cast<float*>(h_B), nb * 4}, {slot->dA, const_cast<float*>(h_A), na * 4}};
+        TB_TRY(copy_h2d(in, 2, nullptr));
+        std::lock_guard<std::mutex> lock(gemm_mutex);
+        TB_TRY(product(0, (size_t)M, false));
+        TB_TRY(device_error_request(ctx, nullptr));
+        const CopySpan out = {slot->dC, h_C, nc * 4};
+        TB_TRY(copy_d2h(&out, 1, nullptr));
+        return device_error_result(ctx);
+    }
+    TB_TRY(slot->streams());
+    const size_t per = (((size_t)M + blocks - 1) / blocks + 127) / 128 * 128;      // so that `blocks` of them reach M
+    CopySpan in[kMatmulBlocks + 1], out[kMatmulBlocks];
+    size_t first[kMatmulBlocks + 1];
+    in[0] = {slot->dB, const_cast<float*>(h_B), nb * 4};
+    int n = 0;
+    for (size_t r = 0; r < (size_t)M; r += per, ++n) {
+        const size_t rows = std::min(per, (size_t)M - r);
+        first[n] = r;
+        in[n + 1] = {slot->dA + r * K, const_cast<float*>(h_A) + r * K, rows * K * 4};
+        out[n] = {slot->dC + r * N, h_C + r * N, rows * N * 4};
+    }
+    first[n] = (size_t)M;
     std::lock_guard<std::mutex> lock(gemm_mutex);
-    TB_TRY(gemm_f32_impl(TB_GEMM_NN, slot->dA, slot->dB, slot->dC, M, N, K, K, N, N, 1, 0, 0, 0, 1.0f, 0.0f, nullptr,
-                         nullptr, precision, nullptr));
-    TB_TRY(check_device_error(ctx, nullptr));
-    TB_CUDA(cudaMemcpy(h_C, slot->dC, nc * 4, cudaMemcpyDeviceToHost));
-    return 0;
+    const std::function<int(int)> ready = [&](int span) -> int {
+        if (span == 0) return 0;                             // (B: in front of block 0 on the same stream)
+        const int i = span - 1;
+        TB_CUDA(cudaEventRecord(slot->arrived[i], slot->in));
+        TB_CUDA(cudaStreamWaitEvent(nullptr, slot->arrived[i], 0));
+        TB_TRY(product(first[i], first[i + 1] - first[i], i > 0));
+        if (i == n - 1) TB_TRY(device_error_request(ctx, nullptr));
+        TB_CUDA(cudaEventRecord(slot->done[i], nullptr));
+        return 0;
+    };
+    TB_TRY(copy_h2d(in, n + 1, slot->in, &ready));
+    TB_TRY(copy_d2h(out, n, slot->out, slot->done));
+    return device_error_result(ctx);
 }
 
 }  // extern "C"

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <cstdio>
+#include <functional>
 #include <vector>
 
 namespace tb {
@@ -52,6 +53,17 @@ const char* last_error();
         TB_CUDA(cudaStreamSynchronize(cudaStreamLegacy));                        \
     } while (0)
 
+// ---- copies between pageable host memory and the device through pinned buffers (host_copy.cu)
+struct CopySpan { void* dev; void* host; size_t bytes; };
+// All spans, in stream order on `st`; on return the host memory has been read, the copies themselves may be on their way.
+// ready (optional) is called span by span, in order, when all of a span's copies have been handed to the stream.
+int copy_h2d(const CopySpan* spans, int count, cudaStream_t st, const std::function<int(int)>* ready = nullptr);
+// On return the data is in host memory (and what was in front of the copies on `st` has finished).
+// after (optional): an event per span that its copies wait for.
+int copy_d2h(const CopySpan* spans, int count, cudaStream_t st, const cudaEvent_t* after = nullptr);
+// frees the pinned buffers and ends the helper threads
+int copy_give_back();
+
 // ---- optional per-launch timing: one event in front of a launch (prof_mark) and one behind it
 // (prof_close); the difference is the kernel's own time even when the host is the bottleneck.
 struct ProfRec { const char* tag; cudaEvent_t ev; cudaEvent_t ev_end; double flops; double bytes; };
@@ -84,6 +96,10 @@ int get_ctx(DeviceCtx** out);
 int ensure_scratch(DeviceCtx* ctx, size_t bytes);
 // Reads and clears the device error word (synchronises the stream first).
 int check_device_error(DeviceCtx* ctx, cudaStream_t stream);
+// The same in two halves, for a caller that waits for the stream itself in between: the word's copy to the host is issued
+// / what it brought is looked at.
+int device_error_request(DeviceCtx* ctx, cudaStream_t stream);
+int device_error_result(DeviceCtx* ctx);
 
 // ---- GEMM on BF16 operands (gemm_tcgen05.cu)
 enum GemmKind { GEMM_NN = 0, GEMM_NT = 1, GEMM_TN = 2 };

@@ -109,10 +109,24 @@ void prof_close(DeviceCtx* ctx, cudaStream_t stream) {
     cudaEventRecord(r.ev_end, stream);
 }
 
-int check_device_error(DeviceCtx* ctx, cudaStream_t stream) {
-    int h = 0;
-    TB_CUDA(cudaStreamSynchronize(stream));
-    TB_CUDA(cudaMemcpy(&h, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+namespace {
+// where a calling thread receives the error word: pinned, so that the copy waits for nothing but its stream (the same copy
+// to pageable memory took 12 us after the stream had drained)
+struct ErrWord {
+    int* p = nullptr;
+    ~ErrWord() { if (p) cudaFreeHost(p); }
+};
+thread_local ErrWord t_err;
+}  // namespace
+
+int device_error_request(DeviceCtx* ctx, cudaStream_t stream) {
+    if (!t_err.p) TB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&t_err.p), sizeof(int), cudaHostAllocPortable));
+    TB_CUDA(cudaMemcpyAsync(t_err.p, ctx->d_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    return 0;
+}
+
+int device_error_result(DeviceCtx* ctx) {
+    const int h = *static_cast<volatile int*>(t_err.p);
     if (h != 0) {
         // the ticket words and packed maxima behind the error word go back to zero as well: a kernel that
         // gave up may have left them half-way
@@ -122,6 +136,12 @@ int check_device_error(DeviceCtx* ctx, cudaStream_t stream) {
         return -3;
     }
     return 0;
+}
+
+int check_device_error(DeviceCtx* ctx, cudaStream_t stream) {
+    TB_TRY(device_error_request(ctx, stream));
+    TB_CUDA(cudaStreamSynchronize(stream));
+    return device_error_result(ctx);
 }
 
 }  // namespace tb

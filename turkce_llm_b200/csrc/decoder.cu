@@ -368,11 +368,11 @@ int tb_decoder_generate(TbDecoder* g, int n) {
 // Copies the generated tokens [S, count] (count = tokens generated so far) to the host.
 int tb_decoder_read_tokens(TbDecoder* g, uint32_t* h_out, int count) {
     TB_CHECK(count >= 0 && count <= g->generated, "only %d tokens have been generated", g->generated);
+    if (count > 0)      // (the prompt's staging buffer has room for every row, and its own copy is long done)
+        TB_CUDA(cudaMemcpy2DAsync(g->h_pinned, (size_t)count * 4, g->out, (size_t)g->cap * 4, (size_t)count * 4, g->S,
+                                  cudaMemcpyDeviceToHost, g->stream));
     TB_TRY(check_device_error(g->ctx, g->stream));
-    std::vector<uint32_t> tmp((size_t)g->S * g->cap);
-    TB_CUDA(cudaMemcpy(tmp.data(), g->out, tmp.size() * 4, cudaMemcpyDeviceToHost));
-    for (int s = 0; s < g->S; ++s)
-        for (int i = 0; i < count; ++i) h_out[(size_t)s * count + i] = tmp[(size_t)s * g->cap + i];
+    std::memcpy(h_out, g->h_pinned, (size_t)g->S * count * 4);
     return 0;
 }
 
@@ -381,12 +381,11 @@ int tb_decoder_read_tokens(TbDecoder* g, uint32_t* h_out, int count) {
 int tb_decoder_read_logits(TbDecoder* g, float* h_logits) {
     TB_CHECK(g->head_rows > 0, "tb_decoder_read_logits: no step has run yet");
     if (g->fused_head) TB_TRY(head_logits(g, g->head_rows));
-    TB_CUDA(cudaStreamSynchronize(g->stream));
-    TB_TRY(check_device_error(g->ctx, g->stream));
-    std::vector<float> tmp((size_t)g->S * g->Vp);
-    TB_CUDA(cudaMemcpy(tmp.data(), g->logits, tmp.size() * 4, cudaMemcpyDeviceToHost));
-    for (int s = 0; s < g->S; ++s) std::memcpy(h_logits + (size_t)s * g->V, tmp.data() + (size_t)s * g->Vp, (size_t)g->V * 4);
-    return 0;
+    TB_TRY(device_error_request(g->ctx, g->stream));
+    std::vector<CopySpan> rows((size_t)g->S);           // (rows are padded on the device only)
+    for (int s = 0; s < g->S; ++s) rows[s] = {g->logits + (size_t)s * g->Vp, h_logits + (size_t)s * g->V, (size_t)g->V * 4};
+    TB_TRY(copy_d2h(rows.data(), g->S, g->stream));
+    return device_error_result(g->ctx);
 }
 
 void* tb_decoder_stream(TbDecoder* g) { return g->stream; }
