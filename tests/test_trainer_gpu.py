@@ -244,3 +244,22 @@ def test_loss_trajectory_200_steps(tb, oracle, precision):
     assert worst <= 1e-2, worst
     assert loss_c < np.log(V) - 0.3       # it actually trained
     g.destroy()
+
+
+@pytest.mark.parametrize("cfg", [(97, 64, 2, 2, 128, 45, 3, 1e-5), (97, 128, 2, 1, 128, 77, 2, 1e-5), (97, 128, 2, 1, 64, 9, 5, 1e-5)],
+                         ids=["head_dim_32", "head_dim_64", "several_sequences_in_32_rows"])
+def test_positions_of_sequences_that_end_inside_a_tile(tb, oracle, cfg):
+    """Context lengths that are no multiple of 32: the QKV projection rotates and splits its rows sequence by sequence."""
+    from turkce_llm_b200.gpu_train import GRADS
+    V, D, H, L, F, T, B, eps = cfg
+    g, p, off, num = make_params(oracle, cfg, 3)
+    rng = np.random.default_rng(4)
+    ids, tgt = (rng.integers(0, V, B * T).astype(np.uint32) for _ in range(2))
+    g.upload(p)
+    loss = g.forward_backward(ids, tgt)
+    grads = g.download(GRADS)
+    want_loss, want_grads, _ = oracle.model_forward_backward(cfg, p, ids, tgt, mode=FP32)
+    assert abs(loss - want_loss) <= 1e-4 * abs(want_loss)
+    for i, (o, n) in enumerate(zip(off, num)):
+        assert compare_tensor_bad(grads[o:o + n], want_grads[o:o + n], GRAD_TOL) == 0, "parameter %d" % i
+    g.destroy()

@@ -80,10 +80,17 @@ struct AttFwdParams {
 };
 
 // ------------------------------------------------------------------------------------ forward
-// CTA = 6 warps: TMA producer, MMA issuer (owns TMEM: two score buffers of 64 key columns and two
-// P V buffers of 64 head-dim columns), four softmax warps (thread = query row).  Keys are taken in
-// half blocks of 64 and the steps are software-pipelined: while the softmax warps work on half block
-// i, the tensor core computes the scores of i+1 and P V of i-1.  Two CTAs fit per SM on top of that.
+// CTA = 6 warps: TMA producer, MMA issuer (owns TMEM: two score buffers of 64 key columns and the output accumulator of
+// 64 head-dim columns), four softmax warps (thread = query row).  Keys are taken in half blocks of 64 and the steps are
+// software-pipelined: while the softmax warps work on half block i, the tensor core computes the scores of i+1 and adds
+// P V of i-1.  Two CTAs fit per SM on top of that.
+// The softmax warps bound the kernel (a half block of a CTA is 8192 exponentials, 512 clocks at 16 per clock), so the running
+// output stays in tensor memory: the row maximum that the exponentials are taken against is only moved when it has grown by
+// more than 2^8 (kLazyMax), and only then is the accumulator read, rescaled and written back.  The probabilities then reach
+// 2^8 instead of 1, with the same relative error in bf16, and the row sum is kept against the same maximum.  Reading every
+// P V back and folding it in with a factor of its own, as before, was a third of a softmax warp's instructions.
+constexpr float kLazyMax = 8.0f;        // in units of log2
+
 __global__ void __launch_bounds__(192, 2)
 attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -106,8 +113,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     uint64_t* s_full = bars + 7;      // 2: score buffer b holds Q K^T of a 64-key half block
     uint64_t* s_free = bars + 9;      // 2
     uint64_t* p_full = bars + 11;     // 2: probability buffer b written
-    uint64_t* o_full = bars + 13;     // 2: P V of a half block landed in output buffer b
-    uint64_t* o_free = bars + 15;     // 2
+    uint64_t* o_full = bars + 13;     // 2: P V of a half block of parity b has been added
     uint64_t* out_full = bars + 18;   // 4 arrivals: the output tile is staged in shared memory
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -125,7 +131,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int i = 0; i < 2; ++i) { mbar_init(&k_full[i], 1); mbar_init(&v_full[i], 1); mbar_init(&kv_empty[i], 1); }
         for (int i = 0; i < 2; ++i) {
             mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 4); mbar_init(&p_full[i], 4);
-            mbar_init(&o_full[i], 1); mbar_init(&o_free[i], 4);
+            mbar_init(&o_full[i], 1);
         }
         mbar_init(out_full, 4);
         *abort_flag = 0;
@@ -137,7 +143,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();                 // everything above is independent of earlier kernels' results
-    // TMEM: two score buffers of 64 key columns, two output buffers of 64 head-dim columns
+    // TMEM: two score buffers of 64 key columns, the output accumulator of 64 head-dim columns
     const uint32_t tS = tmem_base, tO = tmem_base + 128;
     const int nsub = 2 * nkv;                         // 64-key half blocks
 
@@ -186,13 +192,12 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 const uint32_t par = (uint32_t)((i >> 1) & 1);
                 if (!mbar_wait(&p_full[b], par, abort_flag)) { ok = false; break; }
                 if (b == 0 && !mbar_wait(&v_full[st], (uint32_t)((j >> 1) & 1), abort_flag)) { ok = false; break; }
-                if (!mbar_wait(&o_free[b], par ^ 1u, abort_flag)) { ok = false; break; }
                 tc_fence_after();
                 const uint64_t dP = dP0 + (uint64_t)b * TILESTEP;
                 const uint64_t dV = dV0 + (uint64_t)st * TILESTEP + (uint64_t)b * (4 * MNSTEP);
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    umma_bf16(tO + (uint32_t)(b * 64), dP + k * KSTEP, dV + k * MNSTEP, idesc_o, k > 0 ? 1u : 0u);
+                    umma_bf16(tO, dP + k * KSTEP, dV + k * MNSTEP, idesc_o, (i | k) != 0 ? 1u : 0u);
                 umma_commit(&o_full[b]);
                 if (b == 1) umma_commit(&kv_empty[st]);          // both halves of the K/V tile are consumed
                 if (i + 2 < nsub) ok = issue_scores(i + 2);
@@ -204,33 +209,9 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         const int r = q * 32 + lane;                 // row of the tile = TMEM lane
         const int qi = q0 + r;                       // query position
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
-        float m = -INFINITY, l = 0.0f;
-        float O[ATT_HD];
-#pragma unroll
-        for (int d = 0; d < ATT_HD; ++d) O[d] = 0.0f;
+        float m = -INFINITY, l = 0.0f;               // the maximum the exponentials are taken against, and their sum
         bool ok = true;
-        float alpha_prev = 0.0f;                     // rescale factor of the half block whose P V is still due
-        // adds P V of half block i (output buffer i&1) into the running output: O = O * alpha_i + P_i V_i
-        uint32_t va[32], vb[32];                     // one half block's scores (or one P V result) per row
-        auto accumulate = [&](int i, float alpha) -> bool {
-            const int b = i & 1;
-            if (!mbar_wait(&o_full[b], (uint32_t)((i >> 1) & 1), abort_flag)) return false;
-            tc_fence_after();
-            tmem_ld32(tO + lane_base + (uint32_t)(b * 64), va);
-            tmem_ld32(tO + lane_base + (uint32_t)(b * 64 + 32), vb);
-            tmem_ld_wait();
-            const float2 al2 = make_float2(alpha, alpha);
-#pragma unroll
-            for (int e = 0; e < 32; e += 2) {
-                const float2 o0 = __ffma2_rn(make_float2(O[e], O[e + 1]), al2, pair_of(va[e], va[e + 1]));
-                const float2 o1 = __ffma2_rn(make_float2(O[32 + e], O[33 + e]), al2, pair_of(vb[e], vb[e + 1]));
-                O[e] = o0.x; O[e + 1] = o0.y; O[32 + e] = o1.x; O[33 + e] = o1.y;
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&o_free[b]);
-            return true;
-        };
+        uint32_t va[32], vb[32];                     // one half block's scores (or the accumulator) of this row
         for (int i = 0; i < nsub && ok; ++i) {
             const int b = i & 1;
             if (!mbar_wait(&s_full[b], (uint32_t)((i >> 1) & 1), abort_flag)) { ok = false; break; }
@@ -263,11 +244,16 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
             }
             const float m_new = fmaxf(m, mx * p.scale_log2);
-            const float alpha = fast_exp2(m - m_new);        // 0 on the first block (m = -inf)
-            l *= alpha;
+            float alpha = 1.0f;
+            if (m_new > m + kLazyMax) {                       // (each row for itself: a row does not depend on its neighbours)
+                alpha = fast_exp2(m - m_new);                // 0 on the first block (m = -inf)
+                l *= alpha;
+                m = m_new;
+            }
+            const bool move = __any_sync(0xffffffffu, alpha != 1.0f);
             // p = 2^(s*c - m), row sum, bf16 P into shared memory (K-major, 128B swizzle)
             float pa[32], pb[32];
-            const float2 c2 = make_float2(p.scale_log2, p.scale_log2), nm2 = make_float2(-m_new, -m_new);
+            const float2 c2 = make_float2(p.scale_log2, p.scale_log2), nm2 = make_float2(-m, -m);
             float2 la = make_float2(0.f, 0.f), lb = make_float2(0.f, 0.f);
 #pragma unroll
             for (int e = 0; e < 32; e += 2) {
@@ -283,18 +269,36 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 lb = __fadd2_rn(lb, make_float2(pb[e], pb[e + 1]));
             }
             l += (la.x + la.y) + (lb.x + lb.y);
+            if (move && i > 0) {
+                // P V of the half blocks so far, against the old maximum: rescaled once the last of them has been added
+                if (!mbar_wait(&o_full[b ^ 1], (uint32_t)(((i - 1) >> 1) & 1), abort_flag)) { ok = false; break; }
+                tc_fence_after();
+#pragma unroll
+                for (int h2 = 0; h2 < 2; ++h2) {
+                    tmem_ld32(tO + lane_base + (uint32_t)(h2 * 32), va);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) va[e] = __float_as_uint(__uint_as_float(va[e]) * alpha);
+                    tmem_st32(tO + lane_base + (uint32_t)(h2 * 32), va);
+                }
+                tmem_st_wait();
+            }
+            // the probabilities of two half blocks ago have been multiplied
+            if (i >= 2 && !mbar_wait(&o_full[b], (uint32_t)(((i >> 1) - 1) & 1), abort_flag)) { ok = false; break; }
             store_chunk_bf16(sP, r, 2 * b, pa);
             store_chunk_bf16(sP, r, 2 * b + 1, pb);
             tc_fence_before();
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) { mbar_arrive(&s_free[b]); mbar_arrive(&p_full[b]); }
-            // the previous half block's P V has had this whole softmax to finish: add it now
-            if (i > 0) ok = accumulate(i - 1, alpha_prev);
-            alpha_prev = alpha;
-            m = m_new;
         }
-        if (ok) ok = accumulate(nsub - 1, alpha_prev);
+        if (ok) ok = mbar_wait(&o_full[(nsub - 1) & 1], (uint32_t)(((nsub - 1) >> 1) & 1), abort_flag);
+        if (ok) {
+            tc_fence_after();
+            tmem_ld32(tO + lane_base, va);
+            tmem_ld32(tO + lane_base + 32u, vb);
+            tmem_ld_wait();
+        }
         if (ok) {
             // O / l as bf16 into the Q tile (every product has completed), one TMA store for the 128 rows: a thread per
             // row storing to global memory directly touches 32 different rows per instruction
@@ -305,11 +309,12 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
                 for (int d = 0; d < ATT_HD; d += 8) {
                     if (d >= p.hd) break;
+                    float o[8];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) o[e] = __uint_as_float(d < 32 ? va[(d + e) & 31] : vb[(d + e) & 31]) * inv;
                     uint4 pk;
-                    __nv_bfloat162 h0 = __floats2bfloat162_rn(O[d + 0] * inv, O[d + 1] * inv);
-                    __nv_bfloat162 h1 = __floats2bfloat162_rn(O[d + 2] * inv, O[d + 3] * inv);
-                    __nv_bfloat162 h2 = __floats2bfloat162_rn(O[d + 4] * inv, O[d + 5] * inv);
-                    __nv_bfloat162 h3 = __floats2bfloat162_rn(O[d + 6] * inv, O[d + 7] * inv);
+                    __nv_bfloat162 h0 = __floats2bfloat162_rn(o[0], o[1]), h1 = __floats2bfloat162_rn(o[2], o[3]);
+                    __nv_bfloat162 h2 = __floats2bfloat162_rn(o[4], o[5]), h3 = __floats2bfloat162_rn(o[6], o[7]);
                     pk.x = *reinterpret_cast<uint32_t*>(&h0); pk.y = *reinterpret_cast<uint32_t*>(&h1);
                     pk.z = *reinterpret_cast<uint32_t*>(&h2); pk.w = *reinterpret_cast<uint32_t*>(&h3);
                     *reinterpret_cast<uint4*>(row + (((d >> 3) ^ (r & 7)) << 4)) = pk;

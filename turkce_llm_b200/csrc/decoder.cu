@@ -297,8 +297,18 @@ int tb_decoder_prefill(TbDecoder* g, const uint32_t* h_ids, int prompt_len) {
     TB_TRY(launch_embed_fwd(c, P32(g, 0), g->ids, g->x, N, D, st));
     for (int l = 0; l < g->L; ++l) {
         TB_TRY(launch_rmsnorm_fwd(c, g->x, P32(g, pidx(l, PK_ATTN_NORM)), g->n, g->r, N, D, g->eps, st));
-        TB_TRY(linear(g, g->n, P16(g, pidx(l, PK_WQKV)), P32(g, pidx(l, PK_BQKV)), nullptr, g->qkv, N, 3 * D, D));
-        TB_TRY(launch_rope_split(c, g->qkv, g->cos_t, g->sin_t, g->Q, g->Kc[l], g->Vc[l], S, T, H, hd, g->cap, st));
+        if (hd == 32 || hd == 64) {
+            // rotation, head split and the cache append in the projection's epilogue
+            GemmArgs s;
+            s.kind = GEMM_NN; s.A = g->n; s.B = P16(g, pidx(l, PK_WQKV)); s.M = N; s.N = 3 * D; s.K = D; s.lda = D; s.ldb = 3 * D;
+            s.bias = P32(g, pidx(l, PK_BQKV)); s.splits = 1;
+            s.rope_qkv = g->Q; s.rope_k = g->Kc[l]; s.rope_v = g->Vc[l]; s.rope_kv_rows = g->cap;
+            s.rope_cos = g->cos_t; s.rope_sin = g->sin_t; s.rope_T = T; s.rope_H = H; s.rope_hd = hd;
+            TB_TRY(launch_gemm_bf16_ws(c, s, g->splitk_ws, g->splitk_floats, st));
+        } else {
+            TB_TRY(linear(g, g->n, P16(g, pidx(l, PK_WQKV)), P32(g, pidx(l, PK_BQKV)), nullptr, g->qkv, N, 3 * D, D));
+            TB_TRY(launch_rope_split(c, g->qkv, g->cos_t, g->sin_t, g->Q, g->Kc[l], g->Vc[l], S, T, H, hd, g->cap, st));
+        }
         TB_TRY(launch_attention_fwd(c, g->Q, g->Kc[l], g->Vc[l], g->att, nullptr, S, H, T, hd, g->scale, st, g->cap));
         TB_TRY(layer_tail(g, l, N));
     }

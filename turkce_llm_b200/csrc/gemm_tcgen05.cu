@@ -79,6 +79,9 @@ struct GemmParams {
                                 // 4: softmax statistics only (cross-entropy pass 1), nothing stored
                                 // 5: bf16 tiles into [3][B][H][T][hd] with q, k rotated (tmC is a 5-D map)
     const float* rope_cos; const float* rope_sin; int rope_T, rope_H, rope_hd;
+    int rope_direct;            // the tiles leave by ordinary stores, row by row: sequences whose length is no multiple of 32,
+    bf16 *rope_q, *rope_k, *rope_v;   // or K and V in a cache with rope_kv_rows rows per head
+    int rope_kv_rows;
     int ce_mode;                // 2: bf16 tile stores carry (exp(z - lse[row]) - onehot) * ce_scale
     const uint32_t* ce_targets; float* ce_stats; float* ce_ztarget; const float* ce_lse; float ce_scale;
     int pair_off;               // mode 3: F; tile columns [0,BN/2) are gate columns n0/2.., [BN/2,BN) up columns F + n0/2..
@@ -523,7 +526,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             // mode 5: position of this thread's row, and of the 32-row chunk, inside its sequence (once per tile)
             const int rope_D = p.rope_H * p.rope_hd, rope_shift = p.rope_hd == 64 ? 6 : 5;
             int rope_b = 0, rope_t0 = 0, rope_t = 0;
-            if (m_rope) { rope_b = gm0 / p.rope_T; rope_t0 = gm0 - rope_b * p.rope_T; rope_t = rope_t0 + lane; }
+            if (m_rope) {
+                rope_b = gm0 / p.rope_T; rope_t0 = gm0 - rope_b * p.rope_T; rope_t = rope_t0 + lane;
+                if (rope_t >= p.rope_T) rope_t %= p.rope_T;          // (only where 32 rows can lie in two sequences)
+            }
             if (m_res && lane == 0 && rows_in && col0 < p.N) {
                 mbar_expect_tx(rbar, 4096);
                 tma_load_4d(rbuf, &tmR, rbar, col0, gm0, 0, c.z);
@@ -698,6 +704,29 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     }
                 }
                 if (paired && !second) continue;              // the unit leaves after its second chunk
+                if (m_rope && p.rope_direct) {
+                    // row by row: 8 (head dim 64) or 4 adjacent lanes write a row's values of one head, 128 or 64 bytes
+                    __syncwarp();
+                    const int g0 = paired ? gn0 - 32 : gn0;
+                    if (rows_in && g0 < p.N) {
+                        const int which = g0 >= 2 * rope_D ? 2 : (g0 >= rope_D ? 1 : 0), cin = g0 - which * rope_D, head = cin >> rope_shift;
+                        bf16* base = which == 0 ? p.rope_q : which == 1 ? p.rope_k : p.rope_v;
+                        const int per = which == 0 ? p.rope_T : p.rope_kv_rows;
+                        const int lanes = paired ? 8 : 4, piece = lane & (lanes - 1);
+                        const uint8_t* src = obuf + b * 4096;
+#pragma unroll 2
+                        for (int row = lane / lanes; row < 32 && gm0 + row < p.M; row += 32 / lanes) {
+                            int t = rope_t0 + row, sq = rope_b;
+                            while (t >= p.rope_T) { t -= p.rope_T; ++sq; }
+                            const uint4 v4 = *reinterpret_cast<const uint4*>(paired ? src + row * 128 + ((piece ^ (row & 7)) << 4)
+                                                                                    : src + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4));
+                            *reinterpret_cast<uint4*>(base + (((long long)sq * p.rope_H + head) * per + t) * p.rope_hd +
+                                                      (cin & (p.rope_hd - 1)) + piece * 8) = v4;
+                        }
+                    }
+                    ++cnt;
+                    continue;
+                }
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0 && paired) {
@@ -1097,6 +1126,7 @@ static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
     };
     if (a.swiglu_h)      // paired gate/up tile: 128 wide, or 256 wide on a CTA pair
         return ((a.bn == 256 || (a.bn == 0 && pair_ok && cost_of(256) < cost_of(128))) && a.N % 256 == 0) ? 256 : 128;
+    if (a.rope_qkv && a.bn == 0) return 128;      // the width its epilogue is compiled for (192 and 256 gained nothing)
     if (a.dsw_dgu) return (a.bn == 256 || (a.bn == 0 && pair_ok)) ? 256 : 128;      // its chunks leave in pairs
     if (a.ce_mode != 0) return a.bn == 256 ? 256 : 192;     // the statistics are laid out per tile of this width
     if (a.bn == 64 || a.bn == 128 || a.bn == 192 || a.bn == 256 || a.bn == 384) return a.bn;
@@ -1211,8 +1241,8 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         TB_CHECK(a.kind == GEMM_NN && !a.tf32 && a.batch == 1 && splits == 1 && a.alpha == 1.0f && a.beta == 0.0f &&
                      !a.residual && !a.C32 && !a.C16 && !a.swiglu_h && a.ce_mode == 0 && a.causal == CAUSAL_NONE &&
                      a.rope_cos && a.rope_sin && (a.rope_hd == 32 || a.rope_hd == 64) && a.rope_T > 0 &&
-                     a.rope_T % 32 == 0 && a.M % a.rope_T == 0 && a.N == 3 * a.rope_H * a.rope_hd && aligned16(a.rope_qkv),
-                 "fused QKV + position-embedding GEMM: needs a plain NN bf16 product with N = 3*H*hd, hd 32 or 64, T %% 32 == 0");
+                     a.M % a.rope_T == 0 && a.N == 3 * a.rope_H * a.rope_hd && aligned16(a.rope_qkv) && aligned16(a.rope_k) && aligned16(a.rope_v),
+                 "fused QKV + position-embedding GEMM: needs a plain NN bf16 product with N = 3*H*hd, hd 32 or 64");
     }
     if (a.ce_mode != 0) {
         TB_CHECK(a.kind == GEMM_NT && !a.tf32 && a.batch == 1 && (bn == 192 || bn == 256) && splits == 1 && a.alpha == 1.0f &&
@@ -1294,6 +1324,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
     p.ce_lse = a.ce_lse; p.ce_scale = a.ce_scale;
     p.bias_vec = p.bias && aligned16(p.bias);
     p.rope_cos = a.rope_cos; p.rope_sin = a.rope_sin; p.rope_T = a.rope_T; p.rope_H = a.rope_H; p.rope_hd = a.rope_hd;
+    p.rope_direct = 0;
     if (a.ce_mode == 1) {
         p.tma_mode = 4;
     } else if (a.rope_qkv) {
@@ -1304,6 +1335,11 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         cuuint64_t strides[4] = {hd * 2, T * hd * 2, H * T * hd * 2, Bn * H * T * hd * 2};
         // head dim 64 on 128- or 256-column tiles: a warp's chunk pairs are whole heads and leave in rows of 128 bytes
         const bool wide = a.rope_hd == 64 && (bn == 128 || bn == 256) && getenv("TB_GEMM_NO_WIDE16") == nullptr;
+        p.rope_direct = (a.rope_T % 32 != 0 || a.rope_kv_rows > 0) ? 1 : 0;
+        p.rope_q = a.rope_qkv;
+        p.rope_k = a.rope_k ? a.rope_k : a.rope_qkv + (long long)a.M * a.rope_H * a.rope_hd;
+        p.rope_v = a.rope_v ? a.rope_v : a.rope_qkv + 2LL * a.M * a.rope_H * a.rope_hd;
+        p.rope_kv_rows = a.rope_kv_rows > 0 ? a.rope_kv_rows : a.rope_T;
         cuuint32_t box[5] = {wide ? 64u : 32u, 32u, 1u, 1u, 1u};
         cuuint32_t estr[5] = {1u, 1u, 1u, 1u, 1u};
         CUresult r = enc(&tmC, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, a.rope_qkv, dims, strides, box, estr,

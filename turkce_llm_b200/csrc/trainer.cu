@@ -92,7 +92,7 @@ struct TbTrainer {
     std::vector<Segment> segments;
     bool graphs_on = true;
     bool fused_attention = true;   // head_dim <= 64: scores stay on chip
-    bool fused_rope = true;        // T % 32 == 0, head_dim 32 or 64: rotation and head split in the QKV GEMM epilogue
+    bool fused_rope = true;        // head_dim 32 or 64: rotation and head split in the QKV GEMM epilogue
     bool fused_ce = true;          // cross-entropy inside the LM-head GEMM epilogues: no [N, V] logits
     bool fused_dswiglu = false;    // SwiGLU backward in the epilogue of the down-projection's input-gradient GEMM
     bool fused_swiglu = true;      // d_ff % 64 == 0: silu(gate) * up formed in the gate|up GEMM's epilogue
@@ -599,7 +599,7 @@ int tb_trainer_create_prec(TbTrainer** out, int V, int D, int H, int L, int F, i
     TB_CHECK(!g->tf32 || g->fused_attention, "the TF32 mode needs head_dim <= 64 (the attention core is the fused bf16 kernel)");
     g->fused_swiglu = !g->tf32 && F % 64 == 0 && getenv("TB_NO_FUSED_SWIGLU") == nullptr;
     g->fused_dswiglu = g->fused_swiglu && getenv("TB_NO_FUSED_DSWIGLU") == nullptr;
-    g->fused_rope = !g->tf32 && T % 32 == 0 && (D / H == 32 || D / H == 64) && getenv("TB_NO_FUSED_ROPE") == nullptr;
+    g->fused_rope = !g->tf32 && (D / H == 32 || D / H == 64) && getenv("TB_NO_FUSED_ROPE") == nullptr;
     g->V = V; g->D = D; g->H = H; g->L = L; g->F = F; g->T = T; g->B = B; g->N = B * T; g->hd = D / H;
     g->Vp = round_up(V, 8);
     g->Tp = round_up(T, 8);
