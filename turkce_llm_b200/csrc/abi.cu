@@ -268,8 +268,8 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
         bf16* pb = static_cast<bf16*>(ctx->scratch);
         bf16* pa = reinterpret_cast<bf16*>(static_cast<char*>(ctx->scratch) + b_bytes);
         float* ws = reinterpret_cast<float*>(static_cast<char*>(ctx->scratch) + a_bytes + b_bytes);
-        TB_TRY(launch_pack_bf16(ctx, A, pa, a_rows, a_cols, lda, a_ld, batch, sA, a_stride, stream));
-        if (!same_b) TB_TRY(launch_pack_bf16(ctx, B, pb, b_rows, b_cols, ldb, b_ld, batch, sB, b_stride, stream));
+        ConvSide sides[2] = {{A, pa, a_rows, a_cols, lda, a_ld, sA, a_stride}, {B, pb, b_rows, b_cols, ldb, b_ld, sB, b_stride}};
+        TB_TRY(launch_pack_operands(ctx, sides, same_b ? 1 : 2, batch, stream));
         g.A = pa; g.B = pb;
         return launch_gemm_bf16_ws(ctx, g, ws, ws_floats, stream);
     }
@@ -299,11 +299,15 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
     float* pa = reinterpret_cast<float*>(static_cast<char*>(ctx->scratch) + b_bytes);
     float* ws = reinterpret_cast<float*>(static_cast<char*>(ctx->scratch) + a_bytes + b_bytes);
     if (split3) {
-        TB_TRY(launch_split3_f32(ctx, A, pa, a_rows, a_cols, lda, a_ld, a_cat_cols ? 1 : 0, 0, batch, sA, a_stride, stream));
-        if (!same_b) TB_TRY(launch_split3_f32(ctx, B, pb, b_rows, b_cols, ldb, b_ld, b_cat_cols ? 1 : 0, 1, batch, sB, b_stride, stream));
+        ConvSide sides[2] = {{A, pa, a_rows, a_cols, lda, a_ld, sA, a_stride, a_cat_cols ? 1 : 0, 0},
+                             {B, pb, b_rows, b_cols, ldb, b_ld, sB, b_stride, b_cat_cols ? 1 : 0, 1}};
+        TB_TRY(launch_split3_operands(ctx, sides, same_b ? 1 : 2, batch, stream));
     } else {
-        if (!a_inplace) TB_TRY(launch_copy_f32(ctx, A, pa, a_rows, a_cols, lda, a_ld, batch, sA, a_stride, stream));
-        if (!b_inplace && !same_b) TB_TRY(launch_copy_f32(ctx, B, pb, b_rows, b_cols, ldb, b_ld, batch, sB, b_stride, stream));
+        ConvSide sides[2] = {};
+        int n = 0;
+        if (!a_inplace) sides[n++] = {A, pa, a_rows, a_cols, lda, a_ld, sA, a_stride};
+        if (!b_inplace && !same_b) sides[n++] = {B, pb, b_rows, b_cols, ldb, b_ld, sB, b_stride};
+        if (n) TB_TRY(launch_copy_operands(ctx, sides, n, batch, stream));
     }
     g.A = a_inplace ? static_cast<const void*>(A) : pa;
     g.B = b_inplace ? static_cast<const void*>(B) : pb;

@@ -211,15 +211,21 @@ int launch_decode_cluster(DeviceCtx* ctx, DecodeCluster* m, const uint32_t* tok,
                           bf16* out, cudaStream_t st);
 
 // ---- operand packing (pack.cu)
-// float32 [rows, cols] -> float32 copy with another leading dimension (makes a matrix TMA-addressable)
-int launch_copy_f32(DeviceCtx* ctx, const float* src, float* dst, int rows, int cols, long long ld_src,
-                    long long ld_dst, int batch, long long stride_src, long long stride_dst, cudaStream_t stream);
-// float32 x -> three tf32-exact pieces for the 3xTF32 product: hi = x truncated to tf32, lo = x - hi.
-// along_cols: dst [rows, 3*cols] = [p0 | p1 | p2], else dst [3*rows, cols] = [p0 ; p1 ; p2];
-// pattern 0: (hi, hi, lo)   pattern 1: (hi, lo, hi)
-int launch_split3_f32(DeviceCtx* ctx, const float* src, float* dst, int rows, int cols, long long ld_src,
-                      long long ld_dst, int along_cols, int pattern, int batch, long long stride_src,
-                      long long stride_dst, cudaStream_t stream);
+// One float32 matrix on its way to an operand.  along_cols, pattern: for the pieces of the 3xTF32 product, hi = x
+// truncated to tf32 and lo = x - hi: dst [rows, 3*cols] = [p0 | p1 | p2], else dst [3*rows, cols] = [p0 ; p1 ; p2];
+// pattern 0: (hi, hi, lo)   pattern 1: (hi, lo, hi).  vec and blocks are filled in by the launcher.
+struct ConvSide {
+    const float* src; void* dst;
+    int rows, cols;
+    long long ld_src, ld_dst, stride_src, stride_dst;
+    int along_cols, pattern;
+    int vec, blocks;
+};
+// one or both operands of a product (`batch` matrices each) in one launch: as bf16, as float32 with another leading
+// dimension (makes a matrix TMA-addressable), as the pieces of the 3xTF32 product.  `sides` has room for two.
+int launch_pack_operands(DeviceCtx* ctx, ConvSide* sides, int count, int batch, cudaStream_t stream);
+int launch_copy_operands(DeviceCtx* ctx, ConvSide* sides, int count, int batch, cudaStream_t stream);
+int launch_split3_operands(DeviceCtx* ctx, ConvSide* sides, int count, int batch, cudaStream_t stream);
 // float32 [rows, cols] (ld) -> bf16 [rows, cols] (ld_out), batched
 // Decode-time LM head with fused greedy choice (lmhead_decode.cu): tok[s] = argmax_v <X[s,:], E[v,:]>,
 // S <= 64 rows of X [S, K] bf16, E [V, K] bf16; best (64 words) and ticket (1 word) are zeroed device
@@ -253,18 +259,23 @@ static inline long long round_up(long long x, long long m) { return (x + m - 1) 
 // ---- launches with programmatic dependent launch: the next kernel of the stream may be scheduled
 // and run its prologue while this one drains; every kernel of this library therefore executes
 // pdl_wait() before it touches global memory (a no-op for a launch without the attribute).
-int pdl_mode();     // 0 off, 1 every launch, 2 only launches with >= 64 KB of dynamic shared memory
+// Mode 2 (the default) gives the attribute to the kernels that have a prologue worth hiding (64 KB of dynamic shared memory
+// or more) and to grids of up to 64 blocks: those fit beside what is still running, and in a chain of small launches
+// the hand-over is most of the time (a training step of 61 launches: 238 -> 228 us).  A larger grid's waiting blocks take
+// the thread slots of the kernel they wait for, or of one on another stream (attention at 16 x 1024 with it everywhere:
+// 147 -> 162 us; up to 148 blocks: TF32 step of 28 x 128 tokens 4394 -> 4468 us).
+constexpr long long kEarlyBlocks = 64;
+int pdl_mode();     // 0 off, 1 every launch, 2 by the rule above
 
 // cluster_x > 1: thread-block clusters of that many CTAs along x (the grid must be a multiple of it)
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_kernel_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                         cudaStream_t stream, int cluster_x, Args&&... args) {
+inline cudaError_t launch_kernel_as(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                    cudaStream_t stream, int cluster_x, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int n = 0;
-    const int mode = pdl_mode();
-    if (mode == 1 || (mode == 2 && smem >= 65536)) {
+    if (early && pdl_mode() != 0) {
         attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n].val.programmaticStreamSerializationAllowed = 1;
         ++n;
@@ -280,9 +291,23 @@ inline cudaError_t launch_kernel_cluster(void (*kernel)(KArgs...), dim3 grid, di
 }
 
 template <typename... KArgs, typename... Args>
+inline cudaError_t launch_kernel_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                         cudaStream_t stream, int cluster_x, Args&&... args) {
+    const bool early = pdl_mode() == 1 || smem >= 65536 || (long long)grid.x * grid.y * grid.z <= kEarlyBlocks;
+    return launch_kernel_as(early, kernel, grid, block, smem, stream, cluster_x, static_cast<Args&&>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
 inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                  Args&&... args) {
     return launch_kernel_cluster(kernel, grid, block, smem, stream, 1, static_cast<Args&&>(args)...);
+}
+
+// whatever the grid: short kernels between GEMMs (one CTA per SM), which leave the thread slots free
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_kernel_early(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                       Args&&... args) {
+    return launch_kernel_as(true, kernel, grid, block, smem, stream, 1, static_cast<Args&&>(args)...);
 }
 
 #ifdef __CUDACC__

@@ -910,7 +910,9 @@ __global__ void reduce_splits_kernel(const float* __restrict__ part, float* __re
     for (long long iv = (long long)blockIdx.x * blockDim.x + threadIdx.x; iv < nvec;
          iv += (long long)gridDim.x * blockDim.x) {
         const long long i = iv * VEC;
-        const int r = (int)(i / N), cidx = (int)(i % N);
+        int r, cidx;
+        if (per < (1LL << 31)) { r = (int)((unsigned)i / (unsigned)N); cidx = (int)((unsigned)i - (unsigned)r * (unsigned)N); }
+        else { r = (int)(i / N); cidx = (int)(i % N); }
         const float* src = part + ((long long)z * splits) * per + i;
         float s[VEC];
 #pragma unroll
@@ -1449,11 +1451,14 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         if (blocks > 8 * ctx->sm_count) blocks = 8 * ctx->sm_count;
         if (blocks < 1) blocks = 1;
         dim3 grid(blocks, a.batch);
+        // (alone on its SMs behind the product it may be launched early whatever its grid; beside another product it would
+        // take that one's thread slots)
+        const bool early = a.max_ctas == 0 || (long long)blocks * a.batch <= kEarlyBlocks;
         prof_mark(ctx, "splitk_reduce", 0.0, (double)(splits + 2) * per * a.batch * 4.0, stream);
         if (vec4)
-            TB_CUDA(launch_kernel((reduce_splits_kernel<4>), dim3(grid), dim3(256), 0, stream, ws, a.C32, a.C16, a.M, a.N, a.ldc32, a.ldc16, splits, a.strideC32, a.strideC16, a.beta, a.bias));
+            TB_CUDA(launch_kernel_as(early, (reduce_splits_kernel<4>), dim3(grid), dim3(256), 0, stream, 1, ws, a.C32, a.C16, a.M, a.N, a.ldc32, a.ldc16, splits, a.strideC32, a.strideC16, a.beta, a.bias));
         else
-            TB_CUDA(launch_kernel((reduce_splits_kernel<1>), dim3(grid), dim3(256), 0, stream, ws, a.C32, a.C16, a.M, a.N, a.ldc32, a.ldc16, splits, a.strideC32, a.strideC16, a.beta, a.bias));
+            TB_CUDA(launch_kernel_as(early, (reduce_splits_kernel<1>), dim3(grid), dim3(256), 0, stream, 1, ws, a.C32, a.C16, a.M, a.N, a.ldc32, a.ldc16, splits, a.strideC32, a.strideC16, a.beta, a.bias));
         TB_CUDA(cudaGetLastError());
         ctx->launches++;
         prof_close(ctx, stream);
