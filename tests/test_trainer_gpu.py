@@ -263,3 +263,28 @@ def test_positions_of_sequences_that_end_inside_a_tile(tb, oracle, cfg):
     for i, (o, n) in enumerate(zip(off, num)):
         assert compare_tensor_bad(grads[o:o + n], want_grads[o:o + n], GRAD_TOL) == 0, "parameter %d" % i
     g.destroy()
+
+
+@pytest.mark.parametrize("precision", ["bf16", "tf32"])
+@pytest.mark.parametrize("cfg", [(97, 384, 6, 2, 256, 256, 40, 1e-5),      # more row blocks than clusters at once
+                                 (97, 256, 4, 2, 64, 33, 5, 1e-5),         # rows that end inside a 32-row strip
+                                 (97, 192, 3, 1, 64, 7, 1, 1e-5),          # one CTA holds the row
+                                 (97, 768, 12, 1, 64, 100, 2, 1e-5)],      # four CTAs
+                         ids=["waves", "ragged", "one_cta", "four_ctas"])
+def test_rmsnorm_in_the_projection_epilogues(tb, oracle, monkeypatch, cfg, precision):
+    """RMSNorm of the out- and down-projections' results inside their epilogues against the separate kernel."""
+    from turkce_llm_b200.gpu_train import GRADS
+    V, D, H, L, F, T, B, eps = cfg
+    rng = np.random.default_rng(4)
+    ids, tgt = (rng.integers(0, V, B * T).astype(np.uint32) for _ in range(2))
+    got = []
+    for separate in (False, True):
+        if separate:
+            monkeypatch.setenv("TB_NO_FUSED_NORM", "1")
+        g, p, off, num = make_params(oracle, cfg, 3, tb.PREC_TF32 if precision == "tf32" else tb.PREC_BF16)
+        g.upload(p)
+        got.append((g.forward_backward(ids, tgt), g.download(GRADS)))
+        g.destroy()
+    assert abs(got[0][0] - got[1][0]) <= 2e-5 * abs(got[1][0])
+    for i, (o, n) in enumerate(zip(off, num)):
+        assert rel_to_maxabs(got[0][1][o:o + n], got[1][1][o:o + n]) <= 1e-2, "parameter %d" % i

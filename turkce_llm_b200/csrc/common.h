@@ -159,6 +159,10 @@ struct GemmArgs {
     // K and V elsewhere (both, with rope_kv_rows >= T rows per head): a KV cache.  rope_qkv then receives Q alone.
     bf16 *rope_k = nullptr, *rope_v = nullptr;
     int rope_kv_rows = 0;
+    // RMSNorm of the result in the epilogue (kind NN with a residual, C32 = the residual stream): norm16 or norm32 [M, N] =
+    // C32 * norm_w / sqrt(mean(C32^2) + norm_eps), norm_rinv [M] (optional) = 1 / sqrt(..).  gemm_norm_supported(N).
+    const float* norm_w = nullptr; float norm_eps = 0.f;
+    float* norm_rinv = nullptr; bf16* norm16 = nullptr; float* norm32 = nullptr;
     int ce_mode = 0;
     const uint32_t* ce_targets = nullptr;
     float* ce_stats = nullptr;
@@ -168,6 +172,8 @@ struct GemmArgs {
 };
 
 int launch_gemm_bf16(DeviceCtx* ctx, const GemmArgs& a, cudaStream_t stream);
+// whether rows of N columns can be split into tiles over the CTAs of a cluster (GemmArgs::norm_w)
+bool gemm_norm_supported(const DeviceCtx* ctx, int N);
 // split-K with caller-provided partial-sum storage (needs splits*batch*M*N floats)
 int launch_gemm_bf16_ws(DeviceCtx* ctx, const GemmArgs& a, float* workspace, size_t workspace_floats,
                         cudaStream_t stream);

@@ -78,21 +78,25 @@ inline float* P32(TbDecoder* g, long long i) { return g->params + g->offsets[i];
 inline bf16* P16(TbDecoder* g, long long i) { return g->params16 + g->offsets[i]; }
 
 // C[M,N] = A[M,K] @ W[K,N] + bias (+ residual), float32 out
+// norm_w (optional): the result's RMSNorm -> g->n as well
 int linear(TbDecoder* g, const bf16* A, const bf16* W, const float* bias, const float* residual, float* C, int M,
-           int N, int K) {
+           int N, int K, const float* norm_w = nullptr) {
     GemmArgs a;
     a.kind = GEMM_NN; a.A = A; a.B = W; a.M = M; a.N = N; a.K = K; a.lda = K; a.ldb = N;
     a.C32 = C; a.ldc32 = N; a.bias = bias; a.residual = residual; a.ldr = N;
     a.splits = 1;
+    if (norm_w) { a.norm_w = norm_w; a.norm_eps = g->eps; a.norm16 = g->n; }
     return launch_gemm_bf16_ws(g->ctx, a, g->splitk_ws, g->splitk_floats, g->stream);
 }
 
-// the rest of a layer after attention, and the head; rows = number of token rows in flight
-int layer_tail(TbDecoder* g, int l, int rows) {
+// the rest of a layer after attention; rows = number of token rows in flight.  norm: the layer's RMSNorms come out of the
+// projections' epilogues, the one of the next layer (or the head) included.
+int layer_tail(TbDecoder* g, int l, int rows, bool norm) {
     DeviceCtx* c = g->ctx; cudaStream_t st = g->stream;
     const int D = g->D, F = g->F;
-    TB_TRY(linear(g, g->att, P16(g, pidx(l, PK_WO)), P32(g, pidx(l, PK_BO)), g->x, g->x2, rows, D, D));
-    TB_TRY(launch_rmsnorm_fwd(c, g->x2, P32(g, pidx(l, PK_FFN_NORM)), g->n, g->r, rows, D, g->eps, st));
+    TB_TRY(linear(g, g->att, P16(g, pidx(l, PK_WO)), P32(g, pidx(l, PK_BO)), g->x, g->x2, rows, D, D,
+                  norm ? P32(g, pidx(l, PK_FFN_NORM)) : nullptr));
+    if (!norm) TB_TRY(launch_rmsnorm_fwd(c, g->x2, P32(g, pidx(l, PK_FFN_NORM)), g->n, g->r, rows, D, g->eps, st));
     if (F % 64 == 0 && getenv("TB_NO_FUSED_SWIGLU") == nullptr) {
         GemmArgs s;       // h = silu(gate) * up in the projection's epilogue; gate|up themselves are not kept
         s.kind = GEMM_NN; s.A = g->n; s.B = P16(g, pidx(l, PK_WGU)); s.M = rows; s.N = 2 * F; s.K = D; s.lda = D;
@@ -102,7 +106,8 @@ int layer_tail(TbDecoder* g, int l, int rows) {
         TB_TRY(linear(g, g->n, P16(g, pidx(l, PK_WGU)), P32(g, pidx(l, PK_BGU)), nullptr, g->gu, rows, 2 * F, D));
         TB_TRY(launch_swiglu_fwd(c, g->gu, g->h, rows, F, st));
     }
-    TB_TRY(linear(g, g->h, P16(g, pidx(l, PK_WDOWN)), P32(g, pidx(l, PK_BDOWN)), g->x2, g->x, rows, D, F));
+    TB_TRY(linear(g, g->h, P16(g, pidx(l, PK_WDOWN)), P32(g, pidx(l, PK_BDOWN)), g->x2, g->x, rows, D, F,
+                  norm ? P32(g, l + 1 < g->L ? pidx(l + 1, PK_ATTN_NORM) : pidx(g->L, 0)) : nullptr));
     return 0;
 }
 
@@ -176,7 +181,7 @@ int decode_step_body(TbDecoder* g) {
             TB_TRY(launch_rope_attn_decode(c, g->qkv, g->cos_t, g->sin_t, g->Kc[l], g->Vc[l], g->att, g->pos, S, H, hd,
                                            g->cap, g->scale, st));
         }
-        TB_TRY(layer_tail(g, l, S));
+        TB_TRY(layer_tail(g, l, S, false));
     }
     return head(g, g->x, S, 1);
 }
@@ -294,9 +299,11 @@ int tb_decoder_prefill(TbDecoder* g, const uint32_t* h_ids, int prompt_len) {
     int* h_state = reinterpret_cast<int*>(g->h_pinned + N);
     h_state[0] = T; h_state[1] = 0;
     TB_CUDA(cudaMemcpyAsync(g->pos, h_state, 2 * sizeof(int), cudaMemcpyHostToDevice, st));
-    TB_TRY(launch_embed_fwd(c, P32(g, 0), g->ids, g->x, N, D, st));
+    const bool norm = g->L > 0 && gemm_norm_supported(c, D) && getenv("TB_NO_FUSED_NORM") == nullptr;
+    if (norm) TB_TRY(launch_embed_norm(c, P32(g, 0), g->ids, g->x, P32(g, pidx(0, PK_ATTN_NORM)), g->n, nullptr, nullptr, N, D, g->eps, st));
+    else TB_TRY(launch_embed_fwd(c, P32(g, 0), g->ids, g->x, N, D, st));
     for (int l = 0; l < g->L; ++l) {
-        TB_TRY(launch_rmsnorm_fwd(c, g->x, P32(g, pidx(l, PK_ATTN_NORM)), g->n, g->r, N, D, g->eps, st));
+        if (!norm) TB_TRY(launch_rmsnorm_fwd(c, g->x, P32(g, pidx(l, PK_ATTN_NORM)), g->n, g->r, N, D, g->eps, st));
         if (hd == 32 || hd == 64) {
             // rotation, head split and the cache append in the projection's epilogue
             GemmArgs s;
@@ -310,7 +317,7 @@ int tb_decoder_prefill(TbDecoder* g, const uint32_t* h_ids, int prompt_len) {
             TB_TRY(launch_rope_split(c, g->qkv, g->cos_t, g->sin_t, g->Q, g->Kc[l], g->Vc[l], S, T, H, hd, g->cap, st));
         }
         TB_TRY(launch_attention_fwd(c, g->Q, g->Kc[l], g->Vc[l], g->att, nullptr, S, H, T, hd, g->scale, st, g->cap));
-        TB_TRY(layer_tail(g, l, N));
+        TB_TRY(layer_tail(g, l, N, norm));
     }
     TB_TRY(launch_gather_last_rows(c, g->x, g->xl, S, T, D, st));
     // the first generated token sits at position prompt_len; *pos stays there for the first decode step

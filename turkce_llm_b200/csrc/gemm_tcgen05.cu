@@ -22,6 +22,7 @@
 #include "common.h"
 #include "ptx.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -35,6 +36,7 @@ constexpr int BK_TF32 = 32;         // float32 elements of one 128-byte swizzle 
 constexpr int ROW_BYTES = 128;
 constexpr int NUM_THREADS = 320;      // TMA warp, MMA warp, 8 epilogue warps
 constexpr int EPI_WARPS = 8;
+constexpr int NORM_MAX_CTAS = 4;      // CTAs that share a row block in the RMSNorm epilogue
 constexpr int STAGE_LD = 36;        // floats per staging row (32 + 4 pad: conflict-free float4 access)
 
 // PAIR: two CTAs of a cluster share a 256 x BN tile (cta_group::2): each loads its own 128 rows of A and
@@ -43,18 +45,20 @@ constexpr int STAGE_LD = 36;        // floats per staging row (32 + 4 pad: confl
 // the whole N, 40 KB per K slice feed 768 tensor-core cycles (53 B/clk against 64 for 256 x 256 with half of the
 // second tile empty).  The tensor core takes N <= 256, so a K step is three instructions of 128 columns; each CTA
 // loads the 64-column boxes at n0 + 128 j + 64 rank, which keeps accumulator column = output column.  One accumulator.
-template <int BN, bool PAIR = false> struct GemmCfg {
+// NORM: the CTAs of a cluster hold the columns of one row block between them and exchange the rows' sums of squares
+template <int BN, bool PAIR = false, bool NORM = false> struct GemmCfg {
     static constexpr int BN_LOCAL = PAIR ? BN / 2 : BN;   // columns of B this CTA loads
     static constexpr int A_BYTES = BM * ROW_BYTES;      // one K slice: 128-byte rows for either operand type
     static constexpr int B_BYTES = BN_LOCAL * ROW_BYTES;
     static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int STAGES = (PAIR && BN == 384) ? 3 : PAIR ? 4 : (BN == 192) ? 3 : (BN == 128) ? 4 : 5;
+    static constexpr int STAGES = (PAIR && BN == 384) ? 3 : PAIR ? 4 : (BN == 192) ? 3 : (BN == 128) ? (NORM ? 3 : 4) : 5;
     // per epilogue warp: 2 output buffers + 1 residual buffer of 32 rows x 128 B (TMA path);
     // the generic path uses the front of the same region (32 x 36 floats per warp)
     static constexpr int EPI_WARP_BYTES = 3 * 4096;
     static constexpr int STAGING_BYTES = EPI_WARPS * EPI_WARP_BYTES;
     static constexpr int BAR_BYTES = 512;
-    static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + STAGING_BYTES + BAR_BYTES;
+    static constexpr int NORM_BYTES = NORM ? (2 * 2 * NORM_MAX_CTAS * BM + 2 * BN) * 4 : 0;      // [2 tiles][CTA, half][row] partial sums | bias | weight
+    static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + STAGING_BYTES + BAR_BYTES + NORM_BYTES;
     static constexpr int TMEM_COLS = (2 * BN <= 128) ? 128 : (2 * BN <= 256) ? 256 : 512;   // power of two
     // accumulators in TMEM: two (the epilogue of tile i overlaps the main loop of tile i+1) unless one fills it
     static constexpr int NBUF = (2 * BN <= 512) ? 2 : 1;
@@ -89,6 +93,7 @@ struct GemmParams {
     int wide16;                 // bf16 tiles leave two 32-column chunks at a time: 32 rows x 128 bytes per store through the
                                 // 64-column map (tmR; with dsw: tmC), a last odd chunk through the 32-column map tmC
     int dsw;                    // SwiGLU backward: the product is dh; tmR = saved gate|up [M,2F] bf16, tmC = dgu [M,2F] bf16
+    const float* norm_w; float norm_eps, norm_inv_n; float* norm_rinv; bf16* norm16; float* norm32;    // EPI_NORM
     int tma_res;                // TMA path: add res_scale * (tile of tmR) -- the residual, or the old C for beta
     float res_scale;
     int bias_vec;               // bias pointer is 16-byte aligned
@@ -149,7 +154,7 @@ __device__ __forceinline__ TileCoord tile_of(const GemmParams& p, int t, int row
 // a 32-column chunk costs ~0.15 us more in instruction fetches); the other values fix the mode at compile time and
 // drop the rest -- measured on an [8192 x 384 x 1152] launch: last tile's epilogue 2.42 -> 1.89 us (float32 out),
 // 2.02 -> 1.54 us (bf16 out).
-enum { EPI_ANY = 0, EPI_F32, EPI_BF16, EPI_SWIGLU, EPI_CE1, EPI_ROPE, EPI_CE2, EPI_DSW };
+enum { EPI_ANY = 0, EPI_F32, EPI_BF16, EPI_SWIGLU, EPI_CE1, EPI_ROPE, EPI_CE2, EPI_DSW, EPI_NORM };
 
 template <int BN, bool TF32, bool PAIR = false, int EPI = EPI_ANY>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -157,7 +162,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmR,
                  const GemmParams p) {
     static_assert(!(PAIR && TF32), "CTA pairs are built for bf16 operands only");
-    using Cfg = GemmCfg<BN, PAIR>;
+    constexpr bool NORM = EPI == EPI_NORM;
+    using Cfg = GemmCfg<BN, PAIR, NORM>;
     constexpr int STAGES = Cfg::STAGES;
     constexpr int NBUF = Cfg::NBUF;
     constexpr int BNL = Cfg::BN_LOCAL;
@@ -185,6 +191,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint64_t* acc_full = bars + 2 * STAGES;       // [2]
     uint64_t* acc_empty = bars + 2 * STAGES + 2;  // [2]
     uint64_t* res_bar = bars + 2 * STAGES + 4;    // [EPI_WARPS]
+    uint64_t* norm_bar = bars + 40;               // [2]: the partial sums of a tile (by parity) have arrived
+    float* norm_part = reinterpret_cast<float*>(smem + STAGES * Cfg::STAGE_BYTES + Cfg::STAGING_BYTES + Cfg::BAR_BYTES);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4 + EPI_WARPS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -214,6 +222,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         for (int i = 0; i < STAGES; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], PAIR ? 2 * EPI_WARPS : EPI_WARPS); }
         for (int i = 0; i < EPI_WARPS; ++i) mbar_init(&res_bar[i], 1);
+        if (NORM) for (int i = 0; i < 2; ++i) mbar_init(&norm_bar[i], (uint32_t)(p.nt * EPI_WARPS));
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -225,7 +234,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const TileCoord c_first = tile_of<BN, BKE, TILE_M>(p, worker < total_tiles ? worker : 0, row_off);
     tc_fence_before();
     __syncthreads();
-    if (PAIR) cluster_sync();          // both CTAs' barriers exist before either signals the other's
+    if (PAIR || NORM) cluster_sync();  // the other CTAs' barriers exist before either signals the other's
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     if (threadIdx.x == 0) TS(1);
@@ -362,6 +371,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         uint8_t* rbuf = obuf + 8192;
         uint64_t* rbar = res_bar + ew;
         constexpr int NCH = BN / 64;             // chunks of 32 columns per warp and tile
+        float* norm_bias = norm_part + 2 * 2 * NORM_MAX_CTAS * BM;      // [BN] bias | [BN] norm weight of this CTA's columns
+        if constexpr (NORM) {
+            // (a CTA keeps its columns: the tiles of a cluster differ in their rows only)
+            for (int i = threadIdx.x - 64; i < BN; i += EPI_WARPS * 32) {
+                norm_bias[i] = p.bias ? __ldg(p.bias + c_first.n0 + i) : 0.0f;
+                norm_bias[BN + i] = __ldg(p.norm_w + c_first.n0 + i);
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+        }
         uint32_t cnt = 0;                        // chunks produced so far (selects the output buffer)
         uint32_t rphase = 0;
         int it = 0;
@@ -519,6 +537,138 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                         tma_store_commit();
                     }
                 }
+                ++it;
+                continue;
+            }
+            if constexpr (NORM) {
+                // x = product + bias + residual (the residual stream) and, as the next product's operand, its RMSNorm
+                // x w / rms: the rows' sums of squares are exchanged within the cluster, whose CTAs hold the columns
+                // of these rows between them.  x waits in the accumulator meanwhile.  (The norm as a kernel of its own
+                // is a launch, 4 bytes read and as many kept in flight per element: 8.5 us at 3885 rows of 384.)
+                const int col0 = c.n0 + half * (BN / 2);
+                // the residual tile comes in whole beside the main loop, into the buffers that x then leaves from
+                static_assert(!NORM || NCH <= 3, "three buffers per epilogue warp");
+                if (lane == 0) {
+                    tma_store_wait_read<0>();
+                    if (rows_in) {
+                        mbar_expect_tx(rbar, 4096 * NCH);
+                        for (int ch = 0; ch < NCH; ++ch) tma_load_4d(obuf + ch * 4096, &tmR, rbar, col0 + ch * 32, gm0, 0, 0);
+                    }
+                }
+                __syncwarp();
+                if (rows_in) {
+                    if (!mbar_wait(rbar, rphase, abort_flag)) { ok = false; break; }
+                    rphase ^= 1u;
+                }
+                if (!mbar_wait(&acc_full[buf], acc_phase, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + half * (BN / 2));
+                float ss = 0.0f;
+#pragma unroll 1
+                for (int ch = 0; ch < NCH; ++ch) {
+                    const int gn0 = col0 + ch * 32;
+                    uint32_t v[32];
+                    tmem_ld32(t_row + (uint32_t)(ch * 32), v);
+                    tmem_ld_wait();
+                    float o[32];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float4 bb = *reinterpret_cast<const float4*>(norm_bias + half * (BN / 2) + ch * 32 + 4 * j);
+                        o[4 * j] = __uint_as_float(v[4 * j]) + bb.x;         o[4 * j + 1] = __uint_as_float(v[4 * j + 1]) + bb.y;
+                        o[4 * j + 2] = __uint_as_float(v[4 * j + 2]) + bb.z; o[4 * j + 3] = __uint_as_float(v[4 * j + 3]) + bb.w;
+                    }
+                    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+                    uint8_t* orow = obuf + ch * 4096 + lane * 128;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        float4* r4p = reinterpret_cast<float4*>(orow + ((j ^ (lane & 7)) << 4));
+                        if (rows_in) {
+                            const float4 r4 = *r4p;
+                            o[4 * j] += r4.x; o[4 * j + 1] += r4.y; o[4 * j + 2] += r4.z; o[4 * j + 3] += r4.w;
+                        }
+                        s0 += o[4 * j] * o[4 * j];         s1 += o[4 * j + 1] * o[4 * j + 1];
+                        s2 += o[4 * j + 2] * o[4 * j + 2]; s3 += o[4 * j + 3] * o[4 * j + 3];
+                        *r4p = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+                    }
+                    ss += (s0 + s1) + (s2 + s3);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(o[j]);
+                    tmem_st32(t_row + (uint32_t)(ch * 32), v);
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (rows_in) tma_store_4d(&tmC, obuf + ch * 4096, gn0, gm0, 0, 0);
+                        tma_store_commit();
+                    }
+                }
+                tmem_st_wait();
+                // partial sums to every CTA of the cluster; a tile's slots are written again two tiles on, which no CTA
+                // reaches before all have read them
+                const int nc = p.nt, par = it & 1;
+                float* part = norm_part + par * (2 * NORM_MAX_CTAS * BM);
+                const int slot = ((c.n0 / BN) * 2 + half) * BM + q * 32 + lane;
+                for (int d = 0; d < nc; ++d) st_cluster_f32(mapa_cluster(smem_u32(part + slot), (uint32_t)d), ss);
+                __syncwarp();
+                if (lane < nc) mbar_arrive_cluster(mapa_cluster(smem_u32(&norm_bar[par]), (uint32_t)lane));
+                if (!mbar_wait_cluster(&norm_bar[par], (uint32_t)(it >> 1) & 1u, abort_flag)) { ok = false; break; }
+                ss = 0.0f;
+                for (int k = 0; k < 2 * nc; ++k) ss += part[k * BM + q * 32 + lane];
+                const float rinv = 1.0f / __fsqrt_rn(ss * p.norm_inv_n + p.norm_eps);
+                if (p.norm_rinv && c.n0 == 0 && half == 0 && gm0 + lane < p.M) p.norm_rinv[gm0 + lane] = rinv;
+                if (lane == 0) tma_store_wait_read<0>();
+                __syncwarp();
+                // bf16: the whole BN / 2 columns of 32 rows through shared memory (rows 16 bytes apart from a multiple of
+                // 128: no bank conflicts), then rows of 16-byte pieces by adjacent lanes; float32: 32 columns at a time
+                constexpr int PITCH16 = NCH * 64 + 16, PIECES16 = NCH * 4, PITCH32 = 128 + 16;
+#pragma unroll 1
+                for (int ch = 0; ch < NCH; ++ch) {
+                    const int gn0 = col0 + ch * 32;
+                    uint32_t v[32];
+                    tmem_ld32(t_row + (uint32_t)(ch * 32), v);
+                    tmem_ld_wait();
+                    float o[32];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float4 w4 = *reinterpret_cast<const float4*>(norm_bias + BN + half * (BN / 2) + ch * 32 + 4 * j);
+                        o[4 * j] = __uint_as_float(v[4 * j]) * rinv * w4.x;         o[4 * j + 1] = __uint_as_float(v[4 * j + 1]) * rinv * w4.y;
+                        o[4 * j + 2] = __uint_as_float(v[4 * j + 2]) * rinv * w4.z; o[4 * j + 3] = __uint_as_float(v[4 * j + 3]) * rinv * w4.w;
+                    }
+                    if (p.norm32) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            *reinterpret_cast<float4*>(obuf + lane * PITCH32 + j * 16) = make_float4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+                        __syncwarp();
+#pragma unroll 4
+                        for (int i = lane; i < 32 * 8; i += 32)
+                            if (gm0 + (i >> 3) < p.M)
+                                *reinterpret_cast<float4*>(p.norm32 + (long long)(gm0 + (i >> 3)) * p.N + gn0 + (i & 7) * 4) =
+                                    *reinterpret_cast<const float4*>(obuf + (i >> 3) * PITCH32 + (i & 7) * 16);
+                        __syncwarp();
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            __nv_bfloat162 h0 = __floats2bfloat162_rn(o[8 * j], o[8 * j + 1]), h1 = __floats2bfloat162_rn(o[8 * j + 2], o[8 * j + 3]);
+                            __nv_bfloat162 h2 = __floats2bfloat162_rn(o[8 * j + 4], o[8 * j + 5]), h3 = __floats2bfloat162_rn(o[8 * j + 6], o[8 * j + 7]);
+                            *reinterpret_cast<uint4*>(obuf + lane * PITCH16 + ch * 64 + j * 16) =
+                                make_uint4(*reinterpret_cast<uint32_t*>(&h0), *reinterpret_cast<uint32_t*>(&h1),
+                                           *reinterpret_cast<uint32_t*>(&h2), *reinterpret_cast<uint32_t*>(&h3));
+                        }
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[buf]);
+                if (p.norm16) {
+#pragma unroll 4
+                    for (int i = lane; i < 32 * PIECES16; i += 32) {
+                        const int r = i / PIECES16, j = i - r * PIECES16;
+                        if (gm0 + r < p.M)
+                            *reinterpret_cast<uint4*>(p.norm16 + (long long)(gm0 + r) * p.N + col0 + j * 8) =
+                                *reinterpret_cast<const uint4*>(obuf + r * PITCH16 + j * 16);
+                    }
+                }
+                fence_proxy_async();                  // (the buffers are written by the next tile's copies)
+                __syncwarp();
                 ++it;
                 continue;
             }
@@ -887,7 +1037,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     tc_fence_before();
     __syncthreads();
-    if (PAIR) cluster_sync();          // the other CTA has read its accumulators and needs none of this CTA's barriers any more
+    if (PAIR || NORM) cluster_sync();  // the other CTA has read its accumulators and needs none of this CTA's barriers any more
     if (warp == 1) {
         tc_fence_after();
         if (PAIR) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
@@ -1106,7 +1256,28 @@ static int make_map_out(CUtensorMap* map, const void* ptr, int elem_bytes, long 
 
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Width of the tiles whose row sums are exchanged: N / width CTAs of a cluster share a row block.  The widths divide N, so
+// that every CTA of a cluster has a whole tile; the choice weighs waves of clusters against tile width like pick_bn.  Clusters
+// of three or four do not fill the chip (SMs per processor cluster), so they are taken where one wave of them holds all row
+// blocks: D = 384, validation loss of 5 x 777 tokens 911 us on 3 x 128 against 943 on 2 x 192, step of 8 x 1024 4611 against 4429.
+static int pick_norm_bn(const DeviceCtx* ctx, int M, int N) {
+    static const double factor[3] = {1.30, 1.00, 0.95};
+    const long long mt = (M + BM - 1) / BM;
+    int best = 0;
+    double best_cost = 1e30;
+    for (int bn = 64; bn <= 192; bn += 64) {
+        const int nc = N / bn;
+        if (N % bn != 0 || nc > NORM_MAX_CTAS) continue;
+        const long long fit = std::max(1, (nc > 2 ? ctx->sm_count * 4 / 5 : ctx->sm_count) / nc);
+        const double cost = (double)((mt + fit - 1) / fit) * bn * factor[bn / 64 - 1];
+        if (cost < best_cost - 1e-9) { best_cost = cost; best = bn; }
+    }
+    return best;
+}
+bool gemm_norm_supported(const DeviceCtx* ctx, int N) { return pick_norm_bn(ctx, BM, N) > 0; }
+
 static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
+    if (a.norm_w) return pick_norm_bn(ctx, a.M, a.N);
     // time ~ waves x tile width x a factor for how often a tile re-reads its operands from L2
     // (flops per operand byte: 43 for 128x64, 64 for 128x128, 77 for 128x192, 128 for a CTA pair on 256x256).
     // 256 = a CTA pair on a 256 x 256 tile: per output element a CTA pulls 0.6x the operand bytes of a
@@ -1176,7 +1347,7 @@ template <int BN, bool TF32, bool PAIR = false, int EPI = EPI_ANY>
 static int launch_impl(DeviceCtx* ctx, const GemmArgs& a, const GemmParams& p, const CUtensorMap& tmA,
                        const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmR,
                        cudaStream_t stream) {
-    using Cfg = GemmCfg<BN, PAIR>;
+    using Cfg = GemmCfg<BN, PAIR, EPI == EPI_NORM>;
     static bool attr_set[64] = {false};
     if (!attr_set[ctx->device & 63]) {
         TB_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<BN, TF32, PAIR, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1193,8 +1364,9 @@ static int launch_impl(DeviceCtx* ctx, const GemmArgs& a, const GemmParams& p, c
         grid = (int)(total < sms ? total : sms);
     }
     if (grid < 1) grid = PAIR ? 2 : 1;
+    if (EPI == EPI_NORM) grid = p.nt * std::min(p.mt, std::max(1, sms / p.nt));       // whole clusters of p.nt CTAs
     TB_CUDA(launch_kernel_cluster((gemm_bf16_kernel<BN, TF32, PAIR, EPI>), dim3(grid), dim3(NUM_THREADS), Cfg::SMEM_BYTES,
-                                  stream, PAIR ? 2 : 1, tmA, tmB, tmC, tmR, p));
+                                  stream, EPI == EPI_NORM ? p.nt : PAIR ? 2 : 1, tmA, tmB, tmC, tmR, p));
     TB_CUDA(cudaGetLastError());
     ctx->launches++;
     prof_close(ctx, stream);
@@ -1260,6 +1432,13 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
                      aligned16(a.dsw_gu) && aligned16(a.dsw_dgu),
                  "SwiGLU-backward GEMM: needs a plain bf16 product with N = F (a multiple of 64), the saved gate|up "
                  "projection and the output, 16-byte aligned with ldgu %% 8 == 0");
+    }
+    if (a.norm_w) {
+        TB_CHECK(a.kind == GEMM_NN && a.batch == 1 && splits == 1 && bn > 0 && bn <= 192 && a.N % bn == 0 && a.N / bn <= NORM_MAX_CTAS &&
+                     a.alpha == 1.0f && a.beta == 0.0f && a.residual && a.ldr == a.N && a.C32 && a.ldc32 == a.N && !a.C16 && !a.swiglu_h &&
+                     a.ce_mode == 0 && !a.rope_qkv && !a.dsw_dgu && a.causal == CAUSAL_NONE && (a.norm16 != nullptr) != (a.norm32 != nullptr) &&
+                     aligned16(a.C32) && aligned16(a.residual) && aligned16(a.bias) && aligned16(a.norm_w) && aligned16(a.norm16) && aligned16(a.norm32),
+                 "GEMM with RMSNorm epilogue: needs a plain NN product with a residual, contiguous 16-byte aligned rows and a supported width (N=%d)", a.N);
     }
     const bool swiglu = a.swiglu_h != nullptr;
     if (swiglu) {
@@ -1327,6 +1506,8 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
     p.bias_vec = p.bias && aligned16(p.bias);
     p.rope_cos = a.rope_cos; p.rope_sin = a.rope_sin; p.rope_T = a.rope_T; p.rope_H = a.rope_H; p.rope_hd = a.rope_hd;
     p.rope_direct = 0;
+    p.norm_w = a.norm_w; p.norm_eps = a.norm_eps; p.norm_inv_n = 1.0f / (float)a.N; p.norm_rinv = a.norm_rinv;
+    p.norm16 = a.norm16; p.norm32 = a.norm32;
     if (a.ce_mode == 1) {
         p.tma_mode = 4;
     } else if (a.rope_qkv) {
@@ -1415,12 +1596,21 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
             char tag[128];
             static const char* kn[3] = {"NN", "NT", "TN"};
             snprintf(tag, sizeof(tag), "%s:%s:%dx%dx%d:b%d:s%d:c%d:bn%d%s", a.tf32 ? "gemm_tf32" : "gemm_bf16",
-                     kn[(int)a.kind], a.M, a.N, a.K, a.batch, splits, (int)a.causal, bn, swiglu ? ":swiglu" : a.rope_qkv ? ":rope" : a.ce_mode == 1 ? ":ce_stats" : a.ce_mode == 2 ? ":ce_grad" : "");
+                     kn[(int)a.kind], a.M, a.N, a.K, a.batch, splits, (int)a.causal, bn, swiglu ? ":swiglu" : a.rope_qkv ? ":rope" : a.ce_mode == 1 ? ":ce_stats" : a.ce_mode == 2 ? ":ce_grad" : a.norm_w ? ":norm" : "");
             // the second cross-entropy pass repeats pass 1's product: its flops are not algorithmic work
             prof_mark(ctx, prof_intern(tag), a.ce_mode == 2 ? 0.0 : 2.0 * macs, in_bytes + out_bytes, stream);
         }
     }
-    if (pair && bn == 384) {
+    if (a.norm_w) {
+        TB_CHECK(p.tma_mode == 1, "GEMM with RMSNorm epilogue: the output must be 16-byte addressable");
+#define TB_NORM_LAUNCH(W)                                                                                              \
+        (a.tf32 ? launch_impl<W, true, false, EPI_NORM>(ctx, a, p, tmA, tmB, tmC, tmR, stream)                           \
+                : launch_impl<W, false, false, EPI_NORM>(ctx, a, p, tmA, tmB, tmC, tmR, stream))
+        if (bn == 64)       TB_TRY(TB_NORM_LAUNCH(64));
+        else if (bn == 128) TB_TRY(TB_NORM_LAUNCH(128));
+        else                TB_TRY(TB_NORM_LAUNCH(192));
+#undef TB_NORM_LAUNCH
+    } else if (pair && bn == 384) {
         TB_TRY((launch_bf16<384, true>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
     } else if (pair) {
         TB_TRY((launch_bf16<256, true>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));

@@ -191,6 +191,56 @@ __global__ void rmsnorm_fwd_vec_kernel(const float* __restrict__ x, const float*
     }
 }
 
+// Embedding gather and the first RMSNorm in one pass: x = E[ids], out = bf16 (or out32 = float32) of x w / rms.  A warp per row;
+// summation order and rounding are those of rmsnorm_fwd_vec_kernel.
+template <int NV>
+__global__ void embed_norm_kernel(const float* __restrict__ E, const uint32_t* __restrict__ ids, float* __restrict__ x,
+                                  const float* __restrict__ w, bf16* __restrict__ out, float* __restrict__ out32,
+                                  float* __restrict__ rinv, int rows, int cols, float eps) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int lane = threadIdx.x & 31;
+    const int wpb = blockDim.x >> 5;
+    for (long long row = (long long)blockIdx.x * wpb + (threadIdx.x >> 5); row < rows; row += (long long)gridDim.x * wpb) {
+        const float* src = E + (long long)ids[row] * cols;      // ids are range-checked by whoever writes them
+        float4 xv[NV];
+        float ss = 0.0f;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const int j = 4 * (lane + 32 * k);
+            xv[k] = j < cols ? *reinterpret_cast<const float4*>(src + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+            ss += xv[k].x * xv[k].x + xv[k].y * xv[k].y + xv[k].z * xv[k].z + xv[k].w * xv[k].w;
+        }
+        ss = warp_sum(ss);
+        const float r = 1.0f / __fsqrt_rn(ss / (float)cols + eps);
+        if (lane == 0 && rinv) rinv[row] = r;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            const int j = 4 * (lane + 32 * k);
+            if (j < cols) {
+                const float4 wv = *reinterpret_cast<const float4*>(w + j);
+                const float4 y = make_float4(xv[k].x * r * wv.x, xv[k].y * r * wv.y, xv[k].z * r * wv.z, xv[k].w * r * wv.w);
+                *reinterpret_cast<float4*>(x + row * cols + j) = xv[k];
+                if (out) {
+                    __nv_bfloat162 lo = __floats2bfloat162_rn(y.x, y.y), hi = __floats2bfloat162_rn(y.z, y.w);
+                    *reinterpret_cast<uint2*>(out + row * cols + j) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+                }
+                if (out32) *reinterpret_cast<float4*>(out32 + row * cols + j) = y;
+            }
+        }
+    }
+}
+
+int launch_embed_norm(DeviceCtx* ctx, const float* E, const uint32_t* ids, float* x, const float* w, bf16* out, float* out32,
+                      float* rinv, int rows, int cols, float eps, cudaStream_t st) {
+    TB_CHECK(cols % 4 == 0 && cols <= 1024, "embed_norm: rows of up to 1024 columns, a multiple of 4 (got %d)", cols);
+    prof_mark(ctx, "embed_norm", 0.0, 0.0, st);
+    TB_CUDA(launch_kernel(cols <= 384 ? embed_norm_kernel<3> : embed_norm_kernel<8>, dim3(grid_for(rows, 8, ctx)), dim3(256), 0, st, E, ids,
+                          x, w, out, out32, rinv, rows, cols, eps));
+    TB_LAUNCHED(ctx);
+    return 0;
+}
+
 int launch_rmsnorm_fwd(DeviceCtx* ctx, const float* x, const float* w, bf16* out, float* rinv, int rows, int cols,
                        float eps, cudaStream_t st, float* out32) {
     prof_mark(ctx, "rmsnorm_fwd", 0.0, 0.0, st);

@@ -10,6 +10,9 @@
 namespace tb {
 
 int launch_embed_fwd(DeviceCtx*, const float* E, const uint32_t* ids, float* x, int rows, int D, cudaStream_t);
+// x = E[ids] and its RMSNorm (out bf16 or out32 float32; rinv may be NULL) in one pass; D a multiple of 4 up to 1024
+int launch_embed_norm(DeviceCtx*, const float* E, const uint32_t* ids, float* x, const float* w, bf16* out, float* out32,
+                      float* rinv, int rows, int D, float eps, cudaStream_t);
 // (out32, when given, receives the same values unrounded; out may then be NULL)
 int launch_rmsnorm_fwd(DeviceCtx*, const float* x, const float* w, bf16* out, float* rinv, int rows, int cols,
                        float eps, cudaStream_t, float* out32 = nullptr);

@@ -95,6 +95,7 @@ struct TbTrainer {
     bool fused_rope = true;        // head_dim 32 or 64: rotation and head split in the QKV GEMM epilogue
     bool fused_ce = true;          // cross-entropy inside the LM-head GEMM epilogues: no [N, V] logits
     bool fused_dswiglu = false;    // SwiGLU backward in the epilogue of the down-projection's input-gradient GEMM
+    bool fused_norm = false;       // RMSNorm in the epilogues of the out- and down-projections, the first one in the embedding gather
     bool fused_swiglu = true;      // d_ff % 64 == 0: silu(gate) * up formed in the gate|up GEMM's epilogue
     // TF32 mode (TB_PREC_TF32): every linear-layer GEMM (forward, dX, dW, LM head) reads float32 operands as tf32
     // (kind::tf32); weights are the float32 masters, activations and gradients that feed a GEMM are kept in float32.
@@ -143,13 +144,19 @@ inline bool pair_on(const TbTrainer* g) { return g->pair_ctas > 0 && !g->ctx->pr
 
 // C[M,N] = A[M,K] @ W[K,N] + bias (+ residual): the reference's bf16_gemm_bias (gpu_train.c:103-107).
 // Operands are bf16, or float32 read as tf32 in the TF32 mode.
+// norm_w (optional): the result's RMSNorm as well, in the product's epilogue.
 int linear_fwd(TbTrainer* g, const void* A, const void* W, const float* bias, const float* residual, float* C32,
-               bf16* C16, int M, int N, int K) {
+               bf16* C16, int M, int N, int K, const float* norm_w = nullptr, bf16* n16 = nullptr, float* n32 = nullptr,
+               float* rinv = nullptr) {
     GemmArgs a;
     a.kind = GEMM_NN; a.A = A; a.B = W; a.M = M; a.N = N; a.K = K; a.lda = K; a.ldb = N;
     a.C32 = C32; a.ldc32 = N; a.C16 = C16; a.ldc16 = N;
     a.bias = bias; a.residual = residual; a.ldr = N;
     a.splits = 1; a.tf32 = g->tf32;
+    if (norm_w) {
+        a.norm_w = norm_w; a.norm_eps = g->eps; a.norm_rinv = rinv;
+        if (g->tf32) a.norm32 = n32; else a.norm16 = n16;
+    }
     return gemm(g, a);
 }
 
@@ -203,12 +210,26 @@ int forward(TbTrainer* g, bool want_grad) {
     const long long Tp = g->Tp, sTT = (long long)T * Tp, sThd = (long long)T * hd;
 
     float* x0 = g->L > 0 ? g->layers[0].x_in : g->x_final;
-    TB_TRY(launch_embed_fwd(c, P32(g, 0), g->ids, x0, N, D, st));
+    const long long p_final = pidx(g->L, 0);
+    // the normalised rows that follow layer l - 1: the input of layer l, or (behind the last layer) of the head
+    auto norm_of = [&](int l, const float** w, bf16** n16, float** n32, float** r) {
+        const bool head = l == g->L;
+        *w = P32(g, head ? p_final : pidx(l, PK_ATTN_NORM));
+        *n16 = head ? g->nf : g->layers[l].n1; *n32 = head ? g->nf32 : g->layers[l].n1_32; *r = head ? g->rf : g->layers[l].r1;
+    };
+    const float* nw; bf16* n16; float *n32, *nr;
+    if (g->fused_norm) {
+        norm_of(0, &nw, &n16, &n32, &nr);
+        TB_TRY(launch_embed_norm(c, P32(g, 0), g->ids, x0, nw, g->tf32 ? nullptr : n16, n32, nr, N, D, g->eps, st));
+    } else {
+        TB_TRY(launch_embed_fwd(c, P32(g, 0), g->ids, x0, N, D, st));
+    }
 
     for (int l = 0; l < g->L; ++l) {
         LayerActs& a = g->layers[l];
         float* x_out = (l + 1 < g->L) ? g->layers[l + 1].x_in : g->x_final;
-        TB_TRY(launch_rmsnorm_fwd(c, a.x_in, P32(g, pidx(l, PK_ATTN_NORM)), a.n1, a.r1, N, D, g->eps, st, a.n1_32));
+        if (!g->fused_norm)
+            TB_TRY(launch_rmsnorm_fwd(c, a.x_in, P32(g, pidx(l, PK_ATTN_NORM)), a.n1, a.r1, N, D, g->eps, st, a.n1_32));
         if (g->fused_rope) {
             // QKV projection; q and k rotated and all three stored per head as bf16 by the GEMM epilogue
             GemmArgs s;
@@ -245,8 +266,10 @@ int forward(TbTrainer* g, bool want_grad) {
         }
         if (g->tf32) TB_TRY(launch_widen_bf16(c, a.att, g->att32, (long long)N * D, st));
         TB_TRY(linear_fwd(g, g->tf32 ? (const void*)g->att32 : (const void*)a.att, WOP(g, pidx(l, PK_WO)),
-                          P32(g, pidx(l, PK_BO)), a.x_in, a.x2, nullptr, N, D, D));
-        TB_TRY(launch_rmsnorm_fwd(c, a.x2, P32(g, pidx(l, PK_FFN_NORM)), a.n2, a.r2, N, D, g->eps, st, a.n2_32));
+                          P32(g, pidx(l, PK_BO)), a.x_in, a.x2, nullptr, N, D, D,
+                          g->fused_norm ? P32(g, pidx(l, PK_FFN_NORM)) : nullptr, a.n2, a.n2_32, a.r2));
+        if (!g->fused_norm)
+            TB_TRY(launch_rmsnorm_fwd(c, a.x2, P32(g, pidx(l, PK_FFN_NORM)), a.n2, a.r2, N, D, g->eps, st, a.n2_32));
         if (g->fused_swiglu) {
             // gate|up projection with h = silu(gate) * up formed in the GEMM epilogue; gate|up kept in bf16
             GemmArgs s;
@@ -259,12 +282,13 @@ int forward(TbTrainer* g, bool want_grad) {
                               P32(g, pidx(l, PK_BGU)), nullptr, a.gu, nullptr, N, 2 * F, D));
             TB_TRY(launch_swiglu_fwd(c, a.gu, g->tf32 ? nullptr : a.h, N, F, st, a.h32));
         }
+        norm_of(l + 1, &nw, &n16, &n32, &nr);
         TB_TRY(linear_fwd(g, g->tf32 ? (const void*)a.h32 : (const void*)a.h, WOP(g, pidx(l, PK_WDOWN)),
-                          P32(g, pidx(l, PK_BDOWN)), a.x2, x_out, nullptr, N, D, F));
+                          P32(g, pidx(l, PK_BDOWN)), a.x2, x_out, nullptr, N, D, F, g->fused_norm ? nw : nullptr, n16, n32, nr));
     }
 
-    const long long p_final = pidx(g->L, 0);
-    TB_TRY(launch_rmsnorm_fwd(c, g->x_final, P32(g, p_final), g->nf, g->rf, N, D, g->eps, st, g->nf32));
+    if (!g->fused_norm)
+        TB_TRY(launch_rmsnorm_fwd(c, g->x_final, P32(g, p_final), g->nf, g->rf, N, D, g->eps, st, g->nf32));
     if (g->fused_ce) {
         // logits = nf @ E^T (tied head, gpu_train.c:378) never reach HBM: pass 1 keeps per-tile softmax
         // statistics and the target logit, their combination is the loss; pass 2 forms the product again
@@ -600,6 +624,8 @@ int tb_trainer_create_prec(TbTrainer** out, int V, int D, int H, int L, int F, i
     g->fused_swiglu = !g->tf32 && F % 64 == 0 && getenv("TB_NO_FUSED_SWIGLU") == nullptr;
     g->fused_dswiglu = g->fused_swiglu && getenv("TB_NO_FUSED_DSWIGLU") == nullptr;
     g->fused_rope = !g->tf32 && (D / H == 32 || D / H == 64) && getenv("TB_NO_FUSED_ROPE") == nullptr;
+    // (parameters start at multiples of 8 scalars in the flat buffers: d_model, d_ff and head_dim are multiples of 8)
+    g->fused_norm = gemm_norm_supported(g->ctx, D) && getenv("TB_NO_FUSED_NORM") == nullptr;
     g->V = V; g->D = D; g->H = H; g->L = L; g->F = F; g->T = T; g->B = B; g->N = B * T; g->hd = D / H;
     g->Vp = round_up(V, 8);
     g->Tp = round_up(T, 8);
