@@ -18,6 +18,8 @@
 #include "common.h"
 #include "ptx.cuh"
 
+#include <algorithm>
+
 #include <cstdlib>
 
 namespace tb {
@@ -73,6 +75,7 @@ __device__ __forceinline__ void store_chunk_bf16(uint8_t* tiles, int r, int c, c
 struct AttFwdParams {
     int T, H, hd, D;
     int nq;                 // query blocks per head
+    int BH, items;          // heads of all sequences; work items = BH * nq
     float scale_log2;       // 1/sqrt(hd) * log2(e)
     bf16* att;              // [B*T, D]
     float* lse;             // [B*H, T]
@@ -89,7 +92,17 @@ struct AttFwdParams {
 // more than 2^8 (kLazyMax), and only then is the accumulator read, rescaled and written back.  The probabilities then reach
 // 2^8 instead of 1, with the same relative error in bf16, and the row sum is kept against the same maximum.  Reading every
 // P V back and folding it in with a factor of its own, as before, was a third of a softmax warp's instructions.
+// A CTA works through several items (query block, head): a CTA per item spent 5 us outside its loop -- set-up, the first loads,
+// the last products, the store -- while here the next item's query and key tiles and its first scores are under way
+// when the softmax warps finish the item before.  Measured at 16 x 6 heads x 1024: 37.5 us with a CTA per item.
 constexpr float kLazyMax = 8.0f;        // in units of log2
+
+// Item k of worker w of n: heavy items (late query blocks) first, every second round in reverse order, so that the workers'
+// sums of half blocks differ by little; -1: no more.  All heads of a query block are adjacent.
+__device__ __forceinline__ int att_item(int k, int w, int n, int items) {
+    const int i = k * n + ((k & 1) ? n - 1 - w : w);
+    return i < items ? i : -1;
+}
 
 __global__ void __launch_bounds__(192, 2)
 attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -115,16 +128,15 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     uint64_t* p_full = bars + 11;     // 2: probability buffer b written
     uint64_t* o_full = bars + 13;     // 2: P V of a half block of parity b has been added
     uint64_t* out_full = bars + 18;   // 4 arrivals: the output tile is staged in shared memory
+    uint64_t* q_empty = bars + 15;    // 1: the item's last scores have been formed
+    uint64_t* out_done = bars + 16;   // 1: the store has read the staged output
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // blocks are handed out x fastest: all heads' heaviest (last) query block first, the lightest last,
-    // so the long CTAs start together and the short ones fill the tail
-    const int qb = p.nq - 1 - (int)blockIdx.y;
-    const int bh = blockIdx.x;
-    const int q0 = qb * ATT_BM;
-    const int nkv = qb + 1;                           // key blocks 0..qb
+    const int worker = (int)blockIdx.x, workers = (int)gridDim.x;
+    auto q_block = [&](int item) { return p.nq - 1 - item / p.BH; };           // items: last (heaviest) query block first
+    auto half_blocks = [&](int item) { return 2 * (q_block(item) + 1); };       // key blocks 0 .. its own, two halves each
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
@@ -133,7 +145,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 4); mbar_init(&p_full[i], 4);
             mbar_init(&o_full[i], 1);
         }
-        mbar_init(out_full, 4);
+        mbar_init(out_full, 4); mbar_init(q_empty, 1); mbar_init(out_done, 1);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -144,21 +156,27 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();                 // everything above is independent of earlier kernels' results
     // TMEM: two score buffers of 64 key columns, the output accumulator of 64 head-dim columns
+    // Half blocks are counted through all items of the CTA (g): an item has an even number of them, so buffer b = g & 1 is also
+    // the half of the key block, and key block g >> 1 uses stage (g >> 1) & 1.
     const uint32_t tS = tmem_base, tO = tmem_base + 128;
-    const int nsub = 2 * nkv;                         // 64-key half blocks
 
     if (warp == 0) {
         if (elect_one()) {
             bool ok = true;
-            mbar_expect_tx(q_full, TILE_BYTES);
-            tma_load_3d(sQ, &tmQ, q_full, 0, q0, bh);
-            for (int j = 0; j < nkv && ok; ++j) {
-                const int s = j & 1;
-                if (!mbar_wait(&kv_empty[s], (uint32_t)((j >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
-                mbar_expect_tx(&k_full[s], TILE_BYTES);
-                tma_load_3d(sK + s * TILE_BYTES, &tmK, &k_full[s], 0, j * ATT_BN, bh);
-                mbar_expect_tx(&v_full[s], TILE_BYTES);
-                tma_load_3d(sV + s * TILE_BYTES, &tmV, &v_full[s], 0, j * ATT_BN, bh);
+            int jg = 0;
+            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
+                const int qb = q_block(item), bh = item % p.BH;
+                if (!mbar_wait(q_empty, (uint32_t)(k & 1) ^ 1u, abort_flag)) { ok = false; break; }
+                mbar_expect_tx(q_full, TILE_BYTES);
+                tma_load_3d(sQ, &tmQ, q_full, 0, qb * ATT_BM, bh);
+                for (int j = 0; j <= qb; ++j, ++jg) {
+                    const int s = jg & 1;
+                    if (!mbar_wait(&kv_empty[s], (uint32_t)((jg >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
+                    mbar_expect_tx(&k_full[s], TILE_BYTES);
+                    tma_load_3d(sK + s * TILE_BYTES, &tmK, &k_full[s], 0, j * ATT_BN, bh);
+                    mbar_expect_tx(&v_full[s], TILE_BYTES);
+                    tma_load_3d(sV + s * TILE_BYTES, &tmV, &v_full[s], 0, j * ATT_BN, bh);
+                }
             }
             pdl_launch_dependents_now();     // all loads issued: the next kernel may start its prologue
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 11); }
@@ -172,49 +190,64 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             const uint32_t idesc_o = umma_idesc(1u, 0u, 1u, ATT_BM, ATT_HD);     // P V: V is MN-major
             const uint64_t dQ = kmajor_tile(smem_u32(sQ)), dK0 = kmajor_tile(smem_u32(sK)), dP0 = kmajor_tile(smem_u32(sP));
             const uint64_t dV0 = mnmajor_tile(smem_u32(sV), TILE_BYTES);
-            bool ok = mbar_wait(q_full, 0, abort_flag);
-            auto issue_scores = [&](int i) -> bool {
-                const int j = i >> 1, st = j & 1, b = i & 1;
-                if (b == 0 && !mbar_wait(&k_full[st], (uint32_t)((j >> 1) & 1), abort_flag)) return false;
-                if (!mbar_wait(&s_free[b], (uint32_t)((i >> 1) & 1) ^ 1u, abort_flag)) return false;
+            bool ok = true;
+            // the scores run up to two half blocks ahead of P V, across the end of an item
+            int gs = 0, ks = 0, is = 0, ns = half_blocks(att_item(0, worker, workers, p.items));     // ns = 0: no item left
+            auto issue_scores = [&]() -> bool {
+                const int st = (gs >> 1) & 1, b = gs & 1;
+                const uint32_t par = (uint32_t)((gs >> 1) & 1);
+                if (is == 0 && !mbar_wait(q_full, (uint32_t)(ks & 1), abort_flag)) return false;
+                if (b == 0 && !mbar_wait(&k_full[st], (uint32_t)((gs >> 2) & 1), abort_flag)) return false;
+                if (!mbar_wait(&s_free[b], par ^ 1u, abort_flag)) return false;
                 tc_fence_after();
                 const uint64_t dK = dK0 + (uint64_t)st * TILESTEP + (uint64_t)b * (TILESTEP / 2);   // keys 64b.. of the tile
 #pragma unroll
                 for (int k = 0; k < ATT_HD / 16; ++k)
                     umma_bf16(tS + (uint32_t)(b * 64), dQ + k * KSTEP, dK + k * KSTEP, idesc_s, k > 0 ? 1u : 0u);
                 umma_commit(&s_full[b]);
+                ++gs;
+                if (++is == ns) {
+                    umma_commit(q_empty);
+                    const int item = att_item(++ks, worker, workers, p.items);
+                    is = 0; ns = item >= 0 ? half_blocks(item) : 0;
+                }
                 return true;
             };
-            if (ok) ok = issue_scores(0);
-            if (ok && nsub > 1) ok = issue_scores(1);
-            for (int i = 0; i < nsub && ok; ++i) {
-                const int j = i >> 1, st = j & 1, b = i & 1;
-                const uint32_t par = (uint32_t)((i >> 1) & 1);
-                if (!mbar_wait(&p_full[b], par, abort_flag)) { ok = false; break; }
-                if (b == 0 && !mbar_wait(&v_full[st], (uint32_t)((j >> 1) & 1), abort_flag)) { ok = false; break; }
-                tc_fence_after();
-                const uint64_t dP = dP0 + (uint64_t)b * TILESTEP;
-                const uint64_t dV = dV0 + (uint64_t)st * TILESTEP + (uint64_t)b * (4 * MNSTEP);
+            for (int i = 0; i < 2 && ok && ns > 0; ++i) ok = issue_scores();
+            int g = 0;
+            for (int kp = 0, item; ok && (item = att_item(kp, worker, workers, p.items)) >= 0; ++kp) {
+                const int nsub = half_blocks(item);
+                for (int i = 0; i < nsub; ++i, ++g) {
+                    const int st = (g >> 1) & 1, b = g & 1;
+                    if (!mbar_wait(&p_full[b], (uint32_t)((g >> 1) & 1), abort_flag)) { ok = false; break; }
+                    if (b == 0 && !mbar_wait(&v_full[st], (uint32_t)((g >> 2) & 1), abort_flag)) { ok = false; break; }
+                    tc_fence_after();
+                    const uint64_t dP = dP0 + (uint64_t)b * TILESTEP;
+                    const uint64_t dV = dV0 + (uint64_t)st * TILESTEP + (uint64_t)b * (4 * MNSTEP);
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    umma_bf16(tO, dP + k * KSTEP, dV + k * MNSTEP, idesc_o, (i | k) != 0 ? 1u : 0u);
-                umma_commit(&o_full[b]);
-                if (b == 1) umma_commit(&kv_empty[st]);          // both halves of the K/V tile are consumed
-                if (i + 2 < nsub) ok = issue_scores(i + 2);
+                    for (int k = 0; k < 4; ++k)
+                        umma_bf16(tO, dP + k * KSTEP, dV + k * MNSTEP, idesc_o, (i | k) != 0 ? 1u : 0u);
+                    umma_commit(&o_full[b]);
+                    if (b == 1) umma_commit(&kv_empty[st]);          // both halves of the K/V tile are consumed
+                    if (ns > 0 && !issue_scores()) { ok = false; break; }
+                }
             }
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 12); }
         }
     } else {
         const int q = warp & 3;
         const int r = q * 32 + lane;                 // row of the tile = TMEM lane
-        const int qi = q0 + r;                       // query position
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
-        float m = -INFINITY, l = 0.0f;               // the maximum the exponentials are taken against, and their sum
         bool ok = true;
+        int g = 0;
+        for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
+        const int qb = q_block(item), bh = item % p.BH, q0 = qb * ATT_BM, nsub = half_blocks(item);
+        const int qi = q0 + r;                       // query position
+        float m = -INFINITY, l = 0.0f;               // the maximum the exponentials are taken against, and their sum
         uint32_t va[32], vb[32];                     // one half block's scores (or the accumulator) of this row
-        for (int i = 0; i < nsub && ok; ++i) {
+        for (int i = 0; i < nsub && ok; ++i, ++g) {
             const int b = i & 1;
-            if (!mbar_wait(&s_full[b], (uint32_t)((i >> 1) & 1), abort_flag)) { ok = false; break; }
+            if (!mbar_wait(&s_full[b], (uint32_t)((g >> 1) & 1), abort_flag)) { ok = false; break; }
             tc_fence_after();
             const bool diag = ((i >> 1) == qb);
             const int k0 = (i >> 1) * ATT_BN + b * 64;
@@ -271,7 +304,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             l += (la.x + la.y) + (lb.x + lb.y);
             if (move && i > 0) {
                 // P V of the half blocks so far, against the old maximum: rescaled once the last of them has been added
-                if (!mbar_wait(&o_full[b ^ 1], (uint32_t)(((i - 1) >> 1) & 1), abort_flag)) { ok = false; break; }
+                if (!mbar_wait(&o_full[b ^ 1], (uint32_t)(((g - 1) >> 1) & 1), abort_flag)) { ok = false; break; }
                 tc_fence_after();
 #pragma unroll
                 for (int h2 = 0; h2 < 2; ++h2) {
@@ -284,7 +317,11 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 tmem_st_wait();
             }
             // the probabilities of two half blocks ago have been multiplied
-            if (i >= 2 && !mbar_wait(&o_full[b], (uint32_t)(((i >> 1) - 1) & 1), abort_flag)) { ok = false; break; }
+            if (i >= 2 && !mbar_wait(&o_full[b], (uint32_t)(((g >> 1) - 1) & 1), abort_flag)) { ok = false; break; }
+            if (i == 1 && k > 0) {                            // the previous item's output was staged in the second buffer
+                if (q == 0 && lane == 0) { tma_store_wait_read<0>(); mbar_arrive(out_done); }
+                if (!mbar_wait(out_done, (uint32_t)(k & 1) ^ 1u, abort_flag)) { ok = false; break; }
+            }
             store_chunk_bf16(sP, r, 2 * b, pa);
             store_chunk_bf16(sP, r, 2 * b + 1, pb);
             tc_fence_before();
@@ -292,7 +329,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             __syncwarp();
             if (lane == 0) { mbar_arrive(&s_free[b]); mbar_arrive(&p_full[b]); }
         }
-        if (ok) ok = mbar_wait(&o_full[(nsub - 1) & 1], (uint32_t)(((nsub - 1) >> 1) & 1), abort_flag);
+        if (ok) ok = mbar_wait(&o_full[1], (uint32_t)(((g - 1) >> 1) & 1), abort_flag);      // (g: behind the item)
         if (ok) {
             tc_fence_after();
             tmem_ld32(tO + lane_base, va);
@@ -300,12 +337,12 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             tmem_ld_wait();
         }
         if (ok) {
-            // O / l as bf16 into the Q tile (every product has completed), one TMA store for the 128 rows: a thread per
-            // row storing to global memory directly touches 32 different rows per instruction
+            // O / l as bf16 into the second probability buffer (every product has completed), one TMA store for the 128
+            // rows: a thread per row storing to global memory directly touches 32 different rows per instruction
             const float inv = 1.0f / l;
             const int b = bh / p.H, h = bh % p.H;
             if (qi < p.T) {
-                uint8_t* row = sQ + r * 128;
+                uint8_t* row = sP + TILE_BYTES + r * 128;
 #pragma unroll
                 for (int d = 0; d < ATT_HD; d += 8) {
                     if (d >= p.hd) break;
@@ -325,13 +362,15 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             __syncwarp();
             if (lane == 0) mbar_arrive(out_full);
             if (q == 0 && lane == 0) {
-                if (mbar_wait(out_full, 0, abort_flag)) {
-                    tma_store_4d(&tmO, sQ, 0, q0, h, b);          // rows past T are clipped
+                if (mbar_wait(out_full, (uint32_t)(k & 1), abort_flag)) {
+                    tma_store_4d(&tmO, sP + TILE_BYTES, 0, q0, h, b);          // rows past T are clipped
                     tma_store_commit();
-                    tma_store_wait_read<0>();
                 } else ok = false;
             }
+            ok = __all_sync(0xffffffffu, ok);
         }
+        }
+        if (q == 0 && lane == 0) tma_store_wait_read<0>();
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.err, 13); }
     }
 
@@ -968,10 +1007,11 @@ int launch_attention_fwd(DeviceCtx* ctx, const bf16* Q, const bf16* K, const bf1
         TB_CUDA(cudaFuncSetAttribute(attention_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_FWD_SMEM));
         attr_set[ctx->device & 63] = true;
     }
-    dim3 grid(BH, p.nq);
+    p.BH = BH; p.items = BH * p.nq;
+    const int grid = std::min(p.items, 2 * ctx->sm_count);           // two CTAs per SM
     // algorithmic work: the lower triangle of two products of 2*T*T*hd flops each
     prof_mark(ctx, "attention_fwd", 2.0 * (double)BH * T * (double)T * hd, (double)BH * T * hd * 2.0 * 4.0, stream);
-    TB_CUDA(launch_kernel(attention_fwd_kernel, dim3(grid), dim3(192), ATT_FWD_SMEM, stream, tmQ, tmK, tmV, tmO, p));
+    TB_CUDA(launch_kernel(attention_fwd_kernel, dim3((unsigned)grid), dim3(192), ATT_FWD_SMEM, stream, tmQ, tmK, tmV, tmO, p));
     TB_CUDA(cudaGetLastError());
     ctx->launches++;
     prof_close(ctx, stream);
