@@ -389,24 +389,24 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // query blocks below the diagonal (dK, dV), the other owns a query block and walks its key blocks
 // (dQ); both recompute S and dP on the tensor cores.
 
+// delta of row (b, h, t): eight lanes per row, 16 bytes each, so that a warp reads four adjacent heads' pieces of a token (a
+// thread per row read 32 different 128-byte rows per instruction: 13 us at 16 x 6 x 1024, this 8).
 __global__ void attention_delta_kernel(const bf16* __restrict__ att, const bf16* __restrict__ datt,
                                        float* __restrict__ delta, int B, int T, int H, int hd) {
     pdl_wait();
     pdl_launch_dependents();
     const long long total = (long long)B * T * H;
-    const int D = H * hd;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const int h = (int)(i % H);
-        const long long n = i / H;
-        const int t = (int)(n % T);
-        const long long b = n / T;
-        const bf16* o = att + n * D + h * hd;
-        const bf16* d = datt + n * D + h * hd;
+    const int D = H * hd, piece = threadIdx.x & 7;
+    const bool mine = piece * 8 < hd;
+    // (whole groups of eight lanes go round the loop together, and a warp's groups leave it together: the bound is rounded up)
+    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3; i < ((total + 3) & ~3LL); i += (gridDim.x * blockDim.x) >> 3) {
+        const long long n = total < (1LL << 31) ? (long long)((unsigned)i / (unsigned)H) : i / H;
+        const int h = (int)(i - n * H);
         float s = 0.0f;
-        for (int k = 0; k < hd; k += 8) {
-            const uint4 ov = *reinterpret_cast<const uint4*>(o + k);
-            const uint4 dv = *reinterpret_cast<const uint4*>(d + k);
+        if (mine && i < total) {
+            const long long o = n * D + h * hd + piece * 8;
+            const uint4 ov = *reinterpret_cast<const uint4*>(att + o);
+            const uint4 dv = *reinterpret_cast<const uint4*>(datt + o);
             const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&ov);
             const __nv_bfloat162* d2 = reinterpret_cast<const __nv_bfloat162*>(&dv);
 #pragma unroll
@@ -416,7 +416,12 @@ __global__ void attention_delta_kernel(const bf16* __restrict__ att, const bf16*
                 s += a.y * c.y;
             }
         }
-        delta[(b * H + h) * T + t] = s;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (piece == 0 && i < total) {
+            const long long b = total < (1LL << 31) ? (long long)((unsigned)n / (unsigned)T) : n / T;
+            delta[(b * H + h) * T + (n - b * T)] = s;
+        }
     }
 }
 
@@ -517,10 +522,11 @@ __device__ __forceinline__ void p_and_ds(const uint32_t (&sv)[32], const uint32_
     }
 }
 
-constexpr int ATT_BWD_STAGES = 2;       // stages of the (Q, dO) pair in the dK/dV kernel
-constexpr int ATT_BWD_THREADS = 352;     // TMA warp, score-MMA warp, 8 compute warps, gradient-MMA warp
+constexpr int ATT_BWD_STAGES = 3;       // stages of the (Q, dO) pair in the dK/dV kernel
+constexpr int ATT_BWD_THREADS = 608;     // TMA warp, score-MMA warp, 16 compute warps, gradient-MMA warp
+constexpr int ATT_BWD_CW = 16;          // compute warps
 // (two issuing threads on different schedulers: one thread cannot issue a block's 24 UMMAs as fast as the
-//  tensor pipe retires them while eight compute warps compete for the same issue slots)
+//  tensor pipe retires them while the compute warps compete for the same issue slots)
 
 // dK, dV of one key block: walks the query blocks qb = kb .. nq-1.
 __global__ void __launch_bounds__(ATT_BWD_THREADS, 1)
@@ -542,11 +548,11 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     uint64_t* qdo_full = bars + 1;     // ATT_BWD_STAGES
     uint64_t* qdo_empty = bars + 5;    // ATT_BWD_STAGES
     uint64_t* sdp_full = bars + 9;
-    uint64_t* sdp_free = bars + 10;    // 8 arrivals
-    uint64_t* pds_full = bars + 11;    // 8 arrivals
+    uint64_t* sdp_free = bars + 10;    // one arrival per compute warp
+    uint64_t* pds_full = bars + 11;    // one arrival per compute warp
     uint64_t* pds_free = bars + 12;
     uint64_t* acc_full = bars + 13;
-    uint64_t* out_full = bars + 14;    // 8 arrivals: the output tile is staged in shared memory
+    uint64_t* out_full = bars + 14;    // one arrival per compute warp: the output tile is staged in shared memory
     uint64_t* ds_stored = bars + 16;   // 2: the bulk store of dS buffer b has read it
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -561,8 +567,8 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     if (threadIdx.x == 0) {
         mbar_init(kv_full, 1);
         for (int i = 0; i < ATT_BWD_STAGES; ++i) { mbar_init(&qdo_full[i], 1); mbar_init(&qdo_empty[i], 1); }
-        mbar_init(sdp_full, 1); mbar_init(sdp_free, 8); mbar_init(pds_full, 8); mbar_init(pds_free, 1);
-        mbar_init(acc_full, 1); mbar_init(out_full, 8);
+        mbar_init(sdp_full, 1); mbar_init(sdp_free, ATT_BWD_CW); mbar_init(pds_full, ATT_BWD_CW); mbar_init(pds_free, 1);
+        mbar_init(acc_full, 1); mbar_init(out_full, ATT_BWD_CW);
         mbar_init(&ds_stored[0], 1); mbar_init(&ds_stored[1], 1);
         *abort_flag = 0;
         fence_mbar_init();
@@ -617,7 +623,7 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
             for (int it = 0; it + 1 < niter && ok; ++it) ok = issue_sdp(it + 1);
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 22); }
         }
-    } else if (warp == 10) {
+    } else if (warp == 2 + ATT_BWD_CW) {
         // second issuer: dV += P^T dO and dK += dS^T Q once the compute warps have written P and dS
         if (elect_one()) {
             const uint32_t id_t = umma_idesc(1u, 1u, 1u, 128, 64);       // both operands MN-major
@@ -644,9 +650,10 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
                 umma_commit(&qdo_empty[s]);
                 if (it == niter - 1) umma_commit(acc_full);      // the epilogue need not wait for the store below
                 // the dS block leaves for the dQ kernel as it lies in shared memory; its buffer is written again two
-                // steps from now, and this thread has nothing else to do until the next block is ready.  Not before the
-                // products above have completed: a 32 KB read of shared memory beside them delays pds_free, which the
-                // compute warps need ~900 cycles after they sign pds_full
+                // steps from now.  Not before the products above have completed: a 32 KB read of shared memory beside them
+                // delays pds_free, which the compute warps need ~900 cycles after they sign pds_full.  That it has been read
+                // (1,400 clocks) is looked at a step later.
+                if (it > 0) { tma_store_wait_read<0>(); mbar_arrive(&ds_stored[(it - 1) & 1]); }
                 if (!mbar_wait(pds_free, (uint32_t)(it & 1), abort_flag)) { ok = false; break; }
                 {
                     const int qb = kb + it;
@@ -654,15 +661,14 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
                                    ((long long)bh * nblk + (long long)qb * (qb + 1) / 2 + kb) * DS_BLOCK_BYTES;
                     bulk_store(dst, sdS + (it & 1) * DS_BLOCK_BYTES, DS_BLOCK_BYTES);
                     tma_store_commit();
-                    tma_store_wait_read<0>();
-                    mbar_arrive(&ds_stored[it & 1]);
                 }
             }
+            tma_store_wait_read<0>();
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 24); }
         }
     } else {
         const int q = warp & 3;
-        const int half = (warp - 2) >> 2;             // which 64 key columns this warp handles
+        const int cq = (warp - 2) >> 2;               // which 32 key columns this warp handles
         const int r = q * 32 + lane;                  // query row inside the block
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
         bool ok = true;
@@ -670,97 +676,82 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
         float lse_next = INFINITY, dl_next = 0.0f;
         {
             const int qi0 = kb * ATT_BM + r;
-            if (qi0 < p.T) { lse_next = p.lse[(long long)bh * p.T + qi0] * 1.4426950408889634f; dl_next = p.delta[(long long)bh * p.T + qi0]; }
+            if (qi0 < p.T) { lse_next = p.lse[(long long)bh * p.T + qi0]; dl_next = p.delta[(long long)bh * p.T + qi0]; }
         }
         for (int it = 0; it < niter && ok; ++it) {
             const uint32_t pi = (uint32_t)(it & 1);
             const int qb = kb + it;
             const int qi = qb * ATT_BM + r;
             const bool diag = (qb == kb);
-            const float lse2 = lse_next, dl = dl_next;            // +inf for rows past T: P = 0
+            // (the factor is applied here and not where the value is asked for: there it would wait for the load, 600 clocks)
+            const float lse2 = lse_next * 1.4426950408889634f, dl = dl_next;            // +inf for rows past T: P = 0
             lse_next = INFINITY; dl_next = 0.0f;
             if (it + 1 < niter && qi + ATT_BM < p.T) {
-                lse_next = p.lse[(long long)bh * p.T + qi + ATT_BM] * 1.4426950408889634f;
+                lse_next = p.lse[(long long)bh * p.T + qi + ATT_BM];
                 dl_next = p.delta[(long long)bh * p.T + qi + ATT_BM];
             }
             if (!mbar_wait(sdp_full, pi, abort_flag)) { ok = false; break; }
             tc_fence_after();
-            // this thread's 64 scores and 64 dP values in one TMEM round trip, then the tiles are free
-            uint32_t sv0[32], sv1[32], dv0[32], dv1[32];
-            tmem_ld32(tS + lane_base + (half * 2) * 32, sv0);
-            tmem_ld32(tS + lane_base + (half * 2 + 1) * 32, sv1);
-            tmem_ld32(tdP + lane_base + (half * 2) * 32, dv0);
-            tmem_ld32(tdP + lane_base + (half * 2 + 1) * 32, dv1);
+            // this thread's 32 scores and 32 dP values in one TMEM round trip, then the tiles are free
+            uint32_t sv[32], dv[32];
+            tmem_ld32(tS + lane_base + cq * 32, sv);
+            tmem_ld32(tdP + lane_base + cq * 32, dv);
             tmem_ld_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(sdp_free);
             // rows past T get lse2 = +inf, i.e. P = 0; the diagonal block masks keys after the query
             float P[32], dS[32];
-            p_and_ds(sv0, dv0, p.scale_log2, lse2, dl, diag, diag ? qi - (k0 + (half * 2) * 32) : 32, P, dS);
+            p_and_ds(sv, dv, p.scale_log2, lse2, dl, diag, diag ? qi - (k0 + cq * 32) : 32, P, dS);
             if (!mbar_wait(pds_free, pi ^ 1u, abort_flag)) { ok = false; break; }     // previous P, dS consumed
             uint8_t* sdS_it = sdS + pi * DS_BLOCK_BYTES;                                // and this buffer's block stored
             if (!mbar_wait(&ds_stored[pi], (uint32_t)((it >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
-            store_chunk_bf16(sP, r, half * 2, P);
-            store_chunk_bf16(sdS_it, r, half * 2, dS);
-            p_and_ds(sv1, dv1, p.scale_log2, lse2, dl, diag, diag ? qi - (k0 + (half * 2 + 1) * 32) : 32, P, dS);
-            store_chunk_bf16(sP, r, half * 2 + 1, P);
-            store_chunk_bf16(sdS_it, r, half * 2 + 1, dS);
+            store_chunk_bf16(sP, r, cq, P);
+            store_chunk_bf16(sdS_it, r, cq, dS);
             tc_fence_before();
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(pds_full);
         }
+        // dV leaves by the first eight warps (two per lane quarter: head-dim columns 0-31 | 32-63), dK by the others
         const int kj = k0 + r;                        // key row of the accumulators
+        const int half = cq & 1;
+        const bool is_dk = cq >= 2;
         RopeRow rot;                                  // fetched while the last products finish
-        if (ok && kj < p.T && p.dqkv != nullptr)
+        if (ok && is_dk && kj < p.T && p.dqkv != nullptr)
             load_rope_row(rot, p.cos_t + (long long)kj * (p.hd >> 1), p.sin_t + (long long)kj * (p.hd >> 1), half * 32, p.hd);
         if (ok) {
             if (!mbar_wait(acc_full, 0, abort_flag)) ok = false;
         }
         if (ok) {
             tc_fence_after();
-            uint32_t v[32], w[32];
-            tmem_ld32(tdV + lane_base + half * 32, v);
-            tmem_ld32(tdK + lane_base + half * 32, w);
+            uint32_t v[32];
+            tmem_ld32((is_dk ? tdK : tdV) + lane_base + half * 32, v);
             tmem_ld_wait();
             if (p.dqkv != nullptr) {
                 // the P and dS tiles are free (every product has completed): dK into the first, dV into the second
-                if (kj < p.T) {
-                    stage_row_bf16(sP, r, w, half * 32, p.hd, &rot, p.scale);
-                    stage_row_bf16(sP + TILE_BYTES, r, v, half * 32, p.hd, nullptr, 1.0f);
-                }
-                fence_proxy_async();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(out_full);
-                if (warp == 2 && lane == 0) {
-                    if (mbar_wait(out_full, 0, abort_flag)) {
-                        tma_store_4d(&tmoK, sP, 0, k0, h, b);              // rows past T are clipped
-                        tma_store_4d(&tmoV, sP + TILE_BYTES, 0, k0, h, b);
-                        tma_store_commit();
-                        tma_store_wait_read<0>();
-                    } else ok = false;
-                }
+                if (kj < p.T) stage_row_bf16(sP + (is_dk ? 0 : TILE_BYTES), r, v, half * 32, p.hd, is_dk ? &rot : nullptr, is_dk ? p.scale : 1.0f);
             } else {
                 // separate float32 outputs [B*H, T, hd]: dK into the two P tiles (head-dim columns 0-31 | 32-63), dV
                 // into the two Q stages (a dS buffer may still be on its way out); tmoK / tmoV are float32 maps here
-                if (kj < p.T && half * 32 < p.hd) {
-                    stage_row_f32(sP + half * TILE_BYTES, r, w, p.scale);
-                    stage_row_f32(sQ + half * TILE_BYTES, r, v, 1.0f);
+                if (kj < p.T && half * 32 < p.hd) stage_row_f32((is_dk ? sP : sQ) + half * TILE_BYTES, r, v, is_dk ? p.scale : 1.0f);
+            }
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(out_full);
+            if (warp == 2 && lane == 0) {
+                if (!mbar_wait(out_full, 0, abort_flag)) ok = false;
+                else if (p.dqkv != nullptr) {
+                    tma_store_4d(&tmoK, sP, 0, k0, h, b);              // rows past T are clipped
+                    tma_store_4d(&tmoV, sP + TILE_BYTES, 0, k0, h, b);
+                } else {
+                    for (int c = 0; c * 32 < p.hd; ++c) {
+                        tma_store_3d(&tmoK, sP + c * TILE_BYTES, c * 32, k0, bh);
+                        tma_store_3d(&tmoV, sQ + c * TILE_BYTES, c * 32, k0, bh);
+                    }
                 }
-                fence_proxy_async();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(out_full);
-                if (warp == 2 && lane == 0) {
-                    if (mbar_wait(out_full, 0, abort_flag)) {
-                        for (int c = 0; c * 32 < p.hd; ++c) {
-                            tma_store_3d(&tmoK, sP + c * TILE_BYTES, c * 32, k0, bh);
-                            tma_store_3d(&tmoV, sQ + c * TILE_BYTES, c * 32, k0, bh);
-                        }
-                        tma_store_commit();
-                        tma_store_wait_read<0>();
-                    } else ok = false;
-                }
+                tma_store_commit();
+                tma_store_wait_read<0>();
             }
         }
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.err, 23); }
@@ -960,8 +951,8 @@ int launch_attention_bwd(DeviceCtx* ctx, const bf16* Q, const bf16* K, const bf1
     }
     {
         const long long total = (long long)B * T * H;
-        long long blocks = (total + 255) / 256;
-        if (blocks > 16LL * ctx->sm_count) blocks = 16LL * ctx->sm_count;
+        long long blocks = (total + 31) / 32;         // eight lanes per row
+        if (blocks > 8LL * ctx->sm_count) blocks = 8LL * ctx->sm_count;
         prof_mark(ctx, "attention_delta", 0.0, 0.0, stream);
         TB_CUDA(launch_kernel(attention_delta_kernel, dim3((int)blocks), dim3(256), 0, stream, att, datt, delta, B, T, H, hd));
         TB_CUDA(cudaGetLastError());
