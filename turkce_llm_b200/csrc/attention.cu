@@ -428,6 +428,7 @@ __global__ void attention_delta_kernel(const bf16* __restrict__ att, const bf16*
 struct AttBwdParams {
     int T, H, hd;
     int nq;
+    int BH, items;          // heads of all sequences; work items of the dK/dV kernel = BH * nq
     float scale, scale_log2;
     const float* lse;       // [B*H, T]
     const float* delta;     // [B*H, T]
@@ -506,29 +507,54 @@ __device__ __forceinline__ void stage_row_f32(uint8_t* tile, int r, const uint32
                         __uint_as_float(v[4 * g + 2]) * mul, __uint_as_float(v[4 * g + 3]) * mul);
 }
 
-// P = 2^(s*c - lse) and dS' = P * (dP - delta) of 32 scores of one row, two per instruction.  The factor 1/sqrt(hd)
-// of dS is applied to the accumulated dQ and dK instead (they are linear in dS).  lim: columns e <= lim are allowed.
-__device__ __forceinline__ void p_and_ds(const uint32_t (&sv)[32], const uint32_t (&dv)[32], float scale_log2, float lse2,
-                                         float dl, bool diag, int lim, float (&P)[32], float (&dS)[32]) {
+// P = 2^(s*c - lse) and dS' = P * (dP - delta) of scores E0 .. E0 + 15 of one row, two per instruction, as 16 bf16 each.  The
+// factor 1/sqrt(hd) of dS is applied to the accumulated dQ and dK instead (they are linear in dS).  lim: columns e <= lim are
+// allowed.
+template <int E0>
+__device__ __forceinline__ void p_and_ds16(const uint32_t (&sv)[32], const uint32_t (&dv)[32], float scale_log2, float lse2,
+                                           float dl, bool diag, int lim, uint4 (&pP)[2], uint4 (&pD)[2]) {
     const float2 c2 = make_float2(scale_log2, scale_log2), nl2 = make_float2(-lse2, -lse2), nd2 = make_float2(-dl, -dl);
+    uint32_t wp[8], wd[8];
 #pragma unroll
-    for (int e = 0; e < 32; e += 2) {
+    for (int i = 0; i < 8; ++i) {
+        const int e = E0 + 2 * i;
         const float2 x = __ffma2_rn(pair_of(sv[e], sv[e + 1]), c2, nl2);
         float p0 = fast_exp2(x.x), p1 = fast_exp2(x.y);
         if (diag) { p0 = e <= lim ? p0 : 0.0f; p1 = e + 1 <= lim ? p1 : 0.0f; }
         const float2 d = __fmul2_rn(make_float2(p0, p1), __fadd2_rn(pair_of(dv[e], dv[e + 1]), nd2));
-        P[e] = p0; P[e + 1] = p1;
-        dS[e] = d.x; dS[e + 1] = d.y;
+        __nv_bfloat162 hp = __floats2bfloat162_rn(p0, p1), hd = __floats2bfloat162_rn(d.x, d.y);
+        wp[i] = *reinterpret_cast<uint32_t*>(&hp);
+        wd[i] = *reinterpret_cast<uint32_t*>(&hd);
     }
+    pP[0] = make_uint4(wp[0], wp[1], wp[2], wp[3]); pP[1] = make_uint4(wp[4], wp[5], wp[6], wp[7]);
+    pD[0] = make_uint4(wd[0], wd[1], wd[2], wd[3]); pD[1] = make_uint4(wd[4], wd[5], wd[6], wd[7]);
+}
+
+// 16 bf16 of row r, columns 32 c + 16 h .., into a [128 x 128] operand stored as two [128 x 64] tiles
+__device__ __forceinline__ void store_half_chunk(uint8_t* tiles, int r, int c, int h, const uint4 (&v)[2]) {
+    uint8_t* row = tiles + (c >> 1) * TILE_BYTES + r * 128;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(row + ((((c & 1) * 4 + h * 2 + i) ^ (r & 7)) << 4)) = v[i];
 }
 
 constexpr int ATT_BWD_STAGES = 3;       // stages of the (Q, dO) pair in the dK/dV kernel
-constexpr int ATT_BWD_THREADS = 608;     // TMA warp, score-MMA warp, 16 compute warps, gradient-MMA warp
 constexpr int ATT_BWD_CW = 16;          // compute warps
+constexpr int ATT_BWD_THREADS = 128 + 32 * ATT_BWD_CW;      // + TMA warp, score-MMA warp, gradient-MMA warp, store warp
 // (two issuing threads on different schedulers: one thread cannot issue a block's 24 UMMAs as fast as the
 //  tensor pipe retires them while the compute warps compete for the same issue slots)
 
-// dK, dV of one key block: walks the query blocks qb = kb .. nq-1.
+// dK, dV of key blocks: an item is one key block of one head, walking the query blocks qb = kb .. nq-1; a CTA works through
+// several items (att_item: early key blocks, which have the most query blocks, first).
+// What bounds it (cycle stamps, 16 x 6 heads x 1024, a block = 128 queries x 128 keys): 1,024 clocks of 2^x per block, 512 of
+// shared-memory writes of P and dS', ~1,100 from the signal that P is written to the end of the gradient products, and
+// what an item costs outside its loop.  Hence
+//  * sixteen compute warps of 32 key columns (with eight of 64 the chain of one warp took 2,240 clocks a block);
+//  * P is free again after the dV products, which come first, and half of a block's exponentials come behind the stores of
+//    the first half;
+//  * dS' blocks leave through a thread of their own (reading 32 KB out takes 1,400 clocks, a third of a block's time when the
+//    gradient thread waited for it), three stages of Q and dO cover the loads (2,000 clocks under load);
+//  * with a CTA per item the set-up, the first loads and the epilogue took 4.3 us against 1.2 per block; now the next
+//    item's K, V, Q and dO come in, and its first scores are formed, under the last block and the epilogue of the one before.
 __global__ void __launch_bounds__(ATT_BWD_THREADS, 1)
 attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                           const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -542,34 +568,30 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     uint8_t* sQ = smem + 2 * TILE_BYTES;                              // ATT_BWD_STAGES stages
     uint8_t* sdO = smem + (2 + ATT_BWD_STAGES) * TILE_BYTES;          // ATT_BWD_STAGES stages
     uint8_t* sP = smem + (2 + 2 * ATT_BWD_STAGES) * TILE_BYTES;       // [128 q, 128 keys] as two tiles
-    uint8_t* sdS = smem + (4 + 2 * ATT_BWD_STAGES) * TILE_BYTES;      // same, two buffers (one is being stored to HBM)
+    uint8_t* sdS = smem + (4 + 2 * ATT_BWD_STAGES) * TILE_BYTES;      // same, two buffers (one is being stored)
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (8 + 2 * ATT_BWD_STAGES) * TILE_BYTES);
-    uint64_t* kv_full = bars;          // 1
-    uint64_t* qdo_full = bars + 1;     // ATT_BWD_STAGES
-    uint64_t* qdo_empty = bars + 5;    // ATT_BWD_STAGES
-    uint64_t* sdp_full = bars + 9;
-    uint64_t* sdp_free = bars + 10;    // one arrival per compute warp
-    uint64_t* pds_full = bars + 11;    // one arrival per compute warp
-    uint64_t* pds_free = bars + 12;
-    uint64_t* acc_full = bars + 13;
-    uint64_t* out_full = bars + 14;    // one arrival per compute warp: the output tile is staged in shared memory
-    uint64_t* ds_stored = bars + 16;   // 2: the bulk store of dS buffer b has read it
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+    uint64_t* kv_full = bars;
+    uint64_t* kv_empty = bars + 1;
+    uint64_t* qdo_full = bars + 2;     // ATT_BWD_STAGES
+    uint64_t* qdo_empty = bars + 6;    // ATT_BWD_STAGES
+    uint64_t* sdp_full = bars + 10;
+    uint64_t* sdp_free = bars + 11;    // one arrival per compute warp
+    uint64_t* pds_full = bars + 12;    // one arrival per compute warp
+    uint64_t* p_free = bars + 13;      // the dV products of the block have read P
+    uint64_t* ds_free = bars + 14;     // the dK products of the block have read dS'
+    uint64_t* acc_full = bars + 15;    // an item's last products are done
+    uint64_t* out_full = bars + 16;    // one arrival per compute warp: an item's output tiles are staged
+    uint64_t* out_done = bars + 17;    // the store has read them
+    uint64_t* ds_stored = bars + 18;   // 2: the bulk store of dS buffer b has read it
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kb = blockIdx.y;                 // early key blocks have the most query blocks: all heads' first
-    const int bh = blockIdx.x;
-    const int b = bh / p.H, h = bh % p.H;
-    const int k0 = kb * ATT_BN;
-    const int niter = p.nq - kb;
+    const int worker = (int)blockIdx.x, workers = (int)gridDim.x;
+    // Blocks are counted through all items of the CTA (g); item k has nq - kb of them.
 
     if (threadIdx.x == 0) {
-        mbar_init(kv_full, 1);
-        for (int i = 0; i < ATT_BWD_STAGES; ++i) { mbar_init(&qdo_full[i], 1); mbar_init(&qdo_empty[i], 1); }
-        mbar_init(sdp_full, 1); mbar_init(sdp_free, ATT_BWD_CW); mbar_init(pds_full, ATT_BWD_CW); mbar_init(pds_free, 1);
-        mbar_init(acc_full, 1); mbar_init(out_full, ATT_BWD_CW);
-        mbar_init(&ds_stored[0], 1); mbar_init(&ds_stored[1], 1);
+        for (int i = 0; i < 20; ++i) mbar_init(&bars[i], (i == 11 || i == 12 || i == 16) ? ATT_BWD_CW : 1);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -584,43 +606,52 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     if (warp == 0) {
         if (elect_one()) {
             bool ok = true;
-            mbar_expect_tx(kv_full, 2 * TILE_BYTES);
-            tma_load_3d(sK, &tmK, kv_full, 0, k0, bh);
-            tma_load_3d(sV, &tmV, kv_full, 0, k0, bh);
-            for (int it = 0; it < niter && ok; ++it) {
-                const int s = it % ATT_BWD_STAGES;
-                if (!mbar_wait(&qdo_empty[s], (uint32_t)((it / ATT_BWD_STAGES) & 1) ^ 1u, abort_flag)) { ok = false; break; }
-                const int q0 = (kb + it) * ATT_BM;
-                mbar_expect_tx(&qdo_full[s], 2 * TILE_BYTES);
-                tma_load_3d(sQ + s * TILE_BYTES, &tmQ, &qdo_full[s], 0, q0, bh);
-                tma_load_4d(sdO + s * TILE_BYTES, &tmdO, &qdo_full[s], 0, q0, h, b);
+            int g = 0;
+            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
+                const int kb = item / p.BH, bh = item % p.BH, b = bh / p.H, h = bh % p.H;
+                for (int qb = kb; qb < p.nq; ++qb, ++g) {
+                    const int s = g % ATT_BWD_STAGES;
+                    if (!mbar_wait(&qdo_empty[s], (uint32_t)((g / ATT_BWD_STAGES) & 1) ^ 1u, abort_flag)) { ok = false; break; }
+                    mbar_expect_tx(&qdo_full[s], 2 * TILE_BYTES);
+                    tma_load_3d(sQ + s * TILE_BYTES, &tmQ, &qdo_full[s], 0, qb * ATT_BM, bh);
+                    tma_load_4d(sdO + s * TILE_BYTES, &tmdO, &qdo_full[s], 0, qb * ATT_BM, h, b);
+                    if (qb == kb) {             // (behind the first Q and dO, for which there may be room earlier)
+                        if (!mbar_wait(kv_empty, (uint32_t)(k & 1) ^ 1u, abort_flag)) { ok = false; break; }
+                        mbar_expect_tx(kv_full, 2 * TILE_BYTES);
+                        tma_load_3d(sK, &tmK, kv_full, 0, kb * ATT_BN, bh);
+                        tma_load_3d(sV, &tmV, kv_full, 0, kb * ATT_BN, bh);
+                    }
+                }
             }
             pdl_launch_dependents_now();     // all loads issued: the next kernel may start its prologue
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 21); }
         }
     } else if (warp == 1) {
+        // S = Q K^T and dP = dO V^T of every block; may run ahead of the gradient products because the compute warps free
+        // the two score tiles as soon as they hold them in registers
         if (elect_one()) {
-            const uint32_t id_s = umma_idesc(1u, 0u, 0u, 128, 128);      // Q K^T, dO V^T
+            const uint32_t id_s = umma_idesc(1u, 0u, 0u, 128, 128);
             const uint64_t dKk = kmajor_tile(smem_u32(sK)), dVk = kmajor_tile(smem_u32(sV));
             const uint64_t dQk0 = kmajor_tile(smem_u32(sQ)), ddOk0 = kmajor_tile(smem_u32(sdO));
-            bool ok = mbar_wait(kv_full, 0, abort_flag);
-            // S = Q K^T and dP = dO V^T of query block `it`; may run ahead of the accumulation of it-1
-            // because the compute warps free the two score tiles as soon as they hold them in registers
-            auto issue_sdp = [&](int it) -> bool {
-                const int s = it % ATT_BWD_STAGES;
-                const uint64_t dQk = dQk0 + (uint64_t)s * TILESTEP, ddOk = ddOk0 + (uint64_t)s * TILESTEP;
-                if (!mbar_wait(&qdo_full[s], (uint32_t)((it / ATT_BWD_STAGES) & 1), abort_flag)) return false;
-                if (!mbar_wait(sdp_free, (uint32_t)(it & 1) ^ 1u, abort_flag)) return false;
-                tc_fence_after();
+            bool ok = true;
+            int g = 0;
+            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
+                const int n = p.nq - item / p.BH;
+                if (!mbar_wait(kv_full, (uint32_t)(k & 1), abort_flag)) { ok = false; break; }
+                for (int it = 0; it < n; ++it, ++g) {
+                    const int s = g % ATT_BWD_STAGES;
+                    const uint64_t dQk = dQk0 + (uint64_t)s * TILESTEP, ddOk = ddOk0 + (uint64_t)s * TILESTEP;
+                    if (!mbar_wait(&qdo_full[s], (uint32_t)((g / ATT_BWD_STAGES) & 1), abort_flag)) { ok = false; break; }
+                    if (!mbar_wait(sdp_free, (uint32_t)(g & 1) ^ 1u, abort_flag)) { ok = false; break; }
+                    tc_fence_after();
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma_bf16(tS, dQk + k * KSTEP, dKk + k * KSTEP, id_s, k > 0 ? 1u : 0u);
+                    for (int j = 0; j < 4; ++j) umma_bf16(tS, dQk + j * KSTEP, dKk + j * KSTEP, id_s, j > 0 ? 1u : 0u);
 #pragma unroll
-                for (int k = 0; k < 4; ++k) umma_bf16(tdP, ddOk + k * KSTEP, dVk + k * KSTEP, id_s, k > 0 ? 1u : 0u);
-                umma_commit(sdp_full);
-                return true;
-            };
-            if (ok) ok = issue_sdp(0);
-            for (int it = 0; it + 1 < niter && ok; ++it) ok = issue_sdp(it + 1);
+                    for (int j = 0; j < 4; ++j) umma_bf16(tdP, ddOk + j * KSTEP, dVk + j * KSTEP, id_s, j > 0 ? 1u : 0u);
+                    umma_commit(sdp_full);
+                }
+                if (ok) umma_commit(kv_empty);
+            }
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 22); }
         }
     } else if (warp == 2 + ATT_BWD_CW) {
@@ -628,131 +659,160 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
         if (elect_one()) {
             const uint32_t id_t = umma_idesc(1u, 1u, 1u, 128, 64);       // both operands MN-major
             const uint64_t dPm = mnmajor_tile(smem_u32(sP), TILE_BYTES), ddSm0 = mnmajor_tile(smem_u32(sdS), TILE_BYTES);
-            const long long nblk = (long long)p.nq * (p.nq + 1) / 2;
             const uint64_t dQm0 = mnmajor_tile(smem_u32(sQ), TILE_BYTES), ddOm0 = mnmajor_tile(smem_u32(sdO), TILE_BYTES);
             bool ok = true;
-            for (int it = 0; it < niter && ok; ++it) {
-                const int s = it % ATT_BWD_STAGES;
-                const uint64_t dQm = dQm0 + (uint64_t)s * TILESTEP, ddOm = ddOm0 + (uint64_t)s * TILESTEP;
-                if (!mbar_wait(&qdo_full[s], (uint32_t)((it / ATT_BWD_STAGES) & 1), abort_flag)) { ok = false; break; }
-                if (!mbar_wait(pds_full, (uint32_t)(it & 1), abort_flag)) { ok = false; break; }
-                tc_fence_after();
+            int g = 0;
+            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
+                const int n = p.nq - item / p.BH;
+                for (int it = 0; it < n; ++it, ++g) {
+                    const int s = g % ATT_BWD_STAGES;
+                    const uint64_t dQm = dQm0 + (uint64_t)s * TILESTEP, ddOm = ddOm0 + (uint64_t)s * TILESTEP;
+                    const uint64_t ddSm = ddSm0 + (uint64_t)(g & 1) * (2 * TILESTEP);
+                    if (!mbar_wait(&qdo_full[s], (uint32_t)((g / ATT_BWD_STAGES) & 1), abort_flag)) { ok = false; break; }
+                    if (!mbar_wait(pds_full, (uint32_t)(g & 1), abort_flag)) { ok = false; break; }
+                    tc_fence_after();
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    umma_bf16(tdV, dPm + k * MNSTEP, ddOm + k * MNSTEP, id_t, (it > 0 || k > 0) ? 1u : 0u);
-                const uint64_t ddSm = ddSm0 + (uint64_t)(it & 1) * (2 * TILESTEP);
+                    for (int j = 0; j < 8; ++j)
+                        umma_bf16(tdV, dPm + j * MNSTEP, ddOm + j * MNSTEP, id_t, (it > 0 || j > 0) ? 1u : 0u);
+                    umma_commit(p_free);
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    umma_bf16(tdK, ddSm + k * MNSTEP, dQm + k * MNSTEP, id_t, (it > 0 || k > 0) ? 1u : 0u);
-                umma_commit(pds_free);
-                // S and dP of this block (the other issuer's) completed before the compute warps could sign
-                // pds_full, so this commit covers every read of the stage
-                umma_commit(&qdo_empty[s]);
-                if (it == niter - 1) umma_commit(acc_full);      // the epilogue need not wait for the store below
-                // the dS block leaves for the dQ kernel as it lies in shared memory; its buffer is written again two
-                // steps from now.  Not before the products above have completed: a 32 KB read of shared memory beside them
-                // delays pds_free, which the compute warps need ~900 cycles after they sign pds_full.  That it has been read
-                // (1,400 clocks) is looked at a step later.
-                if (it > 0) { tma_store_wait_read<0>(); mbar_arrive(&ds_stored[(it - 1) & 1]); }
-                if (!mbar_wait(pds_free, (uint32_t)(it & 1), abort_flag)) { ok = false; break; }
-                {
-                    const int qb = kb + it;
-                    uint8_t* dst = reinterpret_cast<uint8_t*>(p.ds) +
-                                   ((long long)bh * nblk + (long long)qb * (qb + 1) / 2 + kb) * DS_BLOCK_BYTES;
-                    bulk_store(dst, sdS + (it & 1) * DS_BLOCK_BYTES, DS_BLOCK_BYTES);
+                    for (int j = 0; j < 8; ++j)
+                        umma_bf16(tdK, ddSm + j * MNSTEP, dQm + j * MNSTEP, id_t, (it > 0 || j > 0) ? 1u : 0u);
+                    umma_commit(ds_free);
+                    // S and dP of this block (the other issuer's) completed before the compute warps could sign
+                    // pds_full, so this commit covers every read of the stage
+                    umma_commit(&qdo_empty[s]);
+                }
+                if (ok) umma_commit(acc_full);
+            }
+            if (!ok) { *abort_flag = 1; atomicExch(p.err, 24); }
+        }
+    } else if (warp == 3 + ATT_BWD_CW) {
+        // the dS blocks leave for the dQ kernel as they lie in shared memory.  Not before the products that read them have
+        // completed: a 32 KB read of shared memory beside those would delay them.
+        if (elect_one()) {
+            const long long nblk = (long long)p.nq * (p.nq + 1) / 2;
+            bool ok = true;
+            int g = 0;
+            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
+                const int kb = item / p.BH, bh = item % p.BH;
+                for (int qb = kb; qb < p.nq; ++qb, ++g) {
+                    if (!mbar_wait(ds_free, (uint32_t)(g & 1), abort_flag)) { ok = false; break; }
+                    bulk_store(reinterpret_cast<uint8_t*>(p.ds) + ((long long)bh * nblk + (long long)qb * (qb + 1) / 2 + kb) * DS_BLOCK_BYTES,
+                               sdS + (g & 1) * DS_BLOCK_BYTES, DS_BLOCK_BYTES);
                     tma_store_commit();
+                    tma_store_wait_read<0>();
+                    mbar_arrive(&ds_stored[g & 1]);
                 }
             }
-            tma_store_wait_read<0>();
-            if (!ok) { *abort_flag = 1; atomicExch(p.err, 24); }
+            if (!ok) { *abort_flag = 1; atomicExch(p.err, 25); }
         }
     } else {
         const int q = warp & 3;
         const int cq = (warp - 2) >> 2;               // which 32 key columns this warp handles
         const int r = q * 32 + lane;                  // query row inside the block
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
+        const int half = cq & 1;                      // epilogue: dV leaves by the first eight warps (two per lane quarter:
+        const bool is_dk = cq >= 2;                   // head-dim columns 0-31 | 32-63), dK by the others
         bool ok = true;
-        // the row's log-sum-exp and delta of the NEXT query block are fetched while this one is worked on
+        int g = 0;
+        // the row's log-sum-exp and delta of the NEXT query block are asked for while this one is worked on
         float lse_next = INFINITY, dl_next = 0.0f;
-        {
-            const int qi0 = kb * ATT_BM + r;
-            if (qi0 < p.T) { lse_next = p.lse[(long long)bh * p.T + qi0]; dl_next = p.delta[(long long)bh * p.T + qi0]; }
-        }
-        for (int it = 0; it < niter && ok; ++it) {
-            const uint32_t pi = (uint32_t)(it & 1);
-            const int qb = kb + it;
+        auto fetch_row = [&](int item, int qb) {
             const int qi = qb * ATT_BM + r;
-            const bool diag = (qb == kb);
-            // (the factor is applied here and not where the value is asked for: there it would wait for the load, 600 clocks)
-            const float lse2 = lse_next * 1.4426950408889634f, dl = dl_next;            // +inf for rows past T: P = 0
-            lse_next = INFINITY; dl_next = 0.0f;
-            if (it + 1 < niter && qi + ATT_BM < p.T) {
-                lse_next = p.lse[(long long)bh * p.T + qi + ATT_BM];
-                dl_next = p.delta[(long long)bh * p.T + qi + ATT_BM];
+            lse_next = INFINITY; dl_next = 0.0f;      // rows past T: P = 0
+            if (qi < p.T) {
+                const long long o = (long long)(item % p.BH) * p.T + qi;
+                lse_next = p.lse[o]; dl_next = p.delta[o];
             }
-            if (!mbar_wait(sdp_full, pi, abort_flag)) { ok = false; break; }
-            tc_fence_after();
-            // this thread's 32 scores and 32 dP values in one TMEM round trip, then the tiles are free
-            uint32_t sv[32], dv[32];
-            tmem_ld32(tS + lane_base + cq * 32, sv);
-            tmem_ld32(tdP + lane_base + cq * 32, dv);
-            tmem_ld_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(sdp_free);
-            // rows past T get lse2 = +inf, i.e. P = 0; the diagonal block masks keys after the query
-            float P[32], dS[32];
-            p_and_ds(sv, dv, p.scale_log2, lse2, dl, diag, diag ? qi - (k0 + cq * 32) : 32, P, dS);
-            if (!mbar_wait(pds_free, pi ^ 1u, abort_flag)) { ok = false; break; }     // previous P, dS consumed
-            uint8_t* sdS_it = sdS + pi * DS_BLOCK_BYTES;                                // and this buffer's block stored
-            if (!mbar_wait(&ds_stored[pi], (uint32_t)((it >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
-            store_chunk_bf16(sP, r, cq, P);
-            store_chunk_bf16(sdS_it, r, cq, dS);
-            tc_fence_before();
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(pds_full);
-        }
-        // dV leaves by the first eight warps (two per lane quarter: head-dim columns 0-31 | 32-63), dK by the others
-        const int kj = k0 + r;                        // key row of the accumulators
-        const int half = cq & 1;
-        const bool is_dk = cq >= 2;
-        RopeRow rot;                                  // fetched while the last products finish
-        if (ok && is_dk && kj < p.T && p.dqkv != nullptr)
-            load_rope_row(rot, p.cos_t + (long long)kj * (p.hd >> 1), p.sin_t + (long long)kj * (p.hd >> 1), half * 32, p.hd);
-        if (ok) {
-            if (!mbar_wait(acc_full, 0, abort_flag)) ok = false;
-        }
-        if (ok) {
-            tc_fence_after();
-            uint32_t v[32];
-            tmem_ld32((is_dk ? tdK : tdV) + lane_base + half * 32, v);
-            tmem_ld_wait();
-            if (p.dqkv != nullptr) {
-                // the P and dS tiles are free (every product has completed): dK into the first, dV into the second
-                if (kj < p.T) stage_row_bf16(sP + (is_dk ? 0 : TILE_BYTES), r, v, half * 32, p.hd, is_dk ? &rot : nullptr, is_dk ? p.scale : 1.0f);
-            } else {
-                // separate float32 outputs [B*H, T, hd]: dK into the two P tiles (head-dim columns 0-31 | 32-63), dV
-                // into the two Q stages (a dS buffer may still be on its way out); tmoK / tmoV are float32 maps here
-                if (kj < p.T && half * 32 < p.hd) stage_row_f32((is_dk ? sP : sQ) + half * TILE_BYTES, r, v, is_dk ? p.scale : 1.0f);
+        };
+        int item = att_item(0, worker, workers, p.items);
+        fetch_row(item, item / p.BH);
+        for (int k = 0; ok && item >= 0; ++k) {
+            const int kb = item / p.BH, bh = item % p.BH, k0 = kb * ATT_BN;
+            const int next_item = att_item(k + 1, worker, workers, p.items);
+            for (int qb = kb; qb < p.nq; ++qb, ++g) {
+                const uint32_t pi = (uint32_t)(g & 1);
+                const bool diag = qb == kb;
+                // (the factor is applied here and not where the value is asked for: there it would wait for the load)
+                const float lse2 = lse_next * 1.4426950408889634f, dl = dl_next;
+                if (!mbar_wait(sdp_full, pi, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                // this thread's 32 scores and 32 dP values in one TMEM round trip, then the tiles are free
+                uint32_t sv[32], dv[32];
+                tmem_ld32(tS + lane_base + cq * 32, sv);
+                tmem_ld32(tdP + lane_base + cq * 32, dv);
+                tmem_ld_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(sdp_free);
+                if (qb + 1 < p.nq) fetch_row(item, qb + 1);
+                else if (next_item >= 0) fetch_row(next_item, next_item / p.BH);
+                // the dS buffer's block of two steps ago has left; at an item's start, so have the staged outputs
+                uint8_t* sdS_g = sdS + pi * DS_BLOCK_BYTES;
+                if (!mbar_wait(&ds_stored[pi], (uint32_t)((g >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
+                if (diag && k > 0 && !mbar_wait(out_done, (uint32_t)(k & 1) ^ 1u, abort_flag)) { ok = false; break; }
+                // the diagonal block masks keys after the query: columns e <= lim are allowed
+                const int lim = diag ? r - cq * 32 : 32;
+                uint4 pP[2], pD[2];
+                p_and_ds16<0>(sv, dv, p.scale_log2, lse2, dl, diag, lim, pP, pD);
+                if (!mbar_wait(p_free, pi ^ 1u, abort_flag)) { ok = false; break; }          // the previous block's P is read
+                store_half_chunk(sP, r, cq, 0, pP);
+                store_half_chunk(sdS_g, r, cq, 0, pD);
+                p_and_ds16<16>(sv, dv, p.scale_log2, lse2, dl, diag, lim, pP, pD);
+                store_half_chunk(sP, r, cq, 1, pP);
+                store_half_chunk(sdS_g, r, cq, 1, pD);
+                tc_fence_before();
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(pds_full);
             }
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(out_full);
-            if (warp == 2 && lane == 0) {
-                if (!mbar_wait(out_full, 0, abort_flag)) ok = false;
-                else if (p.dqkv != nullptr) {
-                    tma_store_4d(&tmoK, sP, 0, k0, h, b);              // rows past T are clipped
-                    tma_store_4d(&tmoV, sP + TILE_BYTES, 0, k0, h, b);
+            const int kj = k0 + r;                        // key row of the accumulators
+            RopeRow rot;                                  // fetched while the last products finish
+            if (ok && is_dk && kj < p.T && p.dqkv != nullptr)
+                load_rope_row(rot, p.cos_t + (long long)kj * (p.hd >> 1), p.sin_t + (long long)kj * (p.hd >> 1), half * 32, p.hd);
+            if (ok && !mbar_wait(acc_full, (uint32_t)(k & 1), abort_flag)) ok = false;
+            // the float32 dV tiles go into the dS buffer that the next item's first block will use (g is behind the last)
+            uint8_t* spare = sdS + (g & 1) * DS_BLOCK_BYTES;
+            if (ok && p.dqkv == nullptr && g >= 2 && !mbar_wait(&ds_stored[g & 1], (uint32_t)((g >> 1) & 1) ^ 1u, abort_flag)) ok = false;
+            if (ok) {
+                tc_fence_after();
+                uint32_t v[32];
+                tmem_ld32((is_dk ? tdK : tdV) + lane_base + half * 32, v);
+                tmem_ld_wait();
+                tc_fence_before();
+                if (p.dqkv != nullptr) {
+                    // the P tiles are free (every product has completed): dK into the first, dV into the second
+                    if (kj < p.T) stage_row_bf16(sP + (is_dk ? 0 : TILE_BYTES), r, v, half * 32, p.hd, is_dk ? &rot : nullptr, is_dk ? p.scale : 1.0f);
                 } else {
-                    for (int c = 0; c * 32 < p.hd; ++c) {
-                        tma_store_3d(&tmoK, sP + c * TILE_BYTES, c * 32, k0, bh);
-                        tma_store_3d(&tmoV, sQ + c * TILE_BYTES, c * 32, k0, bh);
-                    }
+                    // separate float32 outputs [B*H, T, hd]: dK into the two P tiles (head-dim columns 0-31 | 32-63), dV
+                    // into the spare dS buffer; tmoK / tmoV are float32 maps here
+                    if (kj < p.T && half * 32 < p.hd) stage_row_f32((is_dk ? sP : spare) + half * TILE_BYTES, r, v, is_dk ? p.scale : 1.0f);
                 }
-                tma_store_commit();
-                tma_store_wait_read<0>();
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(out_full);
+                if (warp == 2) {
+                    if (lane == 0) {
+                        if (!mbar_wait(out_full, (uint32_t)(k & 1), abort_flag)) ok = false;
+                        else if (p.dqkv != nullptr) {
+                            const int b = bh / p.H, h = bh % p.H;
+                            tma_store_4d(&tmoK, sP, 0, k0, h, b);              // rows past T are clipped
+                            tma_store_4d(&tmoV, sP + TILE_BYTES, 0, k0, h, b);
+                        } else {
+                            for (int c = 0; c * 32 < p.hd; ++c) {
+                                tma_store_3d(&tmoK, sP + c * TILE_BYTES, c * 32, k0, bh);
+                                tma_store_3d(&tmoV, spare + c * TILE_BYTES, c * 32, k0, bh);
+                            }
+                        }
+                        tma_store_commit();
+                        tma_store_wait_read<0>();
+                        mbar_arrive(out_done);
+                    }
+                    ok = __all_sync(0xffffffffu, ok);
+                }
             }
+            item = next_item;
         }
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.err, 23); }
     }
@@ -962,7 +1022,8 @@ int launch_attention_bwd(DeviceCtx* ctx, const bf16* Q, const bf16* K, const bf1
     dim3 grid(BH, p.nq);
     const double tri = (double)BH * T * (double)T * hd;      // one lower-triangular product = tri flops
     prof_mark(ctx, "attention_bwd_dkdv", 4.0 * tri, (double)BH * T * hd * (2.0 * 4 + 8.0), stream);
-    TB_CUDA(launch_kernel(attention_bwd_dkdv_kernel, dim3(grid), dim3(ATT_BWD_THREADS), ATT_DKDV_SMEM, stream, tmQ, tmK, tmV, tmdO, tmoK, tmoV, p));
+    p.BH = BH; p.items = BH * p.nq;
+    TB_CUDA(launch_kernel(attention_bwd_dkdv_kernel, dim3((unsigned)std::min(p.items, ctx->sm_count)), dim3(ATT_BWD_THREADS), ATT_DKDV_SMEM, stream, tmQ, tmK, tmV, tmdO, tmoK, tmoV, p));
     TB_CUDA(cudaGetLastError());
     ctx->launches++;
     prof_close(ctx, stream);
