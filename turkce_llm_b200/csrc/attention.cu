@@ -577,13 +577,12 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     uint64_t* sdp_full = bars + 10;
     uint64_t* sdp_free = bars + 11;    // one arrival per compute warp
     uint64_t* pds_full = bars + 12;    // one arrival per compute warp
-    uint64_t* p_free = bars + 13;      // the dV products of the block have read P
+    uint64_t* w_free = bars + 13;      // 2 arrivals: block g's dV products have read P, block g - 1's dS buffer has been read out
     uint64_t* ds_free = bars + 14;     // the dK products of the block have read dS'
     uint64_t* acc_full = bars + 15;    // an item's last products are done
     uint64_t* out_full = bars + 16;    // one arrival per compute warp: an item's output tiles are staged
     uint64_t* out_done = bars + 17;    // the store has read them
-    uint64_t* ds_stored = bars + 18;   // 2: the bulk store of dS buffer b has read it
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -591,7 +590,7 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     // Blocks are counted through all items of the CTA (g); item k has nq - kb of them.
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 20; ++i) mbar_init(&bars[i], (i == 11 || i == 12 || i == 16) ? ATT_BWD_CW : 1);
+        for (int i = 0; i < 18; ++i) mbar_init(&bars[i], (i == 11 || i == 12 || i == 16) ? ATT_BWD_CW : i == 13 ? 2 : 1);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -674,7 +673,7 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         umma_bf16(tdV, dPm + j * MNSTEP, ddOm + j * MNSTEP, id_t, (it > 0 || j > 0) ? 1u : 0u);
-                    umma_commit(p_free);
+                    umma_commit(w_free);
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         umma_bf16(tdK, ddSm + j * MNSTEP, dQm + j * MNSTEP, id_t, (it > 0 || j > 0) ? 1u : 0u);
@@ -689,21 +688,37 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
         }
     } else if (warp == 3 + ATT_BWD_CW) {
         // the dS blocks leave for the dQ kernel as they lie in shared memory.  Not before the products that read them have
-        // completed: a 32 KB read of shared memory beside those would delay them.
+        // completed: a 32 KB read of shared memory beside those would delay them.  An item's output tiles leave here too:
+        // no compute warp waits for them to be read out.
         if (elect_one()) {
             const long long nblk = (long long)p.nq * (p.nq + 1) / 2;
             bool ok = true;
             int g = 0;
+            mbar_arrive(w_free);                      // in front of block 0: no buffer to be read out
             for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
-                const int kb = item / p.BH, bh = item % p.BH;
+                const int kb = item / p.BH, bh = item % p.BH, b = bh / p.H, h = bh % p.H;
                 for (int qb = kb; qb < p.nq; ++qb, ++g) {
                     if (!mbar_wait(ds_free, (uint32_t)(g & 1), abort_flag)) { ok = false; break; }
                     bulk_store(reinterpret_cast<uint8_t*>(p.ds) + ((long long)bh * nblk + (long long)qb * (qb + 1) / 2 + kb) * DS_BLOCK_BYTES,
                                sdS + (g & 1) * DS_BLOCK_BYTES, DS_BLOCK_BYTES);
                     tma_store_commit();
                     tma_store_wait_read<0>();
-                    mbar_arrive(&ds_stored[g & 1]);
+                    mbar_arrive(w_free);
                 }
+                if (!ok || !mbar_wait(out_full, (uint32_t)(k & 1), abort_flag)) { ok = false; break; }
+                if (p.dqkv != nullptr) {
+                    tma_store_4d(&tmoK, sP, 0, kb * ATT_BN, h, b);              // rows past T are clipped
+                    tma_store_4d(&tmoV, sP + TILE_BYTES, 0, kb * ATT_BN, h, b);
+                } else {
+                    uint8_t* spare = sdS + (g & 1) * DS_BLOCK_BYTES;
+                    for (int c = 0; c * 32 < p.hd; ++c) {
+                        tma_store_3d(&tmoK, sP + c * TILE_BYTES, c * 32, kb * ATT_BN, bh);
+                        tma_store_3d(&tmoV, spare + c * TILE_BYTES, c * 32, kb * ATT_BN, bh);
+                    }
+                }
+                tma_store_commit();
+                tma_store_wait_read<0>();
+                mbar_arrive(out_done);
             }
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 25); }
         }
@@ -748,15 +763,15 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
                 if (lane == 0) mbar_arrive(sdp_free);
                 if (qb + 1 < p.nq) fetch_row(item, qb + 1);
                 else if (next_item >= 0) fetch_row(next_item, next_item / p.BH);
-                // the dS buffer's block of two steps ago has left; at an item's start, so have the staged outputs
                 uint8_t* sdS_g = sdS + pi * DS_BLOCK_BYTES;
-                if (!mbar_wait(&ds_stored[pi], (uint32_t)((g >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
-                if (diag && k > 0 && !mbar_wait(out_done, (uint32_t)(k & 1) ^ 1u, abort_flag)) { ok = false; break; }
                 // the diagonal block masks keys after the query: columns e <= lim are allowed
                 const int lim = diag ? r - cq * 32 : 32;
                 uint4 pP[2], pD[2];
                 p_and_ds16<0>(sv, dv, p.scale_log2, lse2, dl, diag, lim, pP, pD);
-                if (!mbar_wait(p_free, pi ^ 1u, abort_flag)) { ok = false; break; }          // the previous block's P is read
+                // the previous block's P has been read, the one before has left this dS buffer; at an item's start the staged
+                // outputs have left both
+                if (!mbar_wait(w_free, pi ^ 1u, abort_flag)) { ok = false; break; }
+                if (diag && k > 0 && !mbar_wait(out_done, (uint32_t)(k & 1) ^ 1u, abort_flag)) { ok = false; break; }
                 store_half_chunk(sP, r, cq, 0, pP);
                 store_half_chunk(sdS_g, r, cq, 0, pD);
                 p_and_ds16<16>(sv, dv, p.scale_log2, lse2, dl, diag, lim, pP, pD);
@@ -772,9 +787,9 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
             if (ok && is_dk && kj < p.T && p.dqkv != nullptr)
                 load_rope_row(rot, p.cos_t + (long long)kj * (p.hd >> 1), p.sin_t + (long long)kj * (p.hd >> 1), half * 32, p.hd);
             if (ok && !mbar_wait(acc_full, (uint32_t)(k & 1), abort_flag)) ok = false;
-            // the float32 dV tiles go into the dS buffer that the next item's first block will use (g is behind the last)
+            // the float32 dV tiles go into the dS buffer that the next item's first block will use (g is behind the last block)
             uint8_t* spare = sdS + (g & 1) * DS_BLOCK_BYTES;
-            if (ok && p.dqkv == nullptr && g >= 2 && !mbar_wait(&ds_stored[g & 1], (uint32_t)((g >> 1) & 1) ^ 1u, abort_flag)) ok = false;
+            if (ok && p.dqkv == nullptr && !mbar_wait(w_free, (uint32_t)(g & 1) ^ 1u, abort_flag)) ok = false;
             if (ok) {
                 tc_fence_after();
                 uint32_t v[32];
@@ -792,25 +807,6 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(out_full);
-                if (warp == 2) {
-                    if (lane == 0) {
-                        if (!mbar_wait(out_full, (uint32_t)(k & 1), abort_flag)) ok = false;
-                        else if (p.dqkv != nullptr) {
-                            const int b = bh / p.H, h = bh % p.H;
-                            tma_store_4d(&tmoK, sP, 0, k0, h, b);              // rows past T are clipped
-                            tma_store_4d(&tmoV, sP + TILE_BYTES, 0, k0, h, b);
-                        } else {
-                            for (int c = 0; c * 32 < p.hd; ++c) {
-                                tma_store_3d(&tmoK, sP + c * TILE_BYTES, c * 32, k0, bh);
-                                tma_store_3d(&tmoV, spare + c * TILE_BYTES, c * 32, k0, bh);
-                            }
-                        }
-                        tma_store_commit();
-                        tma_store_wait_read<0>();
-                        mbar_arrive(out_done);
-                    }
-                    ok = __all_sync(0xffffffffu, ok);
-                }
             }
             item = next_item;
         }
