@@ -822,43 +822,40 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
 
 // dQ of one query block: dQ = scale * sum over its key blocks kb = 0 .. qb of dS'(qb, kb) K(kb), the dS' blocks read
 // back as the dK/dV kernel stored them.  No exponentials and no compute warps in the loop: a loader, a tensor-core
-// issuer and four epilogue warps (thread = query row); two stages of 48 KB, so two CTAs share an SM and the prologue
-// and epilogue of one hide behind the loop of the other.  Sums are formed in key-block order: fixed, no atomics.
+// issuer and four epilogue warps (thread = query row).  A CTA works through several (query block, head) items (att_item) with
+// four stages of 48 KB running through all of them and two accumulators, so that an item's epilogue lies beside the next
+// one's loop (two CTAs per SM with an item each and two stages took 31 us at 16 x 6 heads x 1024: the set-up, first loads
+// and epilogue of an item are as long as its 4.5 blocks).  Sums are formed in key-block order: fixed, no atomics.
 constexpr int ATT_DQ_THREADS = 192;
-constexpr int ATT_DQ_STAGES = 2;
+constexpr int ATT_DQ_STAGES = 4;
 constexpr int ATT_DQ_STAGE_BYTES = DS_BLOCK_BYTES + TILE_BYTES;
 
-__global__ void __launch_bounds__(ATT_DQ_THREADS, 2)
+__global__ void __launch_bounds__(ATT_DQ_THREADS, 1)
 attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmoQ,
                         const AttBwdParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
-    const uint32_t pad = (1024u - (raw_addr & 1023u)) & 1023u;
-    uint8_t* smem = smem_raw + pad;
-    // stage s: dS block (two [128 x 64] tiles) then the K tile.  The request is 1 KB + the stages: the barriers go
-    // behind the stages when the alignment pad leaves room there (the usual case: pad 0), else into the pad itself
-    uint64_t* bars = reinterpret_cast<uint64_t*>(pad <= 768u ? smem + ATT_DQ_STAGES * ATT_DQ_STAGE_BYTES : smem_raw);
+    uint8_t* smem = smem_raw + ((1024u - (raw_addr & 1023u)) & 1023u);
+    // stage s: dS block (two [128 x 64] tiles) then the K tile; behind the stages two tiles for the output
+    uint8_t* out = smem + ATT_DQ_STAGES * ATT_DQ_STAGE_BYTES;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(out + 2 * TILE_BYTES);
     uint64_t* full = bars;             // ATT_DQ_STAGES
-    uint64_t* empty = bars + 2;        // ATT_DQ_STAGES
-    uint64_t* acc_full = bars + 4;
-    uint64_t* out_full = bars + 5;     // 4 arrivals
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 6);
+    uint64_t* empty = bars + 4;        // ATT_DQ_STAGES
+    uint64_t* acc_full = bars + 8;     // 2
+    uint64_t* acc_empty = bars + 10;   // 2, four arrivals
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qb = p.nq - 1 - (int)blockIdx.y;       // heaviest query blocks of all heads first
-    const int bh = blockIdx.x;
-    const int b = bh / p.H, h = bh % p.H;
-    const int q0 = qb * ATT_BM;
-    const int niter = qb + 1;
+    const int worker = (int)blockIdx.x, workers = (int)gridDim.x;
+    auto q_block = [&](int item) { return p.nq - 1 - item / p.BH; };       // heaviest query blocks of all heads first
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < ATT_DQ_STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
-        mbar_init(acc_full, 1); mbar_init(out_full, 4);
+        for (int i = 0; i < 12; ++i) mbar_init(&bars[i], i >= 10 ? 4 : 1);
         *abort_flag = 0;
         fence_mbar_init();
     }
-    if (warp == 1) { tmem_alloc(tmem_slot, 64); tmem_relinquish(); }
+    if (warp == 1) { tmem_alloc(tmem_slot, 128); tmem_relinquish(); }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -869,15 +866,19 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         if (elect_one()) {
             bool ok = true;
             const long long nblk = (long long)p.nq * (p.nq + 1) / 2;
-            const uint8_t* src = reinterpret_cast<const uint8_t*>(p.ds) +
-                                 ((long long)bh * nblk + (long long)qb * (qb + 1) / 2) * DS_BLOCK_BYTES;
-            for (int it = 0; it < niter && ok; ++it) {
-                const int s = it % ATT_DQ_STAGES;
-                if (!mbar_wait(&empty[s], (uint32_t)((it / ATT_DQ_STAGES) & 1) ^ 1u, abort_flag)) { ok = false; break; }
-                uint8_t* st = smem + s * ATT_DQ_STAGE_BYTES;
-                mbar_expect_tx(&full[s], ATT_DQ_STAGE_BYTES);
-                bulk_load(st, src + (long long)it * DS_BLOCK_BYTES, DS_BLOCK_BYTES, &full[s]);
-                tma_load_3d(st + DS_BLOCK_BYTES, &tmK, &full[s], 0, it * ATT_BN, bh);
+            int g = 0;
+            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
+                const int qb = q_block(item), bh = item % p.BH;
+                const uint8_t* src = reinterpret_cast<const uint8_t*>(p.ds) +
+                                     ((long long)bh * nblk + (long long)qb * (qb + 1) / 2) * DS_BLOCK_BYTES;
+                for (int it = 0; it <= qb; ++it, ++g) {
+                    const int s = g % ATT_DQ_STAGES;
+                    if (!mbar_wait(&empty[s], (uint32_t)((g / ATT_DQ_STAGES) & 1) ^ 1u, abort_flag)) { ok = false; break; }
+                    uint8_t* st = smem + s * ATT_DQ_STAGE_BYTES;
+                    mbar_expect_tx(&full[s], ATT_DQ_STAGE_BYTES);
+                    bulk_load(st, src + (long long)it * DS_BLOCK_BYTES, DS_BLOCK_BYTES, &full[s]);
+                    tma_load_3d(st + DS_BLOCK_BYTES, &tmK, &full[s], 0, it * ATT_BN, bh);
+                }
             }
             pdl_launch_dependents_now();     // all loads issued: the next kernel may start its prologue
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 31); }
@@ -886,44 +887,54 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         if (elect_one()) {
             const uint32_t id_q = umma_idesc(1u, 0u, 1u, 128, 64);       // dS (K-major) x K block (MN-major)
             bool ok = true;
-            for (int it = 0; it < niter && ok; ++it) {
-                const int s = it % ATT_DQ_STAGES;
-                const uint32_t st = smem_u32(smem + s * ATT_DQ_STAGE_BYTES);
-                const uint64_t ddSk = kmajor_tile(st);
-                const uint64_t dKm = mnmajor_tile(st + DS_BLOCK_BYTES, TILE_BYTES);
-                if (!mbar_wait(&full[s], (uint32_t)((it / ATT_DQ_STAGES) & 1), abort_flag)) { ok = false; break; }
+            int g = 0;
+            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
+                const int qb = q_block(item);
+                if (!mbar_wait(&acc_empty[k & 1], (uint32_t)((k >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
                 tc_fence_after();
+                for (int it = 0; it <= qb; ++it, ++g) {
+                    const int s = g % ATT_DQ_STAGES;
+                    const uint32_t st = smem_u32(smem + s * ATT_DQ_STAGE_BYTES);
+                    const uint64_t ddSk = kmajor_tile(st);
+                    const uint64_t dKm = mnmajor_tile(st + DS_BLOCK_BYTES, TILE_BYTES);
+                    if (!mbar_wait(&full[s], (uint32_t)((g / ATT_DQ_STAGES) & 1), abort_flag)) { ok = false; break; }
+                    tc_fence_after();
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    umma_bf16(tdQ, ddSk + (uint64_t)(k >> 2) * TILESTEP + (uint64_t)(k & 3) * KSTEP, dKm + k * MNSTEP, id_q,
-                              (it > 0 || k > 0) ? 1u : 0u);
-                umma_commit(&empty[s]);
+                    for (int j = 0; j < 8; ++j)
+                        umma_bf16(tdQ + (uint32_t)((k & 1) * 64), ddSk + (uint64_t)(j >> 2) * TILESTEP + (uint64_t)(j & 3) * KSTEP,
+                                  dKm + j * MNSTEP, id_q, (it > 0 || j > 0) ? 1u : 0u);
+                    umma_commit(&empty[s]);
+                }
+                if (ok) umma_commit(&acc_full[k & 1]);
             }
-            if (ok) umma_commit(acc_full);
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 32); }
         }
     } else {
         const int q = warp & 3;
         const int r = q * 32 + lane;
-        const int qi = q0 + r;
-        const bool valid = qi < p.T;
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
         bool ok = true;
-        RopeRow rot0, rot1;                           // fetched while the products run
-        if (valid && p.dqkv != nullptr) {
-            const float* cs = p.cos_t + (long long)qi * (p.hd >> 1);
-            const float* sn = p.sin_t + (long long)qi * (p.hd >> 1);
-            load_rope_row(rot0, cs, sn, 0, p.hd);
-            load_rope_row(rot1, cs, sn, 32, p.hd);
-        }
-        if (!mbar_wait(acc_full, 0, abort_flag)) ok = false;
-        if (ok) {
+        for (int k = 0, item; (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
+            const int qb = q_block(item), bh = item % p.BH, q0 = qb * ATT_BM, qi = q0 + r;
+            const bool valid = qi < p.T;
+            RopeRow rot0, rot1;                           // fetched while the products run
+            if (valid && p.dqkv != nullptr) {
+                const float* cs = p.cos_t + (long long)qi * (p.hd >> 1);
+                const float* sn = p.sin_t + (long long)qi * (p.hd >> 1);
+                load_rope_row(rot0, cs, sn, 0, p.hd);
+                load_rope_row(rot1, cs, sn, 32, p.hd);
+            }
+            // (a thread whose wait gave up goes on with the others to the barriers below; every later wait returns at once)
+            if (!mbar_wait(&acc_full[k & 1], (uint32_t)((k >> 1) & 1), abort_flag)) { ok = false; *abort_flag = 1; }
             tc_fence_after();
             uint32_t v0[32], v1[32];
-            tmem_ld32(tdQ + lane_base, v0);
-            tmem_ld32(tdQ + lane_base + 32, v1);
+            tmem_ld32(tdQ + (uint32_t)((k & 1) * 64) + lane_base, v0);
+            tmem_ld32(tdQ + (uint32_t)((k & 1) * 64) + lane_base + 32, v1);
             tmem_ld_wait();
-            uint8_t* out = smem;                      // stage 0 is free: every product has completed
+            tc_fence_before();
+            if (q == 0 && lane == 0) tma_store_wait_read<0>();       // the previous item's rows have left the output tiles
+            asm volatile("bar.sync 1, 128;" ::: "memory");
+            if (lane == 0) mbar_arrive(&acc_empty[k & 1]);
             if (p.dqkv != nullptr) {
                 if (valid) {
                     stage_row_bf16(out, r, v0, 0, p.hd, &rot0, p.scale);
@@ -934,17 +945,15 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
                 if (p.hd > 32) stage_row_f32(out + TILE_BYTES, r, v1, p.scale);
             }
             fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(out_full);
+            asm volatile("bar.sync 1, 128;" ::: "memory");
             if (q == 0 && lane == 0) {
-                if (mbar_wait(out_full, 0, abort_flag)) {
-                    if (p.dqkv != nullptr) tma_store_4d(&tmoQ, out, 0, q0, h, b);          // rows past T are clipped
-                    else for (int c = 0; c * 32 < p.hd; ++c) tma_store_3d(&tmoQ, out + c * TILE_BYTES, c * 32, q0, bh);
-                    tma_store_commit();
-                    tma_store_wait_read<0>();
-                } else ok = false;
+                const int b = bh / p.H, h = bh % p.H;
+                if (p.dqkv != nullptr) tma_store_4d(&tmoQ, out, 0, q0, h, b);          // rows past T are clipped
+                else for (int c = 0; c * 32 < p.hd; ++c) tma_store_3d(&tmoQ, out + c * TILE_BYTES, c * 32, q0, bh);
+                tma_store_commit();
             }
         }
+        if (q == 0 && lane == 0) tma_store_wait_read<0>();
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.err, 33); }
     }
 
@@ -952,11 +961,11 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     if (*abort_flag) for (int i = 0; i < 64; ++i) __nanosleep(1000);
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) { tc_fence_after(); tmem_dealloc(tdQ, 64); }
+    if (warp == 1) { tc_fence_after(); tmem_dealloc(tdQ, 128); }
 }
 
 constexpr int ATT_DKDV_SMEM = 1024 + (8 + 2 * ATT_BWD_STAGES) * TILE_BYTES + 256;
-constexpr int ATT_DQ_SMEM = 1024 + ATT_DQ_STAGES * ATT_DQ_STAGE_BYTES;
+constexpr int ATT_DQ_SMEM = 1024 + ATT_DQ_STAGES * ATT_DQ_STAGE_BYTES + 2 * TILE_BYTES + 256;
 
 size_t attention_bwd_ds_bytes(int B, int H, int T) {
     const long long nq = (T + ATT_BM - 1) / ATT_BM;
@@ -1015,16 +1024,16 @@ int launch_attention_bwd(DeviceCtx* ctx, const bf16* Q, const bf16* K, const bf1
         ctx->launches++;
         prof_close(ctx, stream);
     }
-    dim3 grid(BH, p.nq);
+    p.BH = BH; p.items = BH * p.nq;
+    const dim3 grid((unsigned)std::min(p.items, ctx->sm_count));
     const double tri = (double)BH * T * (double)T * hd;      // one lower-triangular product = tri flops
     prof_mark(ctx, "attention_bwd_dkdv", 4.0 * tri, (double)BH * T * hd * (2.0 * 4 + 8.0), stream);
-    p.BH = BH; p.items = BH * p.nq;
-    TB_CUDA(launch_kernel(attention_bwd_dkdv_kernel, dim3((unsigned)std::min(p.items, ctx->sm_count)), dim3(ATT_BWD_THREADS), ATT_DKDV_SMEM, stream, tmQ, tmK, tmV, tmdO, tmoK, tmoV, p));
+    TB_CUDA(launch_kernel(attention_bwd_dkdv_kernel, grid, dim3(ATT_BWD_THREADS), ATT_DKDV_SMEM, stream, tmQ, tmK, tmV, tmdO, tmoK, tmoV, p));
     TB_CUDA(cudaGetLastError());
     ctx->launches++;
     prof_close(ctx, stream);
     prof_mark(ctx, "attention_bwd_dq", 1.0 * tri, (double)BH * T * hd * (2.0 * 4 + 4.0), stream);
-    TB_CUDA(launch_kernel(attention_bwd_dq_kernel, dim3(grid), dim3(ATT_DQ_THREADS), ATT_DQ_SMEM, stream, tmK, tmoQ, p));
+    TB_CUDA(launch_kernel(attention_bwd_dq_kernel, grid, dim3(ATT_DQ_THREADS), ATT_DQ_SMEM, stream, tmK, tmoQ, p));
     TB_CUDA(cudaGetLastError());
     ctx->launches++;
     prof_close(ctx, stream);
