@@ -75,7 +75,6 @@ __device__ __forceinline__ void store_chunk_bf16(uint8_t* tiles, int r, int c, c
 struct AttFwdParams {
     int T, H, hd, D;
     int nq;                 // query blocks per head
-    int BH, items;          // heads of all sequences; work items = BH * nq
     float scale_log2;       // 1/sqrt(hd) * log2(e)
     bf16* att;              // [B*T, D]
     float* lse;             // [B*H, T]
@@ -92,17 +91,7 @@ struct AttFwdParams {
 // more than 2^8 (kLazyMax), and only then is the accumulator read, rescaled and written back.  The probabilities then reach
 // 2^8 instead of 1, with the same relative error in bf16, and the row sum is kept against the same maximum.  Reading every
 // P V back and folding it in with a factor of its own, as before, was a third of a softmax warp's instructions.
-// A CTA works through several items (query block, head): a CTA per item spent 5 us outside its loop -- set-up, the first loads,
-// the last products, the store -- while here the next item's query and key tiles and its first scores are under way
-// when the softmax warps finish the item before.  Measured at 16 x 6 heads x 1024: 37.5 us with a CTA per item.
 constexpr float kLazyMax = 8.0f;        // in units of log2
-
-// Item k of worker w of n: heavy items (late query blocks) first, every second round in reverse order, so that the workers'
-// sums of half blocks differ by little; -1: no more.  All heads of a query block are adjacent.
-__device__ __forceinline__ int att_item(int k, int w, int n, int items) {
-    const int i = k * n + ((k & 1) ? n - 1 - w : w);
-    return i < items ? i : -1;
-}
 
 __global__ void __launch_bounds__(192, 2)
 attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -128,15 +117,16 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     uint64_t* p_full = bars + 11;     // 2: probability buffer b written
     uint64_t* o_full = bars + 13;     // 2: P V of a half block of parity b has been added
     uint64_t* out_full = bars + 18;   // 4 arrivals: the output tile is staged in shared memory
-    uint64_t* q_empty = bars + 15;    // 1: the item's last scores have been formed
-    uint64_t* out_done = bars + 16;   // 1: the store has read the staged output
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int worker = (int)blockIdx.x, workers = (int)gridDim.x;
-    auto q_block = [&](int item) { return p.nq - 1 - item / p.BH; };           // items: last (heaviest) query block first
-    auto half_blocks = [&](int item) { return 2 * (q_block(item) + 1); };       // key blocks 0 .. its own, two halves each
+    // blocks are handed out x fastest: all heads' heaviest (last) query block first, the lightest last,
+    // so the long CTAs start together and the short ones fill the tail
+    const int qb = p.nq - 1 - (int)blockIdx.y;
+    const int bh = blockIdx.x;
+    const int q0 = qb * ATT_BM;
+    const int nkv = qb + 1;                           // key blocks 0..qb
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
@@ -145,7 +135,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 4); mbar_init(&p_full[i], 4);
             mbar_init(&o_full[i], 1);
         }
-        mbar_init(out_full, 4); mbar_init(q_empty, 1); mbar_init(out_done, 1);
+        mbar_init(out_full, 4);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -156,27 +146,21 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();                 // everything above is independent of earlier kernels' results
     // TMEM: two score buffers of 64 key columns, the output accumulator of 64 head-dim columns
-    // Half blocks are counted through all items of the CTA (g): an item has an even number of them, so buffer b = g & 1 is also
-    // the half of the key block, and key block g >> 1 uses stage (g >> 1) & 1.
     const uint32_t tS = tmem_base, tO = tmem_base + 128;
+    const int nsub = 2 * nkv;                         // 64-key half blocks
 
     if (warp == 0) {
         if (elect_one()) {
             bool ok = true;
-            int jg = 0;
-            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
-                const int qb = q_block(item), bh = item % p.BH;
-                if (!mbar_wait(q_empty, (uint32_t)(k & 1) ^ 1u, abort_flag)) { ok = false; break; }
-                mbar_expect_tx(q_full, TILE_BYTES);
-                tma_load_3d(sQ, &tmQ, q_full, 0, qb * ATT_BM, bh);
-                for (int j = 0; j <= qb; ++j, ++jg) {
-                    const int s = jg & 1;
-                    if (!mbar_wait(&kv_empty[s], (uint32_t)((jg >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
-                    mbar_expect_tx(&k_full[s], TILE_BYTES);
-                    tma_load_3d(sK + s * TILE_BYTES, &tmK, &k_full[s], 0, j * ATT_BN, bh);
-                    mbar_expect_tx(&v_full[s], TILE_BYTES);
-                    tma_load_3d(sV + s * TILE_BYTES, &tmV, &v_full[s], 0, j * ATT_BN, bh);
-                }
+            mbar_expect_tx(q_full, TILE_BYTES);
+            tma_load_3d(sQ, &tmQ, q_full, 0, q0, bh);
+            for (int j = 0; j < nkv && ok; ++j) {
+                const int s = j & 1;
+                if (!mbar_wait(&kv_empty[s], (uint32_t)((j >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
+                mbar_expect_tx(&k_full[s], TILE_BYTES);
+                tma_load_3d(sK + s * TILE_BYTES, &tmK, &k_full[s], 0, j * ATT_BN, bh);
+                mbar_expect_tx(&v_full[s], TILE_BYTES);
+                tma_load_3d(sV + s * TILE_BYTES, &tmV, &v_full[s], 0, j * ATT_BN, bh);
             }
             pdl_launch_dependents_now();     // all loads issued: the next kernel may start its prologue
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 11); }
@@ -190,64 +174,49 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             const uint32_t idesc_o = umma_idesc(1u, 0u, 1u, ATT_BM, ATT_HD);     // P V: V is MN-major
             const uint64_t dQ = kmajor_tile(smem_u32(sQ)), dK0 = kmajor_tile(smem_u32(sK)), dP0 = kmajor_tile(smem_u32(sP));
             const uint64_t dV0 = mnmajor_tile(smem_u32(sV), TILE_BYTES);
-            bool ok = true;
-            // the scores run up to two half blocks ahead of P V, across the end of an item
-            int gs = 0, ks = 0, is = 0, ns = half_blocks(att_item(0, worker, workers, p.items));     // ns = 0: no item left
-            auto issue_scores = [&]() -> bool {
-                const int st = (gs >> 1) & 1, b = gs & 1;
-                const uint32_t par = (uint32_t)((gs >> 1) & 1);
-                if (is == 0 && !mbar_wait(q_full, (uint32_t)(ks & 1), abort_flag)) return false;
-                if (b == 0 && !mbar_wait(&k_full[st], (uint32_t)((gs >> 2) & 1), abort_flag)) return false;
-                if (!mbar_wait(&s_free[b], par ^ 1u, abort_flag)) return false;
+            bool ok = mbar_wait(q_full, 0, abort_flag);
+            auto issue_scores = [&](int i) -> bool {
+                const int j = i >> 1, st = j & 1, b = i & 1;
+                if (b == 0 && !mbar_wait(&k_full[st], (uint32_t)((j >> 1) & 1), abort_flag)) return false;
+                if (!mbar_wait(&s_free[b], (uint32_t)((i >> 1) & 1) ^ 1u, abort_flag)) return false;
                 tc_fence_after();
                 const uint64_t dK = dK0 + (uint64_t)st * TILESTEP + (uint64_t)b * (TILESTEP / 2);   // keys 64b.. of the tile
 #pragma unroll
                 for (int k = 0; k < ATT_HD / 16; ++k)
                     umma_bf16(tS + (uint32_t)(b * 64), dQ + k * KSTEP, dK + k * KSTEP, idesc_s, k > 0 ? 1u : 0u);
                 umma_commit(&s_full[b]);
-                ++gs;
-                if (++is == ns) {
-                    umma_commit(q_empty);
-                    const int item = att_item(++ks, worker, workers, p.items);
-                    is = 0; ns = item >= 0 ? half_blocks(item) : 0;
-                }
                 return true;
             };
-            for (int i = 0; i < 2 && ok && ns > 0; ++i) ok = issue_scores();
-            int g = 0;
-            for (int kp = 0, item; ok && (item = att_item(kp, worker, workers, p.items)) >= 0; ++kp) {
-                const int nsub = half_blocks(item);
-                for (int i = 0; i < nsub; ++i, ++g) {
-                    const int st = (g >> 1) & 1, b = g & 1;
-                    if (!mbar_wait(&p_full[b], (uint32_t)((g >> 1) & 1), abort_flag)) { ok = false; break; }
-                    if (b == 0 && !mbar_wait(&v_full[st], (uint32_t)((g >> 2) & 1), abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint64_t dP = dP0 + (uint64_t)b * TILESTEP;
-                    const uint64_t dV = dV0 + (uint64_t)st * TILESTEP + (uint64_t)b * (4 * MNSTEP);
+            if (ok) ok = issue_scores(0);
+            if (ok && nsub > 1) ok = issue_scores(1);
+            for (int i = 0; i < nsub && ok; ++i) {
+                const int j = i >> 1, st = j & 1, b = i & 1;
+                const uint32_t par = (uint32_t)((i >> 1) & 1);
+                if (!mbar_wait(&p_full[b], par, abort_flag)) { ok = false; break; }
+                if (b == 0 && !mbar_wait(&v_full[st], (uint32_t)((j >> 1) & 1), abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                const uint64_t dP = dP0 + (uint64_t)b * TILESTEP;
+                const uint64_t dV = dV0 + (uint64_t)st * TILESTEP + (uint64_t)b * (4 * MNSTEP);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        umma_bf16(tO, dP + k * KSTEP, dV + k * MNSTEP, idesc_o, (i | k) != 0 ? 1u : 0u);
-                    umma_commit(&o_full[b]);
-                    if (b == 1) umma_commit(&kv_empty[st]);          // both halves of the K/V tile are consumed
-                    if (ns > 0 && !issue_scores()) { ok = false; break; }
-                }
+                for (int k = 0; k < 4; ++k)
+                    umma_bf16(tO, dP + k * KSTEP, dV + k * MNSTEP, idesc_o, (i | k) != 0 ? 1u : 0u);
+                umma_commit(&o_full[b]);
+                if (b == 1) umma_commit(&kv_empty[st]);          // both halves of the K/V tile are consumed
+                if (i + 2 < nsub) ok = issue_scores(i + 2);
             }
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 12); }
         }
     } else {
         const int q = warp & 3;
         const int r = q * 32 + lane;                 // row of the tile = TMEM lane
-        const uint32_t lane_base = (uint32_t)(q * 32) << 16;
-        bool ok = true;
-        int g = 0;
-        for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
-        const int qb = q_block(item), bh = item % p.BH, q0 = qb * ATT_BM, nsub = half_blocks(item);
         const int qi = q0 + r;                       // query position
+        const uint32_t lane_base = (uint32_t)(q * 32) << 16;
         float m = -INFINITY, l = 0.0f;               // the maximum the exponentials are taken against, and their sum
+        bool ok = true;
         uint32_t va[32], vb[32];                     // one half block's scores (or the accumulator) of this row
-        for (int i = 0; i < nsub && ok; ++i, ++g) {
+        for (int i = 0; i < nsub && ok; ++i) {
             const int b = i & 1;
-            if (!mbar_wait(&s_full[b], (uint32_t)((g >> 1) & 1), abort_flag)) { ok = false; break; }
+            if (!mbar_wait(&s_full[b], (uint32_t)((i >> 1) & 1), abort_flag)) { ok = false; break; }
             tc_fence_after();
             const bool diag = ((i >> 1) == qb);
             const int k0 = (i >> 1) * ATT_BN + b * 64;
@@ -304,7 +273,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             l += (la.x + la.y) + (lb.x + lb.y);
             if (move && i > 0) {
                 // P V of the half blocks so far, against the old maximum: rescaled once the last of them has been added
-                if (!mbar_wait(&o_full[b ^ 1], (uint32_t)(((g - 1) >> 1) & 1), abort_flag)) { ok = false; break; }
+                if (!mbar_wait(&o_full[b ^ 1], (uint32_t)(((i - 1) >> 1) & 1), abort_flag)) { ok = false; break; }
                 tc_fence_after();
 #pragma unroll
                 for (int h2 = 0; h2 < 2; ++h2) {
@@ -317,11 +286,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 tmem_st_wait();
             }
             // the probabilities of two half blocks ago have been multiplied
-            if (i >= 2 && !mbar_wait(&o_full[b], (uint32_t)(((g >> 1) - 1) & 1), abort_flag)) { ok = false; break; }
-            if (i == 1 && k > 0) {                            // the previous item's output was staged in the second buffer
-                if (q == 0 && lane == 0) { tma_store_wait_read<0>(); mbar_arrive(out_done); }
-                if (!mbar_wait(out_done, (uint32_t)(k & 1) ^ 1u, abort_flag)) { ok = false; break; }
-            }
+            if (i >= 2 && !mbar_wait(&o_full[b], (uint32_t)(((i >> 1) - 1) & 1), abort_flag)) { ok = false; break; }
             store_chunk_bf16(sP, r, 2 * b, pa);
             store_chunk_bf16(sP, r, 2 * b + 1, pb);
             tc_fence_before();
@@ -329,7 +294,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             __syncwarp();
             if (lane == 0) { mbar_arrive(&s_free[b]); mbar_arrive(&p_full[b]); }
         }
-        if (ok) ok = mbar_wait(&o_full[1], (uint32_t)(((g - 1) >> 1) & 1), abort_flag);      // (g: behind the item)
+        if (ok) ok = mbar_wait(&o_full[(nsub - 1) & 1], (uint32_t)(((nsub - 1) >> 1) & 1), abort_flag);
         if (ok) {
             tc_fence_after();
             tmem_ld32(tO + lane_base, va);
@@ -337,12 +302,12 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             tmem_ld_wait();
         }
         if (ok) {
-            // O / l as bf16 into the second probability buffer (every product has completed), one TMA store for the 128
-            // rows: a thread per row storing to global memory directly touches 32 different rows per instruction
+            // O / l as bf16 into the Q tile (every product has completed), one TMA store for the 128 rows: a thread per
+            // row storing to global memory directly touches 32 different rows per instruction
             const float inv = 1.0f / l;
             const int b = bh / p.H, h = bh % p.H;
             if (qi < p.T) {
-                uint8_t* row = sP + TILE_BYTES + r * 128;
+                uint8_t* row = sQ + r * 128;
 #pragma unroll
                 for (int d = 0; d < ATT_HD; d += 8) {
                     if (d >= p.hd) break;
@@ -362,15 +327,13 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             __syncwarp();
             if (lane == 0) mbar_arrive(out_full);
             if (q == 0 && lane == 0) {
-                if (mbar_wait(out_full, (uint32_t)(k & 1), abort_flag)) {
-                    tma_store_4d(&tmO, sP + TILE_BYTES, 0, q0, h, b);          // rows past T are clipped
+                if (mbar_wait(out_full, 0, abort_flag)) {
+                    tma_store_4d(&tmO, sQ, 0, q0, h, b);          // rows past T are clipped
                     tma_store_commit();
+                    tma_store_wait_read<0>();
                 } else ok = false;
             }
-            ok = __all_sync(0xffffffffu, ok);
         }
-        }
-        if (q == 0 && lane == 0) tma_store_wait_read<0>();
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.err, 13); }
     }
 
@@ -425,10 +388,82 @@ __global__ void attention_delta_kernel(const bf16* __restrict__ att, const bf16*
     }
 }
 
+// ---- work items of the two gradient kernels
+// An item is one (key or query block, head); the grid has a CTA per item, heaviest first, all heads of a block adjacent.  A CTA
+// that has started takes over items whose CTAs have not (cluster launch control), so that the next item's loads lie under
+// this one's work, and SMs that another kernel still holds simply take no part.  The next item is asked for with the last
+// block's loads: a CTA that asks at its start takes items from SMs that are still empty (5 x 6 heads x 777: 31 us against 26).
+// One thread asks for the items and hands them to the roles of the CTA through a ring of four; -1 ends the CTA.
+constexpr int ITEM_RING = 4;
+struct ItemRing {
+    uint64_t *full, *empty, *answered;      // [ITEM_RING], [ITEM_RING], 1
+    volatile int* items;                    // [ITEM_RING]
+    uint8_t* answer;                        // 16 bytes, 16-byte aligned
+};
+__device__ __forceinline__ ItemRing item_ring(uint8_t* mem) {       // 104 bytes
+    ItemRing r;
+    r.answer = mem;
+    r.full = reinterpret_cast<uint64_t*>(mem + 16);
+    r.empty = r.full + ITEM_RING;
+    r.answered = r.empty + ITEM_RING;
+    r.items = reinterpret_cast<volatile int*>(r.answered + 1);
+    return r;
+}
+__device__ __forceinline__ void item_ring_init(const ItemRing& r, uint32_t takers) {
+    for (int i = 0; i < ITEM_RING; ++i) { mbar_init(&r.full[i], 1); mbar_init(&r.empty[i], takers); }
+    mbar_init(r.answered, 1);
+}
+// the asking thread: item k for everybody
+__device__ __forceinline__ bool item_put(const ItemRing& r, int k, int item, volatile int* abort_flag) {
+    const int s = k % ITEM_RING;
+    if (!mbar_wait(&r.empty[s], (uint32_t)((k / ITEM_RING) & 1) ^ 1u, abort_flag)) return false;
+    r.items[s] = item;
+    mbar_arrive(&r.full[s]);
+    return true;
+}
+// everybody else: item k, or -1 (also when a wait gave up: the abort flag is up then).  A warp takes it with all lanes.
+__device__ __forceinline__ int item_get(const ItemRing& r, int k, bool one_thread, volatile int* abort_flag) {
+    const int s = k % ITEM_RING;
+    if (!mbar_wait(&r.full[s], (uint32_t)((k / ITEM_RING) & 1), abort_flag)) { *abort_flag = 1; return -1; }
+    const int item = r.items[s];
+    if (!one_thread) __syncwarp();
+    if (one_thread || (threadIdx.x & 31) == 0) mbar_arrive(&r.empty[s]);
+    return item;
+}
+// asks for a CTA that has not started ..
+__device__ __forceinline__ void item_ask(const ItemRing& r) {
+    fence_proxy_async();                                 // (the last answer was read by ordinary loads)
+    mbar_expect_tx(r.answered, 16);
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+                 ::"r"(smem_u32(r.answer)), "r"(smem_u32(r.answered)) : "memory");
+}
+// .. and the answer to request number k: its index, or -1 when all have started (nothing is asked after that)
+__device__ __forceinline__ int item_answer(const ItemRing& r, int k, volatile int* abort_flag) {
+    if (!mbar_wait(r.answered, (uint32_t)(k & 1), abort_flag)) { *abort_flag = 1; return -1; }
+    uint32_t got, x;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
+        "ld.shared.b128 h, [%2];\n\t"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\tmov.b32 %1, 0;\n\t"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+        : "=r"(got), "=r"(x) : "r"(smem_u32(r.answer)) : "memory");
+    return got ? (int)x : -1;
+}
+// items = rounds of BH heads: i / BH by multiplication with ceil(2^32 / BH) where that is exact (magic != 0; a division by a
+// run-time value is ~150 clocks in front of an item's first load)
+__device__ __forceinline__ int att_round(int i, int BH, unsigned magic) {
+    return magic ? (int)__umulhi((unsigned)i, magic) : i / BH;
+}
+inline unsigned att_magic(long long BH, long long items) {
+    return (BH > 1 && BH * items < (1LL << 32)) ? (unsigned)(((1ULL << 32) + BH - 1) / BH) : 0u;
+}
+
 struct AttBwdParams {
     int T, H, hd;
     int nq;
-    int BH, items;          // heads of all sequences; work items of the dK/dV kernel = BH * nq
+    int BH;                 // heads of all sequences; work items = BH * nq
+    unsigned bh_magic;
     float scale, scale_log2;
     const float* lse;       // [B*H, T]
     const float* delta;     // [B*H, T]
@@ -544,7 +579,7 @@ constexpr int ATT_BWD_THREADS = 128 + 32 * ATT_BWD_CW;      // + TMA warp, score
 //  tensor pipe retires them while the compute warps compete for the same issue slots)
 
 // dK, dV of key blocks: an item is one key block of one head, walking the query blocks qb = kb .. nq-1; a CTA works through
-// several items (att_item: early key blocks, which have the most query blocks, first).
+// several items (early key blocks, which have the most query blocks, first).
 // What bounds it (cycle stamps, 16 x 6 heads x 1024, a block = 128 queries x 128 keys): 1,024 clocks of 2^x per block, 512 of
 // shared-memory writes of P and dS', ~1,100 from the signal that P is written to the end of the gradient products, and
 // what an item costs outside its loop.  Hence
@@ -584,13 +619,14 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     uint64_t* out_done = bars + 17;    // the store has read them
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const ItemRing ring = item_ring(reinterpret_cast<uint8_t*>(bars + 20));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int worker = (int)blockIdx.x, workers = (int)gridDim.x;
     // Blocks are counted through all items of the CTA (g); item k has nq - kb of them.
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 18; ++i) mbar_init(&bars[i], (i == 11 || i == 12 || i == 16) ? ATT_BWD_CW : i == 13 ? 2 : 1);
+        item_ring_init(ring, 3 + ATT_BWD_CW);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -606,10 +642,13 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
         if (elect_one()) {
             bool ok = true;
             int g = 0;
-            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
-                const int kb = item / p.BH, bh = item % p.BH, b = bh / p.H, h = bh % p.H;
+            for (int k = 0, item = (int)blockIdx.x; ok; ++k) {
+                if (!item_put(ring, k, item, abort_flag)) { ok = false; break; }
+                if (item < 0) break;
+                const int kb = att_round(item, p.BH, p.bh_magic), bh = item - kb * p.BH, b = bh / p.H, h = bh % p.H;
                 for (int qb = kb; qb < p.nq; ++qb, ++g) {
                     const int s = g % ATT_BWD_STAGES;
+                    if (qb == p.nq - 1) item_ask(ring);
                     if (!mbar_wait(&qdo_empty[s], (uint32_t)((g / ATT_BWD_STAGES) & 1) ^ 1u, abort_flag)) { ok = false; break; }
                     mbar_expect_tx(&qdo_full[s], 2 * TILE_BYTES);
                     tma_load_3d(sQ + s * TILE_BYTES, &tmQ, &qdo_full[s], 0, qb * ATT_BM, bh);
@@ -621,6 +660,7 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
                         tma_load_3d(sV, &tmV, kv_full, 0, kb * ATT_BN, bh);
                     }
                 }
+                if (ok) item = item_answer(ring, k, abort_flag);
             }
             pdl_launch_dependents_now();     // all loads issued: the next kernel may start its prologue
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 21); }
@@ -634,8 +674,8 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
             const uint64_t dQk0 = kmajor_tile(smem_u32(sQ)), ddOk0 = kmajor_tile(smem_u32(sdO));
             bool ok = true;
             int g = 0;
-            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
-                const int n = p.nq - item / p.BH;
+            for (int k = 0, item; ok && (item = item_get(ring, k, true, abort_flag)) >= 0; ++k) {
+                const int n = p.nq - att_round(item, p.BH, p.bh_magic);
                 if (!mbar_wait(kv_full, (uint32_t)(k & 1), abort_flag)) { ok = false; break; }
                 for (int it = 0; it < n; ++it, ++g) {
                     const int s = g % ATT_BWD_STAGES;
@@ -661,8 +701,8 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
             const uint64_t dQm0 = mnmajor_tile(smem_u32(sQ), TILE_BYTES), ddOm0 = mnmajor_tile(smem_u32(sdO), TILE_BYTES);
             bool ok = true;
             int g = 0;
-            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
-                const int n = p.nq - item / p.BH;
+            for (int k = 0, item; ok && (item = item_get(ring, k, true, abort_flag)) >= 0; ++k) {
+                const int n = p.nq - att_round(item, p.BH, p.bh_magic);
                 for (int it = 0; it < n; ++it, ++g) {
                     const int s = g % ATT_BWD_STAGES;
                     const uint64_t dQm = dQm0 + (uint64_t)s * TILESTEP, ddOm = ddOm0 + (uint64_t)s * TILESTEP;
@@ -695,8 +735,8 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
             bool ok = true;
             int g = 0;
             mbar_arrive(w_free);                      // in front of block 0: no buffer to be read out
-            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
-                const int kb = item / p.BH, bh = item % p.BH, b = bh / p.H, h = bh % p.H;
+            for (int k = 0, item; ok && (item = item_get(ring, k, true, abort_flag)) >= 0; ++k) {
+                const int kb = att_round(item, p.BH, p.bh_magic), bh = item - kb * p.BH, b = bh / p.H, h = bh % p.H;
                 for (int qb = kb; qb < p.nq; ++qb, ++g) {
                     if (!mbar_wait(ds_free, (uint32_t)(g & 1), abort_flag)) { ok = false; break; }
                     bulk_store(reinterpret_cast<uint8_t*>(p.ds) + ((long long)bh * nblk + (long long)qb * (qb + 1) / 2 + kb) * DS_BLOCK_BYTES,
@@ -737,15 +777,15 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
             const int qi = qb * ATT_BM + r;
             lse_next = INFINITY; dl_next = 0.0f;      // rows past T: P = 0
             if (qi < p.T) {
-                const long long o = (long long)(item % p.BH) * p.T + qi;
+                const long long o = (long long)(item - att_round(item, p.BH, p.bh_magic) * p.BH) * p.T + qi;
                 lse_next = p.lse[o]; dl_next = p.delta[o];
             }
         };
-        int item = att_item(0, worker, workers, p.items);
-        fetch_row(item, item / p.BH);
+        int item = item_get(ring, 0, false, abort_flag);
+        if (item >= 0) fetch_row(item, att_round(item, p.BH, p.bh_magic));
         for (int k = 0; ok && item >= 0; ++k) {
-            const int kb = item / p.BH, bh = item % p.BH, k0 = kb * ATT_BN;
-            const int next_item = att_item(k + 1, worker, workers, p.items);
+            const int kb = att_round(item, p.BH, p.bh_magic), k0 = kb * ATT_BN;
+            int next_item = -1;
             for (int qb = kb; qb < p.nq; ++qb, ++g) {
                 const uint32_t pi = (uint32_t)(g & 1);
                 const bool diag = qb == kb;
@@ -762,7 +802,8 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
                 __syncwarp();
                 if (lane == 0) mbar_arrive(sdp_free);
                 if (qb + 1 < p.nq) fetch_row(item, qb + 1);
-                else if (next_item >= 0) fetch_row(next_item, next_item / p.BH);
+                else if ((next_item = item_get(ring, k + 1, false, abort_flag)) >= 0)
+                    fetch_row(next_item, att_round(next_item, p.BH, p.bh_magic));
                 uint8_t* sdS_g = sdS + pi * DS_BLOCK_BYTES;
                 // the diagonal block masks keys after the query: columns e <= lim are allowed
                 const int lim = diag ? r - cq * 32 : 32;
@@ -822,7 +863,7 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
 
 // dQ of one query block: dQ = scale * sum over its key blocks kb = 0 .. qb of dS'(qb, kb) K(kb), the dS' blocks read
 // back as the dK/dV kernel stored them.  No exponentials and no compute warps in the loop: a loader, a tensor-core
-// issuer and four epilogue warps (thread = query row).  A CTA works through several (query block, head) items (att_item) with
+// issuer and four epilogue warps (thread = query row).  A CTA works through several (query block, head) items with
 // four stages of 48 KB running through all of them and two accumulators, so that an item's epilogue lies beside the next
 // one's loop (two CTAs per SM with an item each and two stages took 31 us at 16 x 6 heads x 1024: the set-up, first loads
 // and epilogue of an item are as long as its 4.5 blocks).  Sums are formed in key-block order: fixed, no atomics.
@@ -845,13 +886,14 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     uint64_t* acc_empty = bars + 10;   // 2, four arrivals
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const ItemRing ring = item_ring(reinterpret_cast<uint8_t*>(bars + 14));
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int worker = (int)blockIdx.x, workers = (int)gridDim.x;
-    auto q_block = [&](int item) { return p.nq - 1 - item / p.BH; };       // heaviest query blocks of all heads first
+    auto q_block = [&](int item) { return p.nq - 1 - att_round(item, p.BH, p.bh_magic); };       // heaviest query blocks of all heads first
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < 12; ++i) mbar_init(&bars[i], i >= 10 ? 4 : 1);
+        item_ring_init(ring, 5);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -867,18 +909,22 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             bool ok = true;
             const long long nblk = (long long)p.nq * (p.nq + 1) / 2;
             int g = 0;
-            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
-                const int qb = q_block(item), bh = item % p.BH;
+            for (int k = 0, item = (int)blockIdx.x; ok; ++k) {
+                if (!item_put(ring, k, item, abort_flag)) { ok = false; break; }
+                if (item < 0) break;
+                const int qb = q_block(item), bh = item - (p.nq - 1 - qb) * p.BH;
                 const uint8_t* src = reinterpret_cast<const uint8_t*>(p.ds) +
                                      ((long long)bh * nblk + (long long)qb * (qb + 1) / 2) * DS_BLOCK_BYTES;
                 for (int it = 0; it <= qb; ++it, ++g) {
                     const int s = g % ATT_DQ_STAGES;
+                    if (it == qb) item_ask(ring);
                     if (!mbar_wait(&empty[s], (uint32_t)((g / ATT_DQ_STAGES) & 1) ^ 1u, abort_flag)) { ok = false; break; }
                     uint8_t* st = smem + s * ATT_DQ_STAGE_BYTES;
                     mbar_expect_tx(&full[s], ATT_DQ_STAGE_BYTES);
                     bulk_load(st, src + (long long)it * DS_BLOCK_BYTES, DS_BLOCK_BYTES, &full[s]);
                     tma_load_3d(st + DS_BLOCK_BYTES, &tmK, &full[s], 0, it * ATT_BN, bh);
                 }
+                if (ok) item = item_answer(ring, k, abort_flag);
             }
             pdl_launch_dependents_now();     // all loads issued: the next kernel may start its prologue
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 31); }
@@ -888,7 +934,7 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
             const uint32_t id_q = umma_idesc(1u, 0u, 1u, 128, 64);       // dS (K-major) x K block (MN-major)
             bool ok = true;
             int g = 0;
-            for (int k = 0, item; ok && (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
+            for (int k = 0, item; ok && (item = item_get(ring, k, true, abort_flag)) >= 0; ++k) {
                 const int qb = q_block(item);
                 if (!mbar_wait(&acc_empty[k & 1], (uint32_t)((k >> 1) & 1) ^ 1u, abort_flag)) { ok = false; break; }
                 tc_fence_after();
@@ -914,8 +960,8 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
         const int r = q * 32 + lane;
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
         bool ok = true;
-        for (int k = 0, item; (item = att_item(k, worker, workers, p.items)) >= 0; ++k) {
-            const int qb = q_block(item), bh = item % p.BH, q0 = qb * ATT_BM, qi = q0 + r;
+        for (int k = 0, item; (item = item_get(ring, k, false, abort_flag)) >= 0; ++k) {
+            const int qb = q_block(item), bh = item - (p.nq - 1 - qb) * p.BH, q0 = qb * ATT_BM, qi = q0 + r;
             const bool valid = qi < p.T;
             RopeRow rot0, rot1;                           // fetched while the products run
             if (valid && p.dqkv != nullptr) {
@@ -964,8 +1010,8 @@ attention_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_co
     if (warp == 1) { tc_fence_after(); tmem_dealloc(tdQ, 128); }
 }
 
-constexpr int ATT_DKDV_SMEM = 1024 + (8 + 2 * ATT_BWD_STAGES) * TILE_BYTES + 256;
-constexpr int ATT_DQ_SMEM = 1024 + ATT_DQ_STAGES * ATT_DQ_STAGE_BYTES + 2 * TILE_BYTES + 256;
+constexpr int ATT_DKDV_SMEM = 1024 + (8 + 2 * ATT_BWD_STAGES) * TILE_BYTES + 384;
+constexpr int ATT_DQ_SMEM = 1024 + ATT_DQ_STAGES * ATT_DQ_STAGE_BYTES + 2 * TILE_BYTES + 384;
 
 size_t attention_bwd_ds_bytes(int B, int H, int T) {
     const long long nq = (T + ATT_BM - 1) / ATT_BM;
@@ -1024,8 +1070,8 @@ int launch_attention_bwd(DeviceCtx* ctx, const bf16* Q, const bf16* K, const bf1
         ctx->launches++;
         prof_close(ctx, stream);
     }
-    p.BH = BH; p.items = BH * p.nq;
-    const dim3 grid((unsigned)std::min(p.items, ctx->sm_count));
+    p.BH = BH; p.bh_magic = att_magic(BH, (long long)BH * p.nq);
+    const dim3 grid((unsigned)(BH * p.nq));
     const double tri = (double)BH * T * (double)T * hd;      // one lower-triangular product = tri flops
     prof_mark(ctx, "attention_bwd_dkdv", 4.0 * tri, (double)BH * T * hd * (2.0 * 4 + 8.0), stream);
     TB_CUDA(launch_kernel(attention_bwd_dkdv_kernel, grid, dim3(ATT_BWD_THREADS), ATT_DKDV_SMEM, stream, tmQ, tmK, tmV, tmdO, tmoK, tmoV, p));
@@ -1064,11 +1110,10 @@ int launch_attention_fwd(DeviceCtx* ctx, const bf16* Q, const bf16* K, const bf1
         TB_CUDA(cudaFuncSetAttribute(attention_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ATT_FWD_SMEM));
         attr_set[ctx->device & 63] = true;
     }
-    p.BH = BH; p.items = BH * p.nq;
-    const int grid = std::min(p.items, 2 * ctx->sm_count);           // two CTAs per SM
+    dim3 grid(BH, p.nq);
     // algorithmic work: the lower triangle of two products of 2*T*T*hd flops each
     prof_mark(ctx, "attention_fwd", 2.0 * (double)BH * T * (double)T * hd, (double)BH * T * hd * 2.0 * 4.0, stream);
-    TB_CUDA(launch_kernel(attention_fwd_kernel, dim3((unsigned)grid), dim3(192), ATT_FWD_SMEM, stream, tmQ, tmK, tmV, tmO, p));
+    TB_CUDA(launch_kernel(attention_fwd_kernel, dim3(grid), dim3(192), ATT_FWD_SMEM, stream, tmQ, tmK, tmV, tmO, p));
     TB_CUDA(cudaGetLastError());
     ctx->launches++;
     prof_close(ctx, stream);
