@@ -61,6 +61,13 @@ def test_attention_fwd_bwd_matches_oracle(tb, oracle, dims):
         assert rel_to_maxabs(g, want_a) <= TOL_BWD, name
 
 
+@pytest.mark.parametrize("dims", [(2, 1, 2, 8), (1, 3, 16, 40), (2, 2, 17, 32), (1, 2, 64, 64), (3, 1, 127, 64), (50, 6, 128, 64)])
+def test_attention_of_one_block(tb, oracle, dims):
+    """Sequences of up to 128 positions have a backward kernel of their own: edges of its products' 16-row steps and of
+    the block, narrow heads, more heads than fit on the device at a time."""
+    test_attention_fwd_bwd_matches_oracle(tb, oracle, dims)
+
+
 def test_attention_properties_at_benchmark_size(tb):
     """B=16, H=6, T=1024, hd=64 (the attention configuration of the benchmark): rows of P sum to 1
     (V = 1 gives O = 1), and a change in later keys/values leaves earlier outputs bit-identical."""
