@@ -88,6 +88,13 @@ def test_tf32_and_fp32_modes(tb, oracle, kind, shape):
     assert rel_to_maxabs(got, want32) <= TOL_FP32_MODE
 
 
+@pytest.mark.parametrize("kind", ["NN", "NT", "TN"])
+@pytest.mark.parametrize("shape", [(513, 1030, 44), (777, 384, 2112), (1024, 300, 2080), (2049, 700, 260), (512, 384, 2048)])
+def test_tf32_and_fp32_modes_on_pair_tiles(tb, oracle, kind, shape):
+    """Sizes at which float32 operands take 256 x 256 and 256 x 384 tiles of a CTA pair, ragged in every dimension."""
+    test_tf32_and_fp32_modes(tb, oracle, kind, shape)
+
+
 def test_modes_with_bias_residual_batch(tb, oracle):
     """Strided, batched, alpha/beta and bias+residual forms in the TF32 and FP32 modes."""
     rng = np.random.default_rng(33)

@@ -260,7 +260,7 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
         const size_t a_bytes = round_up((size_t)a_stride * batch * 2, 256);
         const size_t b_bytes = round_up((size_t)b_stride * batch * 2, 256);
         g.lda = a_ld; g.ldb = b_ld; g.strideA = a_stride; g.strideB = b_stride;
-        const int splits = residual ? 1 : choose_splits(ctx, g, (N <= 64) ? 64 : 128);
+        const int splits = planned_splits(ctx, g);
         g.splits = splits;
         const size_t ws_floats = splits > 1 ? (size_t)splits * batch * M * N : 0;
         if (a_bytes + b_bytes + ws_floats * sizeof(float) > ctx->scratch_bytes) same_b = false;      // the scratch memory moves
@@ -290,7 +290,7 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
     const size_t b_bytes = b_inplace ? 0 : round_up((size_t)b_stride * batch * 4, 256);
     if (split3) g.K = 3 * K;
     g.lda = a_ld; g.ldb = b_ld; g.strideA = a_stride; g.strideB = b_stride;
-    const int splits = residual ? 1 : choose_splits(ctx, g, (N <= 64) ? 64 : 128);
+    const int splits = planned_splits(ctx, g);
     g.splits = splits;
     const size_t ws_floats = splits > 1 ? (size_t)splits * batch * M * N : 0;
     if (a_bytes + b_bytes + ws_floats * sizeof(float) > ctx->scratch_bytes) same_b = false;      // the scratch memory moves

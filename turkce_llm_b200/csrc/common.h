@@ -177,7 +177,7 @@ bool gemm_norm_supported(const DeviceCtx* ctx, int N);
 // split-K with caller-provided partial-sum storage (needs splits*batch*M*N floats)
 int launch_gemm_bf16_ws(DeviceCtx* ctx, const GemmArgs& a, float* workspace, size_t workspace_floats,
                         cudaStream_t stream);
-int choose_splits(const DeviceCtx* ctx, const GemmArgs& a, int bn);
+int planned_splits(const DeviceCtx* ctx, const GemmArgs& a);
 // TMA map over a bf16 matrix seen as (inner, rows, batch) with a 64-element x box_rows box, 128B swizzle
 int make_operand_map(CUtensorMap* map, const bf16* ptr, long long inner, long long rows, long long ld, int batch,
                      long long batch_stride, int box_rows);

@@ -161,7 +161,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmR,
                  const GemmParams p) {
-    static_assert(!(PAIR && TF32), "CTA pairs are built for bf16 operands only");
     constexpr bool NORM = EPI == EPI_NORM;
     using Cfg = GemmCfg<BN, PAIR, NORM>;
     constexpr int STAGES = Cfg::STAGES;
@@ -271,7 +270,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     } else {
 #pragma unroll
                         for (int j = 0; j < BNL / MNW; ++j) {
-                            int n = BN == 384 ? c.n0 + 128 * j + 64 * (int)rank : nb0 + j * MNW;
+                            int n = BN == 384 ? c.n0 + 128 * (j * MNW / 64) + 64 * (int)rank + j * MNW % 64 : nb0 + j * MNW;
                             if (m_swiglu) {            // paired tile: first half gate columns, second half their up columns
                                 const int jj = (int)rank * (BNL / MNW) + j;      // box index inside the whole tile
                                 n = (c.n0 >> 1) + (jj < BN / MNW / 2 ? jj * MNW : p.pair_off + (jj - BN / MNW / 2) * MNW);
@@ -300,8 +299,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             constexpr int UMMA_N = BN == 384 ? 128 : BN;       // columns per tensor-core instruction
             constexpr int NSUB = BN / UMMA_N;
             const uint32_t idesc = umma_idesc(TF32 ? 2u : 1u, (uint32_t)p.a_mn, (uint32_t)p.b_mn, TILE_M, UMMA_N);
-            // (BN = 384: instruction j takes the j-th 64-column box of B in either CTA and accumulator columns 128 j ..)
-            constexpr uint64_t B_SUB_STEP = (uint64_t)(MN_BOX_BYTES >> 4);
+            // (BN = 384: instruction j takes the j-th 64 columns of B in either CTA and accumulator columns 128 j ..)
+            constexpr uint64_t B_SUB_STEP = (uint64_t)((64 / MNW * MN_BOX_BYTES) >> 4);
             // Shared-memory descriptors are built once: the descriptor of stage 0, the step between stages
             // and the step between the four UMMAs of a K slice are all that changes (the start address sits
             // in the low 14 bits, in 16-byte units, and never carries out of them below 256 KB).  One thread
@@ -335,13 +334,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     tc_fence_after();
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {          // 4 UMMAs of 32 bytes of K per 128-byte slice
-                        if (TF32)      umma_tf32(d_tmem, a_desc + k * a_kstep, b_desc + k * b_kstep, idesc, (kb > c.kb0 || k > 0) ? 1u : 0u);
-                        else if (PAIR) {
+                        if (PAIR) {
 #pragma unroll
-                            for (int j = 0; j < NSUB; ++j)
-                                umma_bf16_pair(d_tmem + (uint32_t)(j * UMMA_N), a_desc + k * a_kstep, b_desc + k * b_kstep + j * B_SUB_STEP,
-                                               idesc, (kb > c.kb0 || k > 0) ? 1u : 0u);
+                            for (int j = 0; j < NSUB; ++j) {
+                                const uint32_t d = d_tmem + (uint32_t)(j * UMMA_N), acc = (kb > c.kb0 || k > 0) ? 1u : 0u;
+                                if (TF32) umma_tf32_pair(d, a_desc + k * a_kstep, b_desc + k * b_kstep + j * B_SUB_STEP, idesc, acc);
+                                else      umma_bf16_pair(d, a_desc + k * a_kstep, b_desc + k * b_kstep + j * B_SUB_STEP, idesc, acc);
+                            }
                         }
+                        else if (TF32) umma_tf32(d_tmem, a_desc + k * a_kstep, b_desc + k * b_kstep, idesc, (kb > c.kb0 || k > 0) ? 1u : 0u);
                         else           umma_bf16(d_tmem, a_desc + k * a_kstep, b_desc + k * b_kstep, idesc, (kb > c.kb0 || k > 0) ? 1u : 0u);
                     }
                     if (PAIR) umma_commit_pair(&empty_bar[stage]);   // stage reusable (in both CTAs) once these MMAs have read it
@@ -1282,7 +1283,7 @@ static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
     // (flops per operand byte: 43 for 128x64, 64 for 128x128, 77 for 128x192, 128 for a CTA pair on 256x256).
     // 256 = a CTA pair on a 256 x 256 tile: per output element a CTA pulls 0.6x the operand bytes of a
     // 128 x 192 tile through its L2 port (the limit of the main loop); its waves are counted in CTA pairs.
-    const bool pair_ok = !a.tf32 && a.batch == 1 && a.causal == CAUSAL_NONE && a.c_inner <= 1 && a.M >= 512 &&
+    const bool pair_ok = a.batch == 1 && a.causal == CAUSAL_NONE && a.c_inner <= 1 && a.M >= 512 &&
                          getenv("TB_GEMM_NO_PAIR") == nullptr;
     const long long mt = (a.M + BM - 1) / BM;
     auto cost_of = [&](int width) -> double {
@@ -1291,7 +1292,7 @@ static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
             const long long tiles = ((a.M + 2 * BM - 1) / (2 * BM)) * ((a.N + 255) / 256);
             const long long pairs = ctx->sm_count / 2;
             // a narrow output wastes part of the second 256-wide column of tiles; only a long K loop pays for that
-            const double narrow = (a.N < 512 && a.K < 4096) ? 1.15 : 1.0;
+            const double narrow = (a.N < 512 && a.K < 64 * (a.tf32 ? BK_TF32 : BK)) ? 1.15 : 1.0;
             return (double)((tiles + pairs - 1) / pairs) * 256 * factor[3] * narrow;
         }
         const long long tiles = mt * ((a.N + width - 1) / width) * a.batch;
@@ -1303,9 +1304,14 @@ static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
     if (a.dsw_dgu) return (a.bn == 256 || (a.bn == 0 && pair_ok)) ? 256 : 128;      // its chunks leave in pairs
     if (a.ce_mode != 0) return a.bn == 256 ? 256 : 192;     // the statistics are laid out per tile of this width
     if (a.bn == 64 || a.bn == 128 || a.bn == 192 || a.bn == 256 || a.bn == 384) return a.bn;
-    // one 256 x 384 pair tile over the whole N where K is long (the LM-head gradients: dE 225 -> ~125 us)
-    if (pair_ok && a.kind != GEMM_NT && a.N > 256 && a.N <= 384 && a.K >= 4096 && !a.swiglu_h && !a.rope_qkv &&
-        getenv("TB_GEMM_NO_384") == nullptr)
+    // one 256 x 384 pair tile over the whole N where every pair gets a long main loop (the LM-head gradients: dE 225 -> ~125 us,
+    // with float32 operands 218 -> 149).  The line is at 30 K slices per pair: its tiles are few, so short products are
+    // split many times along K and pay in the reduction (us, this tile against the rule below, slices per pair in brackets:
+    // 1024 x 384 x 3584 tf32 20.4 : 15.6 [6], 2048 x 384 x 4096 bf16 25.3 : 21.4 [7], tf32 21.1 : 19.5 [14], 1024 x 384 x 3584
+    // in three tf32 products 38.3 : 35.7 [18], 2048 x 384 x 4096 66.8 : 76.3 [42])
+    const long long kb = (a.K + (a.tf32 ? BK_TF32 : BK) - 1) / (a.tf32 ? BK_TF32 : BK);
+    if (pair_ok && a.kind != GEMM_NT && a.N > 256 && a.N <= 384 && kb >= 64 && !a.swiglu_h && !a.rope_qkv &&
+        ((a.M + 2 * BM - 1) / (2 * BM)) * kb >= 30LL * (ctx->sm_count / 2) && getenv("TB_GEMM_NO_384") == nullptr)
         return 384;
     if (a.N <= 64) return 64;
     const long long t128 = mt * ((a.N + 127) / 128) * a.batch;
@@ -1327,7 +1333,7 @@ static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
     return best;
 }
 
-int choose_splits(const DeviceCtx* ctx, const GemmArgs& a, int bn) {
+static int choose_splits(const DeviceCtx* ctx, const GemmArgs& a, int bn) {
     if (a.causal != CAUSAL_NONE) return 1;
     const int tile_m = bn >= 256 ? 2 * BM : BM;                     // a CTA pair owns 256 rows
     const int sms = (a.max_ctas > 0 && a.max_ctas < ctx->sm_count) ? a.max_ctas : ctx->sm_count;
@@ -1341,6 +1347,10 @@ int choose_splits(const DeviceCtx* ctx, const GemmArgs& a, int bn) {
     if (s < 1) s = 1;
     const int kb_per = (kb_total + s - 1) / s;
     return (kb_total + kb_per - 1) / kb_per;     // no empty split
+}
+
+int planned_splits(const DeviceCtx* ctx, const GemmArgs& a) {
+    return (a.residual || a.c_inner > 1) ? 1 : choose_splits(ctx, a, pick_bn(ctx, a));
 }
 
 template <int BN, bool TF32, bool PAIR = false, int EPI = EPI_ANY>
@@ -1457,8 +1467,8 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
     else       TB_TRY(make_operand_map_es(&tmA, a.A, es, a.M, a.K, a.lda, a.batch, a.strideA, bke, true));
     const bool pair = bn == 256 || bn == 384;
     if (pair)
-        TB_CHECK(!a.tf32 && a.batch == 1 && a.causal == CAUSAL_NONE && a.c_inner <= 1,
-                 "256-wide CTA-pair tiles take one plain bf16 product (no batch, no causal mode)");
+        TB_CHECK(a.batch == 1 && a.causal == CAUSAL_NONE && a.c_inner <= 1,
+                 "256-wide CTA-pair tiles take one plain product (no batch, no causal mode)");
     if (bn == 384)
         TB_CHECK(b_mn && !a.swiglu_h && a.ce_mode == 0 && !a.rope_qkv,
                  "384-wide CTA-pair tiles take B stored [K, N] (kinds NN and TN) and a plain epilogue");
@@ -1610,10 +1620,6 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         else if (bn == 128) TB_TRY(TB_NORM_LAUNCH(128));
         else                TB_TRY(TB_NORM_LAUNCH(192));
 #undef TB_NORM_LAUNCH
-    } else if (pair && bn == 384) {
-        TB_TRY((launch_bf16<384, true>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
-    } else if (pair) {
-        TB_TRY((launch_bf16<256, true>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
     } else if (a.tf32) {
         // (float32 operands read as tf32: plain float32 / bf16 tiles have instantiations of their own, the rest is general)
         static const bool general_only = getenv("TB_GEMM_GENERAL_KERNEL") != nullptr;
@@ -1622,10 +1628,20 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         (epi == EPI_F32    ? launch_impl<W, true, false, EPI_F32>(ctx, a, p, tmA, tmB, tmC, tmR, stream)                 \
          : epi == EPI_BF16 ? launch_impl<W, true, false, EPI_BF16>(ctx, a, p, tmA, tmB, tmC, tmR, stream)                \
                            : launch_impl<W, true, false, EPI_ANY>(ctx, a, p, tmA, tmB, tmC, tmR, stream))
+#define TB_TF32_PAIR(W)                                                                                                \
+        (epi == EPI_F32 ? launch_impl<W, true, true, EPI_F32>(ctx, a, p, tmA, tmB, tmC, tmR, stream)                     \
+                        : launch_impl<W, true, true, EPI_ANY>(ctx, a, p, tmA, tmB, tmC, tmR, stream))
         if (bn == 64)       TB_TRY(TB_TF32_LAUNCH(64));
         else if (bn == 192) TB_TRY(TB_TF32_LAUNCH(192));
+        else if (bn == 256) TB_TRY(TB_TF32_PAIR(256));
+        else if (bn == 384) TB_TRY(TB_TF32_PAIR(384));
         else                TB_TRY(TB_TF32_LAUNCH(128));
 #undef TB_TF32_LAUNCH
+#undef TB_TF32_PAIR
+    } else if (pair && bn == 384) {
+        TB_TRY((launch_bf16<384, true>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
+    } else if (pair) {
+        TB_TRY((launch_bf16<256, true>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
     } else {
         if (bn == 64)       TB_TRY((launch_bf16<64, false>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
         else if (bn == 192) TB_TRY((launch_bf16<192, false>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
