@@ -265,6 +265,25 @@ def test_positions_of_sequences_that_end_inside_a_tile(tb, oracle, cfg):
     g.destroy()
 
 
+@pytest.mark.parametrize("cfg", [(4097, 64, 2, 1, 64, 1, 1, 1e-5), (5003, 128, 2, 1, 64, 77, 5, 1e-5), (32768, 64, 1, 1, 64, 50, 3, 1e-5)],
+                         ids=["one_row", "several_rows_per_cta", "widest"])
+def test_tf32_cross_entropy_of_whole_rows_and_rotation(tb, oracle, cfg):
+    """TF32: the cross-entropy kernel that holds a row of logits (edges of its vocabulary range), and the QKV epilogue."""
+    from turkce_llm_b200.gpu_train import GRADS
+    V, D, H, L, F, T, B, eps = cfg
+    g, p, off, num = make_params(oracle, cfg, 3, tb.PREC_TF32)
+    rng = np.random.default_rng(4)
+    ids, tgt = (rng.integers(0, V, B * T).astype(np.uint32) for _ in range(2))
+    g.upload(p)
+    loss = g.forward_backward(ids, tgt)
+    grads = g.download(GRADS)
+    want_loss, want_grads, _ = oracle.model_forward_backward(cfg, p, ids, tgt, mode=FP32)
+    assert abs(loss - want_loss) <= 1e-4 * abs(want_loss)
+    for i, (o, n) in enumerate(zip(off, num)):
+        assert compare_tensor_bad(grads[o:o + n], want_grads[o:o + n], GRAD_TOL) == 0, "parameter %d" % i
+    g.destroy()
+
+
 @pytest.mark.parametrize("precision", ["bf16", "tf32"])
 @pytest.mark.parametrize("cfg", [(97, 384, 6, 2, 256, 256, 40, 1e-5),      # more row blocks than clusters at once
                                  (97, 256, 4, 2, 64, 33, 5, 1e-5),         # rows that end inside a 32-row strip

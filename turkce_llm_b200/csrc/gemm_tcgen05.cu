@@ -1422,11 +1422,11 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
     TB_CHECK(a.A && a.B && (a.C32 || a.C16 || a.swiglu_h || a.ce_mode == 1 || a.rope_qkv || a.dsw_dgu),
              "GEMM needs A, B and at least one output");
     if (a.rope_qkv) {
-        TB_CHECK(a.kind == GEMM_NN && !a.tf32 && a.batch == 1 && splits == 1 && a.alpha == 1.0f && a.beta == 0.0f &&
+        TB_CHECK(a.kind == GEMM_NN && a.batch == 1 && splits == 1 && a.alpha == 1.0f && a.beta == 0.0f &&
                      !a.residual && !a.C32 && !a.C16 && !a.swiglu_h && a.ce_mode == 0 && a.causal == CAUSAL_NONE &&
                      a.rope_cos && a.rope_sin && (a.rope_hd == 32 || a.rope_hd == 64) && a.rope_T > 0 &&
                      a.M % a.rope_T == 0 && a.N == 3 * a.rope_H * a.rope_hd && aligned16(a.rope_qkv) && aligned16(a.rope_k) && aligned16(a.rope_v),
-                 "fused QKV + position-embedding GEMM: needs a plain NN bf16 product with N = 3*H*hd, hd 32 or 64");
+                 "fused QKV + position-embedding GEMM: needs a plain NN product with N = 3*H*hd, hd 32 or 64");
     }
     if (a.ce_mode != 0) {
         TB_CHECK(a.kind == GEMM_NT && !a.tf32 && a.batch == 1 && (bn == 192 || bn == 256) && splits == 1 && a.alpha == 1.0f &&
@@ -1621,7 +1621,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         else                TB_TRY(TB_NORM_LAUNCH(192));
 #undef TB_NORM_LAUNCH
     } else if (a.tf32) {
-        // (float32 operands read as tf32: plain float32 / bf16 tiles have instantiations of their own, the rest is general)
+        // (float32 operands read as tf32: plain float32 / bf16 tiles and the QKV epilogue have instantiations of their own, the rest is general)
         static const bool general_only = getenv("TB_GEMM_GENERAL_KERNEL") != nullptr;
         const int epi = general_only ? EPI_ANY : p.tma_mode == 1 ? EPI_F32 : (p.tma_mode == 2 && p.ce_mode == 0 && !p.dsw) ? EPI_BF16 : EPI_ANY;
 #define TB_TF32_LAUNCH(W)                                                                                              \
@@ -1635,6 +1635,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         else if (bn == 192) TB_TRY(TB_TF32_LAUNCH(192));
         else if (bn == 256) TB_TRY(TB_TF32_PAIR(256));
         else if (bn == 384) TB_TRY(TB_TF32_PAIR(384));
+        else if (p.tma_mode == 5 && !general_only) TB_TRY((launch_impl<128, true, false, EPI_ROPE>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
         else                TB_TRY(TB_TF32_LAUNCH(128));
 #undef TB_TF32_LAUNCH
 #undef TB_TF32_PAIR

@@ -233,7 +233,8 @@ int forward(TbTrainer* g, bool want_grad) {
         if (g->fused_rope) {
             // QKV projection; q and k rotated and all three stored per head as bf16 by the GEMM epilogue
             GemmArgs s;
-            s.kind = GEMM_NN; s.A = a.n1; s.B = P16(g, pidx(l, PK_WQKV)); s.M = N; s.N = 3 * D; s.K = D; s.lda = D;
+            s.kind = GEMM_NN; s.A = g->tf32 ? (const void*)a.n1_32 : (const void*)a.n1; s.B = WOP(g, pidx(l, PK_WQKV)); s.tf32 = g->tf32;
+            s.M = N; s.N = 3 * D; s.K = D; s.lda = D;
             s.ldb = 3 * D; s.bias = P32(g, pidx(l, PK_BQKV)); s.splits = 1;
             s.rope_qkv = a.Q; s.rope_cos = g->cos_t; s.rope_sin = g->sin_t; s.rope_T = T; s.rope_H = H; s.rope_hd = hd;
             if (const char* e = getenv("TB_ROPE_BN")) s.bn = atoi(e);
@@ -623,7 +624,7 @@ int tb_trainer_create_prec(TbTrainer** out, int V, int D, int H, int L, int F, i
     TB_CHECK(!g->tf32 || g->fused_attention, "the TF32 mode needs head_dim <= 64 (the attention core is the fused bf16 kernel)");
     g->fused_swiglu = !g->tf32 && F % 64 == 0 && getenv("TB_NO_FUSED_SWIGLU") == nullptr;
     g->fused_dswiglu = g->fused_swiglu && getenv("TB_NO_FUSED_DSWIGLU") == nullptr;
-    g->fused_rope = !g->tf32 && (D / H == 32 || D / H == 64) && getenv("TB_NO_FUSED_ROPE") == nullptr;
+    g->fused_rope = (D / H == 32 || D / H == 64) && getenv("TB_NO_FUSED_ROPE") == nullptr;
     // (parameters start at multiples of 8 scalars in the flat buffers: d_model, d_ff and head_dim are multiples of 8)
     g->fused_norm = gemm_norm_supported(g->ctx, D) && getenv("TB_NO_FUSED_NORM") == nullptr;
     g->V = V; g->D = D; g->H = H; g->L = L; g->F = F; g->T = T; g->B = B; g->N = B * T; g->hd = D / H;
