@@ -55,23 +55,6 @@ __device__ __forceinline__ float fast_exp2(float x) {
 __device__ __forceinline__ float2 pair_of(uint32_t a, uint32_t b) { return make_float2(__uint_as_float(a), __uint_as_float(b)); }
 
 
-// 32 consecutive values of row r -> bf16 in a [128 x 128] operand stored as two [128 x 64] tiles
-__device__ __forceinline__ void store_chunk_bf16(uint8_t* tiles, int r, int c, const float (&x)[32]) {
-    uint8_t* row = tiles + (c >> 1) * TILE_BYTES + r * 128;
-#pragma unroll
-    for (int g = 0; g < 4; ++g) {
-        uint4 pk;
-        __nv_bfloat162 h0 = __floats2bfloat162_rn(x[8 * g + 0], x[8 * g + 1]);
-        __nv_bfloat162 h1 = __floats2bfloat162_rn(x[8 * g + 2], x[8 * g + 3]);
-        __nv_bfloat162 h2 = __floats2bfloat162_rn(x[8 * g + 4], x[8 * g + 5]);
-        __nv_bfloat162 h3 = __floats2bfloat162_rn(x[8 * g + 6], x[8 * g + 7]);
-        pk.x = *reinterpret_cast<uint32_t*>(&h0); pk.y = *reinterpret_cast<uint32_t*>(&h1);
-        pk.z = *reinterpret_cast<uint32_t*>(&h2); pk.w = *reinterpret_cast<uint32_t*>(&h3);
-        const int chunk = (c & 1) * 4 + g;
-        *reinterpret_cast<uint4*>(row + ((chunk ^ (r & 7)) << 4)) = pk;
-    }
-}
-
 struct AttFwdParams {
     int T, H, hd, D;
     int nq;                 // query blocks per head
@@ -82,18 +65,21 @@ struct AttFwdParams {
 };
 
 // ------------------------------------------------------------------------------------ forward
-// CTA = 6 warps: TMA producer, MMA issuer (owns TMEM: two score buffers of 64 key columns and the output accumulator of
-// 64 head-dim columns), four softmax warps (thread = query row).  Keys are taken in half blocks of 64 and the steps are
-// software-pipelined: while the softmax warps work on half block i, the tensor core computes the scores of i+1 and adds
-// P V of i-1.  Two CTAs fit per SM on top of that.
-// The softmax warps bound the kernel (a half block of a CTA is 8192 exponentials, 512 clocks at 16 per clock), so the running
-// output stays in tensor memory: the row maximum that the exponentials are taken against is only moved when it has grown by
-// more than 2^8 (kLazyMax), and only then is the accumulator read, rescaled and written back.  The probabilities then reach
-// 2^8 instead of 1, with the same relative error in bf16, and the row sum is kept against the same maximum.  Reading every
-// P V back and folding it in with a factor of its own, as before, was a third of a softmax warp's instructions.
+// CTA = 10 warps: TMA producer, MMA issuer (owns TMEM), and two groups of four softmax warps (thread = query row).  Keys are
+// taken in half blocks of 64: group b takes the half blocks of parity b, with a score buffer, a probability buffer, a running
+// maximum, a sum and an output accumulator of its own; the two are put together at the end.  While a group works on its half
+// block, the tensor core forms the scores of its next one (the buffer is free as soon as the scores are in registers) and
+// adds P V of its last one.  Two CTAs fit per SM on top of that.
+// A half block is a chain of score load, maximum, exponentials, stores and a round trip through the tensor core, ~2,500 clocks
+// for 512 of the 2^x unit, so what counts is the number of chains side by side: with one group per CTA (two warps per
+// scheduler) 16 x 6 heads x 1024 took 35.0 us, 5 x 6 x 777 16.3; now 30.4 and 13.9.
+// The running output stays in tensor memory: the row maximum that the exponentials are taken against is only moved when it
+// has grown by more than 2^8 (kLazyMax), and only then is the accumulator read, rescaled and written back.  The probabilities
+// then reach 2^8 instead of 1, with the same relative error in bf16, and the row sum is kept against the same maximum.
 constexpr float kLazyMax = 8.0f;        // in units of log2
 
-__global__ void __launch_bounds__(192, 2)
+constexpr int ATT_FWD_THREADS = 320;
+__global__ void __launch_bounds__(ATT_FWD_THREADS, 2)
 attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
                      const AttFwdParams p) {
@@ -115,8 +101,8 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     uint64_t* s_full = bars + 7;      // 2: score buffer b holds Q K^T of a 64-key half block
     uint64_t* s_free = bars + 9;      // 2
     uint64_t* p_full = bars + 11;     // 2: probability buffer b written
-    uint64_t* o_full = bars + 13;     // 2: P V of a half block of parity b has been added
-    uint64_t* out_full = bars + 18;   // 4 arrivals: the output tile is staged in shared memory
+    uint64_t* o_full = bars + 13;     // 2: P V of a half block of parity b has been added to its accumulator
+    uint64_t* out_full = bars + 18;   // 8 arrivals: the output tile is staged in shared memory
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -135,7 +121,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 4); mbar_init(&p_full[i], 4);
             mbar_init(&o_full[i], 1);
         }
-        mbar_init(out_full, 4);
+        mbar_init(out_full, 8);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -145,7 +131,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();                 // everything above is independent of earlier kernels' results
-    // TMEM: two score buffers of 64 key columns, the output accumulator of 64 head-dim columns
+    // TMEM: two score buffers of 64 key columns, two output accumulators of 64 head-dim columns
     const uint32_t tS = tmem_base, tO = tmem_base + 128;
     const int nsub = 2 * nkv;                         // 64-key half blocks
 
@@ -167,9 +153,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
     } else if (warp == 1) {
         if (elect_one()) {
-            // Half blocks of 64 keys, software-pipelined: the scores of half block i+2 are issued as soon
-            // as the softmax warps have drained buffer i&1, so the tensor core works on Q K^T (i+1, i+2)
-            // and P V (i-1) while the softmax of i runs -- no step waits for a full round trip.
+            // the scores of half block i+2 are issued as soon as its group has drained the buffer, while it works on i
             const uint32_t idesc_s = umma_idesc(1u, 0u, 0u, ATT_BM, 64);         // Q K^T: both K-major
             const uint32_t idesc_o = umma_idesc(1u, 0u, 1u, ATT_BM, ATT_HD);     // P V: V is MN-major
             const uint64_t dQ = kmajor_tile(smem_u32(sQ)), dK0 = kmajor_tile(smem_u32(sK)), dP0 = kmajor_tile(smem_u32(sP));
@@ -192,6 +176,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             for (int i = 0; i < nsub && ok; ++i) {
                 const int j = i >> 1, st = j & 1, b = i & 1;
                 const uint32_t par = (uint32_t)((i >> 1) & 1);
+                if (i + 2 < nsub && !issue_scores(i + 2)) { ok = false; break; }
                 if (!mbar_wait(&p_full[b], par, abort_flag)) { ok = false; break; }
                 if (b == 0 && !mbar_wait(&v_full[st], (uint32_t)((j >> 1) & 1), abort_flag)) { ok = false; break; }
                 tc_fence_after();
@@ -199,49 +184,50 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 const uint64_t dV = dV0 + (uint64_t)st * TILESTEP + (uint64_t)b * (4 * MNSTEP);
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    umma_bf16(tO, dP + k * KSTEP, dV + k * MNSTEP, idesc_o, (i | k) != 0 ? 1u : 0u);
+                    umma_bf16(tO + (uint32_t)(b * 64), dP + k * KSTEP, dV + k * MNSTEP, idesc_o, (i > 1 || k > 0) ? 1u : 0u);
                 umma_commit(&o_full[b]);
                 if (b == 1) umma_commit(&kv_empty[st]);          // both halves of the K/V tile are consumed
-                if (i + 2 < nsub) ok = issue_scores(i + 2);
             }
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 12); }
         }
     } else {
         const int q = warp & 3;
+        const int b = (warp - 2) >> 2;               // this group's half blocks: i = b, b + 2, ..
         const int r = q * 32 + lane;                 // row of the tile = TMEM lane
         const int qi = q0 + r;                       // query position
         const uint32_t lane_base = (uint32_t)(q * 32) << 16;
+        const uint32_t ts = tS + lane_base + (uint32_t)(b * 64), to = tO + lane_base + (uint32_t)(b * 64);
         float m = -INFINITY, l = 0.0f;               // the maximum the exponentials are taken against, and their sum
         bool ok = true;
-        uint32_t va[32], vb[32];                     // one half block's scores (or the accumulator) of this row
-        for (int i = 0; i < nsub && ok; ++i) {
-            const int b = i & 1;
-            if (!mbar_wait(&s_full[b], (uint32_t)((i >> 1) & 1), abort_flag)) { ok = false; break; }
+        uint32_t v[2][32];                           // one half block's scores (or the accumulators) of this row
+        for (int j = 0; j < nkv && ok; ++j) {
+            if (!mbar_wait(&s_full[b], (uint32_t)(j & 1), abort_flag)) { ok = false; break; }
             tc_fence_after();
-            const bool diag = ((i >> 1) == qb);
-            const int k0 = (i >> 1) * ATT_BN + b * 64;
-            const uint32_t ts = tS + lane_base + (uint32_t)(b * 64);
-            // all 64 scores of the row in one TMEM round trip; the registers are reused for the probabilities
-            tmem_ld32(ts, va);
-            tmem_ld32(ts + 32, vb);
+            // all 64 scores of the row in one TMEM round trip, then the buffer is free
+            tmem_ld32(ts, v[0]);
+            tmem_ld32(ts + 32, v[1]);
             tmem_ld_wait();
-            const int lim = diag ? qi - k0 : 64;               // columns e <= lim are allowed
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_free[b]);
+            const bool diag = j == qb;
+            const int lim = diag ? r - b * 64 : 64;            // columns e <= lim are allowed
             float mx = -INFINITY;
             if (diag) {
 #pragma unroll
                 for (int e = 0; e < 32; ++e) {
-                    mx = fmaxf(mx, e <= lim ? __uint_as_float(va[e]) : -INFINITY);
-                    mx = fmaxf(mx, e + 32 <= lim ? __uint_as_float(vb[e]) : -INFINITY);
+                    mx = fmaxf(mx, e <= lim ? __uint_as_float(v[0][e]) : -INFINITY);
+                    mx = fmaxf(mx, e + 32 <= lim ? __uint_as_float(v[1][e]) : -INFINITY);
                 }
             } else {
                 // four chains instead of one of 32 dependent maxima
                 float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
 #pragma unroll
                 for (int e = 0; e < 32; e += 4) {
-                    m0 = fmaxf(m0, fmaxf(__uint_as_float(va[e]), __uint_as_float(vb[e])));
-                    m1 = fmaxf(m1, fmaxf(__uint_as_float(va[e + 1]), __uint_as_float(vb[e + 1])));
-                    m2 = fmaxf(m2, fmaxf(__uint_as_float(va[e + 2]), __uint_as_float(vb[e + 2])));
-                    m3 = fmaxf(m3, fmaxf(__uint_as_float(va[e + 3]), __uint_as_float(vb[e + 3])));
+                    m0 = fmaxf(m0, fmaxf(__uint_as_float(v[0][e]), __uint_as_float(v[1][e])));
+                    m1 = fmaxf(m1, fmaxf(__uint_as_float(v[0][e + 1]), __uint_as_float(v[1][e + 1])));
+                    m2 = fmaxf(m2, fmaxf(__uint_as_float(v[0][e + 2]), __uint_as_float(v[1][e + 2])));
+                    m3 = fmaxf(m3, fmaxf(__uint_as_float(v[0][e + 3]), __uint_as_float(v[1][e + 3])));
                 }
                 mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
             }
@@ -253,82 +239,93 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                 m = m_new;
             }
             const bool move = __any_sync(0xffffffffu, alpha != 1.0f);
+            // the group's last probabilities have been multiplied: their buffer is free and the accumulator is complete
+            if (j > 0 && !mbar_wait(&o_full[b], (uint32_t)((j - 1) & 1), abort_flag)) { ok = false; break; }
             // p = 2^(s*c - m), row sum, bf16 P into shared memory (K-major, 128B swizzle)
-            float pa[32], pb[32];
             const float2 c2 = make_float2(p.scale_log2, p.scale_log2), nm2 = make_float2(-m, -m);
-            float2 la = make_float2(0.f, 0.f), lb = make_float2(0.f, 0.f);
+            float2 ls[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+            uint8_t* prow = sP + b * TILE_BYTES + r * 128;
 #pragma unroll
-            for (int e = 0; e < 32; e += 2) {
-                const float2 xa = __ffma2_rn(pair_of(va[e], va[e + 1]), c2, nm2);
-                const float2 xb = __ffma2_rn(pair_of(vb[e], vb[e + 1]), c2, nm2);
-                pa[e] = fast_exp2(xa.x); pa[e + 1] = fast_exp2(xa.y);
-                pb[e] = fast_exp2(xb.x); pb[e + 1] = fast_exp2(xb.y);
-                if (diag) {
-                    pa[e] = e <= lim ? pa[e] : 0.0f;           pa[e + 1] = e + 1 <= lim ? pa[e + 1] : 0.0f;
-                    pb[e] = e + 32 <= lim ? pb[e] : 0.0f;      pb[e + 1] = e + 33 <= lim ? pb[e + 1] : 0.0f;
+            for (int c = 0; c < 2; ++c) {
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) {
+                        const int e = 8 * g + 2 * h;
+                        const float2 x = __ffma2_rn(pair_of(v[c][e], v[c][e + 1]), c2, nm2);
+                        float2 pr = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+                        if (diag) {
+                            pr.x = e + 32 * c <= lim ? pr.x : 0.0f;
+                            pr.y = e + 1 + 32 * c <= lim ? pr.y : 0.0f;
+                        }
+                        ls[h & 1] = __fadd2_rn(ls[h & 1], pr);
+                        __nv_bfloat162 hp = __floats2bfloat162_rn(pr.x, pr.y);
+                        w[h] = *reinterpret_cast<uint32_t*>(&hp);
+                    }
+                    *reinterpret_cast<uint4*>(prow + (((4 * c + g) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
-                la = __fadd2_rn(la, make_float2(pa[e], pa[e + 1]));
-                lb = __fadd2_rn(lb, make_float2(pb[e], pb[e + 1]));
             }
-            l += (la.x + la.y) + (lb.x + lb.y);
-            if (move && i > 0) {
-                // P V of the half blocks so far, against the old maximum: rescaled once the last of them has been added
-                if (!mbar_wait(&o_full[b ^ 1], (uint32_t)(((i - 1) >> 1) & 1), abort_flag)) { ok = false; break; }
+            l += (ls[0].x + ls[0].y) + (ls[1].x + ls[1].y);
+            if (move && j > 0) {
+                // P V so far, against the old maximum
                 tc_fence_after();
 #pragma unroll
                 for (int h2 = 0; h2 < 2; ++h2) {
-                    tmem_ld32(tO + lane_base + (uint32_t)(h2 * 32), va);
+                    tmem_ld32(to + (uint32_t)(h2 * 32), v[0]);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int e = 0; e < 32; ++e) va[e] = __float_as_uint(__uint_as_float(va[e]) * alpha);
-                    tmem_st32(tO + lane_base + (uint32_t)(h2 * 32), va);
+                    for (int e = 0; e < 32; ++e) v[0][e] = __float_as_uint(__uint_as_float(v[0][e]) * alpha);
+                    tmem_st32(to + (uint32_t)(h2 * 32), v[0]);
                 }
                 tmem_st_wait();
             }
-            // the probabilities of two half blocks ago have been multiplied
-            if (i >= 2 && !mbar_wait(&o_full[b], (uint32_t)(((i >> 1) - 1) & 1), abort_flag)) { ok = false; break; }
-            store_chunk_bf16(sP, r, 2 * b, pa);
-            store_chunk_bf16(sP, r, 2 * b + 1, pb);
             tc_fence_before();
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) { mbar_arrive(&s_free[b]); mbar_arrive(&p_full[b]); }
+            if (lane == 0) mbar_arrive(&p_full[b]);
         }
-        if (ok) ok = mbar_wait(&o_full[(nsub - 1) & 1], (uint32_t)(((nsub - 1) >> 1) & 1), abort_flag);
+        // every product has completed (in this order: a group is at most one half block behind the other); the probability
+        // tiles then hold the groups' maxima and sums
+        if (ok) ok = mbar_wait(&o_full[0], (uint32_t)((nkv - 1) & 1), abort_flag) && mbar_wait(&o_full[1], (uint32_t)((nkv - 1) & 1), abort_flag);
+        float2* stat = reinterpret_cast<float2*>(sP);
+        if (ok) stat[b * ATT_BM + r] = make_float2(m, l);
+        asm volatile("bar.sync 1, 256;" ::: "memory");       // (a thread whose wait gave up comes here as well)
         if (ok) {
+            // head-dim columns 32 b .. of O = (O_0 2^(m_0 - M) + O_1 2^(m_1 - M)) / l.  (m_0 is finite: key 0 is allowed.)
             tc_fence_after();
-            tmem_ld32(tO + lane_base, va);
-            tmem_ld32(tO + lane_base + 32u, vb);
+            tmem_ld32(tO + lane_base + (uint32_t)(b * 32), v[0]);
+            tmem_ld32(tO + lane_base + 64u + (uint32_t)(b * 32), v[1]);
+            const float2 s0 = stat[r], s1 = stat[ATT_BM + r];
+            const float M = fmaxf(s0.x, s1.x), e0 = fast_exp2(s0.x - M), e1 = fast_exp2(s1.x - M);
+            const float lt = s0.y * e0 + s1.y * e1, inv = 1.0f / lt;
+            const float w0 = e0 * inv, w1 = e1 * inv;
             tmem_ld_wait();
-        }
-        if (ok) {
-            // O / l as bf16 into the Q tile (every product has completed), one TMA store for the 128 rows: a thread per
-            // row storing to global memory directly touches 32 different rows per instruction
-            const float inv = 1.0f / l;
-            const int b = bh / p.H, h = bh % p.H;
+            // as bf16 into the Q tile, one TMA store for the 128 rows: a thread per row storing to global memory directly
+            // touches 32 different rows per instruction
             if (qi < p.T) {
                 uint8_t* row = sQ + r * 128;
 #pragma unroll
-                for (int d = 0; d < ATT_HD; d += 8) {
-                    if (d >= p.hd) break;
-                    float o[8];
+                for (int d = 0; d < 32; d += 8) {
+                    if (32 * b + d >= p.hd) break;
+                    uint32_t w[4];
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) o[e] = __uint_as_float(d < 32 ? va[(d + e) & 31] : vb[(d + e) & 31]) * inv;
-                    uint4 pk;
-                    __nv_bfloat162 h0 = __floats2bfloat162_rn(o[0], o[1]), h1 = __floats2bfloat162_rn(o[2], o[3]);
-                    __nv_bfloat162 h2 = __floats2bfloat162_rn(o[4], o[5]), h3 = __floats2bfloat162_rn(o[6], o[7]);
-                    pk.x = *reinterpret_cast<uint32_t*>(&h0); pk.y = *reinterpret_cast<uint32_t*>(&h1);
-                    pk.z = *reinterpret_cast<uint32_t*>(&h2); pk.w = *reinterpret_cast<uint32_t*>(&h3);
-                    *reinterpret_cast<uint4*>(row + (((d >> 3) ^ (r & 7)) << 4)) = pk;
+                    for (int e = 0; e < 4; ++e) {
+                        const int c = d + 2 * e;
+                        __nv_bfloat162 h2 = __floats2bfloat162_rn(__uint_as_float(v[0][c]) * w0 + __uint_as_float(v[1][c]) * w1,
+                                                                  __uint_as_float(v[0][c + 1]) * w0 + __uint_as_float(v[1][c + 1]) * w1);
+                        w[e] = *reinterpret_cast<uint32_t*>(&h2);
+                    }
+                    *reinterpret_cast<uint4*>(row + (((4 * b + (d >> 3)) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
-                if (p.lse) p.lse[(long long)bh * p.T + qi] = (m + log2f(l)) * 0.6931471805599453f;
+                if (p.lse && b == 0) p.lse[(long long)bh * p.T + qi] = (M + log2f(lt)) * 0.6931471805599453f;
             }
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive(out_full);
-            if (q == 0 && lane == 0) {
+            if (warp == 2 && lane == 0) {
                 if (mbar_wait(out_full, 0, abort_flag)) {
-                    tma_store_4d(&tmO, sQ, 0, q0, h, b);          // rows past T are clipped
+                    tma_store_4d(&tmO, sQ, 0, q0, bh % p.H, bh / p.H);          // rows past T are clipped
                     tma_store_commit();
                     tma_store_wait_read<0>();
                 } else ok = false;
@@ -1338,7 +1335,7 @@ int launch_attention_fwd(DeviceCtx* ctx, const bf16* Q, const bf16* K, const bf1
     dim3 grid(BH, p.nq);
     // algorithmic work: the lower triangle of two products of 2*T*T*hd flops each
     prof_mark(ctx, "attention_fwd", 2.0 * (double)BH * T * (double)T * hd, (double)BH * T * hd * 2.0 * 4.0, stream);
-    TB_CUDA(launch_kernel(attention_fwd_kernel, dim3(grid), dim3(192), ATT_FWD_SMEM, stream, tmQ, tmK, tmV, tmO, p));
+    TB_CUDA(launch_kernel(attention_fwd_kernel, dim3(grid), dim3(ATT_FWD_THREADS), ATT_FWD_SMEM, stream, tmQ, tmK, tmV, tmO, p));
     TB_CUDA(cudaGetLastError());
     ctx->launches++;
     prof_close(ctx, stream);
