@@ -31,7 +31,7 @@ namespace {
 enum { PK_ATTN_NORM = 0, PK_WQKV, PK_BQKV, PK_WO, PK_BO, PK_FFN_NORM, PK_WGU, PK_BGU, PK_WDOWN, PK_BDOWN };
 
 struct LayerActs {
-    float *n1_32 = nullptr, *n2_32 = nullptr, *h32 = nullptr;    // TF32 mode: float32 GEMM operands
+    float *n1_32 = nullptr, *n2_32 = nullptr, *h32 = nullptr, *att32 = nullptr;    // TF32 mode: float32 GEMM operands
     float* x_in;  bf16* n1; float* r1;
     bf16 *Q, *K, *V, *P, *att;     // P [BH,T,T] only on the unfused attention path
     float* lse;                    // [BH,T] on the fused path
@@ -102,7 +102,7 @@ struct TbTrainer {
     // The attention core stays the fused bf16 kernel (the reference's attention products are bf16 as well);
     // its outputs are widened.  The fused epilogues are those of the bf16 path and are switched off here.
     bool tf32 = false;
-    float *nf32 = nullptr, *dlogits32 = nullptr, *dgu32 = nullptr, *dqkv32 = nullptr, *att32 = nullptr;
+    float *nf32 = nullptr, *dlogits32 = nullptr, *dgu32 = nullptr, *dqkv32 = nullptr;
     float* att_delta = nullptr;
     bf16* att_ds = nullptr;        // dS blocks on their way from the dK/dV kernel to the dQ kernel
     bool owns_stream = false;
@@ -265,8 +265,8 @@ int forward(TbTrainer* g, bool want_grad) {
                 TB_TRY(gemm(g, o));
             }
         }
-        if (g->tf32) TB_TRY(launch_widen_bf16(c, a.att, g->att32, (long long)N * D, st));
-        TB_TRY(linear_fwd(g, g->tf32 ? (const void*)g->att32 : (const void*)a.att, WOP(g, pidx(l, PK_WO)),
+        if (g->tf32) TB_TRY(launch_widen_bf16(c, a.att, a.att32, (long long)N * D, st));
+        TB_TRY(linear_fwd(g, g->tf32 ? (const void*)a.att32 : (const void*)a.att, WOP(g, pidx(l, PK_WO)),
                           P32(g, pidx(l, PK_BO)), a.x_in, a.x2, nullptr, N, D, D,
                           g->fused_norm ? P32(g, pidx(l, PK_FFN_NORM)) : nullptr, a.n2, a.n2_32, a.r2));
         if (!g->fused_norm)
@@ -377,16 +377,15 @@ int backward_layer(TbTrainer* g, int l) {
     }
     const void* dgu_op = g->tf32 ? (const void*)g->dgu32 : (const void*)g->dgu;
     TB_TRY(linear_dw(g, g->tf32 ? (const void*)a.n2_32 : (const void*)a.n2, dgu_op, G32(g, pidx(l, PK_WGU)), N, 2 * F, D, 1));
-    if (g->fused_dswiglu) {
+    {
         // on the weight gradients' stream when the pair runs side by side (in order behind the product above and ahead
         // of the layer's last weight gradient, whose event the layer's end waits for); with a scratch buffer of its
         // own, because the main stream's column sum of dqkv may run at the same time
+        // (the unfused bf16 SwiGLU backward sums the columns itself)
         cudaStream_t cs = pair_on(g) ? g->side : st;
-        TB_TRY(launch_colsum_bf16(c, g->dgu, G32(g, pidx(l, PK_BGU)), g->colsum_partial2, N, 2 * F, cs));
-    }
-    if (!g->fused_swiglu) {
-        if (g->tf32) TB_TRY(launch_colsum_f32(c, g->dgu32, G32(g, pidx(l, PK_BGU)), g->colsum_partial, N, 2 * F, st));
-        else TB_TRY(launch_colsum_bf16(c, g->dgu, G32(g, pidx(l, PK_BGU)), g->colsum_partial, N, 2 * F, st));
+        if (g->tf32) TB_TRY(launch_colsum_f32(c, g->dgu32, G32(g, pidx(l, PK_BGU)), g->colsum_partial2, N, 2 * F, cs));
+        else if (g->fused_dswiglu || !g->fused_swiglu)
+            TB_TRY(launch_colsum_bf16(c, g->dgu, G32(g, pidx(l, PK_BGU)), g->colsum_partial2, N, 2 * F, cs));
     }
     TB_TRY(linear_dx(g, dgu_op, WOP(g, pidx(l, PK_WGU)), g->dn, nullptr, N, 2 * F, D));
     TB_TRY(pair_wait(g, 0));           // the norm backward overwrites dres16, which the down-projection's dW reads
@@ -394,8 +393,7 @@ int backward_layer(TbTrainer* g, int l) {
                                  G32(g, pidx(l, PK_FFN_NORM)), G32(g, pidx(l, PK_BO)), g->norm_scratch, N, D, 1, st));
 
     // ---- attention: x2 = x + (att @ Wo + bo); dres = dx2
-    if (g->tf32) TB_TRY(launch_widen_bf16(c, a.att, g->att32, (long long)N * D, st));
-    TB_TRY(linear_dw(g, g->tf32 ? (const void*)g->att32 : (const void*)a.att, dres_op, G32(g, pidx(l, PK_WO)), N, D, D, 2));
+    TB_TRY(linear_dw(g, g->tf32 ? (const void*)a.att32 : (const void*)a.att, dres_op, G32(g, pidx(l, PK_WO)), N, D, D, 2));
     // (bo's gradient came with dres as well)
     TB_TRY(linear_dx(g, dres_op, WOP(g, pidx(l, PK_WO)), nullptr, g->datt, N, D, D));
     if (g->fused_attention) {
@@ -438,7 +436,8 @@ int backward_layer(TbTrainer* g, int l) {
     if (g->tf32) TB_TRY(launch_widen_bf16(c, g->dqkv, g->dqkv32, (long long)N * 3 * D, st));
     const void* dqkv_op = g->tf32 ? (const void*)g->dqkv32 : (const void*)g->dqkv;
     TB_TRY(linear_dw(g, g->tf32 ? (const void*)a.n1_32 : (const void*)a.n1, dqkv_op, G32(g, pidx(l, PK_WQKV)), N, 3 * D, D, 3));
-    TB_TRY(launch_colsum_bf16(c, g->dqkv, G32(g, pidx(l, PK_BQKV)), g->colsum_partial, N, 3 * D, st));
+    TB_TRY(launch_colsum_bf16(c, g->dqkv, G32(g, pidx(l, PK_BQKV)), g->colsum_partial2, N, 3 * D, pair_on(g) ? g->side : st));
+    if (pair_on(g)) TB_CUDA(cudaEventRecord(g->ev_done[3], g->side));
     TB_TRY(linear_dx(g, dqkv_op, WOP(g, pidx(l, PK_WQKV)), g->dn, nullptr, N, 3 * D, D));
     TB_TRY(pair_wait(g, 2));           // the norm backward overwrites dres16, which the out-projection's dW reads
     TB_TRY(launch_rmsnorm_bwd_dw(c, a.x_in, P32(g, pidx(l, PK_ATTN_NORM)), a.r1, g->dn, g->dres, g->dres16,
@@ -670,13 +669,14 @@ int tb_trainer_create_prec(TbTrainer** out, int V, int D, int H, int L, int F, i
         TB_TRY(dalloc(g, &a.h, N * F));
         if (g->tf32) {
             TB_TRY(dalloc(g, &a.n1_32, N * D)); TB_TRY(dalloc(g, &a.n2_32, N * D)); TB_TRY(dalloc(g, &a.h32, N * F));
+            TB_TRY(dalloc(g, &a.att32, N * D));
         }
     }
     TB_TRY(dalloc(g, &g->x_final, N * D)); TB_TRY(dalloc(g, &g->nf, N * D)); TB_TRY(dalloc(g, &g->rf, N));
     g->fused_ce = !g->tf32 && getenv("TB_NO_FUSED_CE") == nullptr;
     if (g->tf32) {
         TB_TRY(dalloc(g, &g->nf32, N * D)); TB_TRY(dalloc(g, &g->dlogits32, N * g->Vp));
-        TB_TRY(dalloc(g, &g->dgu32, N * 2 * F)); TB_TRY(dalloc(g, &g->dqkv32, N * 3 * D)); TB_TRY(dalloc(g, &g->att32, N * D));
+        TB_TRY(dalloc(g, &g->dgu32, N * 2 * F)); TB_TRY(dalloc(g, &g->dqkv32, N * 3 * D));
         TB_CUDA(cudaMemset(g->dlogits32, 0, N * g->Vp * 4));      // the padding columns stay zero
     }
     if (g->fused_ce) {
