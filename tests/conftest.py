@@ -1,4 +1,5 @@
 import os
+import subprocess
 import sys
 
 import numpy as np
@@ -8,6 +9,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
+CSRC = os.path.join(ROOT, "turkce_llm_b200", "csrc")
 GOLDEN = os.path.join(ROOT, "tests", "golden")
 
 
@@ -59,3 +61,13 @@ def compare_tensor_bad(got, want, rel_tol):
     floor = maxabs * rel_tol + 1e-12
     tol = floor + rel_tol * np.abs(want)
     return int((np.abs(got - want) > tol).sum())
+
+
+def compile_and_run(tmp_path, source, *flags):
+    """g++ over a source that includes headers of the library; returns its output, asserts that it exits with 0."""
+    cpp, exe = tmp_path / "check.cpp", tmp_path / "check"
+    cpp.write_text(source)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-I", CSRC, *flags, "-o", str(exe), str(cpp)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+    return r.stdout
