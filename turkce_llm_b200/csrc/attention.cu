@@ -582,6 +582,10 @@ __device__ __forceinline__ void store_half_chunk(uint8_t* tiles, int r, int c, i
 
 constexpr int ATT_BWD_STAGES = 3;       // stages of the (Q, dO) pair in the dK/dV kernel
 constexpr int ATT_BWD_CW = 16;          // compute warps
+// Barriers that say "the dK products of block g have read dS'", in turn.  The store thread lets block g + 1 go on (w_free)
+// before it waits for block g, so at an item's boundary two more blocks can end before it has looked, and with one barrier it
+// would take the second one's phase for its own and wait until its limit.  It holds up the third block, so two are enough.
+constexpr int ATT_DS_FREE = 2;
 constexpr int ATT_BWD_THREADS = 128 + 32 * ATT_BWD_CW;      // + TMA warp, score-MMA warp, gradient-MMA warp, store warp
 // (two issuing threads on different schedulers: one thread cannot issue a block's 24 UMMAs as fast as the
 //  tensor pipe retires them while the compute warps compete for the same issue slots)
@@ -621,11 +625,11 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     uint64_t* sdp_free = bars + 11;    // one arrival per compute warp
     uint64_t* pds_full = bars + 12;    // one arrival per compute warp
     uint64_t* w_free = bars + 13;      // 2 arrivals: block g's dV products have read P, block g - 1's dS buffer has been read out
-    uint64_t* ds_free = bars + 14;     // the dK products of the block have read dS'
-    uint64_t* acc_full = bars + 15;    // an item's last products are done
-    uint64_t* out_full = bars + 16;    // one arrival per compute warp: an item's output tiles are staged
-    uint64_t* out_done = bars + 17;    // the store has read them
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
+    uint64_t* ds_free = bars + 14;     // ATT_DS_FREE
+    uint64_t* acc_full = bars + 14 + ATT_DS_FREE;    // an item's last products are done
+    uint64_t* out_full = bars + 17;    // one arrival per compute warp: an item's output tiles are staged
+    uint64_t* out_done = bars + 18;    // the store has read them
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const ItemRing ring = item_ring(reinterpret_cast<uint8_t*>(bars + 20));
 
@@ -633,7 +637,7 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     // Blocks are counted through all items of the CTA (g); item k has nq - kb of them.
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 18; ++i) mbar_init(&bars[i], (i == 11 || i == 12 || i == 16) ? ATT_BWD_CW : i == 13 ? 2 : 1);
+        for (int i = 0; i < 19; ++i) mbar_init(&bars[i], (i == 11 || i == 12 || i == 17) ? ATT_BWD_CW : i == 13 ? 2 : 1);
         item_ring_init(ring, 3 + ATT_BWD_CW);
         *abort_flag = 0;
         fence_mbar_init();
@@ -725,7 +729,7 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         umma_bf16(tdK, ddSm + j * MNSTEP, dQm + j * MNSTEP, id_t, (it > 0 || j > 0) ? 1u : 0u);
-                    umma_commit(ds_free);
+                    umma_commit(&ds_free[g % ATT_DS_FREE]);
                     // S and dP of this block (the other issuer's) completed before the compute warps could sign
                     // pds_full, so this commit covers every read of the stage
                     umma_commit(&qdo_empty[s]);
@@ -746,7 +750,7 @@ attention_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
             for (int k = 0, item; ok && (item = item_get(ring, k, true, abort_flag)) >= 0; ++k) {
                 const int kb = att_round(item, p.BH, p.bh_magic), bh = item - kb * p.BH, b = bh / p.H, h = bh % p.H;
                 for (int qb = kb; qb < p.nq; ++qb, ++g) {
-                    if (!mbar_wait(ds_free, (uint32_t)(g & 1), abort_flag)) { ok = false; break; }
+                    if (!mbar_wait(&ds_free[g % ATT_DS_FREE], (uint32_t)((g / ATT_DS_FREE) & 1), abort_flag)) { ok = false; break; }
                     bulk_store(reinterpret_cast<uint8_t*>(p.ds) + ((long long)bh * nblk + (long long)qb * (qb + 1) / 2 + kb) * DS_BLOCK_BYTES,
                                sdS + (g & 1) * DS_BLOCK_BYTES, DS_BLOCK_BYTES);
                     tma_store_commit();
