@@ -4,6 +4,7 @@
 // the parallel decomposition is this library's own: one warp per row with shuffle
 // reductions instead of one 256-thread block per row with shared-memory trees.
 #include "step_kernels.h"
+#include "lane_scan.h"
 #include "ptx.cuh"
 
 #include <algorithm>
@@ -897,7 +898,8 @@ int launch_argmax_rows(DeviceCtx* ctx, const float* logits, uint32_t* tok, uint3
 // the row twice with 32 cache lines per load); eight take ~5.  Thread t of CTA c owns `per` adjacent columns (an odd number,
 // so that the threads' walks through shared memory meet no bank conflicts): sums per thread, scanned over the threads,
 // the warps and the CTAs in column order.  The bounds of a thread's share of the running sum are formed so that they tile
-// [0, total] exactly, so just one thread holds r; it walks its columns and writes the token.  The writer of the last
+// [0, total] exactly and never go backwards (lane_scan.h; a sum of non-negative values rounds monotonely from there on), so
+// just one thread holds r; it walks its columns and writes the token.  The writer of the last
 // sequence (a ticket) advances the state, which everybody has read before the cluster's first meeting.
 constexpr int kSampleCtas = 8, kSampleThreads = 512;
 
@@ -947,12 +949,9 @@ sample_rows_kernel(const float* __restrict__ logits, const double* __restrict__ 
         if (staged) e_sh[j] = e;
         local += (double)e;
     }
-    double incl = local;                                  // inclusive scan inside the warp
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
-    }
+    const double incl = monotone_lane_sums(
+        local, [lane](double v, int o) { const double b = __shfl_up_sync(0xffffffffu, v, o); return lane >= o ? v + b : v; },
+        [lane](double v, int o) { const double b = __shfl_up_sync(0xffffffffu, v, o); return lane >= o && b > v ? b : v; });
     if (lane == 31) wsum[warp] = incl;
     __syncthreads();
     double wbefore = 0.0, ctotal = 0.0;
