@@ -1357,7 +1357,8 @@ cross_entropy_row_kernel(const float* __restrict__ logits, const uint32_t* __res
     for (long long row = blockIdx.x; row < rows; row += gridDim.x, phase ^= 1u) {
         const int t = (int)targets[row];
         if (!__syncthreads_and(mbar_wait(full, phase, &gave_up))) {
-            if (threadIdx.x == 0) atomicExch(err, 51);
+            if (threadIdx.x == 0) atomicExch(err, 61);
+            for (int i = 0; i < 64; ++i) __nanosleep(1000);          // the copy lands before the shared memory is released
             return;
         }
         float4 v[8];
