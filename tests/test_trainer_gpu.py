@@ -284,6 +284,19 @@ def test_tf32_cross_entropy_of_whole_rows_and_rotation(tb, oracle, cfg):
     g.destroy()
 
 
+def test_a_row_of_infinite_logits_gives_no_finite_loss(tb, oracle):
+    """Logits that are all -inf (a diverged final norm): the row has no softmax, and the columns that pad it to the threads of
+    the cross-entropy kernel must not stand in for one."""
+    cfg = V, D, H, L, F, T, B, eps = (4097, 64, 2, 1, 64, 8, 1, 1e-5)
+    g, p, off, num = make_params(oracle, cfg, 3, tb.PREC_TF32)
+    p[:V * D] = np.abs(p[:V * D]) + 0.5                      # embedding: positive, and large beside the layer's output
+    p[off[-1]] = -np.inf                                     # final norm: dimension 0
+    g.upload(p)
+    ids = np.arange(T, dtype=np.uint32)
+    assert np.isnan(g.forward_backward(ids, ids))
+    g.destroy()
+
+
 @pytest.mark.parametrize("precision", ["bf16", "tf32"])
 @pytest.mark.parametrize("cfg", [(97, 384, 6, 2, 256, 256, 40, 1e-5),      # more row blocks than clusters at once
                                  (97, 256, 4, 2, 64, 33, 5, 1e-5),         # rows that end inside a 32-row strip

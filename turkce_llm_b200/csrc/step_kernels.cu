@@ -1366,10 +1366,11 @@ cross_entropy_row_kernel(const float* __restrict__ logits, const uint32_t* __res
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int j = (threadIdx.x + k * 1024) * 4;
-            v[k] = j < V ? *reinterpret_cast<const float4*>(z + j) : make_float4(-3.0e38f, -3.0e38f, -3.0e38f, -3.0e38f);
-            if (j + 1 >= V) v[k].y = -3.0e38f;
-            if (j + 2 >= V) v[k].z = -3.0e38f;
-            if (j + 3 >= V) v[k].w = -3.0e38f;
+            // (-inf and not a large number: against the smallest maximum there is, it still counts for nothing)
+            v[k] = j < V ? *reinterpret_cast<const float4*>(z + j) : make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+            if (j + 1 >= V) v[k].y = -INFINITY;
+            if (j + 2 >= V) v[k].z = -INFINITY;
+            if (j + 3 >= V) v[k].w = -INFINITY;
             mx = fmaxf(mx, fmaxf(fmaxf(v[k].x, v[k].y), fmaxf(v[k].z, v[k].w)));
         }
         const float zt = z[t];
