@@ -68,6 +68,28 @@ def test_attention_of_one_block(tb, oracle, dims):
     test_attention_fwd_bwd_matches_oracle(tb, oracle, dims)
 
 
+@pytest.mark.parametrize("dims", [(2, 6, 1024, 64), (3, 6, 777, 64), (4, 3, 200, 32), (8, 6, 1000, 16)])
+def test_probabilities_are_rounded_against_the_rows_maximum(tb, dims):
+    """Rows in which a few keys have most of the weight (q four times as large): the largest probability is 1 and exact in
+    bf16, so what is left of the forward pass's error is mostly the rounding of its bf16 output.  That is uniform within half a
+    unit in the last place, 2^-8 of a power of two: 2^-8 / sqrt(3) times the root of the mean of 1 / m^2 over mantissas m
+    whose logarithm is uniform, 0.736, so 1.66e-3 in the 2-norm.  The roundings of P may add half as much in quadrature; with P
+    taken against an older maximum they add 0.65 times as much at 777 keys and up."""
+    B, H, T, hd = dims
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v = (torch.randn(B * H, T, hd, device="cuda", generator=gen) for _ in range(3))
+    q, k, v = (4 * q).bfloat16(), k.bfloat16(), v.bfloat16()
+    att = torch.empty(B * T, H * hd, device="cuda", dtype=torch.bfloat16)
+    lse = torch.empty(B * H, T, device="cuda")
+    tb.attention_fwd(q, k, v, att, lse, B, H, T, hd, float(hd) ** -0.5)
+    tb.sync_check()
+    s = (q.double() @ k.double().transpose(1, 2)) * float(hd) ** -0.5
+    s = s.masked_fill(torch.ones(T, T, device="cuda", dtype=torch.bool).triu(1), float("-inf"))
+    want = (s.softmax(-1) @ v.double()).view(B, H, T, hd).transpose(1, 2).reshape(B * T, H * hd)
+    output_rounding = 2.0 ** -8 / np.sqrt(3.0) * 0.736
+    assert float((att.double() - want).norm() / want.norm()) <= output_rounding * np.sqrt(1 + 0.5 ** 2)
+
+
 def test_attention_properties_at_benchmark_size(tb):
     """B=16, H=6, T=1024, hd=64 (the attention configuration of the benchmark): rows of P sum to 1
     (V = 1 gives O = 1), and a change in later keys/values leaves earlier outputs bit-identical."""

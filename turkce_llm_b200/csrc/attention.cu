@@ -72,11 +72,12 @@ struct AttFwdParams {
 // adds P V of its last one.  Two CTAs fit per SM on top of that.
 // A half block is a chain of score load, maximum, exponentials, stores and a round trip through the tensor core, ~2,500 clocks
 // for 512 of the 2^x unit, so what counts is the number of chains side by side: with one group per CTA (two warps per
-// scheduler) 16 x 6 heads x 1024 took 35.0 us, 5 x 6 x 777 16.3; now 30.4 and 13.9.
-// The running output stays in tensor memory: the row maximum that the exponentials are taken against is only moved when it
-// has grown by more than 2^8 (kLazyMax), and only then is the accumulator read, rescaled and written back.  The probabilities
-// then reach 2^8 instead of 1, with the same relative error in bf16, and the row sum is kept against the same maximum.
-constexpr float kLazyMax = 8.0f;        // in units of log2
+// scheduler) and the output sums in registers 16 x 6 heads x 1024 took 36.2 us, 5 x 6 x 777 16.2; now 31.2 and 14.0.
+// The running output stays in tensor memory and is read, rescaled and written back where the maximum of one of a warp's rows has
+// grown.  The exponentials are always taken against the maximum so far, so that the largest probability of a row is 1 and exact
+// in bf16: taken against an older maximum (rescaling only at a growth of 2^8) that one is rounded like the others, and where a
+// row has one or a few keys that matter the output is further off (2-norm against float64, 16 x 6 heads x 1024: 1.99e-3 instead
+// of 1.71e-3 with q four times as large, 2.02e-3 instead of 1.98e-3 as it is; 29.6 us instead of 31.2).
 
 constexpr int ATT_FWD_THREADS = 320;
 __global__ void __launch_bounds__(ATT_FWD_THREADS, 2)
@@ -233,7 +234,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             }
             const float m_new = fmaxf(m, mx * p.scale_log2);
             float alpha = 1.0f;
-            if (m_new > m + kLazyMax) {                       // (each row for itself: a row does not depend on its neighbours)
+            if (m_new > m) {                                 // (each row for itself: a row does not depend on its neighbours)
                 alpha = fast_exp2(m - m_new);                // 0 on the first block (m = -inf)
                 l *= alpha;
                 m = m_new;
