@@ -8,112 +8,25 @@
 // as it would for the bus).  They are made on the first large transfer, hold 2 x 512 KB per thread whatever the size of a
 // transfer, and are given back by tb_shutdown or when the process ends.
 #include "common.h"
+#include "copy_helpers.h"
 
 #include <algorithm>
 #include <atomic>
-#include <chrono>
-#include <condition_variable>
 #include <cstring>
 #include <functional>
 #include <mutex>
-#include <system_error>
-#include <thread>
 #include <vector>
-
-#include <unistd.h>
 
 namespace tb {
 
 namespace {
 
-constexpr int kCopyThreads = 4;                       // the caller and three helpers: 64 GB/s between them, more gained nothing
+constexpr int kCopyThreads = kHelperSlots;
 constexpr size_t kPiece = 512 * 1024;
 constexpr size_t kThreadedFrom = 1024 * 1024;         // waking the helpers takes ~10 us, in which one thread copies 200 KB
 
-class Helpers {
-public:
-    ~Helpers() { stop(); }
-
-    // body(0) on the calling thread, body(1 .. kCopyThreads - 1) on the helpers; returns when all are done
-    void run(const std::function<void(int)>& body) {
-        if (!start()) {                                 // no threads to be had: one after the other
-            for (int t = 0; t < kCopyThreads; ++t) body(t);
-            return;
-        }
-        {
-            std::lock_guard<std::mutex> lock(m_);
-            body_ = &body;
-            left_ = kCopyThreads - 1;
-            ++generation_;
-        }
-        wake_.notify_all();
-        body(0);
-        std::unique_lock<std::mutex> lock(m_);
-        done_.wait(lock, [this] { return left_ == 0; });
-        body_ = nullptr;
-    }
-
-    void stop() {
-        if (!started_ || pid_ != getpid()) return;     // (a forked child has no helpers)
-        {
-            std::lock_guard<std::mutex> lock(m_);
-            quit_ = true;
-        }
-        wake_.notify_all();
-        for (std::thread& t : threads_) if (t.joinable()) t.join();
-        started_ = false; quit_ = false;
-    }
-
-private:
-    bool start() {
-        if (started_) return pid_ == getpid();
-        pid_ = getpid();
-        const uint64_t seen = generation_;
-        try {
-            for (int i = 1; i < kCopyThreads; ++i) threads_[i] = std::thread([this, i, seen] { loop(i, seen); });
-        } catch (const std::system_error&) {
-            started_ = true;
-            stop();
-            return false;
-        }
-        started_ = true;
-        return true;
-    }
-    // a helper waits for the next body for a tenth of a millisecond with open eyes, then asleep
-    void loop(int index, uint64_t seen) {
-        while (true) {
-            const std::function<void(int)>* body;
-            // (the way back of a product follows its way in by less than a sleeping thread takes to wake)
-            const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(100);
-            while (generation_.load(std::memory_order_acquire) == seen && !quit_.load(std::memory_order_relaxed) &&
-                   std::chrono::steady_clock::now() < until) {}
-            {
-                std::unique_lock<std::mutex> lock(m_);
-                wake_.wait(lock, [&] { return quit_ || generation_ != seen; });
-                if (quit_) return;
-                seen = generation_;
-                body = body_;
-            }
-            (*body)(index);
-            std::lock_guard<std::mutex> lock(m_);
-            if (--left_ == 0) done_.notify_one();
-        }
-    }
-
-    std::mutex m_;
-    std::condition_variable wake_, done_;
-    std::thread threads_[kCopyThreads];
-    const std::function<void(int)>* body_ = nullptr;
-    std::atomic<uint64_t> generation_{0};
-    int left_ = 0;
-    bool started_ = false;
-    std::atomic<bool> quit_{false};
-    pid_t pid_ = 0;
-};
-
 struct Staging {
     std::mutex busy;                                    // one transfer at a time
-    Helpers helpers;
     int device = -1;                                    // the events belong to it; the pinned memory serves every device
     char* buf[kCopyThreads][2] = {};
     cudaEvent_t ev[kCopyThreads][2] = {};
@@ -141,7 +54,7 @@ struct Staging {
         return 0;
     }
     int give_back() {
-        helpers.stop();
+        helpers().stop();
         TB_TRY(drop_events());
         for (int t = 0; t < kCopyThreads; ++t)
             for (int b = 0; b < 2; ++b) {
@@ -212,7 +125,7 @@ int transfer(const CopySpan* spans, int count, bool to_device, cudaStream_t st, 
             }
         if (before_at && ok(cudaEventSynchronize(g.ev[t][b ^ 1]))) std::memcpy(before_at, g.buf[t][b ^ 1], before);
     };
-    if (threads > 1) g.helpers.run(body);
+    if (threads > 1) helpers().run(body);
     else body(0);
     for (cudaError_t e : err) TB_CUDA(e);
     if (ready) tell();
