@@ -433,6 +433,57 @@ def test_matmul_host_from_several_threads(tb, oracle):
     assert not errors, errors
 
 
+@pytest.mark.parametrize("precision", ["bf16", "fp32"])
+def test_matmul_host_in_row_blocks_beside_other_calls(tb, oracle, precision):
+    """Products large enough for row blocks from several threads, with shapes that shrink and grow, while another thread has
+    the device's scratch memory packed with operands of its own."""
+    import threading
+    import torch
+    prec = {"bf16": tb.PREC_BF16, "fp32": tb.PREC_FP32}[precision]
+    tol = {"bf16": 2e-2, "fp32": 1e-5}[precision]
+    rng = np.random.default_rng(78)
+    cases = []
+    for M, K, N in ((1024, 512, 700), (700, 1024, 1024), (129, 64, 40), (2000, 300, 512)):
+        A, B = rng.standard_normal((M, K)).astype(np.float32), (rng.standard_normal((K, N)) * 0.05).astype(np.float32)
+        cases.append((A, B, A.astype(np.float64) @ B.astype(np.float64)))
+    errors, done = [], threading.Event()
+
+    def worker(order):
+        try:
+            for _ in range(6):
+                for i in order:
+                    A, B, want = cases[i]
+                    out = np.zeros(want.shape, np.float32)
+                    tb.matmul_host(A, B, out, A.shape[0], A.shape[1], B.shape[1], prec)
+                    if rel_to_maxabs(out, want) > tol:
+                        errors.append((i, rel_to_maxabs(out, want)))
+        except Exception as e:          # noqa: BLE001 -- reported by the assertion below
+            errors.append(repr(e))
+
+    x, w = torch.randn(640, 500, device="cuda"), torch.randn(500, 330, device="cuda") * 0.05
+    y, want_y = torch.empty(640, 330, device="cuda"), x.double() @ w.double()
+
+    def device_calls():
+        try:
+            while not done.is_set():
+                tb.gemm_f32(tb.NN, x, w, y, 640, 330, 500, 500, 330, 330, precision=prec)
+                err = float((y.double() - want_y).abs().max() / want_y.abs().max())
+                if err > tol:
+                    errors.append(("device", err))
+        except Exception as e:          # noqa: BLE001
+            errors.append(repr(e))
+    tb.gemm_f32(tb.NN, x, w, y, 640, 330, 500, 500, 330, 330, precision=prec)      # (sizes the device's scratch memory)
+    threads = [threading.Thread(target=worker, args=(o,)) for o in ([0, 1, 2, 3], [3, 2, 1, 0], [1, 3, 0, 2])]
+    beside = threading.Thread(target=device_calls)
+    for t in threads + [beside]:
+        t.start()
+    for t in threads:
+        t.join()
+    done.set()
+    beside.join()
+    assert not errors, errors
+
+
 @pytest.mark.parametrize("precision", ["bf16", "tf32", "fp32"])
 @pytest.mark.parametrize("shape", [(255, 1031, 900), (257, 2000, 1025), (1030, 701, 777), (128, 300, 20000), (2049, 513, 1)])
 def test_matmul_host_in_row_blocks(tb, oracle, shape, precision):

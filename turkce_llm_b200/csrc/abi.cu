@@ -232,13 +232,38 @@ static inline bool tma_ok_f32(const float* p, long long ld, int batch, long long
     return (reinterpret_cast<uintptr_t>(p) & 15u) == 0 && ld % 4 == 0 && (batch == 1 || stride % 4 == 0);
 }
 
+// Packed operands and split-K partial sums of a caller that does not use the device's scratch memory
+struct OwnScratch { float* mem = nullptr; size_t floats = 0; };
+
+static int grow(float** p, size_t* cap, size_t need) {
+    if (need <= *cap) return 0;
+    if (*p) TB_CUDA(cudaFree(*p));
+    *p = nullptr; *cap = 0;
+    const size_t want = need + need / 4;
+    TB_CUDA(cudaMalloc(p, want * sizeof(float)));
+    *cap = want;
+    return 0;
+}
+
 static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int M, int N, int K,
                          long long lda, long long ldb, long long ldc, int batch, long long sA, long long sB,
                          long long sC, float alpha, float beta, const float* bias, const float* residual,
-                         int precision, cudaStream_t stream, bool same_b = false) {
-    // (same_b: B is what the call before it on this stream had, and is still packed in the scratch memory)
+                         int precision, cudaStream_t stream, OwnScratch* own = nullptr, bool same_b = false) {
+    // (same_b: B is what the call before it with this scratch memory, its caller's own, had, and is still packed there)
     DeviceCtx* ctx;
     TB_TRY(get_ctx(&ctx));
+    char* scratch = nullptr;
+    auto take_scratch = [&](size_t bytes) -> int {
+        if (own == nullptr) {
+            TB_TRY(ensure_scratch(ctx, bytes));
+            scratch = static_cast<char*>(ctx->scratch);
+            return 0;
+        }
+        if (bytes > own->floats * sizeof(float)) same_b = false;      // it moves
+        TB_TRY(grow(&own->mem, &own->floats, (bytes + sizeof(float) - 1) / sizeof(float)));
+        scratch = reinterpret_cast<char*>(own->mem);
+        return 0;
+    };
     TB_CHECK(kind >= 0 && kind <= 2, "unknown GEMM kind %d", kind);
     TB_CHECK(precision >= TB_PREC_BF16 && precision <= TB_PREC_FP32, "unknown precision %d", precision);
     TB_CHECK(M > 0 && N > 0 && K > 0 && batch > 0, "GEMM dims must be positive");
@@ -263,11 +288,10 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
         const int splits = planned_splits(ctx, g);
         g.splits = splits;
         const size_t ws_floats = splits > 1 ? (size_t)splits * batch * M * N : 0;
-        if (a_bytes + b_bytes + ws_floats * sizeof(float) > ctx->scratch_bytes) same_b = false;      // the scratch memory moves
-        TB_TRY(ensure_scratch(ctx, a_bytes + b_bytes + ws_floats * sizeof(float)));
-        bf16* pb = static_cast<bf16*>(ctx->scratch);
-        bf16* pa = reinterpret_cast<bf16*>(static_cast<char*>(ctx->scratch) + b_bytes);
-        float* ws = reinterpret_cast<float*>(static_cast<char*>(ctx->scratch) + a_bytes + b_bytes);
+        TB_TRY(take_scratch(a_bytes + b_bytes + ws_floats * sizeof(float)));
+        bf16* pb = reinterpret_cast<bf16*>(scratch);
+        bf16* pa = reinterpret_cast<bf16*>(scratch + b_bytes);
+        float* ws = reinterpret_cast<float*>(scratch + a_bytes + b_bytes);
         ConvSide sides[2] = {{A, pa, a_rows, a_cols, lda, a_ld, sA, a_stride}, {B, pb, b_rows, b_cols, ldb, b_ld, sB, b_stride}};
         TB_TRY(launch_pack_operands(ctx, sides, same_b ? 1 : 2, batch, stream));
         g.A = pa; g.B = pb;
@@ -293,11 +317,10 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
     const int splits = planned_splits(ctx, g);
     g.splits = splits;
     const size_t ws_floats = splits > 1 ? (size_t)splits * batch * M * N : 0;
-    if (a_bytes + b_bytes + ws_floats * sizeof(float) > ctx->scratch_bytes) same_b = false;      // the scratch memory moves
-    TB_TRY(ensure_scratch(ctx, a_bytes + b_bytes + ws_floats * sizeof(float)));
-    float* pb = static_cast<float*>(ctx->scratch);
-    float* pa = reinterpret_cast<float*>(static_cast<char*>(ctx->scratch) + b_bytes);
-    float* ws = reinterpret_cast<float*>(static_cast<char*>(ctx->scratch) + a_bytes + b_bytes);
+    TB_TRY(take_scratch(a_bytes + b_bytes + ws_floats * sizeof(float)));
+    float* pb = reinterpret_cast<float*>(scratch);
+    float* pa = reinterpret_cast<float*>(scratch + b_bytes);
+    float* ws = reinterpret_cast<float*>(scratch + a_bytes + b_bytes);
     if (split3) {
         ConvSide sides[2] = {{A, pa, a_rows, a_cols, lda, a_ld, sA, a_stride, a_cat_cols ? 1 : 0, 0},
                              {B, pb, b_rows, b_cols, ldb, b_ld, sB, b_stride, b_cat_cols ? 1 : 0, 1}};
@@ -332,13 +355,15 @@ int tb_gemm_bias_f32(const float* d_A, const float* d_B, const float* d_bias, co
 // (model/gpu_ops.c:31-46,118-160); the slot of a call is the calling thread's (gpu_ops_set_worker_id stores it in a
 // thread-local, :100-102).  Here every host thread that calls tb_matmul_host owns one such slot per device: buffers
 // grow on demand and live until the thread ends, so the steady state allocates nothing, and threads never share a
-// slot (no lock on the data path, as the reference's worker slots).
+// slot.  The packed operands are in the slot as well: B stays packed from row block to row block while host copies run in
+// between, and nothing that another thread does with the device's scratch memory reaches it.
 namespace {
 constexpr int kMatmulBlocks = 4;
 struct MatmulSlot {
     int device = -1;
     float *dA = nullptr, *dB = nullptr, *dC = nullptr;
     size_t capA = 0, capB = 0, capC = 0;
+    OwnScratch packed;
     cudaStream_t in = nullptr, out = nullptr;            // the copies of a product in blocks
     cudaEvent_t arrived[kMatmulBlocks + 1] = {}, done[kMatmulBlocks] = {};
     ~MatmulSlot() {
@@ -346,7 +371,7 @@ struct MatmulSlot {
         int cur = -1;
         if (cudaGetDevice(&cur) != cudaSuccess) return;      // the runtime is already shutting down
         cudaSetDevice(device);
-        cudaFree(dA); cudaFree(dB); cudaFree(dC);
+        cudaFree(dA); cudaFree(dB); cudaFree(dC); cudaFree(packed.mem);
         if (in) cudaStreamDestroy(in);
         if (out) cudaStreamDestroy(out);
         for (cudaEvent_t e : arrived) if (e) cudaEventDestroy(e);
@@ -363,16 +388,6 @@ struct MatmulSlot {
     }
 };
 thread_local MatmulSlot t_slots[8];
-
-int grow(float** p, size_t* cap, size_t need) {
-    if (need <= *cap) return 0;
-    if (*p) TB_CUDA(cudaFree(*p));
-    *p = nullptr; *cap = 0;
-    const size_t want = need + need / 4;
-    TB_CUDA(cudaMalloc(p, want * sizeof(float)));
-    *cap = want;
-    return 0;
-}
 }  // namespace
 
 int tb_matmul_host(const float* h_A, const float* h_B, float* h_C, int M, int K, int N, int precision) {
@@ -388,11 +403,12 @@ int tb_matmul_host(const float* h_A, const float* h_B, float* h_C, int M, int K,
     TB_TRY(grow(&slot->dA, &slot->capA, na));
     TB_TRY(grow(&slot->dB, &slot->capB, nb));
     TB_TRY(grow(&slot->dC, &slot->capC, nc));
-    // the library scratch (operand packing, split-K partials) is one per device: calls of different threads take turns
-    static std::mutex gemm_mutex;
+    // (the launches of one product stay together, as the profile's marks around them do; nothing waits for a copy under the lock)
+    static std::mutex launch_mutex;
     auto product = [&](size_t row0, size_t rows, bool same_b) {
+        std::lock_guard<std::mutex> lock(launch_mutex);
         return gemm_f32_impl(TB_GEMM_NN, slot->dA + row0 * K, slot->dB, slot->dC + row0 * N, (int)rows, N, K, K, N, N, 1, 0, 0, 0, 1.0f, 0.0f,
-                             nullptr, nullptr, precision, nullptr, same_b);
+                             nullptr, nullptr, precision, nullptr, &slot->packed, same_b);
     };
     // A large product goes by row blocks: block i is multiplied and on its way back while block i + 1 comes in, so that the
     // two directions of the bus and the product overlap (1024 x 1024 x 1024: the copies in, 8 MB, are ~170 us at the bus
@@ -402,7 +418,6 @@ int tb_matmul_host(const float* h_A, const float* h_B, float* h_C, int M, int K,
     if (blocks < 2) {
         const CopySpan in[2] = {{slot->dB, const_cast<float*>(h_B), nb * 4}, {slot->dA, const_cast<float*>(h_A), na * 4}};
         TB_TRY(copy_h2d(in, 2, nullptr));
-        std::lock_guard<std::mutex> lock(gemm_mutex);
         TB_TRY(product(0, (size_t)M, false));
         TB_TRY(device_error_request(ctx, nullptr));
         const CopySpan out = {slot->dC, h_C, nc * 4};
@@ -422,7 +437,6 @@ int tb_matmul_host(const float* h_A, const float* h_B, float* h_C, int M, int K,
         out[n] = {slot->dC + r * N, h_C + r * N, rows * N * 4};
     }
     first[n] = (size_t)M;
-    std::lock_guard<std::mutex> lock(gemm_mutex);
     const std::function<int(int)> ready = [&](int span) -> int {
         if (span == 0) return 0;                             // (B: in front of block 0 on the same stream)
         const int i = span - 1;
