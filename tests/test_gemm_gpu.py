@@ -433,6 +433,36 @@ def test_matmul_host_from_several_threads(tb, oracle):
     assert not errors, errors
 
 
+def test_matmul_host_from_more_threads_than_there_are_copy_buffers(tb):
+    """Sixteen threads with products of one row block and of several: more transfers at a time than there are helper threads or
+    pinned buffers, so that all three ways to copy are taken."""
+    import threading
+    rng = np.random.default_rng(79)
+    cases = []
+    for M, K, N in ((600, 900, 1000), (300, 400, 500), (64, 64, 64)):
+        A, B = rng.standard_normal((M, K)).astype(np.float32), (rng.standard_normal((K, N)) * 0.05).astype(np.float32)
+        cases.append((A, B, A.astype(np.float64) @ B.astype(np.float64)))
+    errors, start = [], threading.Barrier(16)
+
+    def worker(first):
+        try:
+            start.wait()
+            for i in range(30):
+                A, B, want = cases[(first + i) % len(cases)]
+                out = np.zeros(want.shape, np.float32)
+                tb.matmul_host(A, B, out, A.shape[0], A.shape[1], B.shape[1], tb.PREC_FP32)
+                if rel_to_maxabs(out, want) > 1e-5:
+                    errors.append(rel_to_maxabs(out, want))
+        except Exception as e:          # noqa: BLE001 -- reported by the assertion below
+            errors.append(repr(e))
+    threads = [threading.Thread(target=worker, args=(t,)) for t in range(16)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+
+
 @pytest.mark.parametrize("precision", ["bf16", "fp32"])
 def test_matmul_host_in_row_blocks_beside_other_calls(tb, oracle, precision):
     """Products large enough for row blocks from several threads, with shapes that shrink and grow, while another thread has

@@ -97,6 +97,28 @@ private:
     pid_t pid_ = 0;
 };
 
+// N numbered things that are handed out without ever waiting for one.
+template <int N>
+class Handout {
+public:
+    // up to `want` of the free ones -> which[]; how many
+    int take(int want, int* which) {
+        std::lock_guard<std::mutex> lock(m_);
+        int n = 0;
+        for (int i = 0; i < N && n < want; ++i)
+            if (!taken_[i]) { taken_[i] = true; which[n++] = i; }
+        return n;
+    }
+    void give(const int* which, int n) {
+        std::lock_guard<std::mutex> lock(m_);
+        for (int i = 0; i < n; ++i) taken_[which[i]] = false;
+    }
+
+private:
+    std::mutex m_;
+    bool taken_[N] = {};
+};
+
 inline Helpers& helpers() {
     static Helpers* const h = new Helpers();
     return *h;
