@@ -433,6 +433,38 @@ def test_matmul_host_from_several_threads(tb, oracle):
     assert not errors, errors
 
 
+@pytest.mark.parametrize("pinned", [(1, 1, 1), (1, 0, 0), (0, 1, 0), (0, 0, 1)])
+@pytest.mark.parametrize("shape", [(300, 200, 100), (1030, 701, 777)])
+def test_matmul_host_with_pinned_arrays(tb, shape, pinned):
+    """Pinned host memory is copied as it is, each operand for itself; the arrays may change as soon as the call is back."""
+    import torch
+    M, K, N = shape
+    a, b, c = (torch.empty(s, pin_memory=bool(p)) for s, p in zip(((M, K), (K, N), (M, N)), pinned))
+    gen = torch.Generator().manual_seed(3)
+    for _ in range(3):
+        a.normal_(generator=gen), b.normal_(generator=gen)
+        want = a.double() @ b.double()
+        tb.matmul_host(a, b, c, M, K, N, tb.PREC_FP32)
+        a.fill_(float("nan")), b.fill_(float("nan"))
+        assert rel_to_maxabs(c, want) <= 1e-5
+
+
+def test_pinned_arrays_are_not_staged(tb):
+    """The copies of 48 MB from and to pinned memory take the bus's time: well under what the staging threads' copies add."""
+    import time
+    import torch
+    M = N = 3000
+    K = 40
+    best = {}
+    for pin in (False, True):
+        a, b, c = (torch.zeros(s, pin_memory=pin) for s in ((M, K), (K, N), (M, N)))
+        for _ in range(8):
+            t0 = time.perf_counter()
+            tb.matmul_host(a, b, c, M, K, N, tb.PREC_BF16)
+            best[pin] = min(best.get(pin, 1e9), time.perf_counter() - t0)
+    assert best[True] < 0.8 * best[False], best
+
+
 def test_matmul_host_from_more_threads_than_there_are_copy_buffers(tb):
     """Sixteen threads with products of one row block and of several: more transfers at a time than there are helper threads or
     pinned buffers, so that all three ways to copy are taken."""

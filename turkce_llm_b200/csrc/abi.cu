@@ -417,11 +417,12 @@ int tb_matmul_host(const float* h_A, const float* h_B, float* h_C, int M, int K,
     const int blocks = (int)std::min<size_t>({(size_t)kMatmulBlocks, moved >> 20, (size_t)M / 128});
     if (blocks < 2) {
         const CopySpan in[2] = {{slot->dB, const_cast<float*>(h_B), nb * 4}, {slot->dA, const_cast<float*>(h_A), na * 4}};
-        TB_TRY(copy_h2d(in, 2, nullptr));
-        TB_TRY(product(0, (size_t)M, false));
-        TB_TRY(device_error_request(ctx, nullptr));
         const CopySpan out = {slot->dC, h_C, nc * 4};
-        TB_TRY(copy_d2h(&out, 1, nullptr));
+        int rc = copy_h2d(in, 2, nullptr);
+        if (rc == 0) rc = product(0, (size_t)M, false);
+        if (rc == 0) rc = device_error_request(ctx, nullptr);
+        if (rc == 0) rc = copy_d2h(&out, 1, nullptr);
+        if (rc != 0) { cudaStreamSynchronize(nullptr); return rc; }      // (no copy from or to the caller's memory goes on behind its back)
         return device_error_result(ctx);
     }
     TB_TRY(slot->streams());
@@ -447,8 +448,12 @@ int tb_matmul_host(const float* h_A, const float* h_B, float* h_C, int M, int K,
         TB_CUDA(cudaEventRecord(slot->done[i], nullptr));
         return 0;
     };
-    TB_TRY(copy_h2d(in, n + 1, slot->in, &ready));
-    TB_TRY(copy_d2h(out, n, slot->out, slot->done));
+    int rc = copy_h2d(in, n + 1, slot->in, &ready);
+    if (rc == 0) rc = copy_d2h(out, n, slot->out, slot->done);
+    if (rc != 0) {
+        for (cudaStream_t st : {slot->in, static_cast<cudaStream_t>(nullptr), slot->out}) cudaStreamSynchronize(st);
+        return rc;
+    }
     return device_error_result(ctx);
 }
 

@@ -53,9 +53,10 @@ const char* last_error();
         TB_CUDA(cudaStreamSynchronize(cudaStreamLegacy));                        \
     } while (0)
 
-// ---- copies between pageable host memory and the device through pinned buffers (host_copy.cu)
+// ---- copies between host memory and the device, pageable memory through pinned buffers (host_copy.cu)
 struct CopySpan { void* dev; void* host; size_t bytes; };
-// All spans, in stream order on `st`; on return the host memory has been read, the copies themselves may be on their way.
+// All spans, in stream order on `st`; on return pageable memory has been read, the copies themselves may be on their way.  Pinned
+// memory is read by those copies: the caller waits for the stream before it lets go of it, on its way out with an error too.
 // ready (optional) is called span by span, in order, when all of a span's copies have been handed to the stream.
 int copy_h2d(const CopySpan* spans, int count, cudaStream_t st, const std::function<int(int)>* ready = nullptr);
 // On return the data is in host memory (and what was in front of the copies on `st` has finished).

@@ -401,7 +401,7 @@ int tb_decoder_read_logits(TbDecoder* g, float* h_logits) {
     TB_TRY(device_error_request(g->ctx, g->stream));
     std::vector<CopySpan> rows((size_t)g->S);           // (rows are padded on the device only)
     for (int s = 0; s < g->S; ++s) rows[s] = {g->logits + (size_t)s * g->Vp, h_logits + (size_t)s * g->V, (size_t)g->V * 4};
-    TB_TRY(copy_d2h(rows.data(), g->S, g->stream));
+    if (const int rc = copy_d2h(rows.data(), g->S, g->stream)) { cudaStreamSynchronize(g->stream); return rc; }
     return device_error_result(g->ctx);
 }
 
