@@ -339,7 +339,8 @@ def test_lean_decode_step_matches_general_step(tb, oracle, monkeypatch):
 
 
 @pytest.mark.parametrize("dims", [(500, 256, 4, 3, 1024, 64, 9, 6), (300, 128, 2, 2, 256, 5, 20, 6),
-                                  (31769, 384, 6, 12, 1024, 64, 16, 4)])
+                                  (31769, 384, 6, 12, 1024, 64, 16, 4),
+                                  (500, 384, 8, 3, 1024, 40, 70, 6), (300, 96, 2, 2, 128, 20, 60, 6)])      # head dim 48
 def test_one_kernel_decode_step_matches_launch_per_kernel_step(tb, oracle, monkeypatch, dims):
     """The default decode step runs every layer in one cooperative kernel (three launches per token with the final
     norm and the head); TB_DECODE_NO_MEGA=1 selects the launch-per-kernel step.  Same bf16 operands and the same

@@ -320,7 +320,9 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
         const int gpp_shift = pairs <= 1 ? 3 : pairs <= 2 ? 2 : pairs <= 4 ? 1 : 0, gpp = 1 << gpp_shift;
         const int pr = warp >> (1 + gpp_shift), sub = (warp >> 1) & (gpp - 1);
         const int nparts = 2 * min(gpp, nblk);
-        const size_t kv_at = ((size_t)(row0 * H + pair0 + tid / (HD / 2)) * p.cap + t) * HD + 2 * (tid % (HD / 2));   // new cache row
+        // one thread per rotated pair of the new row, HP threads per (sequence, head): a power of two, so that their sums are shuffles
+        constexpr int HALF = HD / 2, HP = HD == 48 ? 32 : HALF;
+        const size_t kv_at = ((size_t)(row0 * H + pair0 + tid / HP) * p.cap + t) * HD + 2 * (tid % HP);              // new cache row
         // RMSNorm: places of this lane's columns 4 (lane + 32 k), k < 4, in a row of xbuf
         uint32_t x_at[4];
 #pragma unroll
@@ -483,14 +485,14 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                     float* rv = rq + p.P * HD;
                     float* snew = rv + p.P * HD;
                     if (pairs > 0) {
-                        constexpr int HALF = HD / 2;
-                        const int i = tid / HALF, k = tid % HALF;
+                        const int i = tid / HP, k = tid % HP;
+                        const bool mine = i < pairs && k < HALF;
                         float c = 0.f, sn = 0.f;
-                        if (i < pairs) { c = __ldg(p.cos_t + t * HALF + k); sn = __ldg(p.sin_t + t * HALF + k); }
+                        if (mine) { c = __ldg(p.cos_t + t * HALF + k); sn = __ldg(p.sin_t + t * HALF + k); }
                         wait(qkv_bar, (uint32_t)l & 1u);
                         if (tid == DC_COMPUTE - 1) mbar_expect_tx(qkv_bar, (uint32_t)(pairs * 3 * HD * 4));
                         float dot = 0.0f;                                        // score of the new key
-                        if (i < pairs) {
+                        if (mine) {
                             const float* in = qkv_in + i * 3 * HD + 2 * k;
                             const float q0 = in[0], q1 = in[1], k0 = in[HD], k1 = in[HD + 1], v0 = in[2 * HD], v1 = in[2 * HD + 1];
                             const float r0 = (q0 * c - q1 * sn) * p.qscale, r1 = (q0 * sn + q1 * c) * p.qscale;
@@ -504,16 +506,16 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
                             dot = r0 * __bfloat162float(kn.x) + r1 * __bfloat162float(kn.y);
                             *reinterpret_cast<float2*>(rv + i * HD + 2 * k) = make_float2(__bfloat162float(vn.x), __bfloat162float(vn.y));
                         }
-                        if (warp * 32 < pairs * HALF) {
+                        if (warp * 32 < pairs * HP) {
 #pragma unroll
-                            for (int o = HALF / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+                            for (int o = HP / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
                             if (i < pairs && k == 0) snew[i] = dot;
                         }
                     }
                     compute_sync();
                     if (l + 1 < p.L) fetch_vec(l + 1);
                     // ------------------------------------------------------ attention over the cached rows
-                    constexpr int VL = HD / 8;                                   // lanes that cover a value row
+                    constexpr int VL = HD == 48 ? 8 : HD / 8;                    // lanes that cover a value row (of 48: two have its zero padding)
                     constexpr int VK = 32 / VL;                                  // value rows per pass of the warp
                     if (pr < pairs) {
                         const float* q = rq + pr * HD;
@@ -578,7 +580,7 @@ __global__ void __launch_bounds__(DC_THREADS, 1) decode_cluster_kernel(const __g
 #pragma unroll
                         for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
                         float* part = stage + (pr * 2 * gpp + sub * 2 + (warp & 1)) * PART_LD;
-                        if (lane < VL) {
+                        if (lane < HD / 8) {
                             *reinterpret_cast<float4*>(part + lane * 8) = make_float4(acc[0].x, acc[0].y, acc[1].x, acc[1].y);
                             *reinterpret_cast<float4*>(part + lane * 8 + 4) = make_float4(acc[2].x, acc[2].y, acc[3].x, acc[3].y);
                         }
@@ -732,7 +734,7 @@ __global__ void vec_layout_kernel(const float* __restrict__ bq, const float* __r
 
 typedef void (*DcKernel)(const DcParams);
 DcKernel dc_kernel(int hd) {
-    return hd == 64 ? decode_cluster_kernel<64> : hd == 32 ? decode_cluster_kernel<32> : decode_cluster_kernel<16>;
+    return hd == 64 ? decode_cluster_kernel<64> : hd == 48 ? decode_cluster_kernel<48> : hd == 32 ? decode_cluster_kernel<32> : decode_cluster_kernel<16>;
 }
 
 cudaLaunchConfig_t dc_config(const DcParams& p, size_t smem, cudaStream_t st, cudaLaunchAttribute* attr) {
@@ -761,7 +763,7 @@ struct DecodeCluster {
 
 bool decode_cluster_supported(int D, int H, int F) {
     const int hd = H > 0 ? D / H : 0;
-    return D % 16 == 0 && F % 16 == 0 && D <= 1024 && F <= 1024 && (hd == 16 || hd == 32 || hd == 64);
+    return D % 16 == 0 && F % 16 == 0 && D <= 1024 && F <= 1024 && hd % 16 == 0 && hd >= 16 && hd <= 64;
 }
 
 // *out stays NULL when the shape does not fit a cluster (the caller keeps the launch-per-kernel step).
