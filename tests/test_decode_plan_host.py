@@ -49,3 +49,32 @@ int main() {
 
 def test_every_plan_keeps_to_instruction_shapes_and_memory(tmp_path):
     print(compile_and_run(tmp_path, CHECK))
+
+
+RULE = r"""
+#include "decode_plan.h"
+#include <cstdio>
+using namespace tb;
+int main() {
+    struct { int D, H, F, S; bool cluster; } shapes[] = {
+        {384, 6, 1024, 1, true}, {384, 6, 1024, 64, true}, {384, 6, 1024, 112, true}, {384, 6, 1024, 200, true}, {384, 6, 1024, 336, true},
+        {384, 6, 1024, 448, false}, {384, 12, 1024, 200, true}, {384, 24, 1024, 128, false}, {64, 2, 128, 112, true}, {64, 2, 128, 256, false},
+        {768, 12, 1024, 64, true}, {768, 12, 1024, 128, false}, {1024, 16, 1024, 100, true}, {1024, 16, 1024, 128, false},
+        {1024, 64, 1024, 28, true}, {1024, 64, 1024, 32, false}, {1024, 64, 1024, 64, false}};
+    int wrong = 0;
+    for (auto& s : shapes) {
+        const int fit = 7;                                   // clusters of 16 on a B200
+        DcPlan p;
+        size_t smem;
+        bool found = false;
+        for (int R = std::min(16, ceil_div(s.S, fit)); R >= 1 && !found; --R) found = dc_plan(&p, &smem, s.S, s.D, s.H, s.F, 16, R);
+        if (!found || dc_pays(p, fit) != s.cluster) { printf("D %d H %d F %d S %d: R %d\n", s.D, s.H, s.F, s.S, found ? p.R : 0); ++wrong; }
+    }
+    return wrong;
+}
+"""
+
+
+def test_the_cluster_kernel_is_taken_where_it_is_faster(tmp_path):
+    """(the shapes that the rule was measured on)"""
+    compile_and_run(tmp_path, RULE)

@@ -207,7 +207,7 @@ size_t attention_bwd_ds_bytes(int B, int H, int T);
 
 // ---- the decode step of all layers, sequences spread over thread-block clusters (decode_cluster.cu)
 struct DecodeCluster;
-// *out stays NULL when the shape does not fit
+// *out stays NULL when the shape does not fit, or the launch-per-kernel step is the better one
 int decode_cluster_create(DeviceCtx* ctx, DecodeCluster** out, int S, int D, int H, int F, int L, int cap, float eps, float scale);
 void decode_cluster_destroy(DecodeCluster* m);
 // operand images of the weights + the per-layer pointer table; offsets = the flat parameter offsets (embedding first)

@@ -766,7 +766,7 @@ bool decode_cluster_supported(int D, int H, int F) {
     return D % 16 == 0 && F % 16 == 0 && D <= 1024 && F <= 1024 && hd % 16 == 0 && hd >= 16 && hd <= 64;
 }
 
-// *out stays NULL when the shape does not fit a cluster (the caller keeps the launch-per-kernel step).
+// *out stays NULL when the shape does not fit a cluster or takes too many of them (the caller keeps the launch-per-kernel step).
 int decode_cluster_create(DeviceCtx* ctx, DecodeCluster** out, int S, int D, int H, int F, int L, int cap, float eps, float scale) {
     *out = nullptr;
     if (!decode_cluster_supported(D, H, F) || L < 1 || S < 1) return 0;
@@ -778,6 +778,7 @@ int decode_cluster_create(DeviceCtx* ctx, DecodeCluster** out, int S, int D, int
     TB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     // 16 CTAs per cluster: half the weight bytes per SM of a cluster of 8, at the price of fewer clusters at a time (7 on a
     // B200 whose processor clusters hold 20, 20, .. 8 SMs).  The sequences are spread over the clusters that fit at once.
+    // (A hidden size of 1024 needs the 16: a CTA of eight would own 256 rows of gate|up.  Sizes between were not measured.)
     bool found = false;
     for (int C = 16; C >= 8 && !found; C /= 2) {
         if (!dc_plan(&p, &smem, S, D, H, F, C, 1)) continue;
@@ -787,6 +788,7 @@ int decode_cluster_create(DeviceCtx* ctx, DecodeCluster** out, int S, int D, int
         int fit = 0;
         if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) != cudaSuccess || fit < 1) { cudaGetLastError(); continue; }
         for (int R = std::min(16, ceil_div(S, fit)); R >= 1 && !found; --R) found = dc_plan(&p, &smem, S, D, H, F, C, R);
+        if (found && !dc_pays(p, fit)) return 0;
     }
     if (!found) return 0;
     DecodeCluster* m = new DecodeCluster();

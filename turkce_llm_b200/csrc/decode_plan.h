@@ -109,4 +109,17 @@ inline bool dc_plan(DcPlan* p, size_t* smem_bytes, int S, int D, int H, int F, i
     return true;
 }
 
+// Whether the plan is better than the launch-per-kernel step, when `fit` clusters run at a time.  A wave of clusters takes a
+// layer's chain of phases whatever it carries (14 us at width 64, 20 at 384, 27 - 35 at 1024), the other step grows slowly with
+// the sequences, so the waves decide.  Cluster kernel : launch-per-kernel step, us per step at 128 cached rows:
+//   one wave    width 384, 6 heads, 12 layers, 112 sequences 248 : 546, width 1024, 16 heads, 4 layers, 32 sequences 118 : 271
+//   two         width 384, 200 sequences 483 : 662, width 1024, 64 heads, 28 sequences 218 : 281, width 768, 48 heads, 16 169 : 169
+//   three       width 384, 336 sequences 721 : 802 (16 sequences per cluster), 12 heads, 200 681 : 687 (10);
+//               width 768, 12 heads, 128 316 : 303 (8), width 1024, 64 heads, 32 322 : 287 (2), width 64, 256 84 : 60
+//   four, five  width 384, 448 sequences 958 : 918, width 1024, 64 heads, 64 sequences 530 : 344
+inline bool dc_pays(const DcPlan& p, int fit) {
+    const int waves = ceil_div(ceil_div(p.S, p.R), fit);
+    return waves <= 2 || (waves == 3 && p.R >= 10 && p.D >= 256);
+}
+
 }  // namespace tb
