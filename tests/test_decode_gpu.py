@@ -423,3 +423,30 @@ def test_sampling_over_small_and_large_vocabularies(tb, oracle, V):
                 r = u[s, step] * c[-1]
                 assert abs(int(tok[s]) - want) == 1 and abs(c[min(tok[s], want)] - r) <= 1e-6 * c[-1], (step, s)
     dec.destroy()
+
+
+@pytest.mark.parametrize("launches", [False, True], ids=["one_kernel", "launch_per_kernel"])
+@pytest.mark.parametrize("dims", [(211, 128, 2, 2, 256, 3), (211, 96, 2, 1, 128, 20), (211, 64, 2, 2, 128, 1)])
+def test_what_an_earlier_sequence_left_in_the_cache_has_no_effect(tb, oracle, monkeypatch, dims, launches):
+    """A generation whose keys and values were not finite (diverged weights) leaves them behind in the cache; a later one with
+    good weights gives what a new decoder gives, bit for bit, although its own rows end inside the same blocks."""
+    from turkce_llm_b200.decode import Decoder
+    if launches:
+        monkeypatch.setenv("TB_DECODE_NO_MEGA", "1")
+    V, D, H, L, F, S = dims
+    p = make_params(oracle, (V, D, H, L, F, 1, 1, 1e-5), 5)
+    prompts = np.random.default_rng(6).integers(0, V, (S, 41)).astype(np.uint32)
+    got = []
+    for used in (True, False):
+        dec = Decoder(V, D, H, L, F, S, 180)
+        if used:
+            dec.upload(np.full(dec.total, np.nan, np.float32))
+            dec.prefill(np.zeros((S, 170), np.uint32))
+            dec.generate(4)
+        dec.upload(p)
+        dec.prefill(prompts)
+        dec.generate(30)                     # from row 41 to row 70, across the end of a block
+        got.append((dec.tokens(31), dec.logits()))
+        dec.destroy()
+    assert np.isfinite(got[0][1]).all()
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])

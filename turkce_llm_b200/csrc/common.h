@@ -213,6 +213,8 @@ void decode_cluster_destroy(DecodeCluster* m);
 // operand images of the weights + the per-layer pointer table; offsets = the flat parameter offsets (embedding first)
 int decode_cluster_set_weights(DeviceCtx* ctx, DecodeCluster* m, const float* params, const bf16* params16, const long long* offsets,
                                bf16* const* Kc, bf16* const* Vc, cudaStream_t st);
+// value rows from .. to - 1 of all sequences and layers to zero: at the start of a prompt that is shorter than what is in the cache
+int decode_cluster_clear_values(DeviceCtx* ctx, DecodeCluster* m, int from, int to, cudaStream_t st);
 // out (bf16 [S, D]) = the final norm's output for the tokens tok at position *pos; K and V rows appended to the caches
 int launch_decode_cluster(DeviceCtx* ctx, DecodeCluster* m, const uint32_t* tok, const int* pos, const float* cos_t, const float* sin_t,
                           bf16* out, cudaStream_t st);

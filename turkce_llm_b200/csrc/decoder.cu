@@ -54,6 +54,7 @@ struct TbDecoder {
     uint32_t* h_pinned = nullptr;
     float* splitk_ws = nullptr; size_t splitk_floats = 0;
     int prompt_len = 0, generated = 0;
+    int cached_rows = 0;                       // rows per head that hold keys and values of this sequence or an earlier one
     float temperature = 0.f;                   // > 0: temperature sampling with the uniforms in sample_u
     double* sample_u = nullptr;                // [cap, S]: draw of sequence s for generated token i at i * S + s
     cudaGraphExec_t step_graph = nullptr;
@@ -296,6 +297,8 @@ int tb_decoder_prefill(TbDecoder* g, const uint32_t* h_ids, int prompt_len) {
     std::memcpy(g->h_pinned, h_ids, (size_t)N * 4);
     TB_CUDA(cudaMemcpyAsync(g->ids, g->h_pinned, (size_t)N * 4, cudaMemcpyHostToDevice, st));
     g->prompt_len = T; g->generated = 0;
+    if (g->cluster && g->cached_rows > T) TB_TRY(decode_cluster_clear_values(c, g->cluster, T, g->cached_rows, st));
+    g->cached_rows = T;
     int* h_state = reinterpret_cast<int*>(g->h_pinned + N);
     h_state[0] = T; h_state[1] = 0;
     TB_CUDA(cudaMemcpyAsync(g->pos, h_state, 2 * sizeof(int), cudaMemcpyHostToDevice, st));
@@ -357,6 +360,7 @@ int tb_decoder_generate(TbDecoder* g, int n) {
     // (with the one-kernel step there are two or three launches per token: nothing for a graph to save)
     const bool use_graph = getenv("TB_NO_GRAPH") == nullptr && !g->ctx->prof_on && g->cluster == nullptr;
     for (int i = 0; i < n; ++i) {
+        g->cached_rows = g->prompt_len + g->generated;
         if (!use_graph || g->step_state == 0) {
             TB_TRY(decode_step_body(g));
             if (use_graph) g->step_state = 1;
