@@ -450,3 +450,19 @@ def test_what_an_earlier_sequence_left_in_the_cache_has_no_effect(tb, oracle, mo
         dec.destroy()
     assert np.isfinite(got[0][1]).all()
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
+def test_a_decode_step_without_weights_is_an_error(tb):
+    """The one-kernel step reads tables that the upload makes: without one it is refused before anything is launched."""
+    from turkce_llm_b200 import lib
+    from turkce_llm_b200.decode import Decoder
+    dec = Decoder(97, 64, 2, 1, 128, 2, 16)
+    dec.prefill(np.zeros((2, 4), np.uint32))
+    with pytest.raises(lib.TbError, match="tb_decoder_upload"):
+        dec.generate(1)
+    dec.prefill(np.zeros((2, 3), np.uint32))
+    dec.upload(np.zeros(dec.total, np.float32))
+    dec.prefill(np.zeros((2, 4), np.uint32))
+    dec.generate(1)
+    assert np.array_equal(dec.tokens(2), np.zeros((2, 2)))       # all logits equal: the lowest token
+    dec.destroy()

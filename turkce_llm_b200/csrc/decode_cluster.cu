@@ -878,6 +878,7 @@ int decode_cluster_clear_values(DeviceCtx* ctx, DecodeCluster* m, int from, int 
 // tok [S] at position *pos -> out [S, D]: the final-norm output of the step, bf16; K and V rows appended to the caches.
 int launch_decode_cluster(DeviceCtx* ctx, DecodeCluster* m, const uint32_t* tok, const int* pos, const float* cos_t, const float* sin_t,
                           bf16* out, cudaStream_t st) {
+    TB_CHECK(m->p.embed != nullptr, "the decoder has no weights: call tb_decoder_upload first");      // (nor the kernel its tables)
     DcParams p = m->p;
     p.tok = tok; p.pos = pos; p.cos_t = cos_t; p.sin_t = sin_t; p.out = out;
     const DcKernel kernel = dc_kernel(p.D / p.H);
