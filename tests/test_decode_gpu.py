@@ -374,17 +374,25 @@ def test_one_kernel_decode_step_matches_launch_per_kernel_step(tb, oracle, monke
     assert np.array_equal(toks[0][same_so_far & clear, -1], toks[1][same_so_far & clear, -1])
 
 
-@pytest.mark.parametrize("dims", [(97, 32, 2, 2, 48, 3, 5, 4),          # head dim 16, K shorter than one 64-column block
+@pytest.mark.parametrize("dims", [(97, 32, 2, 2, 80, 17, 5, 4),         # head dim 16, K shorter than one 64-column block
                                   (211, 96, 3, 2, 80, 17, 62, 5),       # columns that do not fill the CTAs; cache across a 64-row block
-                                  (300, 192, 3, 1, 1024, 9, 127, 3),    # three slices of K; more than eight sequences in a cluster
+                                  (300, 192, 3, 1, 1024, 9, 127, 3),    # three slices of K
+                                  (300, 192, 3, 3, 1024, 70, 62, 5),    # and more than eight sequences in a cluster
+                                  (300, 384, 6, 2, 576, 50, 30, 3),     # three slices in both, an odd number of groups of eight
+                                  (300, 96, 2, 2, 80, 100, 20, 3),      # head dim 48, 15 sequences in a cluster
                                   (300, 768, 12, 1, 1008, 7, 64, 3),    # two tiles for the QKV columns
                                   (300, 64, 2, 2, 128, 1, 1, 70),       # one sequence from a one-token prompt
-                                  (97, 128, 2, 1, 256, 100, 9, 3)])     # more sequences than the clusters hold at once
+                                  (97, 128, 2, 1, 256, 100, 9, 3),      # up to 16 sequences in a cluster
+                                  (97, 128, 2, 2, 256, 200, 9, 3)])     # more sequences than the clusters hold at once
 def test_one_kernel_decode_step_at_the_edges_of_its_tiles(tb, oracle, monkeypatch, dims):
-    """The cluster kernel against the launch-per-kernel step where its tiles, slices and row groups end."""
+    """The cluster kernel against the launch-per-kernel step where its tiles, slices and row groups end: the same tokens and, within
+    rounding, the same logits for every sequence.  (The embeddings are large beside what the layers add, so that no choice
+    hangs on the last bits of a sum.)"""
+    from turkce_llm_b200 import lib
     from turkce_llm_b200.decode import Decoder
     V, D, H, L, F, S, prompt_len, n_new = dims
     p = make_params(oracle, (V, D, H, L, F, 1, 1, 1e-5), 5)
+    p[:V * D] *= 10.0
     prompts = np.random.default_rng(6).integers(0, V, (S, prompt_len)).astype(np.uint32)
     outs, toks = [], []
     for off in (False, True):
@@ -393,13 +401,15 @@ def test_one_kernel_decode_step_at_the_edges_of_its_tiles(tb, oracle, monkeypatc
         dec = Decoder(V, D, H, L, F, S, prompt_len + n_new + 2)
         dec.upload(p)
         dec.prefill(prompts)
+        before = lib.launch_count()
         dec.generate(n_new - 1)
+        assert (lib.launch_count() - before <= 4 * (n_new - 1)) == (not off)
         outs.append(dec.logits())
         toks.append(dec.tokens(n_new))
         dec.destroy()
-    same_so_far = (toks[0][:, :-1] == toks[1][:, :-1]).all(axis=1)
-    assert same_so_far.mean() >= 0.6, same_so_far.mean()
-    assert rel_to_maxabs(outs[0][same_so_far], outs[1][same_so_far]) <= 1e-2
+    assert np.array_equal(toks[0], toks[1])
+    worst = np.abs(outs[0] - outs[1]).max(axis=1) / np.abs(outs[1]).max(axis=1)          # per sequence
+    assert worst.max() <= 1e-2, worst
 
 
 @pytest.mark.parametrize("V", [1, 2, 4095, 4096 * 3 + 1, 470_000])
