@@ -298,11 +298,12 @@ def test_a_row_of_infinite_logits_gives_no_finite_loss(tb, oracle):
 
 
 @pytest.mark.parametrize("precision", ["bf16", "tf32"])
-@pytest.mark.parametrize("cfg", [(97, 384, 6, 2, 256, 256, 40, 1e-5),      # more row blocks than clusters at once
+@pytest.mark.parametrize("cfg", [(97, 384, 6, 2, 256, 256, 56, 1e-5),      # more row blocks than clusters at once
                                  (97, 256, 4, 2, 64, 33, 5, 1e-5),         # rows that end inside a 32-row strip
-                                 (97, 192, 3, 1, 64, 7, 1, 1e-5),          # one CTA holds the row
-                                 (97, 768, 12, 1, 64, 100, 2, 1e-5)],      # four CTAs
-                         ids=["waves", "ragged", "one_cta", "four_ctas"])
+                                 (97, 192, 3, 1, 64, 7, 1, 1e-5),          # three CTAs hold a row
+                                 (97, 192, 3, 1, 64, 137, 50, 1e-5),       # one CTA
+                                 (97, 768, 12, 1, 64, 231, 8, 1e-5)],      # four CTAs of the widest tiles
+                         ids=["waves", "ragged", "three_ctas", "one_cta", "four_ctas"])
 def test_rmsnorm_in_the_projection_epilogues(tb, oracle, monkeypatch, cfg, precision):
     """RMSNorm of the out- and down-projections' results inside their epilogues against the separate kernel."""
     from turkce_llm_b200.gpu_train import GRADS
@@ -315,8 +316,30 @@ def test_rmsnorm_in_the_projection_epilogues(tb, oracle, monkeypatch, cfg, preci
             monkeypatch.setenv("TB_NO_FUSED_NORM", "1")
         g, p, off, num = make_params(oracle, cfg, 3, tb.PREC_TF32 if precision == "tf32" else tb.PREC_BF16)
         g.upload(p)
-        got.append((g.forward_backward(ids, tgt), g.download(GRADS)))
+        before = tb.launch_count()
+        got.append((g.forward_backward(ids, tgt), g.download(GRADS), tb.launch_count() - before))
         g.destroy()
+    assert got[0][2] == got[1][2] - 2 * L - 1          # (every norm of the forward pass but none of the backward)
     assert abs(got[0][0] - got[1][0]) <= 2e-5 * abs(got[1][0])
     for i, (o, n) in enumerate(zip(off, num)):
         assert rel_to_maxabs(got[0][1][o:o + n], got[1][1][o:o + n]) <= 1e-2, "parameter %d" % i
+
+
+@pytest.mark.parametrize("precision,cfg,fused", [("bf16", (97, 384, 6, 1, 64, 128, 8, 1e-5), True), ("tf32", (97, 384, 6, 1, 64, 128, 8, 1e-5), False),
+                                                 ("bf16", (97, 512, 8, 1, 64, 128, 33, 1e-5), True), ("bf16", (97, 512, 8, 1, 64, 128, 74, 1e-5), False),
+                                                 ("bf16", (97, 768, 12, 1, 64, 128, 64, 1e-5), False), ("tf32", (97, 256, 4, 1, 64, 128, 88, 1e-5), False)])
+def test_rmsnorm_is_in_the_epilogues_where_that_is_faster(tb, oracle, monkeypatch, precision, cfg, fused):
+    """Widths and row counts on either side of the lines that the rule draws (its measurements are beside it)."""
+    V, D, H, L, F, T, B, eps = cfg
+    ids = np.zeros(B * T, np.uint32)
+    launches = []
+    for separate in (False, True):
+        if separate:
+            monkeypatch.setenv("TB_NO_FUSED_NORM", "1")
+        g, p, _, _ = make_params(oracle, cfg, 3, tb.PREC_TF32 if precision == "tf32" else tb.PREC_BF16)
+        g.upload(p)
+        before = tb.launch_count()
+        g.eval_loss(ids, ids)
+        launches.append(tb.launch_count() - before)
+        g.destroy()
+    assert (launches[0] < launches[1]) == fused, launches

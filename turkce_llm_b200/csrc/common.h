@@ -161,7 +161,7 @@ struct GemmArgs {
     bf16 *rope_k = nullptr, *rope_v = nullptr;
     int rope_kv_rows = 0;
     // RMSNorm of the result in the epilogue (kind NN with a residual, C32 = the residual stream): norm16 or norm32 [M, N] =
-    // C32 * norm_w / sqrt(mean(C32^2) + norm_eps), norm_rinv [M] (optional) = 1 / sqrt(..).  gemm_norm_supported(N).
+    // C32 * norm_w / sqrt(mean(C32^2) + norm_eps), norm_rinv [M] (optional) = 1 / sqrt(..).  gemm_norm_pays.
     const float* norm_w = nullptr; float norm_eps = 0.f;
     float* norm_rinv = nullptr; bf16* norm16 = nullptr; float* norm32 = nullptr;
     int ce_mode = 0;
@@ -173,8 +173,9 @@ struct GemmArgs {
 };
 
 int launch_gemm_bf16(DeviceCtx* ctx, const GemmArgs& a, cudaStream_t stream);
-// whether rows of N columns can be split into tiles over the CTAs of a cluster (GemmArgs::norm_w)
-bool gemm_norm_supported(const DeviceCtx* ctx, int N);
+// whether GemmArgs::norm_w is to be used for products of M x N: rows of N columns can be split into tiles over the CTAs of a
+// cluster, and that is faster than a norm kernel behind the product
+bool gemm_norm_pays(const DeviceCtx* ctx, int M, int N, bool tf32);
 // split-K with caller-provided partial-sum storage (needs splits*batch*M*N floats)
 int launch_gemm_bf16_ws(DeviceCtx* ctx, const GemmArgs& a, float* workspace, size_t workspace_floats,
                         cudaStream_t stream);

@@ -302,7 +302,7 @@ int tb_decoder_prefill(TbDecoder* g, const uint32_t* h_ids, int prompt_len) {
     int* h_state = reinterpret_cast<int*>(g->h_pinned + N);
     h_state[0] = T; h_state[1] = 0;
     TB_CUDA(cudaMemcpyAsync(g->pos, h_state, 2 * sizeof(int), cudaMemcpyHostToDevice, st));
-    const bool norm = g->L > 0 && gemm_norm_supported(c, D) && getenv("TB_NO_FUSED_NORM") == nullptr;
+    const bool norm = g->L > 0 && gemm_norm_pays(c, N, D, false) && getenv("TB_NO_FUSED_NORM") == nullptr;
     if (norm) TB_TRY(launch_embed_norm(c, P32(g, 0), g->ids, g->x, P32(g, pidx(0, PK_ATTN_NORM)), g->n, nullptr, nullptr, N, D, g->eps, st));
     else TB_TRY(launch_embed_fwd(c, P32(g, 0), g->ids, g->x, N, D, st));
     for (int l = 0; l < g->L; ++l) {

@@ -1257,11 +1257,18 @@ static int make_map_out(CUtensorMap* map, const void* ptr, int elem_bytes, long 
 
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// Width of the tiles whose row sums are exchanged: N / width CTAs of a cluster share a row block.  The widths divide N, so
-// that every CTA of a cluster has a whole tile; the choice weighs waves of clusters against tile width like pick_bn.  Clusters
-// of three or four do not fill the chip (SMs per processor cluster), so they are taken where one wave of them holds all row
-// blocks: D = 384, validation loss of 5 x 777 tokens 911 us on 3 x 128 against 943 on 2 x 192, step of 8 x 1024 4611 against 4429.
-static int pick_norm_bn(const DeviceCtx* ctx, int M, int N) {
+// Width of the tiles whose row sums are exchanged, or 0 where a product and a norm kernel behind it are faster.  N / width CTAs
+// of a cluster share a row block; the widths divide N, so that every CTA of a cluster has a whole tile.  The choice weighs waves
+// of clusters against tile width like pick_bn.  Figures: forward pass of 6 layers with d_ff 1024, us, this epilogue : separate norms.
+//  * Clusters of three or four do not fill the chip (SMs per processor cluster) and every further wave of them costs a whole one:
+//    in one wave 361 : 410 (width 512, 31 row blocks) and 469 : 554 (768), in more 801 : 667 (512, 74) and 1570 : 1357 (768,
+//    112), so only where one holds all row blocks.
+//  * Float32 operands take twice the time per tile, and a last wave that is nearly empty is not made up for: two CTAs, 88 row
+//    blocks on 74 clusters 1045 : 1007 (width 384) and 859 : 819 (256), 112 on them 1229 : 1273.  (bf16, 88: 619 : 615, 502 : 523.)
+//  * With a handful of row blocks tiles of 128 columns and more leave most of the chip idle, where the separate product takes 64:
+//    bf16 one row block 221 : 217 (384) and 285 : 276 (768), four 233 : 233 and 307 : 330; float32 four 350 : 324 and 457 : 446,
+//    eight 360 : 349 and 480 : 483, sixteen 415 : 412 and 557 : 577.
+static int pick_norm_bn(const DeviceCtx* ctx, int M, int N, bool tf32) {
     static const double factor[3] = {1.30, 1.00, 0.95};
     const long long mt = (M + BM - 1) / BM;
     int best = 0;
@@ -1269,16 +1276,19 @@ static int pick_norm_bn(const DeviceCtx* ctx, int M, int N) {
     for (int bn = 64; bn <= 192; bn += 64) {
         const int nc = N / bn;
         if (N % bn != 0 || nc > NORM_MAX_CTAS) continue;
-        const long long fit = std::max(1, (nc > 2 ? ctx->sm_count * 4 / 5 : ctx->sm_count) / nc);
-        const double cost = (double)((mt + fit - 1) / fit) * bn * factor[bn / 64 - 1];
+        const long long fit = std::max(1, (nc > 2 ? ctx->sm_count * 9 / 10 : ctx->sm_count) / nc), waves = (mt + fit - 1) / fit;
+        if (nc > 2 && waves > 1) continue;
+        if (nc == 2 && tf32 && waves > 1 && mt * 10 < waves * fit * 7) continue;
+        if (bn >= 128 && mt * nc < (tf32 ? 36 : 12)) continue;
+        const double cost = (double)waves * bn * factor[bn / 64 - 1];
         if (cost < best_cost - 1e-9) { best_cost = cost; best = bn; }
     }
     return best;
 }
-bool gemm_norm_supported(const DeviceCtx* ctx, int N) { return pick_norm_bn(ctx, BM, N) > 0; }
+bool gemm_norm_pays(const DeviceCtx* ctx, int M, int N, bool tf32) { return pick_norm_bn(ctx, M, N, tf32) > 0; }
 
 static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
-    if (a.norm_w) return pick_norm_bn(ctx, a.M, a.N);
+    if (a.norm_w) return pick_norm_bn(ctx, a.M, a.N, a.tf32);
     // time ~ waves x tile width x a factor for how often a tile re-reads its operands from L2
     // (flops per operand byte: 43 for 128x64, 64 for 128x128, 77 for 128x192, 128 for a CTA pair on 256x256).
     // 256 = a CTA pair on a 256 x 256 tile: per output element a CTA pulls 0.6x the operand bytes of a

@@ -632,7 +632,7 @@ int tb_trainer_create_prec(TbTrainer** out, int V, int D, int H, int L, int F, i
     g->fused_dswiglu = g->fused_swiglu && getenv("TB_NO_FUSED_DSWIGLU") == nullptr;
     g->fused_rope = (D / H == 32 || D / H == 64) && getenv("TB_NO_FUSED_ROPE") == nullptr;
     // (parameters start at multiples of 8 scalars in the flat buffers: d_model, d_ff and head_dim are multiples of 8)
-    g->fused_norm = gemm_norm_supported(g->ctx, D) && getenv("TB_NO_FUSED_NORM") == nullptr;
+    g->fused_norm = gemm_norm_pays(g->ctx, B * T, D, g->tf32) && getenv("TB_NO_FUSED_NORM") == nullptr;
     g->V = V; g->D = D; g->H = H; g->L = L; g->F = F; g->T = T; g->B = B; g->N = B * T; g->hd = D / H;
     g->Vp = round_up(V, 8);
     g->Tp = round_up(T, 8);
