@@ -465,6 +465,15 @@ def test_pinned_arrays_are_not_staged(tb):
     assert best[True] < 0.8 * best[False], best
 
 
+@pytest.mark.parametrize("missing", [0, 1, 2])
+def test_matmul_host_refuses_a_null_array(tb, missing):
+    """(it is read and written by the host's own copies, not by the driver, which would refuse it)"""
+    arrays = [np.ones((64, 64), np.float32) for _ in range(3)]
+    arrays[missing] = None
+    with pytest.raises(tb.TbError, match="NULL"):
+        tb.matmul_host(*arrays, 64, 64, 64)
+
+
 def test_matmul_host_from_more_threads_than_there_are_copy_buffers(tb):
     """Sixteen threads with products of one row block and of several: more transfers at a time than there are helper threads or
     pinned buffers, so that all three ways to copy are taken."""

@@ -393,6 +393,7 @@ thread_local MatmulSlot t_slots[8];
 int tb_matmul_host(const float* h_A, const float* h_B, float* h_C, int M, int K, int N, int precision) {
     DeviceCtx* ctx;
     TB_TRY(get_ctx(&ctx));
+    TB_CHECK(h_A && h_B && h_C, "tb_matmul_host: NULL array");
     TB_CHECK(M > 0 && N > 0 && K > 0, "matmul dims must be positive");
     const size_t na = (size_t)M * K, nb = (size_t)K * N, nc = (size_t)M * N;
     MatmulSlot* slot = nullptr;
