@@ -8,8 +8,7 @@
 //
 // What bounds it, and what follows from that:
 //  * The chain of dependent phases (five per layer).  With a grid barrier and a re-load of the activations behind it a
-//    phase cost ~6 us (366 us per step of 64 sequences); the exchange through distributed shared memory takes 0.2 us for one
-//    sequence per cluster and 0.8 us for ten (a CTA takes in ~14 bytes per clock from its 15 peers).
+//    phase cost ~6 us (366 us per step of 64 sequences); now all five take 10 us for one sequence per cluster and 15 for ten.
 //  * Bytes: a CTA needs its slice of every weight matrix and the cache rows of its pairs.  None of them depends on the
 //    step's own results (the new cache row is handled apart), so ONE producer warp streams them in the order of use
 //    through a ring of ~130 KB that runs ahead of the chain, instead of in bursts behind each barrier.
@@ -20,9 +19,10 @@
 //    multiplies activation columns a, the off-diagonal blocks are ignored, the diagonal blocks added in a fixed order.
 //  * Attention: one pass over the cache rows, a warp per 32 rows with a key per lane, float32 products of the float32 query and
 //    probability with the bf16 cache rows; the partial results of a pair's warps are merged at the end.
-// Measured, 12 layers of width 384 (host loop of generate() with the LM head behind it): 64 sequences, cache 128 .. 255:
-// 366 -> ~200 us per step; one sequence: 267 -> ~110 us.  What is left is instruction latency: a layer is ~17,000 clocks for
-// one sequence, of which the tensor core works ~4,500 and the exchanges take ~2,000.
+// Measured, 12 layers of width 384, generate() with the LM head behind it: 64 sequences, cache 128 .. 256: 366 -> 207 us per step,
+// 896 .. 1024: 719 -> 390; one sequence 267 -> 127 us.  What is left is latency: 64 sequences are 29,700 clocks per layer under
+// ncu, with the tensor pipe active in 4 % of them, 27 % of the issue slots used and 1.1 TB/s from DRAM; most stalls are at the
+// barriers between the steps of a phase.
 //
 // Replaces, for the decode step, the reference's re-run of lm_forward over the whole window per generated token
 // (training/generate.c:186-212).
