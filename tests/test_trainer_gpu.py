@@ -343,3 +343,23 @@ def test_rmsnorm_is_in_the_epilogues_where_that_is_faster(tb, oracle, monkeypatc
         launches.append(tb.launch_count() - before)
         g.destroy()
     assert (launches[0] < launches[1]) == fused, launches
+
+
+@pytest.mark.parametrize("T,B", [(31, 9), (45, 7), (64, 6), (777, 2)])
+def test_rotation_tables_by_tma(tb, oracle, monkeypatch, T, B):
+    """Cosines and sines that come in by TMA, 32 positions at a time, against those read row by row (64-byte output rows): the same
+    bits, also where 32 rows lie in two sequences and where the last rows are missing."""
+    from turkce_llm_b200.gpu_train import GRADS
+    cfg = (97, 128, 2, 2, 192, T, B, 1e-5)
+    rng = np.random.default_rng(T)
+    ids, tgt = (rng.integers(0, 97, B * T).astype(np.uint32) for _ in range(2))
+    got = []
+    for rows in (False, True):
+        if rows:
+            monkeypatch.setenv("TB_GEMM_NO_WIDE16", "1")
+        g, p, _, _ = make_params(oracle, cfg, 5)
+        g.upload(p)
+        got.append((g.forward_backward(ids, tgt), g.download(GRADS)))
+        g.destroy()
+    assert got[0][0] == got[1][0]
+    assert np.array_equal(got[0][1].view(np.uint32), got[1][1].view(np.uint32))

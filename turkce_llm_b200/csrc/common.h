@@ -157,6 +157,7 @@ struct GemmArgs {
     bf16* rope_qkv = nullptr;
     const float* rope_cos = nullptr; const float* rope_sin = nullptr;
     int rope_T = 0, rope_H = 0, rope_hd = 0;
+    int rope_rows = 0;                      // rows of the tables where rope_sin lies directly behind rope_cos (0: not known)
     // K and V elsewhere (both, with rope_kv_rows >= T rows per head): a KV cache.  rope_qkv then receives Q alone.
     bf16 *rope_k = nullptr, *rope_v = nullptr;
     int rope_kv_rows = 0;

@@ -253,7 +253,8 @@ int tb_decoder_create(TbDecoder** out, int V, int D, int H, int L, int F, int ma
                 ct[(size_t)p * half + k] = cosf(angle);
                 sn[(size_t)p * half + k] = sinf(angle);
             }
-        TB_TRY(dalloc(g, &g->cos_t, ct.size())); TB_TRY(dalloc(g, &g->sin_t, sn.size()));
+        TB_TRY(dalloc(g, &g->cos_t, 2 * ct.size()));          // cosines, then sines: see GemmArgs::rope_rows
+        g->sin_t = g->cos_t + ct.size();
         TB_H2D_SYNC(g->cos_t, ct.data(), ct.size() * 4);
         TB_H2D_SYNC(g->sin_t, sn.data(), sn.size() * 4);
     }
@@ -313,7 +314,7 @@ int tb_decoder_prefill(TbDecoder* g, const uint32_t* h_ids, int prompt_len) {
             s.kind = GEMM_NN; s.A = g->n; s.B = P16(g, pidx(l, PK_WQKV)); s.M = N; s.N = 3 * D; s.K = D; s.lda = D; s.ldb = 3 * D;
             s.bias = P32(g, pidx(l, PK_BQKV)); s.splits = 1;
             s.rope_qkv = g->Q; s.rope_k = g->Kc[l]; s.rope_v = g->Vc[l]; s.rope_kv_rows = g->cap;
-            s.rope_cos = g->cos_t; s.rope_sin = g->sin_t; s.rope_T = T; s.rope_H = H; s.rope_hd = hd;
+            s.rope_cos = g->cos_t; s.rope_sin = g->sin_t; s.rope_T = T; s.rope_H = H; s.rope_hd = hd; s.rope_rows = g->cap;
             TB_TRY(launch_gemm_bf16_ws(c, s, g->splitk_ws, g->splitk_floats, st));
         } else {
             TB_TRY(linear(g, g->n, P16(g, pidx(l, PK_WQKV)), P32(g, pidx(l, PK_BQKV)), nullptr, g->qkv, N, 3 * D, D));

@@ -83,9 +83,10 @@ struct GemmParams {
                                 // 4: softmax statistics only (cross-entropy pass 1), nothing stored
                                 // 5: bf16 tiles into [3][B][H][T][hd] with q, k rotated (tmC is a 5-D map)
     const float* rope_cos; const float* rope_sin; int rope_T, rope_H, rope_hd;
-    int rope_direct;            // the tiles leave by ordinary stores, row by row: sequences whose length is no multiple of 32,
-    bf16 *rope_q, *rope_k, *rope_v;   // or K and V in a cache with rope_kv_rows rows per head
+    int rope_direct;            // 1: 32 rows that lie in two sequences leave by ordinary stores, row by row; 2: all do (K and V in a
+    bf16 *rope_q, *rope_k, *rope_v;   // cache with rope_kv_rows rows per head)
     int rope_kv_rows;
+    int rope_tab;               // the rotation tables of 32 rows come in by TMA (tmR)
     int ce_mode;                // 2: bf16 tile stores carry (exp(z - lse[row]) - onehot) * ce_scale
     const uint32_t* ce_targets; float* ce_stats; float* ce_ztarget; const float* ce_lse; float ce_scale;
     int pair_off;               // mode 3: F; tile columns [0,BN/2) are gate columns n0/2.., [BN/2,BN) up columns F + n0/2..
@@ -677,9 +678,22 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             // mode 5: position of this thread's row, and of the 32-row chunk, inside its sequence (once per tile)
             const int rope_D = p.rope_H * p.rope_hd, rope_shift = p.rope_hd == 64 ? 6 : 5;
             int rope_b = 0, rope_t0 = 0, rope_t = 0;
+            bool rope_direct = false;
+            // Head dim 64: the rotation of these 32 positions, cosines and sines, comes in beside the main loop (8 KB, behind one
+            // output buffer) and serves every head of the tile.  Read by the rows' threads from global memory it was 16 accesses
+            // of 32 different lines each per head and row, and the epilogue took longer than the main loop: QKV projection of
+            // 8192, 3885 and 11200 rows of 384 in the live step 20, 14 and 30 us that way, 16.8, 11.3 and 25 this way.
+            const bool rope_tab = EPI == EPI_ROPE && p.rope_tab != 0;
+            bool rope_wait = false;
             if (m_rope) {
                 rope_b = gm0 / p.rope_T; rope_t0 = gm0 - rope_b * p.rope_T; rope_t = rope_t0 + lane;
                 if (rope_t >= p.rope_T) rope_t %= p.rope_T;          // (only where 32 rows can lie in two sequences)
+                rope_direct = p.rope_direct == 2 || (p.rope_direct == 1 && rope_t0 + 32 > p.rope_T);
+                rope_wait = rope_tab && rows_in && col0 < 2 * rope_D;
+                if (rope_wait && lane == 0) {
+                    mbar_expect_tx(rbar, 8192);
+                    tma_load_3d(obuf + 4096, &tmR, rbar, 0, rope_t0, 0);
+                }
             }
             if (m_res && lane == 0 && rows_in && col0 < p.N) {
                 mbar_expect_tx(rbar, 4096);
@@ -702,11 +716,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 // with dsw a unit fills both output buffers (dg | du), else the units alternate between them
                 const bool paired = m_wide && ((ch & 1) || ch + 1 < NCH);
                 const bool second = paired && (ch & 1);
-                const uint32_t b = m_dsw ? 0u : (cnt & 1u);
+                const uint32_t b = (m_dsw || rope_tab) ? 0u : (cnt & 1u);
                 const int gn0 = col0 + ch * 32;
                 const bool active = rows_in && gn0 < p.N;
                 if (lane == 0 && !second) {                   // the unit's output buffer has been read out
-                    if (m_dsw) tma_store_wait_read<0>(); else tma_store_wait_read<1>();
+                    if (m_dsw || rope_tab) tma_store_wait_read<0>(); else tma_store_wait_read<1>();
                 }
                 __syncwarp();
                 uint32_t v[32];
@@ -757,10 +771,25 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     if (gn0 < 2 * rope_D) {
                         const int d0 = (gn0 - (gn0 >= rope_D ? rope_D : 0)) & (p.rope_hd - 1);
                         const long long off = (long long)rope_t * (p.rope_hd >> 1) + (d0 >> 1);
+                        if (rope_wait) {
+                            if (!mbar_wait(rbar, rphase, abort_flag)) { ok = false; break; }
+                            rphase ^= 1u;
+                            rope_wait = false;
+                        }
+                        // (rows of the next sequence are read where they are)
+                        const bool tab = rope_tab && rows_in && rope_t0 + lane < p.rope_T;
+                        const uint8_t* trow = obuf + 4096 + lane * 128;
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            const float4 c4 = __ldg(reinterpret_cast<const float4*>(p.rope_cos + off) + j);
-                            const float4 s4 = __ldg(reinterpret_cast<const float4*>(p.rope_sin + off) + j);
+                            float4 c4, s4;
+                            if (tab) {
+                                const int so = (((d0 >> 3) + j) ^ (lane & 7)) << 4;
+                                c4 = *reinterpret_cast<const float4*>(trow + so);
+                                s4 = *reinterpret_cast<const float4*>(trow + 4096 + so);
+                            } else {
+                                c4 = __ldg(reinterpret_cast<const float4*>(p.rope_cos + off) + j);
+                                s4 = __ldg(reinterpret_cast<const float4*>(p.rope_sin + off) + j);
+                            }
                             const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
                             for (int i = 0; i < 4; ++i) {
@@ -855,8 +884,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     }
                 }
                 if (paired && !second) continue;              // the unit leaves after its second chunk
-                if (m_rope && p.rope_direct) {
+                if (m_rope && rope_direct) {
                     // row by row: 8 (head dim 64) or 4 adjacent lanes write a row's values of one head, 128 or 64 bytes
+                    fence_proxy_async();              // (the tables' place is written by the next tile's copy)
                     __syncwarp();
                     const int g0 = paired ? gn0 - 32 : gn0;
                     if (rows_in && g0 < p.N) {
@@ -1525,7 +1555,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
     p.ce_lse = a.ce_lse; p.ce_scale = a.ce_scale;
     p.bias_vec = p.bias && aligned16(p.bias);
     p.rope_cos = a.rope_cos; p.rope_sin = a.rope_sin; p.rope_T = a.rope_T; p.rope_H = a.rope_H; p.rope_hd = a.rope_hd;
-    p.rope_direct = 0;
+    p.rope_direct = 0; p.rope_tab = 0;
     p.norm_w = a.norm_w; p.norm_eps = a.norm_eps; p.norm_inv_n = 1.0f / (float)a.N; p.norm_rinv = a.norm_rinv;
     p.norm16 = a.norm16; p.norm32 = a.norm32;
     if (a.ce_mode == 1) {
@@ -1538,7 +1568,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         cuuint64_t strides[4] = {hd * 2, T * hd * 2, H * T * hd * 2, Bn * H * T * hd * 2};
         // head dim 64 on 128- or 256-column tiles: a warp's chunk pairs are whole heads and leave in rows of 128 bytes
         const bool wide = a.rope_hd == 64 && (bn == 128 || bn == 256) && getenv("TB_GEMM_NO_WIDE16") == nullptr;
-        p.rope_direct = (a.rope_T % 32 != 0 || a.rope_kv_rows > 0) ? 1 : 0;
+        p.rope_direct = a.rope_kv_rows > 0 ? 2 : a.rope_T % 32 != 0 ? 1 : 0;
         p.rope_q = a.rope_qkv;
         p.rope_k = a.rope_k ? a.rope_k : a.rope_qkv + (long long)a.M * a.rope_H * a.rope_hd;
         p.rope_v = a.rope_v ? a.rope_v : a.rope_qkv + 2LL * a.M * a.rope_H * a.rope_hd;
@@ -1551,6 +1581,17 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         p.wide16 = wide ? 1 : 0;
         TB_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled (QKV output) failed with code %d", (int)r);
         p.tma_mode = 5;
+        // The tables come in by TMA where they are one array, the sines behind the cosines (the trainer's and the decoder's are); a
+        // map whose outer stride spans two allocations is not used.
+        if (wide && a.rope_sin == a.rope_cos + (size_t)a.rope_rows * (hd / 2) && a.rope_rows >= a.rope_T && aligned16(a.rope_cos)) {
+            const cuuint64_t rows = (cuuint64_t)a.rope_rows;
+            cuuint64_t tdims[3] = {hd / 2, rows, 2}, tstrides[2] = {hd * 2, rows * hd * 2};
+            cuuint32_t tbox[3] = {32u, 32u, 2u};
+            r = enc(&tmR, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(a.rope_cos), tdims, tstrides, tbox, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            TB_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled (rotation tables) failed with code %d", (int)r);
+            p.rope_tab = 1;
+        }
     } else if (a.dsw_dgu) {
         TB_CHECK(bn == 128 || bn == 256, "SwiGLU-backward GEMM: tiles of 128 or 256 columns (chunks leave in pairs)");
         TB_TRY(make_map_out(&tmC, a.dsw_dgu, 2, 2 * a.N, a.M, a.ldgu, 1, 0, 1, 0, true));

@@ -236,7 +236,7 @@ int forward(TbTrainer* g, bool want_grad) {
             s.kind = GEMM_NN; s.A = g->tf32 ? (const void*)a.n1_32 : (const void*)a.n1; s.B = WOP(g, pidx(l, PK_WQKV)); s.tf32 = g->tf32;
             s.M = N; s.N = 3 * D; s.K = D; s.lda = D;
             s.ldb = 3 * D; s.bias = P32(g, pidx(l, PK_BQKV)); s.splits = 1;
-            s.rope_qkv = a.Q; s.rope_cos = g->cos_t; s.rope_sin = g->sin_t; s.rope_T = T; s.rope_H = H; s.rope_hd = hd;
+            s.rope_qkv = a.Q; s.rope_cos = g->cos_t; s.rope_sin = g->sin_t; s.rope_T = T; s.rope_H = H; s.rope_hd = hd; s.rope_rows = T;
             if (const char* e = getenv("TB_ROPE_BN")) s.bn = atoi(e);
             TB_TRY(gemm(g, s));
         } else {
@@ -779,7 +779,8 @@ int tb_trainer_create_prec(TbTrainer** out, int V, int D, int H, int L, int F, i
                 ct[(size_t)pos * half + k] = cosf(angle);
                 sn[(size_t)pos * half + k] = sinf(angle);
             }
-        TB_TRY(dalloc(g, &g->cos_t, ct.size())); TB_TRY(dalloc(g, &g->sin_t, sn.size()));
+        TB_TRY(dalloc(g, &g->cos_t, 2 * ct.size()));          // cosines, then sines: see GemmArgs::rope_rows
+        g->sin_t = g->cos_t + ct.size();
         TB_H2D_SYNC(g->cos_t, ct.data(), ct.size() * 4);
         TB_H2D_SYNC(g->sin_t, sn.data(), sn.size() * 4);
     }
