@@ -363,3 +363,30 @@ def test_rotation_tables_by_tma(tb, oracle, monkeypatch, T, B):
         g.destroy()
     assert got[0][0] == got[1][0]
     assert np.array_equal(got[0][1].view(np.uint32), got[1][1].view(np.uint32))
+
+
+@pytest.mark.parametrize("precision", ["bf16", "tf32"])
+@pytest.mark.parametrize("T,B", [(128, 64), (777, 11)], ids=["whole_tiles", "ragged"])
+def test_tiles_over_the_whole_width_beside_another_product(tb, oracle, monkeypatch, T, B, precision):
+    """256 x 384 tiles of the input gradients and, formed the other way round, of the weight gradients against the narrower tiles:
+    the same operands summed in another order.  A gradient passes through bf16 (8 bits) a few times on its way, so where a sum falls
+    on the other side of a rounding it moves by 2^-9 of itself."""
+    from turkce_llm_b200.gpu_train import GRADS
+    cfg = V, D, H, L, F, _, _, eps = (97, 384, 6, 2, 1024, T, B, 1e-5)
+    rng = np.random.default_rng(4)
+    ids, tgt = (rng.integers(0, V, B * T).astype(np.uint32) for _ in range(2))
+    got = []
+    for narrow in (False, True):
+        if narrow:
+            monkeypatch.setenv("TB_GEMM_NO_384", "1")
+        g, p, off, num = make_params(oracle, cfg, 3, tb.PREC_TF32 if precision == "tf32" else tb.PREC_BF16)
+        g.upload(p)
+        loss = g.forward_backward(ids, tgt)
+        grads = g.download(GRADS)
+        g.zero_grads()
+        assert g.forward_backward(ids, tgt) == loss and np.array_equal(g.download(GRADS), grads)
+        got.append((loss, grads))
+        g.destroy()
+    assert got[0][0] == got[1][0]
+    for i, (o, n) in enumerate(zip(off, num)):
+        assert rel_to_maxabs(got[0][1][o:o + n], got[1][1][o:o + n]) <= 2.0 ** -9, "parameter %d" % i

@@ -199,6 +199,7 @@ int tb_gemm_bf16(int kind, const void* d_A, const void* d_B, int M, int N, int K
     a.alpha = alpha; a.beta = beta;
     a.causal = static_cast<CausalMode>(causal);
     a.splits = splits; a.bn = tile_n;
+    TB_CHECK(!(tile_n == 384 && kind == GEMM_NT), "384-wide CTA-pair tiles take B stored [K, N] (kinds NN and TN)");
     return launch_gemm_bf16(ctx, a, S(stream));
 }
 
@@ -286,7 +287,7 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
         const size_t b_bytes = round_up((size_t)b_stride * batch * 2, 256);
         g.lda = a_ld; g.ldb = b_ld; g.strideA = a_stride; g.strideB = b_stride;
         const int splits = planned_splits(ctx, g);
-        g.splits = splits;
+        g.splits = splits; g.planned = true;
         const size_t ws_floats = splits > 1 ? (size_t)splits * batch * M * N : 0;
         TB_TRY(take_scratch(a_bytes + b_bytes + ws_floats * sizeof(float)));
         bf16* pb = reinterpret_cast<bf16*>(scratch);
@@ -315,7 +316,7 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
     if (split3) g.K = 3 * K;
     g.lda = a_ld; g.ldb = b_ld; g.strideA = a_stride; g.strideB = b_stride;
     const int splits = planned_splits(ctx, g);
-    g.splits = splits;
+    g.splits = splits; g.planned = true;
     const size_t ws_floats = splits > 1 ? (size_t)splits * batch * M * N : 0;
     TB_TRY(take_scratch(a_bytes + b_bytes + ws_floats * sizeof(float)));
     float* pb = reinterpret_cast<float*>(scratch);

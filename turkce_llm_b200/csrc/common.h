@@ -128,7 +128,9 @@ struct GemmArgs {
     float alpha = 1.0f, beta = 0.0f;        // beta applies to the previous contents of C32
     CausalMode causal = CAUSAL_NONE;
     int splits = 0;                         // 0 = choose; >1 uses scratch for fixed-order partial sums
+    bool planned = false;                   // splits is what planned_splits gave for this product
     int bn = 0;                             // 0 = choose tile width (64, 128 or 192; 256 = a CTA pair on a 256 x 256 tile)
+    bool swapped = false;                   // (set by the launcher) A and B, M and N are exchanged and the reduction turns C^T; splits > 1
     int max_ctas = 0;                       // > 0: at most this many CTAs (two products that share the SMs side by side)
     // SwiGLU backward in the epilogue (bf16 NT product with N = F, the input gradient of the down-projection): the
     // product dh [M, F] is not stored; with the saved gate|up projection dsw_gu [M, 2F] (leading dimension ldgu) the

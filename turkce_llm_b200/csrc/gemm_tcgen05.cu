@@ -266,7 +266,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                         for (int j = 0; j < BM / MNW; ++j) load(sA + j * MN_BOX_BYTES, &tmA, c.m0 + j * MNW, kb * BKE, c.z);
                     }
                     const int nb0 = c.n0 + (int)rank * BNL;          // first B column this CTA loads
-                    if (!p.b_mn) {
+                    if (!p.b_mn && BN == 384) {
+#pragma unroll
+                        for (int j = 0; j < 3; ++j) load(sB + j * 64 * ROW_BYTES, &tmB, kb * BKE, c.n0 + 128 * j + 64 * (int)rank, c.z);
+                    } else if (!p.b_mn) {
                         load(sB, &tmB, kb * BKE, nb0, c.z);
                     } else {
 #pragma unroll
@@ -1136,6 +1139,47 @@ __global__ void reduce_splits_kernel(const float* __restrict__ part, float* __re
     }
 }
 
+// The same for a product formed the other way round (C^T = op(B)^T op(A)^T, GemmArgs::swapped): the partials are [M, N], out is
+// [N, M].  A block turns a 32 x 32 tile through shared memory, so that both sides are read and written in rows of 128 bytes.
+__global__ void __launch_bounds__(256) reduce_splits_turned_kernel(const float* __restrict__ part, float* __restrict__ out, int M, int N,
+                                                                   long long ldc32, int splits, float beta) {
+    __shared__ float tile[32][33];
+    pdl_wait();
+    pdl_launch_dependents();
+    const long long per = (long long)M * N;
+    const int m0 = blockIdx.y * 32, n0 = blockIdx.x * 32;
+    const int hi = threadIdx.x >> 3, lo = (threadIdx.x & 7) * 4;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (m0 + hi < M && n0 + lo < N) {                     // (N is a multiple of 4)
+        const float* src = part + (long long)(m0 + hi) * N + n0 + lo;
+        int k = 0;
+        for (; k + 4 <= splits; k += 4) {
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = *reinterpret_cast<const float4*>(src + (long long)(k + u) * per);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) { s.x += v[u].x; s.y += v[u].y; s.z += v[u].z; s.w += v[u].w; }
+        }
+        for (; k < splits; ++k) {
+            const float4 v = *reinterpret_cast<const float4*>(src + (long long)k * per);
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+    }
+    tile[hi][lo] = s.x; tile[hi][lo + 1] = s.y; tile[hi][lo + 2] = s.z; tile[hi][lo + 3] = s.w;
+    __syncthreads();
+    if (n0 + hi < N) {
+        float* o = out + (long long)(n0 + hi) * ldc32 + m0 + lo;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (m0 + lo + e < M) {
+                float v = tile[lo + e][hi];
+                if (beta != 0.0f) v += beta * o[e];
+                o[e] = v;
+            }
+        }
+    }
+}
+
 // ===================================================================== host side
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1326,17 +1370,18 @@ static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
     const bool pair_ok = a.batch == 1 && a.causal == CAUSAL_NONE && a.c_inner <= 1 && a.M >= 512 &&
                          getenv("TB_GEMM_NO_PAIR") == nullptr;
     const long long mt = (a.M + BM - 1) / BM;
+    const int sms = (a.max_ctas > 0 && a.max_ctas < ctx->sm_count) ? a.max_ctas : ctx->sm_count;
     auto cost_of = [&](int width) -> double {
         static const double factor[4] = {1.30, 1.00, 0.95, 0.70};
         if (width == 256) {
             const long long tiles = ((a.M + 2 * BM - 1) / (2 * BM)) * ((a.N + 255) / 256);
-            const long long pairs = ctx->sm_count / 2;
+            const long long pairs = sms / 2;
             // a narrow output wastes part of the second 256-wide column of tiles; only a long K loop pays for that
             const double narrow = (a.N < 512 && a.K < 64 * (a.tf32 ? BK_TF32 : BK)) ? 1.15 : 1.0;
             return (double)((tiles + pairs - 1) / pairs) * 256 * factor[3] * narrow;
         }
         const long long tiles = mt * ((a.N + width - 1) / width) * a.batch;
-        return (double)((tiles + ctx->sm_count - 1) / ctx->sm_count) * width * factor[width / 64 - 1];
+        return (double)((tiles + sms - 1) / sms) * width * factor[width / 64 - 1];
     };
     if (a.swiglu_h)      // paired gate/up tile: 128 wide, or 256 wide on a CTA pair
         return ((a.bn == 256 || (a.bn == 0 && pair_ok && cost_of(256) < cost_of(128))) && a.N % 256 == 0) ? 256 : 128;
@@ -1362,6 +1407,9 @@ static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
         const long long t192 = mt * ((a.N + 191) / 192) * a.batch;
         return (!a.tf32 && t192 >= 16) ? 192 : 128;
     }
+    // Beside another product, on part of the SMs, tiles are what counts: one 256 x 384 tile over the whole N pulls the operand bytes
+    // of a 128 x 192 one for four times its output, and its longer epilogue (the 1.3) is paid once per wave.
+    const bool wide_ok = pair_ok && a.max_ctas > 0 && a.N > 256 && a.N <= 384 && kb >= 16 && !a.bias && !a.residual && getenv("TB_GEMM_NO_384") == nullptr;
     const int widths[4] = {64, 128, 192, 256};
     int best = 128;
     double best_cost = 1e30;
@@ -1369,6 +1417,7 @@ static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
         const double cost = cost_of(widths[i]);
         if (cost < best_cost - 1e-9) { best_cost = cost; best = widths[i]; }
     }
+    if (wide_ok && (double)(((a.M + 2 * BM - 1) / (2 * BM) + sms / 2 - 1) / (sms / 2)) * 192 * 0.95 * 1.3 < best_cost) best = 384;
     if (a.causal != CAUSAL_NONE && best == 192) best = 128;     // the causal tile rules assume 64 | 128 columns
     return best;
 }
@@ -1389,8 +1438,55 @@ static int choose_splits(const DeviceCtx* ctx, const GemmArgs& a, int bn) {
     return (kb_total + kb_per - 1) / kb_per;     // no empty split
 }
 
-int planned_splits(const DeviceCtx* ctx, const GemmArgs& a) {
-    return (a.residual || a.c_inner > 1) ? 1 : choose_splits(ctx, a, pick_bn(ctx, a));
+// A weight gradient (few tiles, long K, split along it) by the tile that is estimated to take least: operand bytes a CTA pulls at
+// the ~94 KB/us that an SM gets from L2, the last tile's epilogue, and the reduction of the partial slabs at ~6 MB/us.  Candidates
+// are 128- and 192-column tiles and 256 x 384 tiles of a CTA pair, these also with the product formed the other way round
+// (C^T = op(B)^T op(A)^T, turned by the reduction) where it is M that fits 384.  Bytes per flop of the three: 1, 0.83, 0.42.
+// The default rule stays where nothing is expected to beat it by a tenth.
+static GemmArgs arranged(const DeviceCtx* ctx, const GemmArgs& a) {
+    const int bke = a.tf32 ? BK_TF32 : BK;
+    if (a.kind != GEMM_TN || a.bn != 0 || a.swapped || a.batch != 1 || a.causal != CAUSAL_NONE || a.c_inner > 1 || a.bias || a.residual || a.C16 ||
+        !a.C32 || a.N <= 64 || a.K < 16 * bke || (long long)((a.M + BM - 1) / BM) * ((a.N + 127) / 128) * 2 > ctx->sm_count)
+        return a;
+    const int sms = (a.max_ctas > 0 && a.max_ctas < ctx->sm_count) ? a.max_ctas : ctx->sm_count, kb = (a.K + bke - 1) / bke;
+    const int given = a.planned ? 0 : a.splits;
+    auto turned = [&]() {
+        GemmArgs t = a;
+        t.A = a.B; t.B = a.A; t.M = a.N; t.N = a.M; t.lda = a.ldb; t.ldb = a.lda; t.swapped = true;
+        return t;
+    };
+    auto time_of = [&](const GemmArgs& g, int bn) {
+        const bool pair = bn == 384;
+        const int s = given > 0 ? given : choose_splits(ctx, g, bn), per = (kb + s - 1) / s;
+        const long long tiles = (long long)((g.M + (pair ? 2 * BM : BM) - 1) / (pair ? 2 * BM : BM)) * ((g.N + bn - 1) / bn) * s;
+        const int workers = pair ? sms / 2 : sms;
+        const double waves = (double)((tiles + workers - 1) / workers), slab = (double)a.M * a.N * 4e-6;
+        return waves * (per * (bn == 128 ? 32.0 : 40.0) / 94.0 + (pair ? 5.0 : bn == 192 ? 1.8 : 1.2)) +
+               (s == 1 ? 0.0 : 2.0 + (s + 1) * slab / 6.0);
+    };
+    GemmArgs best = a;
+    double least = time_of(a, pick_bn(ctx, a)) * 0.9;
+    auto consider = [&](const GemmArgs& g, int bn) {
+        const double t = time_of(g, bn);
+        if (t < least) { least = t; best = g; best.bn = bn; }
+    };
+    consider(a, 128);
+    if (a.N > 128) consider(a, 192);
+    if (getenv("TB_GEMM_NO_PAIR") == nullptr && getenv("TB_GEMM_NO_384") == nullptr) {
+        if (a.N > 256 && a.N <= 384 && a.M >= 512) consider(a, 384);
+        if (a.M > 256 && a.M <= 384 && a.N >= 512 && a.M % 4 == 0) {
+            const GemmArgs t = turned();
+            const int s = choose_splits(ctx, t, 384);
+            if (s > 1 && (given == 0 || given == s)) consider(t, 384);
+        }
+    }
+    return best;
+}
+
+int planned_splits(const DeviceCtx* ctx, const GemmArgs& a0) {
+    if (a0.residual || a0.c_inner > 1) return 1;
+    const GemmArgs a = arranged(ctx, a0);
+    return choose_splits(ctx, a, pick_bn(ctx, a));
 }
 
 template <int BN, bool TF32, bool PAIR = false, int EPI = EPI_ANY>
@@ -1510,9 +1606,8 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         TB_CHECK(a.batch == 1 && a.causal == CAUSAL_NONE && a.c_inner <= 1,
                  "256-wide CTA-pair tiles take one plain product (no batch, no causal mode)");
     if (bn == 384)
-        TB_CHECK(b_mn && !a.swiglu_h && a.ce_mode == 0 && !a.rope_qkv,
-                 "384-wide CTA-pair tiles take B stored [K, N] (kinds NN and TN) and a plain epilogue");
-    if (!b_mn) TB_TRY(make_operand_map_es(&tmB, a.B, es, a.K, a.N, a.ldb, a.batch, a.strideB, pair ? bn / 2 : bn));
+        TB_CHECK(!a.swiglu_h && a.ce_mode == 0 && !a.rope_qkv, "384-wide CTA-pair tiles take a plain epilogue");
+    if (!b_mn) TB_TRY(make_operand_map_es(&tmB, a.B, es, a.K, a.N, a.ldb, a.batch, a.strideB, bn == 384 ? 64 : pair ? bn / 2 : bn));
     else       TB_TRY(make_operand_map_es(&tmB, a.B, es, a.N, a.K, a.ldb, a.batch, a.strideB, bke, true));
 
     GemmParams p;
@@ -1713,7 +1808,9 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         // take that one's thread slots)
         const bool early = a.max_ctas == 0 || (long long)blocks * a.batch <= kEarlyBlocks;
         prof_mark(ctx, "splitk_reduce", 0.0, (double)(splits + 2) * per * a.batch * 4.0, stream);
-        if (vec4)
+        if (a.swapped)
+            TB_CUDA(launch_kernel_as(early, reduce_splits_turned_kernel, dim3((a.N + 31) / 32, (a.M + 31) / 32), dim3(256), 0, stream, 1, ws, a.C32, a.M, a.N, a.ldc32, splits, a.beta));
+        else if (vec4)
             TB_CUDA(launch_kernel_as(early, (reduce_splits_kernel<4>), dim3(grid), dim3(256), 0, stream, 1, ws, a.C32, a.C16, a.M, a.N, a.ldc32, a.ldc16, splits, a.strideC32, a.strideC16, a.beta, a.bias));
         else
             TB_CUDA(launch_kernel_as(early, (reduce_splits_kernel<1>), dim3(grid), dim3(256), 0, stream, 1, ws, a.C32, a.C16, a.M, a.N, a.ldc32, a.ldc16, splits, a.strideC32, a.strideC16, a.beta, a.bias));
@@ -1735,7 +1832,8 @@ static int check_splits(const GemmArgs& a, int* splits) {
     return 0;
 }
 
-int launch_gemm_bf16(DeviceCtx* ctx, const GemmArgs& a, cudaStream_t stream) {
+int launch_gemm_bf16(DeviceCtx* ctx, const GemmArgs& a0, cudaStream_t stream) {
+    const GemmArgs a = arranged(ctx, a0);
     const int bn = pick_bn(ctx, a);
     int splits = a.splits > 0 ? a.splits : choose_splits(ctx, a, bn);
     TB_TRY(check_splits(a, &splits));
@@ -1748,8 +1846,9 @@ int launch_gemm_bf16(DeviceCtx* ctx, const GemmArgs& a, cudaStream_t stream) {
     return launch_core(ctx, a, bn, splits, ws, stream);
 }
 
-int launch_gemm_bf16_ws(DeviceCtx* ctx, const GemmArgs& a, float* workspace, size_t workspace_floats,
+int launch_gemm_bf16_ws(DeviceCtx* ctx, const GemmArgs& a0, float* workspace, size_t workspace_floats,
                         cudaStream_t stream) {
+    const GemmArgs a = arranged(ctx, a0);
     const int bn = pick_bn(ctx, a);
     int splits = a.splits > 0 ? a.splits : choose_splits(ctx, a, bn);
     TB_TRY(check_splits(a, &splits));
