@@ -572,3 +572,50 @@ def test_matmul_host_in_row_blocks(tb, oracle, shape, precision):
         assert rel_to_maxabs(out, want) <= {"bf16": 2e-2, "tf32": 5e-3, "fp32": 1e-5}[precision]
         A *= -1.0
         want *= -1.0
+
+
+@pytest.mark.parametrize("precision", ["bf16", "tf32"])
+@pytest.mark.parametrize("kind", ["NN", "NT", "TN"])
+@pytest.mark.parametrize("shape", [(200, 72, 1100, 2), (130, 260, 2048, 3), (384, 136, 1024, 5), (64, 64, 4096, 7), (257, 44, 2080, 8), (129, 131, 1500, 0)])
+def test_splits_added_inside_a_cluster(tb, monkeypatch, kind, shape, precision):
+    """Products split along K whose parts a cluster adds: ragged tiles, rows that do not divide by the splits, bias, alpha and beta, a
+    leading dimension that keeps the output from 16-byte accesses, against float64 and the reduction kernel."""
+    M, N, K, splits = shape
+    rng = np.random.default_rng(M + N)
+    A = rng.standard_normal((K, M) if kind == "TN" else (M, K)).astype(np.float32)
+    B = (rng.standard_normal((N, K) if kind == "NT" else (K, N)) * 0.1).astype(np.float32)
+    kn = {"NN": tb.NN, "NT": tb.NT, "TN": tb.TN}[kind]
+    C0 = rng.standard_normal((M, N + 3)).astype(np.float32)
+    got = []
+    for off in (False, True):
+        if off:
+            monkeypatch.setenv("TB_GEMM_NO_CLUSTER_SPLIT", "1")
+        before = tb.launch_count()
+        if precision == "bf16":
+            # (rows of 16 bytes for the operands)
+            pad = lambda X: np.pad(X, ((0, 0), (0, -X.shape[1] % 8)))
+            a, b = torch.from_numpy(pad(A)).cuda().bfloat16(), torch.from_numpy(pad(B)).cuda().bfloat16()
+            C = torch.from_numpy(C0).cuda()
+            bias = torch.from_numpy(C0[0, :N].copy()).cuda()
+            tb.gemm_bf16(kn, a, b, M, N, K, a.shape[1], b.shape[1], C32=C, ldc32=N + 3, bias=bias, alpha=0.5, beta=2.0, splits=splits)
+            want_a, want_b = a.double().cpu().numpy()[:, :A.shape[1]], b.double().cpu().numpy()[:, :B.shape[1]]
+            want = 0.5 * ((want_a.T if kind == "TN" else want_a) @ (want_b.T if kind == "NT" else want_b)) + C0[0, :N].astype(np.float64) + 2.0 * C0[:, :N]
+            launches = 1
+            bound = 2e-5
+        else:
+            C = torch.from_numpy(C0).cuda()
+            tb.gemm_f32(kn, torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda(), C, M, N, K, A.shape[1], B.shape[1], N + 3, alpha=0.5, beta=2.0,
+                        precision=tb.PREC_TF32)
+            want = 0.5 * ((A.T if kind == "TN" else A).astype(np.float64) @ (B.T if kind == "NT" else B).astype(np.float64)) + 2.0 * C0[:, :N]
+            launches = None
+            bound = 5e-3
+        out = C.cpu().numpy()
+        tb.sync_check()
+        if launches is not None and splits:
+            assert tb.launch_count() - before == (2 if off else launches)
+        assert np.abs(out[:, :N] - want).max() <= bound * np.abs(want).max()
+        assert np.array_equal(out[:, N:], C0[:, N:])
+        got.append(out)
+    if precision == "bf16" and splits:
+        # the same parts in the same order, but bias and previous contents are added to other roundings of alpha times the sum
+        assert np.abs(got[0] - got[1]).max() <= 1e-6 * np.abs(got[1]).max()

@@ -23,6 +23,7 @@
 #include "ptx.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -94,6 +95,7 @@ struct GemmParams {
     int wide16;                 // bf16 tiles leave two 32-column chunks at a time: 32 rows x 128 bytes per store through the
                                 // 64-column map (tmR; with dsw: tmC), a last odd chunk through the 32-column map tmC
     int dsw;                    // SwiGLU backward: the product is dh; tmR = saved gate|up [M,2F] bf16, tmC = dgu [M,2F] bf16
+    int csplit;                 // EPI_SPLIT: CTAs of a cluster that share a tile's K slices
     const float* norm_w; float norm_eps, norm_inv_n; float* norm_rinv; bf16* norm16; float* norm32;    // EPI_NORM
     int tma_res;                // TMA path: add res_scale * (tile of tmR) -- the residual, or the old C for beta
     float res_scale;
@@ -155,7 +157,7 @@ __device__ __forceinline__ TileCoord tile_of(const GemmParams& p, int t, int row
 // a 32-column chunk costs ~0.15 us more in instruction fetches); the other values fix the mode at compile time and
 // drop the rest -- measured on an [8192 x 384 x 1152] launch: last tile's epilogue 2.42 -> 1.89 us (float32 out),
 // 2.02 -> 1.54 us (bf16 out).
-enum { EPI_ANY = 0, EPI_F32, EPI_BF16, EPI_SWIGLU, EPI_CE1, EPI_ROPE, EPI_CE2, EPI_DSW, EPI_NORM };
+enum { EPI_ANY = 0, EPI_F32, EPI_BF16, EPI_SWIGLU, EPI_CE1, EPI_ROPE, EPI_CE2, EPI_DSW, EPI_NORM, EPI_SPLIT };
 
 template <int BN, bool TF32, bool PAIR = false, int EPI = EPI_ANY>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
@@ -172,8 +174,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // PAIR: rank in the CTA pair; rank 0 issues the UMMAs and owns the barriers the loads are counted on
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
     const int row_off = (int)rank * BM;
-    const int worker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
-    const int nworkers = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+    // SPLIT: the CTAs of a cluster form one tile, each over its share of the K slices, and add their parts through distributed
+    // shared memory (a cluster per tile: nothing is handed out twice)
+    constexpr bool SPLIT = EPI == EPI_SPLIT;
+    const int srank = SPLIT ? (int)cluster_ctarank() : 0;
+    const int worker = PAIR ? (int)(blockIdx.x >> 1) : SPLIT ? (int)blockIdx.x / p.csplit : (int)blockIdx.x;
+    const int nworkers = PAIR ? (int)(gridDim.x >> 1) : SPLIT ? (int)gridDim.x / p.csplit : (int)gridDim.x;
     constexpr int BKE = TF32 ? BK_TF32 : BK;           // elements per K slice
     constexpr int MNW = TF32 ? 32 : 64;                // elements per 128-byte row of an MN-major box
     constexpr int MN_BOX_BYTES = BKE * ROW_BYTES;      // one MN-major box: BKE rows of 128 bytes
@@ -218,11 +224,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
-        if (!m_generic && !m_ce1) tma_prefetch_desc(&tmC);
+        if (!m_generic && !m_ce1 && EPI != EPI_SPLIT) tma_prefetch_desc(&tmC);
         for (int i = 0; i < STAGES; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], PAIR ? 2 * EPI_WARPS : EPI_WARPS); }
         for (int i = 0; i < EPI_WARPS; ++i) mbar_init(&res_bar[i], 1);
         if (NORM) for (int i = 0; i < 2; ++i) mbar_init(&norm_bar[i], (uint32_t)(p.nt * EPI_WARPS));
+        if (SPLIT) mbar_init(&norm_bar[0], (uint32_t)(p.csplit * EPI_WARPS));
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -231,10 +238,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         else      { tmem_alloc(tmem_slot, Cfg::TMEM_COLS); tmem_relinquish(); }
     }
     // every role's first tile, worked out while the barriers and the tensor memory are being set up
-    const TileCoord c_first = tile_of<BN, BKE, TILE_M>(p, worker < total_tiles ? worker : 0, row_off);
+    TileCoord c_first = tile_of<BN, BKE, TILE_M>(p, worker < total_tiles ? worker : 0, row_off);
+    if (SPLIT) { c_first.kb0 = min(p.kb_total, srank * p.kb_per); c_first.kb1 = min(p.kb_total, c_first.kb0 + p.kb_per); }
     tc_fence_before();
     __syncthreads();
-    if (PAIR || NORM) cluster_sync();  // the other CTAs' barriers exist before either signals the other's
+    if (PAIR || NORM || SPLIT) cluster_sync();  // the other CTAs' barriers exist before either signals the other's
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     if (threadIdx.x == 0) TS(1);
@@ -363,6 +371,80 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             TS(6);
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 2); }
         }
+    } else if (SPLIT) {
+        // ------------------------------------------------ epilogue of a tile that a cluster shares
+        // Every CTA leaves its part in its own ring (all its operands have been read), in blocks of 32 columns with the rows' 16-byte
+        // pieces swizzled; then each adds its share of the rows over all CTAs in rank order.  Sums have a fixed order, partial slabs
+        // in memory and the kernel that reduces them are gone: see choose_splits for both sides' figures.
+        const int q = warp & 3, ew = warp - 2, half = ew >> 2;
+        constexpr int NCH = BN / 64;
+        bool ok = mbar_wait(&acc_full[0], 0, abort_flag);
+        if (ok) {
+            tc_fence_after();
+            const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * (BN / 2));
+            const bool have_acc = c_first.kb1 > c_first.kb0;
+            const int row = q * 32 + lane;
+#pragma unroll 1
+            for (int ch = 0; ch < NCH; ++ch) {
+                uint32_t v[32];
+                if (have_acc) {
+                    tmem_ld32(t_row + (uint32_t)(ch * 32), v);
+                    tmem_ld_wait();
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = 0u;
+                }
+                uint8_t* dst = stage_base + (half * NCH + ch) * (BM * ROW_BYTES) + row * ROW_BYTES;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(dst + ((j ^ (row & 7)) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            }
+            __syncwarp();
+            if (lane < p.csplit) mbar_arrive_cluster(mapa_cluster(smem_u32(&norm_bar[0]), (uint32_t)lane));
+            ok = mbar_wait_cluster(&norm_bar[0], 0, abort_flag);
+        }
+        if (ok) {
+            constexpr int PIECES = BN / 4;                   // 16-byte pieces of a row
+            const int per = (BM + p.csplit - 1) / p.csplit, first = srank * per, rows = min(BM, first + per) - first;
+            const uint32_t base = smem_u32(stage_base);
+#pragma unroll 1
+            for (int i = (int)threadIdx.x - 64; i < rows * PIECES; i += EPI_WARPS * 32) {
+                const int row = first + i / PIECES, c4 = i % PIECES;
+                const uint32_t at = base + (uint32_t)((c4 >> 3) * (BM * ROW_BYTES) + row * ROW_BYTES + (((c4 & 7) ^ (row & 7)) << 4));
+                float4 v[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k) if (k < p.csplit) v[k] = ld_cluster_f32x4(mapa_cluster(at, (uint32_t)k));
+                float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) if (k < p.csplit) { s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
+                const int gm = c_first.m0 + row, gn = c_first.n0 + 4 * c4;
+                if (gm >= p.M || gn >= p.N) continue;
+                float o[4] = {s.x * p.alpha, s.y * p.alpha, s.z * p.alpha, s.w * p.alpha};
+                float* cp = p.C32 + (long long)gm * p.ldc32 + gn;
+                const bool whole = p.C32 && gn + 3 < p.N && p.vec32;
+                if (p.bias) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) if (gn + e < p.N) o[e] += __ldg(p.bias + gn + e);
+                }
+                if (whole) {
+                    if (p.beta != 0.0f) {
+                        const float4 c4v = *reinterpret_cast<const float4*>(cp);
+                        o[0] += p.beta * c4v.x; o[1] += p.beta * c4v.y; o[2] += p.beta * c4v.z; o[3] += p.beta * c4v.w;
+                    }
+                    *reinterpret_cast<float4*>(cp) = make_float4(o[0], o[1], o[2], o[3]);
+                } else if (p.C32) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) if (gn + e < p.N) {
+                        if (p.beta != 0.0f) o[e] += p.beta * cp[e];
+                        cp[e] = o[e];
+                    }
+                }
+                if (p.C16) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) if (gn + e < p.N) p.C16[(long long)gm * p.ldc16 + gn + e] = __float2bfloat16_rn(o[e]);
+                }
+            }
+        }
+        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.err, 3); }
     } else if (!m_generic) {
         // ------------------------------------------------ epilogue, tile stores by TMA
         // Per 32-column chunk: tcgen05.ld -> registers (+bias, +scaled residual tile) -> this warp's
@@ -1071,7 +1153,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     }
     tc_fence_before();
     __syncthreads();
-    if (PAIR || NORM) cluster_sync();  // the other CTA has read its accumulators and needs none of this CTA's barriers any more
+    if (PAIR || NORM || SPLIT) cluster_sync();  // the other CTA has read its accumulators and needs none of this CTA's barriers any more
     if (warp == 1) {
         tc_fence_after();
         if (PAIR) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
@@ -1422,6 +1504,39 @@ static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
     return best;
 }
 
+// How many clusters of s CTAs with a whole SM each run at a time (1 <= s <= 8, the portable sizes).  Processor clusters hold between
+// 16 and 20 SMs, so it is not 148 / s.
+static int cluster_room(const DeviceCtx* ctx, int s) {
+    static std::atomic<int> room[64][9];
+    std::atomic<int>& r = room[ctx->device & 63][s];
+    if (r.load(std::memory_order_relaxed) == 0) {
+        using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GemmParams);
+        const Kernel kernel = gemm_bf16_kernel<128, false, false, EPI_SPLIT>;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)s; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3((unsigned)(s * ctx->sm_count)); cfg.blockDim = dim3(NUM_THREADS);
+        cfg.dynamicSmemBytes = GemmCfg<128, false, false>::SMEM_BYTES;
+        cfg.attrs = attr; cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<128, false, false>::SMEM_BYTES) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess)
+            cudaGetLastError();
+        r.store(n > 0 ? n : -1, std::memory_order_relaxed);
+    }
+    return r.load(std::memory_order_relaxed);
+}
+
+// Whether the splits of a product are added by clusters: one wave of them, alone on the chip (beside another product the SMs of a
+// cluster may not be free together).
+static bool cluster_adds(const DeviceCtx* ctx, const GemmArgs& a, int bn, int splits) {
+    if (splits < 2 || splits > 8 || bn > 192 || a.batch != 1 || a.c_inner > 1 || a.causal != CAUSAL_NONE || a.max_ctas > 0 || (!a.C32 && !a.C16) ||
+        a.residual || a.swapped || getenv("TB_GEMM_NO_CLUSTER_SPLIT") != nullptr)
+        return false;
+    return (long long)((a.M + BM - 1) / BM) * ((a.N + bn - 1) / bn) <= cluster_room(ctx, splits);
+}
+
 static int choose_splits(const DeviceCtx* ctx, const GemmArgs& a, int bn) {
     if (a.causal != CAUSAL_NONE) return 1;
     const int tile_m = bn >= 256 ? 2 * BM : BM;                     // a CTA pair owns 256 rows
@@ -1434,8 +1549,19 @@ static int choose_splits(const DeviceCtx* ctx, const GemmArgs& a, int bn) {
     int s = (int)(workers / tiles);
     if (s > kb_total / 4) s = kb_total / 4;     // at least 4 K slices per split
     if (s < 1) s = 1;
-    const int kb_per = (kb_total + s - 1) / s;
-    return (kb_total + kb_per - 1) / kb_per;     // no empty split
+    auto whole = [&](int n) { const int per = (kb_total + n - 1) / n; return (kb_total + per - 1) / per; };     // no empty split
+    // Fewer splits that a cluster adds against more with a reduction kernel: us at ~94 KB/us of operands per SM, 1.5 for the exchange,
+    // 2 for the launch and 6 MB/us for the slabs.  (Three products of a layer, 1024 rows of 384 : 1152 in float32 pieces 51.0 -> 49.7 us,
+    // 8192 of 384 : 2048 in bf16 60.7 -> 60.0.)
+    const double slice = (bn + 128) * 0.125 / 94.0, slab = (double)a.M * a.N * 4e-6;
+    auto slices = [&](int n) { return (double)((kb_total + n - 1) / n); };
+    const double by_kernel = slices(whole(s)) * slice + 2.0 + (whole(s) + 1) * slab / 6.0;
+    for (int n = s < 8 ? s : 8; n > 1; --n)
+        if (cluster_adds(ctx, a, bn, whole(n))) {
+            if (slices(whole(n)) * slice + 1.5 <= by_kernel) return whole(n);
+            break;
+        }
+    return whole(s);
 }
 
 // A weight gradient (few tiles, long K, split along it) by the tile that is estimated to take least: operand bytes a CTA pulls at
@@ -1462,7 +1588,7 @@ static GemmArgs arranged(const DeviceCtx* ctx, const GemmArgs& a) {
         const int workers = pair ? sms / 2 : sms;
         const double waves = (double)((tiles + workers - 1) / workers), slab = (double)a.M * a.N * 4e-6;
         return waves * (per * (bn == 128 ? 32.0 : 40.0) / 94.0 + (pair ? 5.0 : bn == 192 ? 1.8 : 1.2)) +
-               (s == 1 ? 0.0 : 2.0 + (s + 1) * slab / 6.0);
+               (s == 1 ? 0.0 : cluster_adds(ctx, g, bn, s) ? 1.5 : 2.0 + (s + 1) * slab / 6.0);
     };
     GemmArgs best = a;
     double least = time_of(a, pick_bn(ctx, a)) * 0.9;
@@ -1494,6 +1620,7 @@ static int launch_impl(DeviceCtx* ctx, const GemmArgs& a, const GemmParams& p, c
                        const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmR,
                        cudaStream_t stream) {
     using Cfg = GemmCfg<BN, PAIR, EPI == EPI_NORM>;
+    static_assert(EPI != EPI_SPLIT || Cfg::STAGES * Cfg::STAGE_BYTES >= BM * BN * 4, "a CTA's part of a tile lies in its ring");
     static bool attr_set[64] = {false};
     if (!attr_set[ctx->device & 63]) {
         TB_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<BN, TF32, PAIR, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1510,9 +1637,10 @@ static int launch_impl(DeviceCtx* ctx, const GemmArgs& a, const GemmParams& p, c
         grid = (int)(total < sms ? total : sms);
     }
     if (grid < 1) grid = PAIR ? 2 : 1;
+    if (EPI == EPI_SPLIT) grid = (int)total * p.csplit;
     if (EPI == EPI_NORM) grid = p.nt * std::min(p.mt, std::max(1, sms / p.nt));       // whole clusters of p.nt CTAs
     TB_CUDA(launch_kernel_cluster((gemm_bf16_kernel<BN, TF32, PAIR, EPI>), dim3(grid), dim3(NUM_THREADS), Cfg::SMEM_BYTES,
-                                  stream, EPI == EPI_NORM ? p.nt : PAIR ? 2 : 1, tmA, tmB, tmC, tmR, p));
+                                  stream, EPI == EPI_NORM ? p.nt : EPI == EPI_SPLIT ? p.csplit : PAIR ? 2 : 1, tmA, tmB, tmC, tmR, p));
     TB_CUDA(cudaGetLastError());
     ctx->launches++;
     prof_close(ctx, stream);
@@ -1619,7 +1747,10 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
     p.a_mn = a_mn; p.b_mn = b_mn; p.causal = (int)a.causal;
     p.dsw = 0; p.wide16 = 0;
     p.err = ctx->d_err;
-    if (splits > 1) {
+    const bool in_cluster = cluster_adds(ctx, a, bn, splits);
+    p.csplit = in_cluster ? splits : 0;
+    if (in_cluster) p.splits = 1;
+    if (splits > 1 && !in_cluster) {
         // partial tiles, one [M,N] slab per (batch, split); everything else happens in the reduction
         TB_CHECK(a.c_inner <= 1, "split-K GEMM does not take a two-level output batch stride");
         p.C32 = ws; p.ldc32 = a.N; p.strideC32 = (long long)a.M * a.N; p.strideC32_in = 0;
@@ -1766,6 +1897,14 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         else if (bn == 128) TB_TRY(TB_NORM_LAUNCH(128));
         else                TB_TRY(TB_NORM_LAUNCH(192));
 #undef TB_NORM_LAUNCH
+    } else if (in_cluster) {
+#define TB_SPLIT_LAUNCH(W)                                                                                             \
+        (a.tf32 ? launch_impl<W, true, false, EPI_SPLIT>(ctx, a, p, tmA, tmB, tmC, tmR, stream)                          \
+                : launch_impl<W, false, false, EPI_SPLIT>(ctx, a, p, tmA, tmB, tmC, tmR, stream))
+        if (bn == 64)       TB_TRY(TB_SPLIT_LAUNCH(64));
+        else if (bn == 128) TB_TRY(TB_SPLIT_LAUNCH(128));
+        else                TB_TRY(TB_SPLIT_LAUNCH(192));
+#undef TB_SPLIT_LAUNCH
     } else if (a.tf32) {
         // (float32 operands read as tf32: plain float32 / bf16 tiles and the QKV epilogue have instantiations of their own, the rest is general)
         static const bool general_only = getenv("TB_GEMM_GENERAL_KERNEL") != nullptr;
@@ -1795,7 +1934,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         else                TB_TRY((launch_bf16<128, false>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
     }
 
-    if (splits > 1) {
+    if (splits > 1 && !in_cluster) {
         TB_CHECK(a.residual == nullptr, "split-K GEMM does not take a residual operand");
         const long long per = (long long)a.M * a.N;
         const bool vec4 = a.N % 4 == 0;      // a float4 never straddles a row; partial slabs are 16-byte aligned
