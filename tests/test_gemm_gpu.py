@@ -619,3 +619,44 @@ def test_splits_added_inside_a_cluster(tb, monkeypatch, kind, shape, precision):
     if precision == "bf16" and splits:
         # the same parts in the same order, but bias and previous contents are added to other roundings of alpha times the sum
         assert np.abs(got[0] - got[1]).max() <= 1e-6 * np.abs(got[1]).max()
+
+
+@pytest.mark.parametrize("kind", ["NN", "NT", "TN"])
+@pytest.mark.parametrize("shape", [(4, 4, 192), (100, 68, 228), (132, 132, 420), (200, 72, 1100), (384, 1152, 1024), (1000, 260, 2048), (64, 2048, 384)])
+def test_float32_product_splits_its_slices_on_chip(tb, monkeypatch, kind, shape):
+    """Float32 accuracy in one launch: ragged tiles and slices, clusters of one to eight, an output that is not 16-byte
+    addressable, bias, alpha, beta.  Bound per element: a rest is below 2^-10 of x and loses 2^-10 of itself, the product of two rests
+    2^-20, three times 2^-20 of the sum of magnitudes in all; every addition of eight products may lose 2^-23 of it."""
+    M, N, K = shape
+    rng = np.random.default_rng(M + K)
+    A = rng.standard_normal((K, M) if kind == "TN" else (M, K)).astype(np.float32)
+    B = rng.standard_normal((N, K) if kind == "NT" else (K, N)).astype(np.float32)
+    a64, b64 = (A.T if kind == "TN" else A).astype(np.float64), (B.T if kind == "NT" else B).astype(np.float64)
+    C0 = rng.standard_normal((M, N + 3)).astype(np.float32)
+    want = 0.5 * (a64 @ b64) + 2.0 * C0[:, :N]
+    bound = (3 * 2.0 ** -20 + (K / 8 + 4) * 2.0 ** -23) * (0.5 * (np.abs(a64) @ np.abs(b64)) + 2.0 * np.abs(C0[:, :N]))
+    dA, dB = torch.from_numpy(A).cuda(), torch.from_numpy(B).cuda()
+
+    def run(C):
+        out = torch.from_numpy(C).cuda()
+        before = tb.launch_count()
+        tb.gemm_f32({"NN": tb.NN, "NT": tb.NT, "TN": tb.TN}[kind], dA, dB, out, M, N, K, A.shape[1], B.shape[1], C.shape[1], alpha=0.5, beta=2.0,
+                    precision=tb.PREC_FP32)
+        tb.sync_check()
+        return out.cpu().numpy(), tb.launch_count() - before
+
+    one, launches = run(C0)
+    assert launches == 1
+    assert (np.abs(one[:, :N] - want) <= bound).all()
+    assert np.array_equal(one[:, N:], C0[:, N:])
+    assert np.array_equal(run(np.ascontiguousarray(C0[:, :N]))[0], one[:, :N]) and np.array_equal(run(C0)[0], one)
+    if kind == "NN":
+        bias, y = torch.from_numpy(C0[0, :N].copy()).cuda(), torch.zeros(M, N, device="cuda")
+        tb.gemm_bias_f32(dA, dB, bias, None, y, M, N, K, precision=tb.PREC_FP32)
+        assert (np.abs(y.cpu().numpy() - (a64 @ b64 + C0[0, :N])) <= 2 * bound + 2.0 ** -22 * np.abs(C0[0, :N])).all()
+    # an infinity and a NaN: where the pieces written out in memory give none, none here
+    dA[0, 0], dB[0, 1] = float("inf"), float("nan")
+    special = run(C0)[0]
+    monkeypatch.setenv("TB_GEMM_NO_X3", "1")
+    pieces, launches = run(C0)
+    assert launches >= 2 and np.array_equal(np.isfinite(special), np.isfinite(pieces))

@@ -228,13 +228,14 @@ int tb_attention_bwd(const void* d_Q, const void* d_K, const void* d_V, const vo
 //   TF32: the float32 operands go to the tensor cores as they are (kind::tf32 reads the top 19 bits);
 //         an operand whose rows are not 16-byte addressable is first copied with a padded leading dimension;
 //   FP32: each operand is split into tf32-exact pieces hi + lo and the product is evaluated as
-//         hi*hi + hi*lo + lo*hi in one TF32 GEMM over a 3x longer K (error ~2^-20 of the result).
+//         hi*hi + hi*lo + lo*hi: inside one kernel where plan_gemm_x3 finds that faster, else the pieces are
+//         written to scratch memory for one TF32 GEMM over a 3x longer K (error ~2^-20 of the result).
 static inline bool tma_ok_f32(const float* p, long long ld, int batch, long long stride) {
     return (reinterpret_cast<uintptr_t>(p) & 15u) == 0 && ld % 4 == 0 && (batch == 1 || stride % 4 == 0);
 }
 
 // Packed operands and split-K partial sums of a caller that does not use the device's scratch memory
-struct OwnScratch { float* mem = nullptr; size_t floats = 0; };
+struct OwnScratch { float* mem = nullptr; size_t floats = 0; bool has_b = false; };      // has_b: the last call left its B packed
 
 static int grow(float** p, size_t* cap, size_t need) {
     if (need <= *cap) return 0;
@@ -250,7 +251,9 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
                          long long lda, long long ldb, long long ldc, int batch, long long sA, long long sB,
                          long long sC, float alpha, float beta, const float* bias, const float* residual,
                          int precision, cudaStream_t stream, OwnScratch* own = nullptr, bool same_b = false) {
-    // (same_b: B is what the call before it with this scratch memory, its caller's own, had, and is still packed there)
+    // (same_b: B is what the call before it with this scratch memory, its caller's own, had; it is still packed there if that one did)
+    if (own && !own->has_b) same_b = false;
+    if (own) own->has_b = false;
     DeviceCtx* ctx;
     TB_TRY(get_ctx(&ctx));
     char* scratch = nullptr;
@@ -262,6 +265,7 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
         }
         if (bytes > own->floats * sizeof(float)) same_b = false;      // it moves
         TB_TRY(grow(&own->mem, &own->floats, (bytes + sizeof(float) - 1) / sizeof(float)));
+        own->has_b = true;
         scratch = reinterpret_cast<char*>(own->mem);
         return 0;
     };
@@ -299,6 +303,11 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
         return launch_gemm_bf16_ws(ctx, g, ws, ws_floats, stream);
     }
 
+    if (precision == TB_PREC_FP32 && tma_ok_f32(A, lda, batch, sA) && tma_ok_f32(B, ldb, batch, sB)) {
+        GemmArgs x = g;
+        x.A = A; x.B = B; x.lda = lda; x.ldb = ldb;
+        if (plan_gemm_x3(ctx, &x)) return launch_gemm_x3(ctx, x, stream);
+    }
     g.tf32 = true;
     const bool split3 = precision == TB_PREC_FP32;
     // shapes of the operands the TF32 GEMM sees

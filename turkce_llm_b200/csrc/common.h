@@ -128,6 +128,7 @@ struct GemmArgs {
     float alpha = 1.0f, beta = 0.0f;        // beta applies to the previous contents of C32
     CausalMode causal = CAUSAL_NONE;
     int splits = 0;                         // 0 = choose; >1 uses scratch for fixed-order partial sums
+    bool x3 = false;                        // float32 operands to float32 accuracy (plan_gemm_x3, launch_gemm_x3)
     bool planned = false;                   // splits is what planned_splits gave for this product
     int bn = 0;                             // 0 = choose tile width (64, 128 or 192; 256 = a CTA pair on a 256 x 256 tile)
     bool swapped = false;                   // (set by the launcher) A and B, M and N are exchanged and the reduction turns C^T; splits > 1
@@ -183,6 +184,10 @@ bool gemm_norm_pays(const DeviceCtx* ctx, int M, int N, bool tf32);
 int launch_gemm_bf16_ws(DeviceCtx* ctx, const GemmArgs& a, float* workspace, size_t workspace_floats,
                         cudaStream_t stream);
 int planned_splits(const DeviceCtx* ctx, const GemmArgs& a);
+// The product of float32 operands to float32 accuracy in one launch without scratch memory.  The plan says whether it is the faster
+// way, and fills in tile and splits.
+bool plan_gemm_x3(const DeviceCtx* ctx, GemmArgs* a);
+int launch_gemm_x3(DeviceCtx* ctx, const GemmArgs& a, cudaStream_t stream);
 // TMA map over a bf16 matrix seen as (inner, rows, batch) with a 64-element x box_rows box, 128B swizzle
 int make_operand_map(CUtensorMap* map, const bf16* ptr, long long inner, long long rows, long long ld, int batch,
                      long long batch_stride, int box_rows);

@@ -37,6 +37,7 @@ constexpr int BK_TF32 = 32;         // float32 elements of one 128-byte swizzle 
 constexpr int ROW_BYTES = 128;
 constexpr int NUM_THREADS = 320;      // TMA warp, MMA warp, 8 epilogue warps
 constexpr int EPI_WARPS = 8;
+constexpr int X3_WARPS = 4;           // EPI_X3: warps that form the rests
 constexpr int NORM_MAX_CTAS = 4;      // CTAs that share a row block in the RMSNorm epilogue
 constexpr int STAGE_LD = 36;        // floats per staging row (32 + 4 pad: conflict-free float4 access)
 
@@ -47,20 +48,22 @@ constexpr int STAGE_LD = 36;        // floats per staging row (32 + 4 pad: confl
 // second tile empty).  The tensor core takes N <= 256, so a K step is three instructions of 128 columns; each CTA
 // loads the 64-column boxes at n0 + 128 j + 64 rank, which keeps accumulator column = output column.  One accumulator.
 // NORM: the CTAs of a cluster hold the columns of one row block between them and exchange the rows' sums of squares
-template <int BN, bool PAIR = false, bool NORM = false> struct GemmCfg {
+// X3: a stage holds A | B | rest of B | rest of A (see EPI_X3); its epilogue needs no staging
+template <int BN, bool PAIR = false, bool NORM = false, bool X3 = false> struct GemmCfg {
     static constexpr int BN_LOCAL = PAIR ? BN / 2 : BN;   // columns of B this CTA loads
     static constexpr int A_BYTES = BM * ROW_BYTES;      // one K slice: 128-byte rows for either operand type
     static constexpr int B_BYTES = BN_LOCAL * ROW_BYTES;
-    static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    static constexpr int STAGES = (PAIR && BN == 384) ? 3 : PAIR ? 4 : (BN == 192) ? 3 : (BN == 128) ? (NORM ? 3 : 4) : 5;
+    static constexpr int LOAD_BYTES = A_BYTES + B_BYTES;
+    static constexpr int STAGE_BYTES = (X3 ? 2 : 1) * LOAD_BYTES;
+    static constexpr int STAGES = X3 ? (BN == 128 ? 3 : 4) : (PAIR && BN == 384) ? 3 : PAIR ? 4 : (BN == 192) ? 3 : (BN == 128) ? (NORM ? 3 : 4) : 5;
     // per epilogue warp: 2 output buffers + 1 residual buffer of 32 rows x 128 B (TMA path);
     // the generic path uses the front of the same region (32 x 36 floats per warp)
     static constexpr int EPI_WARP_BYTES = 3 * 4096;
-    static constexpr int STAGING_BYTES = EPI_WARPS * EPI_WARP_BYTES;
+    static constexpr int STAGING_BYTES = X3 ? 0 : EPI_WARPS * EPI_WARP_BYTES;
     static constexpr int BAR_BYTES = 512;
     static constexpr int NORM_BYTES = NORM ? (2 * 2 * NORM_MAX_CTAS * BM + 2 * BN) * 4 : 0;      // [2 tiles][CTA, half][row] partial sums | bias | weight
     static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + STAGING_BYTES + BAR_BYTES + NORM_BYTES;
-    static constexpr int TMEM_COLS = (2 * BN <= 128) ? 128 : (2 * BN <= 256) ? 256 : 512;   // power of two
+    static constexpr int TMEM_COLS = X3 ? 4 * BN : (2 * BN <= 128) ? 128 : (2 * BN <= 256) ? 256 : 512;   // power of two
     // accumulators in TMEM: two (the epilogue of tile i overlaps the main loop of tile i+1) unless one fills it
     static constexpr int NBUF = (2 * BN <= 512) ? 2 : 1;
 };
@@ -157,15 +160,24 @@ __device__ __forceinline__ TileCoord tile_of(const GemmParams& p, int t, int row
 // a 32-column chunk costs ~0.15 us more in instruction fetches); the other values fix the mode at compile time and
 // drop the rest -- measured on an [8192 x 384 x 1152] launch: last tile's epilogue 2.42 -> 1.89 us (float32 out),
 // 2.02 -> 1.54 us (bf16 out).
-enum { EPI_ANY = 0, EPI_F32, EPI_BF16, EPI_SWIGLU, EPI_CE1, EPI_ROPE, EPI_CE2, EPI_DSW, EPI_NORM, EPI_SPLIT };
+enum { EPI_ANY = 0, EPI_F32, EPI_BF16, EPI_SWIGLU, EPI_CE1, EPI_ROPE, EPI_CE2, EPI_DSW, EPI_NORM, EPI_SPLIT, EPI_X3 };
+constexpr int threads_of(int epi) { return NUM_THREADS + (epi == EPI_X3 ? X3_WARPS * 32 : 0); }
 
 template <int BN, bool TF32, bool PAIR = false, int EPI = EPI_ANY>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+__global__ void __launch_bounds__(threads_of(EPI), 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmR,
                  const GemmParams p) {
     constexpr bool NORM = EPI == EPI_NORM;
-    using Cfg = GemmCfg<BN, PAIR, NORM>;
+    // X3: float32 operands to float32 accuracy.  The tensor core reads the top 19 bits of a float32, x = hi + lo with lo exact in
+    // float32, and the product is hi hi + hi lo + lo hi.  Slices come in as they are and serve as hi; four warps write the rests
+    // beside them (element by element, whatever the layout), so neither operand is rewritten in memory and a slice is loaded once
+    // instead of three times.  B's rest lies behind B: one instruction of twice the columns takes A with both, a second A's rest with
+    // B.  The small products have an accumulator of their own, and slices
+    // alternate between two pairs of them: the tensor core rounds every addition towards zero, half as many lose half as much.
+    constexpr bool X3 = EPI == EPI_X3;
+    static_assert(!X3 || (TF32 && !PAIR), "EPI_X3 takes float32 operands on single CTAs");
+    using Cfg = GemmCfg<BN, PAIR, NORM, X3>;
     constexpr int STAGES = Cfg::STAGES;
     constexpr int NBUF = Cfg::NBUF;
     constexpr int BNL = Cfg::BN_LOCAL;
@@ -176,7 +188,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int row_off = (int)rank * BM;
     // SPLIT: the CTAs of a cluster form one tile, each over its share of the K slices, and add their parts through distributed
     // shared memory (a cluster per tile: nothing is handed out twice)
-    constexpr bool SPLIT = EPI == EPI_SPLIT;
+    constexpr bool SPLIT = EPI == EPI_SPLIT || X3;
     const int srank = SPLIT ? (int)cluster_ctarank() : 0;
     const int worker = PAIR ? (int)(blockIdx.x >> 1) : SPLIT ? (int)blockIdx.x / p.csplit : (int)blockIdx.x;
     const int nworkers = PAIR ? (int)(gridDim.x >> 1) : SPLIT ? (int)gridDim.x / p.csplit : (int)gridDim.x;
@@ -197,6 +209,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     uint64_t* acc_full = bars + 2 * STAGES;       // [2]
     uint64_t* acc_empty = bars + 2 * STAGES + 2;  // [2]
     uint64_t* res_bar = bars + 2 * STAGES + 4;    // [EPI_WARPS]
+    uint64_t* lo_bar = bars + 48;                 // [STAGES]: the rests of a stage are written (X3)
     uint64_t* norm_bar = bars + 40;               // [2]: the partial sums of a tile (by parity) have arrived
     float* norm_part = reinterpret_cast<float*>(smem + STAGES * Cfg::STAGE_BYTES + Cfg::STAGING_BYTES + Cfg::BAR_BYTES);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4 + EPI_WARPS);
@@ -224,12 +237,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     if (threadIdx.x == 0) {
         tma_prefetch_desc(&tmA);
         tma_prefetch_desc(&tmB);
-        if (!m_generic && !m_ce1 && EPI != EPI_SPLIT) tma_prefetch_desc(&tmC);
+        if (!m_generic && !m_ce1 && !SPLIT) tma_prefetch_desc(&tmC);
         for (int i = 0; i < STAGES; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], PAIR ? 2 * EPI_WARPS : EPI_WARPS); }
         for (int i = 0; i < EPI_WARPS; ++i) mbar_init(&res_bar[i], 1);
         if (NORM) for (int i = 0; i < 2; ++i) mbar_init(&norm_bar[i], (uint32_t)(p.nt * EPI_WARPS));
         if (SPLIT) mbar_init(&norm_bar[0], (uint32_t)(p.csplit * EPI_WARPS));
+        if (X3) for (int i = 0; i < STAGES; ++i) mbar_init(&lo_bar[i], X3_WARPS);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -261,8 +275,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                     uint8_t* sA = stage_base + stage * Cfg::STAGE_BYTES;
                     uint8_t* sB = sA + Cfg::A_BYTES;
                     // PAIR: both CTAs' bytes are counted on rank 0's barrier, which alone arms it
-                    if (!PAIR) mbar_expect_tx(&full_bar[stage], Cfg::STAGE_BYTES);
-                    else if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * Cfg::STAGE_BYTES);
+                    if (!PAIR) mbar_expect_tx(&full_bar[stage], Cfg::LOAD_BYTES);
+                    else if (rank == 0) mbar_expect_tx(&full_bar[stage], 2 * Cfg::LOAD_BYTES);
                     auto load = [&](void* dst, const CUtensorMap* map, int x, int y, int z) {
                         if (PAIR) tma_load_3d_pair(dst, map, &full_bar[stage], x, y, z);
                         else tma_load_3d(dst, map, &full_bar[stage], x, y, z);
@@ -317,6 +331,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             // and the step between the four UMMAs of a K slice are all that changes (the start address sits
             // in the low 14 bits, in 16-byte units, and never carries out of them below 256 KB).  One thread
             // issues every UMMA of the CTA, so its instruction count per UMMA bounds the tensor pipe.
+            const uint32_t idesc_x3 = umma_idesc(2u, (uint32_t)p.a_mn, (uint32_t)p.b_mn, TILE_M, X3 ? 2 * BN : UMMA_N);
+            constexpr uint64_t A_REST = (uint64_t)((Cfg::A_BYTES + 2 * Cfg::B_BYTES) >> 4);
             const uint32_t a_addr0 = smem_u32(stage_base);
             const uint32_t b_addr0 = a_addr0 + Cfg::A_BYTES;
             const uint64_t a_desc0 = !p.a_mn ? umma_desc_sw128(a_addr0, 16, 1024)
@@ -343,10 +359,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 for (int kb = c.kb0; kb < c.kb1; ++kb) {
                     if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
                     if (it == 0 && kb == c.kb0) TS(4);
+                    if (X3 && !mbar_wait(&lo_bar[stage], phase, abort_flag)) { ok = false; break; }
                     tc_fence_after();
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {          // 4 UMMAs of 32 bytes of K per 128-byte slice
-                        if (PAIR) {
+                        if (X3) {
+                            const uint32_t d = d_tmem + (((kb - c.kb0) & 1) ? 2 * BN : 0);
+                            umma_tf32(d, a_desc + k * a_kstep, b_desc + k * b_kstep, idesc_x3, (kb > c.kb0 + 1 || k > 0) ? 1u : 0u);
+                            umma_tf32(d + BN, a_desc + A_REST + k * a_kstep, b_desc + k * b_kstep, idesc, 1u);
+                        }
+                        else if (PAIR) {
 #pragma unroll
                             for (int j = 0; j < NSUB; ++j) {
                                 const uint32_t d = d_tmem + (uint32_t)(j * UMMA_N), acc = (kb > c.kb0 || k > 0) ? 1u : 0u;
@@ -371,6 +393,29 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             TS(6);
             if (!ok) { *abort_flag = 1; atomicExch(p.err, 2); }
         }
+    } else if (X3 && warp >= 2 + EPI_WARPS) {
+        // ---------------------------------------------------------- the rests of a slice, x - (top 19 bits of x), four warps
+        const int tid = (int)threadIdx.x - NUM_THREADS;
+        int stage = 0; uint32_t phase = 0;
+        bool ok = true;
+        for (int kb = c_first.kb0; kb < c_first.kb1; ++kb) {
+            if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+            uint8_t* base = stage_base + stage * Cfg::STAGE_BYTES;
+            auto rests = [&](const uint8_t* from, uint8_t* to) {
+                const float4 x = *reinterpret_cast<const float4*>(from);
+                auto rest = [](float f) { return f - __uint_as_float(__float_as_uint(f) & 0xFFFFE000u); };
+                *reinterpret_cast<float4*>(to) = make_float4(rest(x.x), rest(x.y), rest(x.z), rest(x.w));
+            };
+#pragma unroll 8
+            for (int i = tid * 16; i < Cfg::B_BYTES; i += X3_WARPS * 512) rests(base + Cfg::A_BYTES + i, base + Cfg::LOAD_BYTES + i);
+#pragma unroll 8
+            for (int i = tid * 16; i < Cfg::A_BYTES; i += X3_WARPS * 512) rests(base + i, base + Cfg::LOAD_BYTES + Cfg::B_BYTES + i);
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&lo_bar[stage]);
+            if (++stage == STAGES) { stage = 0; phase ^= 1u; }
+        }
+        if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.err, 4); }
     } else if (SPLIT) {
         // ------------------------------------------------ epilogue of a tile that a cluster shares
         // Every CTA leaves its part in its own ring (all its operands have been read), in blocks of 32 columns with the rows' 16-byte
@@ -390,6 +435,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 if (have_acc) {
                     tmem_ld32(t_row + (uint32_t)(ch * 32), v);
                     tmem_ld_wait();
+                    if (X3) {
+                        auto add = [&](int col) {
+                            uint32_t w[32];
+                            tmem_ld32(t_row + (uint32_t)(col + ch * 32), w);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+                        };
+                        const bool both = c_first.kb1 > c_first.kb0 + 1;
+                        if (both) add(2 * BN);
+                        add(BN);
+                        if (both) add(3 * BN);
+                    }
                 } else {
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] = 0u;
@@ -1569,11 +1627,11 @@ static int choose_splits(const DeviceCtx* ctx, const GemmArgs& a, int bn) {
 // are 128- and 192-column tiles and 256 x 384 tiles of a CTA pair, these also with the product formed the other way round
 // (C^T = op(B)^T op(A)^T, turned by the reduction) where it is M that fits 384.  Bytes per flop of the three: 1, 0.83, 0.42.
 // The default rule stays where nothing is expected to beat it by a tenth.
-static GemmArgs arranged(const DeviceCtx* ctx, const GemmArgs& a) {
+static bool arranged(const DeviceCtx* ctx, const GemmArgs& a, GemmArgs* out) {
     const int bke = a.tf32 ? BK_TF32 : BK;
     if (a.kind != GEMM_TN || a.bn != 0 || a.swapped || a.batch != 1 || a.causal != CAUSAL_NONE || a.c_inner > 1 || a.bias || a.residual || a.C16 ||
         !a.C32 || a.N <= 64 || a.K < 16 * bke || (long long)((a.M + BM - 1) / BM) * ((a.N + 127) / 128) * 2 > ctx->sm_count)
-        return a;
+        return false;
     const int sms = (a.max_ctas > 0 && a.max_ctas < ctx->sm_count) ? a.max_ctas : ctx->sm_count, kb = (a.K + bke - 1) / bke;
     const int given = a.planned ? 0 : a.splits;
     auto turned = [&]() {
@@ -1590,11 +1648,11 @@ static GemmArgs arranged(const DeviceCtx* ctx, const GemmArgs& a) {
         return waves * (per * (bn == 128 ? 32.0 : 40.0) / 94.0 + (pair ? 5.0 : bn == 192 ? 1.8 : 1.2)) +
                (s == 1 ? 0.0 : cluster_adds(ctx, g, bn, s) ? 1.5 : 2.0 + (s + 1) * slab / 6.0);
     };
-    GemmArgs best = a;
+    int best_bn = 0;
     double least = time_of(a, pick_bn(ctx, a)) * 0.9;
     auto consider = [&](const GemmArgs& g, int bn) {
         const double t = time_of(g, bn);
-        if (t < least) { least = t; best = g; best.bn = bn; }
+        if (t < least) { least = t; *out = g; out->bn = best_bn = bn; }
     };
     consider(a, 128);
     if (a.N > 128) consider(a, 192);
@@ -1606,12 +1664,13 @@ static GemmArgs arranged(const DeviceCtx* ctx, const GemmArgs& a) {
             if (s > 1 && (given == 0 || given == s)) consider(t, 384);
         }
     }
-    return best;
+    return best_bn != 0;
 }
 
 int planned_splits(const DeviceCtx* ctx, const GemmArgs& a0) {
     if (a0.residual || a0.c_inner > 1) return 1;
-    const GemmArgs a = arranged(ctx, a0);
+    GemmArgs other;
+    const GemmArgs& a = arranged(ctx, a0, &other) ? other : a0;
     return choose_splits(ctx, a, pick_bn(ctx, a));
 }
 
@@ -1619,8 +1678,9 @@ template <int BN, bool TF32, bool PAIR = false, int EPI = EPI_ANY>
 static int launch_impl(DeviceCtx* ctx, const GemmArgs& a, const GemmParams& p, const CUtensorMap& tmA,
                        const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmR,
                        cudaStream_t stream) {
-    using Cfg = GemmCfg<BN, PAIR, EPI == EPI_NORM>;
-    static_assert(EPI != EPI_SPLIT || Cfg::STAGES * Cfg::STAGE_BYTES >= BM * BN * 4, "a CTA's part of a tile lies in its ring");
+    using Cfg = GemmCfg<BN, PAIR, EPI == EPI_NORM, EPI == EPI_X3>;
+    constexpr bool SPLIT = EPI == EPI_SPLIT || EPI == EPI_X3;
+    static_assert(!SPLIT || Cfg::STAGES * Cfg::STAGE_BYTES >= BM * BN * 4, "a CTA's part of a tile lies in its ring");
     static bool attr_set[64] = {false};
     if (!attr_set[ctx->device & 63]) {
         TB_CUDA(cudaFuncSetAttribute(gemm_bf16_kernel<BN, TF32, PAIR, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1637,10 +1697,10 @@ static int launch_impl(DeviceCtx* ctx, const GemmArgs& a, const GemmParams& p, c
         grid = (int)(total < sms ? total : sms);
     }
     if (grid < 1) grid = PAIR ? 2 : 1;
-    if (EPI == EPI_SPLIT) grid = (int)total * p.csplit;
+    if (SPLIT) grid = (int)total * p.csplit;
     if (EPI == EPI_NORM) grid = p.nt * std::min(p.mt, std::max(1, sms / p.nt));       // whole clusters of p.nt CTAs
-    TB_CUDA(launch_kernel_cluster((gemm_bf16_kernel<BN, TF32, PAIR, EPI>), dim3(grid), dim3(NUM_THREADS), Cfg::SMEM_BYTES,
-                                  stream, EPI == EPI_NORM ? p.nt : EPI == EPI_SPLIT ? p.csplit : PAIR ? 2 : 1, tmA, tmB, tmC, tmR, p));
+    TB_CUDA(launch_kernel_cluster((gemm_bf16_kernel<BN, TF32, PAIR, EPI>), dim3(grid), dim3(threads_of(EPI)), Cfg::SMEM_BYTES,
+                                  stream, EPI == EPI_NORM ? p.nt : SPLIT ? p.csplit : PAIR ? 2 : 1, tmA, tmB, tmC, tmR, p));
     TB_CUDA(cudaGetLastError());
     ctx->launches++;
     prof_close(ctx, stream);
@@ -1747,7 +1807,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
     p.a_mn = a_mn; p.b_mn = b_mn; p.causal = (int)a.causal;
     p.dsw = 0; p.wide16 = 0;
     p.err = ctx->d_err;
-    const bool in_cluster = cluster_adds(ctx, a, bn, splits);
+    const bool in_cluster = a.x3 || cluster_adds(ctx, a, bn, splits);
     p.csplit = in_cluster ? splits : 0;
     if (in_cluster) p.splits = 1;
     if (splits > 1 && !in_cluster) {
@@ -1882,7 +1942,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         if (ctx->prof_on) {
             char tag[128];
             static const char* kn[3] = {"NN", "NT", "TN"};
-            snprintf(tag, sizeof(tag), "%s:%s:%dx%dx%d:b%d:s%d:c%d:bn%d%s", a.tf32 ? "gemm_tf32" : "gemm_bf16",
+            snprintf(tag, sizeof(tag), "%s:%s:%dx%dx%d:b%d:s%d:c%d:bn%d%s", a.x3 ? "gemm_x3" : a.tf32 ? "gemm_tf32" : "gemm_bf16",
                      kn[(int)a.kind], a.M, a.N, a.K, a.batch, splits, (int)a.causal, bn, swiglu ? ":swiglu" : a.rope_qkv ? ":rope" : a.ce_mode == 1 ? ":ce_stats" : a.ce_mode == 2 ? ":ce_grad" : a.norm_w ? ":norm" : "");
             // the second cross-entropy pass repeats pass 1's product: its flops are not algorithmic work
             prof_mark(ctx, prof_intern(tag), a.ce_mode == 2 ? 0.0 : 2.0 * macs, in_bytes + out_bytes, stream);
@@ -1897,6 +1957,9 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         else if (bn == 128) TB_TRY(TB_NORM_LAUNCH(128));
         else                TB_TRY(TB_NORM_LAUNCH(192));
 #undef TB_NORM_LAUNCH
+    } else if (a.x3) {
+        if (bn == 64) TB_TRY((launch_impl<64, true, false, EPI_X3>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
+        else          TB_TRY((launch_impl<128, true, false, EPI_X3>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
     } else if (in_cluster) {
 #define TB_SPLIT_LAUNCH(W)                                                                                             \
         (a.tf32 ? launch_impl<W, true, false, EPI_SPLIT>(ctx, a, p, tmA, tmB, tmC, tmR, stream)                          \
@@ -1971,8 +2034,44 @@ static int check_splits(const GemmArgs& a, int* splits) {
     return 0;
 }
 
+// Where the product goes this way: one wave of clusters, whose fixed 6.6 (64 columns) or 8.1 us and time per slice the sweep over both
+// widths and 1 - 8 CTAs per cluster gave.  us, pieces written out in memory : split on chip --
+//  * 1024 x 1152 x 384 13.9 : 11.6, 1024 x 384 x 1152 15.6 : 12.2, 64 x 384 x 1152 10.7 : 7.6, 256^3 7.9 : 6.6, 1024^3 23.0 : 17.7,
+//    weight gradients 384 x 1152 x 1024 16.1 : 12.0, of 8192 rows 84.9 : 45.2;
+//  * several waves, each paying the fixed part again: 8192 x 1152 x 384 52 : 62, 8192 x 2048 x 384 69 : 111, 3000 x 1000 x 1000 42 : 55;
+//  * short K, where little is written out: 64 x 256 x 64 5.6 : 6.0, 256 x 256 x 128 7.1 : 7.5, 240 x 70 x 168 6.7 : 6.8, and with most
+//    SMs taken by unsplit tiles (pair tiles are as fast there) 1024 x 2048 x 384 15.7 : 16.1, 2953 x 492 x 192 12.4 : 12.8.
+// A share of K is at most twice as long as the other way's (two pairs of accumulators): the sums are rounded no more often.
+// 64 x 64 x 8192, one cluster of eight against 148 splits: error 1.0e-6 : 1.6e-6.
+bool plan_gemm_x3(const DeviceCtx* ctx, GemmArgs* a) {
+    const int kb = (a->K + BK_TF32 - 1) / BK_TF32;
+    if (kb < 6 || a->batch != 1 || a->residual || !a->C32 || getenv("TB_GEMM_NO_X3") != nullptr) return false;
+    const long long mt = (a->M + BM - 1) / BM;
+    GemmArgs pieces = *a;
+    pieces.K = 3 * a->K; pieces.tf32 = true;
+    const int other = planned_splits(ctx, pieces), longest = 2 * ((3 * kb + other - 1) / other);
+    double least = 1e30;
+    for (int bn = 64; bn <= 128; bn += 64) {
+        const long long tiles = mt * ((a->N + bn - 1) / bn);
+        for (int n = 1; n <= 8; ++n) {
+            const int per = (kb + n - 1) / n, s = (kb + per - 1) / per;
+            if (s != n || per > longest || (s > 1 ? per < 3 : (bn == 128 && 2 * tiles > ctx->sm_count && kb < 16))) continue;
+            if (tiles > (s == 1 ? ctx->sm_count : cluster_room(ctx, s))) continue;
+            const double us = per * (bn == 64 ? 0.53 : 0.58) + (bn == 64 ? 6.6 : 8.1) + (s > 1 ? 0.8 : 0.0);
+            if (us < least) { least = us; a->bn = bn; a->splits = s; }
+        }
+    }
+    a->tf32 = a->x3 = least < 1e30;
+    return a->x3;
+}
+
+int launch_gemm_x3(DeviceCtx* ctx, const GemmArgs& a, cudaStream_t stream) {
+    return launch_core(ctx, a, a.bn, a.splits, nullptr, stream);
+}
+
 int launch_gemm_bf16(DeviceCtx* ctx, const GemmArgs& a0, cudaStream_t stream) {
-    const GemmArgs a = arranged(ctx, a0);
+    GemmArgs other;
+    const GemmArgs& a = arranged(ctx, a0, &other) ? other : a0;
     const int bn = pick_bn(ctx, a);
     int splits = a.splits > 0 ? a.splits : choose_splits(ctx, a, bn);
     TB_TRY(check_splits(a, &splits));
@@ -1987,7 +2086,8 @@ int launch_gemm_bf16(DeviceCtx* ctx, const GemmArgs& a0, cudaStream_t stream) {
 
 int launch_gemm_bf16_ws(DeviceCtx* ctx, const GemmArgs& a0, float* workspace, size_t workspace_floats,
                         cudaStream_t stream) {
-    const GemmArgs a = arranged(ctx, a0);
+    GemmArgs other;
+    const GemmArgs& a = arranged(ctx, a0, &other) ? other : a0;
     const int bn = pick_bn(ctx, a);
     int splits = a.splits > 0 ? a.splits : choose_splits(ctx, a, bn);
     TB_TRY(check_splits(a, &splits));
