@@ -660,3 +660,35 @@ def test_float32_product_splits_its_slices_on_chip(tb, monkeypatch, kind, shape)
     monkeypatch.setenv("TB_GEMM_NO_X3", "1")
     pieces, launches = run(C0)
     assert launches >= 2 and np.array_equal(np.isfinite(special), np.isfinite(pieces))
+
+
+@pytest.mark.parametrize("shape", [(4739, 300, 1190), (7400, 190, 2104), (5000, 1000, 700)])
+@pytest.mark.parametrize("tf32", [False, True], ids=["bf16", "tf32"])
+def test_192_column_tiles_on_cta_pairs(tb, monkeypatch, shape, tf32):
+    """B stored [N, K], tiles of 256 x 192: ragged rows, columns and K, previous contents and bias, against float64 and single CTAs.
+    Operands are exact in either type, so what differs is the sum: every addition of a K step may lose 2^-23 of the magnitudes."""
+    M, N, K = shape
+    rng = np.random.default_rng(M)
+    ld = (K + 7) // 8 * 8
+    A, B = torch.zeros(M, ld, device="cuda", dtype=torch.bfloat16), torch.zeros(N, ld, device="cuda", dtype=torch.bfloat16)
+    A[:, :K] = torch.from_numpy(rng.standard_normal((M, K)).astype(np.float32)).cuda().bfloat16()
+    B[:, :K] = torch.from_numpy(rng.standard_normal((N, K)).astype(np.float32)).cuda().bfloat16()
+    C0 = torch.from_numpy(rng.standard_normal((M, N)).astype(np.float32)).cuda()
+    bias = C0[0].clone()
+    want = A[:, :K].double() @ B[:, :K].double().T + 2.0 * C0.double()
+    bound = (K / 8 + 4) * 2.0 ** -23 * (A[:, :K].double().abs() @ B[:, :K].double().abs().T + 2.0 * C0.abs())
+    if not tf32:
+        want, bound = want + bias, bound + 2.0 ** -22 * bias.abs()
+    a32, b32, got = A.float(), B.float(), []
+    for single in (False, True):
+        if single:
+            monkeypatch.setenv("TB_GEMM_NO_PAIR", "1")
+        C = C0.clone()
+        if tf32:
+            tb.gemm_f32(tb.NT, a32, b32, C, M, N, K, ld, ld, N, beta=2.0, precision=tb.PREC_TF32)
+        else:
+            tb.gemm_bf16(tb.NT, A, B, M, N, K, ld, ld, C32=C, ldc32=N, bias=bias, beta=2.0, tile_n=192)
+        tb.sync_check()
+        assert bool(((C.double() - want).abs() <= bound).all())
+        got.append(C)
+    assert bool(((got[0] - got[1]).abs() <= 2 * bound).all())

@@ -1501,6 +1501,21 @@ static int pick_norm_bn(const DeviceCtx* ctx, int M, int N, bool tf32) {
 }
 bool gemm_norm_pays(const DeviceCtx* ctx, int M, int N, bool tf32) { return pick_norm_bn(ctx, M, N, tf32) > 0; }
 
+// 192-column tiles on CTA pairs (256 x 192): 28 KB of operands per K slice and CTA against 40 on single CTAs.  B has to be stored
+// [N, K] (half a tile of it is 96 rows; stored [K, N] it would be one and a half boxes of 64 columns).  For products that are not
+// split, where the pairs' waves do not eat the gain up and a CTA has 18 slices in all: the pairs' start costs ~0.7 us.  us, single CTAs
+// : pairs (and the width chosen without them): 8192 x 384 x 2048 14.0 : 13.1, 8192 x 768 x 768 13.5 : 12.9 (14.5), 8192 x 576 x 1024
+// 15.4 : 14.1 (18.9; float32 operands, the chosen width, 31.9 : 22.5), 8192 x 1152 x 384 13.8 : 12.8, 8192 x 384 x 384 6.3 : 7.0.
+static bool pairs_of_192(const DeviceCtx* ctx, const GemmArgs& a) {
+    if (a.kind != GEMM_NT || a.batch != 1 || a.causal != CAUSAL_NONE || a.c_inner > 1 || a.M < 512 || a.ce_mode != 0 || a.dsw_dgu || a.norm_w ||
+        a.C32 == nullptr || a.C16 || getenv("TB_GEMM_NO_PAIR") != nullptr)
+        return false;
+    const int sms = (a.max_ctas > 0 && a.max_ctas < ctx->sm_count) ? a.max_ctas : ctx->sm_count;
+    const long long nt = (a.N + 191) / 192, single = (a.M + BM - 1) / BM * nt, pairs = (a.M + 2 * BM - 1) / (2 * BM) * nt;
+    const long long waves = (pairs + sms / 2 - 1) / (sms / 2), kb = (a.K + (a.tf32 ? BK_TF32 : BK) - 1) / (a.tf32 ? BK_TF32 : BK);
+    return single * 2 > sms && waves * kb >= 18 && waves * 28 < (single + sms - 1) / sms * 40;
+}
+
 static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
     if (a.norm_w) return pick_norm_bn(ctx, a.M, a.N, a.tf32);
     // time ~ waves x tile width x a factor for how often a tile re-reads its operands from L2
@@ -1519,6 +1534,10 @@ static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
             // a narrow output wastes part of the second 256-wide column of tiles; only a long K loop pays for that
             const double narrow = (a.N < 512 && a.K < 64 * (a.tf32 ? BK_TF32 : BK)) ? 1.15 : 1.0;
             return (double)((tiles + pairs - 1) / pairs) * 256 * factor[3] * narrow;
+        }
+        if (width == 192 && pairs_of_192(ctx, a)) {
+            const long long tiles = (a.M + 2 * BM - 1) / (2 * BM) * ((a.N + 191) / 192);
+            return (double)((tiles + sms / 2 - 1) / (sms / 2)) * 192 * factor[2] * 0.85;       // (6000 x 384 x 1152 9.5 us, 128 columns 8.1)
         }
         const long long tiles = mt * ((a.N + width - 1) / width) * a.batch;
         return (double)((tiles + sms - 1) / sms) * width * factor[width / 64 - 1];
@@ -1789,7 +1808,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
     const int bke = a.tf32 ? BK_TF32 : BK;
     if (!a_mn) TB_TRY(make_operand_map_es(&tmA, a.A, es, a.K, a.M, a.lda, a.batch, a.strideA, BM));
     else       TB_TRY(make_operand_map_es(&tmA, a.A, es, a.M, a.K, a.lda, a.batch, a.strideA, bke, true));
-    const bool pair = bn == 256 || bn == 384;
+    const bool pair = bn == 256 || bn == 384 || (bn == 192 && splits == 1 && !a.x3 && pairs_of_192(ctx, a));
     if (pair)
         TB_CHECK(a.batch == 1 && a.causal == CAUSAL_NONE && a.c_inner <= 1,
                  "256-wide CTA-pair tiles take one plain product (no batch, no causal mode)");
@@ -1980,7 +1999,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         (epi == EPI_F32 ? launch_impl<W, true, true, EPI_F32>(ctx, a, p, tmA, tmB, tmC, tmR, stream)                     \
                         : launch_impl<W, true, true, EPI_ANY>(ctx, a, p, tmA, tmB, tmC, tmR, stream))
         if (bn == 64)       TB_TRY(TB_TF32_LAUNCH(64));
-        else if (bn == 192) TB_TRY(TB_TF32_LAUNCH(192));
+        else if (bn == 192) TB_TRY(pair ? TB_TF32_PAIR(192) : TB_TF32_LAUNCH(192));
         else if (bn == 256) TB_TRY(TB_TF32_PAIR(256));
         else if (bn == 384) TB_TRY(TB_TF32_PAIR(384));
         else if (p.tma_mode == 5 && !general_only) TB_TRY((launch_impl<128, true, false, EPI_ROPE>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
@@ -1989,6 +2008,9 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
 #undef TB_TF32_PAIR
     } else if (pair && bn == 384) {
         TB_TRY((launch_bf16<384, true>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
+    } else if (pair && bn == 192) {
+        if (p.tma_mode == 1) TB_TRY((launch_impl<192, false, true, EPI_F32>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
+        else                 TB_TRY((launch_impl<192, false, true, EPI_ANY>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
     } else if (pair) {
         TB_TRY((launch_bf16<256, true>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
     } else {
