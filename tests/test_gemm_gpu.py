@@ -621,6 +621,22 @@ def test_splits_added_inside_a_cluster(tb, monkeypatch, kind, shape, precision):
         assert np.abs(got[0] - got[1]).max() <= 1e-6 * np.abs(got[1]).max()
 
 
+@pytest.mark.parametrize("shape", [(384, 1152, 8192), (1024, 384, 8192), (400, 232, 2608), (384, 1152, 2048), (64, 72, 1100)])
+def test_cluster_sums_round_like_the_reduction_kernel(tb, monkeypatch, shape):
+    """Whoever adds them, the parts of a product are as many and come in the same order: the same bits."""
+    M, N, K = shape
+    A, B = (torch.randn(r, c, device="cuda").bfloat16() for r, c in ((M, (K + 7) // 8 * 8), (K, N)))
+    got = []
+    for off in (False, True):
+        if off:
+            monkeypatch.setenv("TB_GEMM_NO_CLUSTER_SPLIT", "1")
+        C = torch.empty(M, N, device="cuda")
+        tb.gemm_bf16(tb.NN, A, B, M, N, K, A.shape[1], N, C32=C, ldc32=N)
+        tb.sync_check()
+        got.append(C)
+    assert torch.equal(*got)
+
+
 @pytest.mark.parametrize("kind", ["NN", "NT", "TN"])
 @pytest.mark.parametrize("shape", [(4, 4, 192), (100, 68, 228), (132, 132, 420), (200, 72, 1100), (384, 1152, 1024), (1000, 260, 2048), (64, 2048, 384)])
 def test_float32_product_splits_its_slices_on_chip(tb, monkeypatch, kind, shape):

@@ -1606,7 +1606,8 @@ static int cluster_room(const DeviceCtx* ctx, int s) {
 }
 
 // Whether the splits of a product are added by clusters: one wave of them, alone on the chip (beside another product the SMs of a
-// cluster may not be free together).
+// cluster may not be free together).  As many splits as with the reduction kernel, so sums are rounded as often.  (Three products of a
+// layer, 1024 rows of 384 : 1152 in float32 pieces 51.0 -> 49.7 us, 8192 of 384 : 2048 in bf16 60.7 -> 60.0.)
 static bool cluster_adds(const DeviceCtx* ctx, const GemmArgs& a, int bn, int splits) {
     if (splits < 2 || splits > 8 || bn > 192 || a.batch != 1 || a.c_inner > 1 || a.causal != CAUSAL_NONE || a.max_ctas > 0 || (!a.C32 && !a.C16) ||
         a.residual || a.swapped || getenv("TB_GEMM_NO_CLUSTER_SPLIT") != nullptr)
@@ -1626,26 +1627,15 @@ static int choose_splits(const DeviceCtx* ctx, const GemmArgs& a, int bn) {
     int s = (int)(workers / tiles);
     if (s > kb_total / 4) s = kb_total / 4;     // at least 4 K slices per split
     if (s < 1) s = 1;
-    auto whole = [&](int n) { const int per = (kb_total + n - 1) / n; return (kb_total + per - 1) / per; };     // no empty split
-    // Fewer splits that a cluster adds against more with a reduction kernel: us at ~94 KB/us of operands per SM, 1.5 for the exchange,
-    // 2 for the launch and 6 MB/us for the slabs.  (Three products of a layer, 1024 rows of 384 : 1152 in float32 pieces 51.0 -> 49.7 us,
-    // 8192 of 384 : 2048 in bf16 60.7 -> 60.0.)
-    const double slice = (bn + 128) * 0.125 / 94.0, slab = (double)a.M * a.N * 4e-6;
-    auto slices = [&](int n) { return (double)((kb_total + n - 1) / n); };
-    const double by_kernel = slices(whole(s)) * slice + 2.0 + (whole(s) + 1) * slab / 6.0;
-    for (int n = s < 8 ? s : 8; n > 1; --n)
-        if (cluster_adds(ctx, a, bn, whole(n))) {
-            if (slices(whole(n)) * slice + 1.5 <= by_kernel) return whole(n);
-            break;
-        }
-    return whole(s);
+    const int kb_per = (kb_total + s - 1) / s;
+    return (kb_total + kb_per - 1) / kb_per;     // no empty split
 }
 
 // A weight gradient (few tiles, long K, split along it) by the tile that is estimated to take least: operand bytes a CTA pulls at
 // the ~94 KB/us that an SM gets from L2, the last tile's epilogue, and the reduction of the partial slabs at ~6 MB/us.  Candidates
 // are 128- and 192-column tiles and 256 x 384 tiles of a CTA pair, these also with the product formed the other way round
 // (C^T = op(B)^T op(A)^T, turned by the reduction) where it is M that fits 384.  Bytes per flop of the three: 1, 0.83, 0.42.
-// The default rule stays where nothing is expected to beat it by a tenth.
+// The default rule stays where nothing is expected to beat it by a tenth, and no choice makes a split's share of K longer than its.
 static bool arranged(const DeviceCtx* ctx, const GemmArgs& a, GemmArgs* out) {
     const int bke = a.tf32 ? BK_TF32 : BK;
     if (a.kind != GEMM_TN || a.bn != 0 || a.swapped || a.batch != 1 || a.causal != CAUSAL_NONE || a.c_inner > 1 || a.bias || a.residual || a.C16 ||
@@ -1658,9 +1648,13 @@ static bool arranged(const DeviceCtx* ctx, const GemmArgs& a, GemmArgs* out) {
         t.A = a.B; t.B = a.A; t.M = a.N; t.N = a.M; t.lda = a.ldb; t.ldb = a.lda; t.swapped = true;
         return t;
     };
+    auto share_of = [&](const GemmArgs& g, int bn) {             // K slices of a split
+        const int s = given > 0 ? given : choose_splits(ctx, g, bn);
+        return (kb + s - 1) / s;
+    };
     auto time_of = [&](const GemmArgs& g, int bn) {
         const bool pair = bn == 384;
-        const int s = given > 0 ? given : choose_splits(ctx, g, bn), per = (kb + s - 1) / s;
+        const int per = share_of(g, bn), s = (kb + per - 1) / per;
         const long long tiles = (long long)((g.M + (pair ? 2 * BM : BM) - 1) / (pair ? 2 * BM : BM)) * ((g.N + bn - 1) / bn) * s;
         const int workers = pair ? sms / 2 : sms;
         const double waves = (double)((tiles + workers - 1) / workers), slab = (double)a.M * a.N * 4e-6;
@@ -1668,10 +1662,11 @@ static bool arranged(const DeviceCtx* ctx, const GemmArgs& a, GemmArgs* out) {
                (s == 1 ? 0.0 : cluster_adds(ctx, g, bn, s) ? 1.5 : 2.0 + (s + 1) * slab / 6.0);
     };
     int best_bn = 0;
+    const int longest = share_of(a, pick_bn(ctx, a));
     double least = time_of(a, pick_bn(ctx, a)) * 0.9;
     auto consider = [&](const GemmArgs& g, int bn) {
         const double t = time_of(g, bn);
-        if (t < least) { least = t; *out = g; out->bn = best_bn = bn; }
+        if (t < least && share_of(g, bn) <= longest) { least = t; *out = g; out->bn = best_bn = bn; }
     };
     consider(a, 128);
     if (a.N > 128) consider(a, 192);
