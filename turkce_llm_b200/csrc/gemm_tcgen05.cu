@@ -468,26 +468,26 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             for (int i = (int)threadIdx.x - 64; i < rows * PIECES; i += EPI_WARPS * 32) {
                 const int row = first + i / PIECES, c4 = i % PIECES;
                 const uint32_t at = base + (uint32_t)((c4 >> 3) * (BM * ROW_BYTES) + row * ROW_BYTES + (((c4 & 7) ^ (row & 7)) << 4));
+                const int gm = c_first.m0 + row, gn = c_first.n0 + 4 * c4;
+                float* cp = p.C32 + (long long)gm * p.ldc32 + gn;
+                const bool in = gm < p.M && gn < p.N, whole = p.C32 && gn + 3 < p.N && p.vec32;
+                // (the previous contents are on their way while the parts are: with beta, 384 x 384 over 1024 rows 7.2 -> 6.4 us, 384 x 2048 over 8192 18.4 -> 17.6)
+                float4 prev = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (in && whole && p.beta != 0.0f) prev = *reinterpret_cast<const float4*>(cp);
                 float4 v[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k) if (k < p.csplit) v[k] = ld_cluster_f32x4(mapa_cluster(at, (uint32_t)k));
                 float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) if (k < p.csplit) { s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
-                const int gm = c_first.m0 + row, gn = c_first.n0 + 4 * c4;
-                if (gm >= p.M || gn >= p.N) continue;
+                if (!in) continue;
                 float o[4] = {s.x * p.alpha, s.y * p.alpha, s.z * p.alpha, s.w * p.alpha};
-                float* cp = p.C32 + (long long)gm * p.ldc32 + gn;
-                const bool whole = p.C32 && gn + 3 < p.N && p.vec32;
                 if (p.bias) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) if (gn + e < p.N) o[e] += __ldg(p.bias + gn + e);
                 }
                 if (whole) {
-                    if (p.beta != 0.0f) {
-                        const float4 c4v = *reinterpret_cast<const float4*>(cp);
-                        o[0] += p.beta * c4v.x; o[1] += p.beta * c4v.y; o[2] += p.beta * c4v.z; o[3] += p.beta * c4v.w;
-                    }
+                    if (p.beta != 0.0f) { o[0] += p.beta * prev.x; o[1] += p.beta * prev.y; o[2] += p.beta * prev.z; o[3] += p.beta * prev.w; }
                     *reinterpret_cast<float4*>(cp) = make_float4(o[0], o[1], o[2], o[3]);
                 } else if (p.C32) {
 #pragma unroll
