@@ -678,6 +678,22 @@ def test_float32_product_splits_its_slices_on_chip(tb, monkeypatch, kind, shape)
     assert launches >= 2 and np.array_equal(np.isfinite(special), np.isfinite(pieces))
 
 
+def test_float32_product_over_its_operand_and_with_rows_that_repeat(tb):
+    """Where C lies over A, or a leading dimension of zero repeats one row, the operands' pieces are written out first, as they were
+    before there was a way without: the same result as with arrays apart."""
+    n = 256
+    A, B = torch.randn(n, n, device="cuda"), torch.randn(n, n, device="cuda")
+    want = A.double() @ B.double()
+    bound = (3 * 2.0 ** -20 + (n / 8 + 4) * 2.0 ** -23) * (A.double().abs() @ B.double().abs())
+    C = A.clone()
+    tb.gemm_f32(tb.NN, C, B, C, n, n, n, n, n, n, precision=tb.PREC_FP32)
+    tb.sync_check()
+    assert bool(((C.double() - want).abs() <= bound).all())
+    tb.gemm_f32(tb.NN, A, B, C, n, n, n, 0, n, n, precision=tb.PREC_FP32)
+    tb.sync_check()
+    assert bool(((C.double() - want[:1]).abs() <= bound[:1]).all())
+
+
 @pytest.mark.parametrize("shape", [(4739, 300, 1190), (7400, 190, 2104), (5000, 1000, 700)])
 @pytest.mark.parametrize("tf32", [False, True], ids=["bf16", "tf32"])
 def test_192_column_tiles_on_cta_pairs(tb, monkeypatch, shape, tf32):

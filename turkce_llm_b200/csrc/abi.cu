@@ -303,7 +303,15 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
         return launch_gemm_bf16_ws(ctx, g, ws, ws_floats, stream);
     }
 
-    if (precision == TB_PREC_FP32 && tma_ok_f32(A, lda, batch, sA) && tma_ok_f32(B, ldb, batch, sB)) {
+    // (Written-out pieces are read before C is written and in whatever way rows lie: a C that lies over an operand, and rows that
+    // lie over one another, stay with them.)
+    auto apart = [&](const float* x, int rows, int cols, long long ld) {
+        const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), x1 = x0 + ((long long)(rows - 1) * ld + cols) * 4;
+        const uintptr_t c0 = reinterpret_cast<uintptr_t>(C), c1 = c0 + ((long long)(M - 1) * ldc + N) * 4;
+        return ld >= cols && (x1 <= c0 || c1 <= x0);
+    };
+    if (precision == TB_PREC_FP32 && tma_ok_f32(A, lda, batch, sA) && tma_ok_f32(B, ldb, batch, sB) && apart(A, a_rows, a_cols, lda) &&
+        apart(B, b_rows, b_cols, ldb)) {
         GemmArgs x = g;
         x.A = A; x.B = B; x.lda = lda; x.ldb = ldb;
         if (plan_gemm_x3(ctx, &x)) return launch_gemm_x3(ctx, x, stream);

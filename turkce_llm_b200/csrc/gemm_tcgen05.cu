@@ -7,17 +7,18 @@
 // a transposed operand is not transposed in memory, it is described to the tensor core
 // as an MN-major shared-memory tile instead of a K-major one.
 //
-// CTA = 6 warps, one CTA per SM, tiles 128 x BN handed out round-robin:
+// CTA = 10 warps, one CTA per SM, tiles 128 x BN handed out round-robin:
 //   warp 0     TMA producer: 64-wide K slices of A and B into a ring of 128B-swizzled stages
 //   warp 1     owns TMEM (2 accumulators of BN columns) and issues tcgen05.mma (one lane)
-//   warps 2-5  epilogue: tcgen05.ld -> registers -> per-warp shared staging -> coalesced
+//   warps 2-9  epilogue: tcgen05.ld -> registers -> per-warp shared staging -> coalesced
 //              global stores with bias / residual / beta*C / bf16 copy fused
 // The two accumulators let the epilogue of tile i overlap the main loop of tile i+1,
 // which matters because K is only 384..1024 here (6..16 slices per tile).
 //
 // Split-K (weight gradients: small M,N, K = tokens) writes one partial tile per split into
 // scratch memory; reduce_splits_kernel then adds the partials in split order, so the result
-// does not depend on scheduling (the reference forbids atomics: train_kernels.cu:17-20).
+// does not depend on scheduling (the reference forbids atomics: train_kernels.cu:17-20).  Where one
+// wave of clusters holds the tiles, a cluster adds the parts in the same order through its shared memory.
 #include "../../include/turkce_b200.h"
 #include "common.h"
 #include "ptx.cuh"
@@ -43,10 +44,10 @@ constexpr int STAGE_LD = 36;        // floats per staging row (32 + 4 pad: confl
 
 // PAIR: two CTAs of a cluster share a 256 x BN tile (cta_group::2): each loads its own 128 rows of A and
 // BN/2 columns of B, so a CTA's shared-memory traffic per output element drops by BN/(128 + BN/2)/(BN/(128+BN)).
-// BN = 384 (PAIR, B stored [K, N]): for products with N <= 384 and a long K (the LM-head gradients): one tile spans
+// BN = 384 (PAIR): for products with N <= 384 and a long K (the LM-head gradients) or beside another product: one tile spans
 // the whole N, 40 KB per K slice feed 768 tensor-core cycles (53 B/clk against 64 for 256 x 256 with half of the
 // second tile empty).  The tensor core takes N <= 256, so a K step is three instructions of 128 columns; each CTA
-// loads the 64-column boxes at n0 + 128 j + 64 rank, which keeps accumulator column = output column.  One accumulator.
+// loads the 64-column boxes (64 rows of B stored [N, K]) at n0 + 128 j + 64 rank: accumulator column = output column.  One accumulator.
 // NORM: the CTAs of a cluster hold the columns of one row block between them and exchange the rows' sums of squares
 // X3: a stage holds A | B | rest of B | rest of A (see EPI_X3); its epilogue needs no staging
 template <int BN, bool PAIR = false, bool NORM = false, bool X3 = false> struct GemmCfg {
