@@ -694,6 +694,21 @@ def test_float32_product_over_its_operand_and_with_rows_that_repeat(tb):
     assert bool(((C.double() - want[:1]).abs() <= bound[:1]).all())
 
 
+@pytest.mark.parametrize("over", ["A", "B"])
+def test_split_product_over_its_operand(tb, over):
+    """A product split along K writes C when its operands have been read, if C lies over one of them: the same bits as apart."""
+    n = 512
+    A, B = torch.randn(n, n, device="cuda"), torch.randn(n, n, device="cuda")
+    got = []
+    for apart in (True, False):
+        a, b = A.clone(), B.clone()
+        C = torch.empty_like(A) if apart else (a if over == "A" else b)
+        tb.gemm_f32(tb.NN, a, b, C, n, n, n, n, n, n, precision=tb.PREC_TF32)
+        tb.sync_check()
+        got.append(C)
+    assert torch.equal(*got)
+
+
 @pytest.mark.parametrize("shape", [(4739, 300, 1190), (7400, 190, 2104), (5000, 1000, 700)])
 @pytest.mark.parametrize("tf32", [False, True], ids=["bf16", "tf32"])
 def test_192_column_tiles_on_cta_pairs(tb, monkeypatch, shape, tf32):

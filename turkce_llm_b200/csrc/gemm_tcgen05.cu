@@ -1616,6 +1616,25 @@ static bool cluster_adds(const DeviceCtx* ctx, const GemmArgs& a, int bn, int sp
     return (long long)((a.M + BM - 1) / BM) * ((a.N + bn - 1) / bn) <= cluster_room(ctx, splits);
 }
 
+// The reduction kernel writes C when both operands have been read, a cluster while others still read them: an output that lies over an
+// operand keeps the kernel.
+static bool output_apart(const GemmArgs& a) {
+    const int es = a.tf32 ? 4 : 2;
+    auto over = [](const void* x, long long rows, long long cols, long long ld, int size, const void* y, long long yrows, long long ycols, long long yld, int ysize) {
+        const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), x1 = x0 + ((rows - 1) * ld + cols) * size;
+        const uintptr_t y0 = reinterpret_cast<uintptr_t>(y), y1 = y0 + ((yrows - 1) * yld + ycols) * ysize;
+        return y != nullptr && x0 < y1 && y0 < x1;
+    };
+    for (int k = 0; k < 2; ++k) {
+        const void* c = k == 0 ? (const void*)a.C32 : (const void*)a.C16;
+        const long long ldc = k == 0 ? a.ldc32 : a.ldc16;
+        if (over(a.A, a.kind == GEMM_TN ? a.K : a.M, a.kind == GEMM_TN ? a.M : a.K, a.lda, es, c, a.M, a.N, ldc, k == 0 ? 4 : 2) ||
+            over(a.B, a.kind == GEMM_NT ? a.N : a.K, a.kind == GEMM_NT ? a.K : a.N, a.ldb, es, c, a.M, a.N, ldc, k == 0 ? 4 : 2))
+            return false;
+    }
+    return true;
+}
+
 static int choose_splits(const DeviceCtx* ctx, const GemmArgs& a, int bn) {
     if (a.causal != CAUSAL_NONE) return 1;
     const int tile_m = bn >= 256 ? 2 * BM : BM;                     // a CTA pair owns 256 rows
@@ -1822,7 +1841,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
     p.a_mn = a_mn; p.b_mn = b_mn; p.causal = (int)a.causal;
     p.dsw = 0; p.wide16 = 0;
     p.err = ctx->d_err;
-    const bool in_cluster = a.x3 || cluster_adds(ctx, a, bn, splits);
+    const bool in_cluster = a.x3 || (cluster_adds(ctx, a, bn, splits) && output_apart(a));
     p.csplit = in_cluster ? splits : 0;
     if (in_cluster) p.splits = 1;
     if (splits > 1 && !in_cluster) {
