@@ -739,3 +739,20 @@ def test_192_column_tiles_on_cta_pairs(tb, monkeypatch, shape, tf32):
         assert bool(((C.double() - want).abs() <= bound).all())
         got.append(C)
     assert bool(((got[0] - got[1]).abs() <= 2 * bound).all())
+
+
+@pytest.mark.parametrize("precision", ["native", "tf32", "fp32"])
+def test_parts_of_a_split_product_are_scaled_before_they_are_added(tb, precision):
+    """Each part is 2^126 or below and eight of them leave float32's range, but not alpha times them: every value here is a power of
+    two or a sum of equal ones, so the result is exact."""
+    n, K = 128, 1024
+    A, B = torch.full((n, K), 2.0 ** 60, device="cuda"), torch.full((K, n), 2.0 ** 59, device="cuda")
+    C = torch.zeros(n, n, device="cuda")
+    before = tb.launch_count()
+    if precision == "native":
+        tb.gemm_bf16(tb.NN, A.bfloat16(), B.bfloat16(), n, n, K, K, n, C32=C, ldc32=n, alpha=2.0 ** -4, splits=8)
+    else:
+        tb.gemm_f32(tb.NN, A, B, C, n, n, K, K, n, n, alpha=2.0 ** -4, precision={"tf32": tb.PREC_TF32, "fp32": tb.PREC_FP32}[precision])
+    tb.sync_check()
+    assert tb.launch_count() - before == 1
+    assert bool((C == 2.0 ** 125).all())

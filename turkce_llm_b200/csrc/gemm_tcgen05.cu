@@ -453,6 +453,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] = 0u;
                 }
+                // (scaled here, part by part, as the slabs are: a sum that only alpha brings back into range stays finite)
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * p.alpha);
                 uint8_t* dst = stage_base + (half * NCH + ch) * (BM * ROW_BYTES) + row * ROW_BYTES;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(dst + ((j ^ (row & 7)) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
@@ -482,7 +485,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 #pragma unroll
                 for (int k = 0; k < 8; ++k) if (k < p.csplit) { s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
                 if (!in) continue;
-                float o[4] = {s.x * p.alpha, s.y * p.alpha, s.z * p.alpha, s.w * p.alpha};
+                float o[4] = {s.x, s.y, s.z, s.w};
                 if (p.bias) {
 #pragma unroll
                     for (int e = 0; e < 4; ++e) if (gn + e < p.N) o[e] += __ldg(p.bias + gn + e);
