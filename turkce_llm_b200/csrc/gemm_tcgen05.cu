@@ -161,7 +161,7 @@ __device__ __forceinline__ TileCoord tile_of(const GemmParams& p, int t, int row
 // a 32-column chunk costs ~0.15 us more in instruction fetches); the other values fix the mode at compile time and
 // drop the rest -- measured on an [8192 x 384 x 1152] launch: last tile's epilogue 2.42 -> 1.89 us (float32 out),
 // 2.02 -> 1.54 us (bf16 out).
-enum { EPI_ANY = 0, EPI_F32, EPI_BF16, EPI_SWIGLU, EPI_CE1, EPI_ROPE, EPI_CE2, EPI_DSW, EPI_NORM, EPI_SPLIT, EPI_X3 };
+enum { EPI_ANY = 0, EPI_F32, EPI_BF16, EPI_SWIGLU, EPI_CE1, EPI_ROPE, EPI_CE2, EPI_DSW, EPI_NORM, EPI_SPLIT, EPI_X3, EPI_ROPE_TAB };
 constexpr int threads_of(int epi) { return NUM_THREADS + (epi == EPI_X3 ? X3_WARPS * 32 : 0); }
 
 template <int BN, bool TF32, bool PAIR = false, int EPI = EPI_ANY>
@@ -225,12 +225,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const bool m_f32 = ANY ? p.tma_mode == 1 : EPI == EPI_F32;           // float32 tiles by TMA
     const bool m_swiglu = ANY ? p.tma_mode == 3 : EPI == EPI_SWIGLU;
     const bool m_ce1 = ANY ? p.tma_mode == 4 : EPI == EPI_CE1;
-    const bool m_rope = ANY ? p.tma_mode == 5 : EPI == EPI_ROPE;
+    constexpr bool ROPE = EPI == EPI_ROPE || EPI == EPI_ROPE_TAB;          // (TAB: with the rotation tables by TMA)
+    const bool m_rope = ANY ? p.tma_mode == 5 : ROPE;
     const bool m_ce2 = ANY ? p.ce_mode == 2 : EPI == EPI_CE2;
     const bool m_dsw = ANY ? p.dsw != 0 : EPI == EPI_DSW;
     const bool m_res = (ANY || EPI == EPI_F32) && p.tma_res != 0;        // a residual / previous-C tile only with float32 tiles
-    const bool m_bias = (ANY || EPI == EPI_F32 || EPI == EPI_BF16 || EPI == EPI_ROPE) && p.bias != nullptr;
-    const bool m_wide = (ANY || EPI == EPI_BF16 || EPI == EPI_ROPE || EPI == EPI_CE2) ? p.wide16 != 0 : EPI == EPI_DSW;
+    const bool m_bias = (ANY || EPI == EPI_F32 || EPI == EPI_BF16 || ROPE) && p.bias != nullptr;
+    const bool m_wide = (ANY || EPI == EPI_BF16 || ROPE || EPI == EPI_CE2) ? p.wide16 != 0 : EPI == EPI_DSW;
     if (threadIdx.x == 0) TS(0);
 
     // Prologue: nothing here reads or writes memory an earlier kernel of the stream produces, so it
@@ -830,7 +831,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             // output buffer) and serves every head of the tile.  Read by the rows' threads from global memory it was 16 accesses
             // of 32 different lines each per head and row, and the epilogue took longer than the main loop: QKV projection of
             // 8192, 3885 and 11200 rows of 384 in the live step 20, 14 and 30 us that way, 16.8, 11.3 and 25 this way.
-            const bool rope_tab = EPI == EPI_ROPE && p.rope_tab != 0;
+            constexpr bool rope_tab = EPI == EPI_ROPE_TAB;
             bool rope_wait = false;
             if (m_rope) {
                 rope_b = gm0 / p.rope_T; rope_t0 = gm0 - rope_b * p.rope_T; rope_t = rope_t0 + lane;
@@ -868,6 +869,35 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 const bool active = rows_in && gn0 < p.N;
                 if (lane == 0 && !second) {                   // the unit's output buffer has been read out
                     if (m_dsw || rope_tab) tma_store_wait_read<0>(); else tma_store_wait_read<1>();
+                }
+                // the angles of this chunk, 32 consecutive head-dim values of one head: all asked for before the accumulator is waited for
+                const bool rotated = m_rope && gn0 < 2 * rope_D;
+                float4 c4[4], s4[4];
+                if (rotated) {
+                    const int d0 = (gn0 - (gn0 >= rope_D ? rope_D : 0)) & (p.rope_hd - 1);
+                    const long long off = (long long)rope_t * (p.rope_hd >> 1) + (d0 >> 1);
+                    if (rope_wait) {
+                        if (!mbar_wait(rbar, rphase, abort_flag)) { ok = false; break; }
+                        rphase ^= 1u;
+                        rope_wait = false;
+                    }
+                    // (rows of the next sequence are read where they are)
+                    const bool tab = rope_tab && rows_in && rope_t0 + lane < p.rope_T;
+                    const uint8_t* trow = obuf + 4096 + lane * 128;
+                    if (tab) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const int so = (((d0 >> 3) + j) ^ (lane & 7)) << 4;
+                            c4[j] = *reinterpret_cast<const float4*>(trow + so);
+                            s4[j] = *reinterpret_cast<const float4*>(trow + 4096 + so);
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            c4[j] = __ldg(reinterpret_cast<const float4*>(p.rope_cos + off) + j);
+                            s4[j] = __ldg(reinterpret_cast<const float4*>(p.rope_sin + off) + j);
+                        }
+                    }
                 }
                 __syncwarp();
                 uint32_t v[32];
@@ -914,30 +944,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 }
                 if (m_rope) {
                     // position embedding on the q and k columns: pairs (2k, 2k+1) of a head rotate by the
-                    // angle of (position, k); this chunk is 32 consecutive head-dim values of one head
-                    if (gn0 < 2 * rope_D) {
-                        const int d0 = (gn0 - (gn0 >= rope_D ? rope_D : 0)) & (p.rope_hd - 1);
-                        const long long off = (long long)rope_t * (p.rope_hd >> 1) + (d0 >> 1);
-                        if (rope_wait) {
-                            if (!mbar_wait(rbar, rphase, abort_flag)) { ok = false; break; }
-                            rphase ^= 1u;
-                            rope_wait = false;
-                        }
-                        // (rows of the next sequence are read where they are)
-                        const bool tab = rope_tab && rows_in && rope_t0 + lane < p.rope_T;
-                        const uint8_t* trow = obuf + 4096 + lane * 128;
+                    // angle of (position, k)
+                    if (rotated) {
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
-                            float4 c4, s4;
-                            if (tab) {
-                                const int so = (((d0 >> 3) + j) ^ (lane & 7)) << 4;
-                                c4 = *reinterpret_cast<const float4*>(trow + so);
-                                s4 = *reinterpret_cast<const float4*>(trow + 4096 + so);
-                            } else {
-                                c4 = __ldg(reinterpret_cast<const float4*>(p.rope_cos + off) + j);
-                                s4 = __ldg(reinterpret_cast<const float4*>(p.rope_sin + off) + j);
-                            }
-                            const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
+                            const float cc[4] = {c4[j].x, c4[j].y, c4[j].z, c4[j].w}, ss[4] = {s4[j].x, s4[j].y, s4[j].z, s4[j].w};
 #pragma unroll
                             for (int i = 0; i < 4; ++i) {
                                 const float a0 = o[8 * j + 2 * i], b0 = o[8 * j + 2 * i + 1];
@@ -1033,7 +1044,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 if (paired && !second) continue;              // the unit leaves after its second chunk
                 if (m_rope && rope_direct) {
                     // row by row: 8 (head dim 64) or 4 adjacent lanes write a row's values of one head, 128 or 64 bytes
-                    fence_proxy_async();              // (the tables' place is written by the next tile's copy)
+                    if (rope_tab) fence_proxy_async();              // (the tables' place is written by the next tile's copy)
                     __syncwarp();
                     const int g0 = paired ? gn0 - 32 : gn0;
                     if (rows_in && g0 < p.N) {
@@ -1772,6 +1783,7 @@ static int launch_bf16(DeviceCtx* ctx, const GemmArgs& a, const GemmParams& p, c
         if (epi == EPI_CE2) return launch_impl<BN, false, PAIR, EPI_CE2>(ctx, a, p, tmA, tmB, tmC, tmR, stream);
     }
     if constexpr (BN == 128) {
+        if (epi == EPI_ROPE && p.rope_tab) return launch_impl<BN, false, PAIR, EPI_ROPE_TAB>(ctx, a, p, tmA, tmB, tmC, tmR, stream);
         if (epi == EPI_ROPE) return launch_impl<BN, false, PAIR, EPI_ROPE>(ctx, a, p, tmA, tmB, tmC, tmR, stream);
     }
     return launch_impl<BN, false, PAIR, EPI_ANY>(ctx, a, p, tmA, tmB, tmC, tmR, stream);
@@ -1905,8 +1917,10 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         TB_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled (QKV output) failed with code %d", (int)r);
         p.tma_mode = 5;
         // The tables come in by TMA where they are one array, the sines behind the cosines (the trainer's and the decoder's are); a
-        // map whose outer stride spans two allocations is not used.
-        if (wide && a.rope_sin == a.rope_cos + (size_t)a.rope_rows * (hd / 2) && a.rope_rows >= a.rope_T && aligned16(a.rope_cos)) {
+        // map whose outer stride spans two allocations is not used.  Where most of 32 rows lie in two sequences, a warp's rows go both
+        // ways and the other instantiation is faster (validation loss of 3800 tokens, 12 layers, us, row by row : by TMA: sequences of 31
+        // 854 : 856, 32 836 : 810, 33 852 : 858, 36 847 : 838, 48 809 : 772).
+        if (wide && (a.rope_T >= 34 || a.rope_T == 32) && a.rope_sin == a.rope_cos + (size_t)a.rope_rows * (hd / 2) && a.rope_rows >= a.rope_T && aligned16(a.rope_cos)) {
             const cuuint64_t rows = (cuuint64_t)a.rope_rows;
             cuuint64_t tdims[3] = {hd / 2, rows, 2}, tstrides[2] = {hd * 2, rows * hd * 2};
             cuuint32_t tbox[3] = {32u, 32u, 2u};
@@ -2020,6 +2034,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         else if (bn == 192) TB_TRY(pair ? TB_TF32_PAIR(192) : TB_TF32_LAUNCH(192));
         else if (bn == 256) TB_TRY(TB_TF32_PAIR(256));
         else if (bn == 384) TB_TRY(TB_TF32_PAIR(384));
+        else if (p.tma_mode == 5 && !general_only && p.rope_tab) TB_TRY((launch_impl<128, true, false, EPI_ROPE_TAB>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
         else if (p.tma_mode == 5 && !general_only) TB_TRY((launch_impl<128, true, false, EPI_ROPE>(ctx, a, p, tmA, tmB, tmC, tmR, stream)));
         else                TB_TRY(TB_TF32_LAUNCH(128));
 #undef TB_TF32_LAUNCH
