@@ -7,6 +7,9 @@ Two comparisons per case, both with the reference's metric max|got-want| / max|w
   * against the float32 oracle -- the BF16-mode bound 2e-2 the task states.
 """
 import json
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -19,6 +22,8 @@ pytestmark = pytest.mark.gpu
 
 TOL_SAME_OPERANDS = 2e-5
 TOL_BF16_MODE = 2e-2
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 KINDS = {"NN": 0, "NT": 1, "TN": 2}
 
@@ -756,3 +761,32 @@ def test_parts_of_a_split_product_are_scaled_before_they_are_added(tb, precision
     tb.sync_check()
     assert tb.launch_count() - before == 1
     assert bool((C == 2.0 ** 125).all())
+
+
+def test_clusters_keep_to_the_sms_that_are_not_reserved():
+    """TB_SM_RESERVE leaves SMs to another library's kernels.  With 40 of them reserved, 15 tiles in clusters of eight do not fit into
+    the rest (two launches instead of one), and a float32 product takes no more CTAs than there are SMs left."""
+    code = """
+import torch
+from turkce_llm_b200 import lib as tb
+tb.init(0)
+left = torch.cuda.get_device_properties(0).multi_processor_count - 40
+A, B, C = torch.randn(1920, 2048, device="cuda").bfloat16(), torch.randn(2048, 128, device="cuda").bfloat16(), torch.zeros(1920, 128, device="cuda")
+before = tb.launch_count()
+tb.gemm_bf16(tb.NN, A, B, 1920, 128, 2048, 2048, 128, C32=C, ldc32=128, splits=8, tile_n=128)
+print("launches", tb.launch_count() - before)
+tb.profile_begin()
+for M, N, K in ((1024, 1152, 384), (1024, 384, 1152), (384, 1152, 1024), (1024, 1024, 1024), (640, 640, 640)):
+    x, w, y = torch.randn(M, K, device="cuda"), torch.randn(K, N, device="cuda"), torch.zeros(M, N, device="cuda")
+    tb.gemm_f32(tb.NN, x, w, y, M, N, K, K, N, N, precision=tb.PREC_FP32)
+for tag in tb.profile_end(torch.cuda.current_stream().cuda_stream):
+    if tag.startswith("gemm_x3"):
+        _, _, shape, _, s, _, bn = tag.split(":")[:7]
+        M, N, K = (int(v) for v in shape.split("x"))
+        ctas = -(-M // 128) * -(-N // int(bn[2:])) * int(s[1:])
+        print("ctas", tag, ctas)
+        assert ctas <= left, tag
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=ROOT, env={**os.environ, "TB_SM_RESERVE": "40"})
+    assert r.returncode == 0, r.stderr
+    assert "launches 2" in r.stdout and "ctas" in r.stdout, r.stdout

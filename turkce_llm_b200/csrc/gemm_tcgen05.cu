@@ -1596,10 +1596,12 @@ static int pick_bn(const DeviceCtx* ctx, const GemmArgs& a) {
     return best;
 }
 
-// How many clusters of s CTAs with a whole SM each run at a time (1 <= s <= 8, the portable sizes).  Processor clusters hold between
-// 16 and 20 SMs, so it is not 148 / s.
+// How many clusters of s CTAs with a whole SM each run at a time (1 <= s <= 8, the portable sizes) on the SMs this library may take
+// (TB_SM_RESERVE).  Processor clusters differ in their SMs, so on the whole chip it is not 148 / s but 74, 45, 33, 26, 22, 15 and 15
+// for 2 .. 8.
 static int cluster_room(const DeviceCtx* ctx, int s) {
     static std::atomic<int> room[64][9];
+    if (s == 1) return ctx->sm_count;
     std::atomic<int>& r = room[ctx->device & 63][s];
     if (r.load(std::memory_order_relaxed) == 0) {
         using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, GemmParams);
@@ -1617,7 +1619,7 @@ static int cluster_room(const DeviceCtx* ctx, int s) {
             cudaGetLastError();
         r.store(n > 0 ? n : -1, std::memory_order_relaxed);
     }
-    return r.load(std::memory_order_relaxed);
+    return std::min(r.load(std::memory_order_relaxed), ctx->sm_count / s);
 }
 
 // Whether the splits of a product are added by clusters: one wave of them, alone on the chip (beside another product the SMs of a
@@ -2111,7 +2113,7 @@ bool plan_gemm_x3(const DeviceCtx* ctx, GemmArgs* a) {
         for (int n = 1; n <= 8; ++n) {
             const int per = (kb + n - 1) / n, s = (kb + per - 1) / per;
             if (s != n || per > longest || (s > 1 ? per < 3 : (bn == 128 && 2 * tiles > ctx->sm_count && kb < 16))) continue;
-            if (tiles > (s == 1 ? ctx->sm_count : cluster_room(ctx, s))) continue;
+            if (tiles > cluster_room(ctx, s)) continue;
             const double us = per * (bn == 64 ? 0.53 : 0.58) + (bn == 64 ? 6.6 : 8.1) + (s > 1 ? 0.8 : 0.0);
             if (us < least) { least = us; a->bn = bn; a->splits = s; }
         }
