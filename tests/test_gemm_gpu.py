@@ -790,3 +790,29 @@ for tag in tb.profile_end(torch.cuda.current_stream().cuda_stream):
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=ROOT, env={**os.environ, "TB_SM_RESERVE": "40"})
     assert r.returncode == 0, r.stderr
     assert "launches 2" in r.stdout and "ctas" in r.stdout, r.stdout
+
+
+@pytest.mark.parametrize("outputs", ["C16", "both"])
+@pytest.mark.parametrize("pad", [0, 3], ids=["by_four", "by_one"])
+@pytest.mark.parametrize("shape", [(3, 72, 1024, 8, 64), (16, 136, 1024, 5, 128), (130, 70, 2048, 3, 64), (129, 388, 1024, 2, 192)])
+def test_cluster_sums_of_few_rows_and_bf16_outputs(tb, monkeypatch, shape, pad, outputs):
+    """Fewer rows than CTAs, a last tile of one or two rows, bf16 outputs that can and cannot be written four at a time, with bias and
+    previous contents: the bits of the reduction kernel, and nothing written past a row's end."""
+    M, N, K, splits, bn = shape
+    A, B = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(K, (N + 7) // 8 * 8, device="cuda").bfloat16()
+    bias, C0 = torch.randn(N, device="cuda"), torch.randn(M, N + pad, device="cuda")
+    got = []
+    for off in (False, True):
+        if off:
+            monkeypatch.setenv("TB_GEMM_NO_CLUSTER_SPLIT", "1")
+        C, C16 = C0.clone(), C0.bfloat16()
+        before = tb.launch_count()
+        tb.gemm_bf16(tb.NN, A, B, M, N, K, K, B.shape[1], C32=C if outputs == "both" else None, ldc32=N + pad, C16=C16, ldc16=N + pad, bias=bias,
+                     alpha=0.75, beta=0.5, splits=splits, tile_n=bn)
+        tb.sync_check()
+        assert tb.launch_count() - before == (2 if off else 1)
+        assert torch.equal(C[:, N:], C0[:, N:]) and torch.equal(C16[:, N:], C0.bfloat16()[:, N:])
+        got.append((C, C16))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    want = 0.75 * (A.double() @ B[:, :N].double()) + bias.double() + (0.5 * C0[:, :N].double() if outputs == "both" else 0.0)
+    assert ((got[0][1][:, :N].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5 * want.abs().max()).all()

@@ -28,6 +28,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 #include <cstring>
 
 namespace tb {
@@ -422,7 +423,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         // ------------------------------------------------ epilogue of a tile that a cluster shares
         // Every CTA leaves its part in its own ring (all its operands have been read), in blocks of 32 columns with the rows' 16-byte
         // pieces swizzled; then each adds its share of the rows over all CTAs in rank order.  Sums have a fixed order, partial slabs
-        // in memory and the kernel that reduces them are gone: see choose_splits for both sides' figures.
+        // in memory and the kernel that reduces them are gone: see cluster_adds for both sides' figures.
         const int q = warp & 3, ew = warp - 2, half = ew >> 2;
         constexpr int NCH = BN / 64;
         bool ok = mbar_wait(&acc_full[0], 0, abort_flag);
@@ -467,44 +468,108 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
         if (ok) {
             constexpr int PIECES = BN / 4;                   // 16-byte pieces of a row
-            const int per = (BM + p.csplit - 1) / p.csplit, first = srank * per, rows = min(BM, first + per) - first;
+            const int there = min(BM, p.M - c_first.m0), per = (there + p.csplit - 1) / p.csplit, first = srank * per;       // (rows that exist)
+            const int rows = min(there, first + per) - first;
             const uint32_t base = smem_u32(stage_base);
-#pragma unroll 1
-            for (int i = (int)threadIdx.x - 64; i < rows * PIECES; i += EPI_WARPS * 32) {
-                const int row = first + i / PIECES, c4 = i % PIECES;
-                const uint32_t at = base + (uint32_t)((c4 >> 3) * (BM * ROW_BYTES) + row * ROW_BYTES + (((c4 & 7) ^ (row & 7)) << 4));
-                const int gm = c_first.m0 + row, gn = c_first.n0 + 4 * c4;
-                float* cp = p.C32 + (long long)gm * p.ldc32 + gn;
-                const bool in = gm < p.M && gn < p.N, whole = p.C32 && gn + 3 < p.N && p.vec32;
-                // (the previous contents are on their way while the parts are: with beta, 384 x 384 over 1024 rows 7.2 -> 6.4 us, 384 x 2048 over 8192 18.4 -> 17.6)
-                float4 prev = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (in && whole && p.beta != 0.0f) prev = *reinterpret_cast<const float4*>(cp);
-                float4 v[8];
+            auto sum_of = [&](uint32_t at) {                 // of a piece over the CTAs, in rank order
+                float4 v[8], s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) if (k < p.csplit) v[k] = ld_cluster_f32x4(mapa_cluster(at, (uint32_t)k));
-                float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int k = 0; k < 8; ++k) if (k < p.csplit) { s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
-                if (!in) continue;
-                float o[4] = {s.x, s.y, s.z, s.w};
-                if (p.bias) {
+                return s;
+            };
+            // Only rows that exist are shared out, and previous contents and bias are on their way while the parts are (us, with a tile's
+            // 128 rows shared out and unaligned contents read behind the sum : now; the reduction kernel in brackets): 16 x 384 x 1152 NT
+            // bf16 5.9 : 4.7 [5.8], 64 x 384 x 1024 6.3 : 5.3 [5.9], 303 x 70 over 519 rows, tf32 with beta, 15.2 : 9.0 [11.5].  The code
+            // runs once per launch and its fetches count: outputs that can be addressed by four columns have a loop of their own.
+            if constexpr (X3) {
+                // (one loop for every output: faster here, 384 x 1152 over 1024 rows 12.8 -> 12.2)
+#pragma unroll 1
+                for (int i = (int)threadIdx.x - 64; i < rows * PIECES; i += EPI_WARPS * 32) {
+                    const int row = first + i / PIECES, c4 = i % PIECES;
+                    const uint32_t at = base + (uint32_t)((c4 >> 3) * (BM * ROW_BYTES) + row * ROW_BYTES + (((c4 & 7) ^ (row & 7)) << 4));
+                    const int gm = c_first.m0 + row, gn = c_first.n0 + 4 * c4;
+                    float* cp = p.C32 + (long long)gm * p.ldc32 + gn;
+                    const bool in = gm < p.M && gn < p.N, whole = p.C32 && gn + 3 < p.N && p.vec32, bias4 = p.bias && p.bias_vec && gn + 3 < p.N;
+                    float4 prev = make_float4(0.f, 0.f, 0.f, 0.f), add = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (in && whole && p.beta != 0.0f) prev = *reinterpret_cast<const float4*>(cp);
+                    else if (in && p.C32 && p.beta != 0.0f) {
+                        prev.x = cp[0];
+                        if (gn + 1 < p.N) prev.y = cp[1];
+                        if (gn + 2 < p.N) prev.z = cp[2];
+                        if (gn + 3 < p.N) prev.w = cp[3];
+                    }
+                    if (bias4) add = __ldg(reinterpret_cast<const float4*>(p.bias + gn));
+                    float4 v[8];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) if (gn + e < p.N) o[e] += __ldg(p.bias + gn + e);
-                }
-                if (whole) {
+                    for (int k = 0; k < 8; ++k) if (k < p.csplit) v[k] = ld_cluster_f32x4(mapa_cluster(at, (uint32_t)k));
+                    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) if (k < p.csplit) { s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
+                    if (!in) continue;
+                    float o[4] = {s.x, s.y, s.z, s.w};
+                    if (bias4) { o[0] += add.x; o[1] += add.y; o[2] += add.z; o[3] += add.w; }
+                    else if (p.bias) {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) if (gn + e < p.N) o[e] += __ldg(p.bias + gn + e);
+                    }
                     if (p.beta != 0.0f) { o[0] += p.beta * prev.x; o[1] += p.beta * prev.y; o[2] += p.beta * prev.z; o[3] += p.beta * prev.w; }
-                    *reinterpret_cast<float4*>(cp) = make_float4(o[0], o[1], o[2], o[3]);
-                } else if (p.C32) {
+                    if (whole) *reinterpret_cast<float4*>(cp) = make_float4(o[0], o[1], o[2], o[3]);
+                    else {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) if (gn + e < p.N) {
-                        if (p.beta != 0.0f) o[e] += p.beta * cp[e];
-                        cp[e] = o[e];
+                        for (int e = 0; e < 4; ++e) if (gn + e < p.N) cp[e] = o[e];
                     }
                 }
-                if (p.C16) {
+            } else {
+                auto add_parts = [&](auto by_four) {
+#pragma unroll 1
+                    for (int i = (int)threadIdx.x - 64; i < rows * PIECES; i += EPI_WARPS * 32) {
+                        const int row = first + i / PIECES, c4 = i % PIECES;
+                        const int gm = c_first.m0 + row, gn = c_first.n0 + 4 * c4, left = p.N - gn;
+                        constexpr bool vec = decltype(by_four)::value;
+                        const bool in = left > 0;
+                        const uint32_t at = base + (uint32_t)((c4 >> 3) * (BM * ROW_BYTES) + row * ROW_BYTES + (((c4 & 7) ^ (row & 7)) << 4));
+                        float* cp = p.C32 + (long long)gm * p.ldc32 + gn;
+                        float prev[4] = {0.f, 0.f, 0.f, 0.f}, add[4] = {0.f, 0.f, 0.f, 0.f};
+                        auto fetch = [&](const float* from, float (&to)[4]) {
+                            if (vec) {
+                                const float4 x = *reinterpret_cast<const float4*>(from);
+                                to[0] = x.x; to[1] = x.y; to[2] = x.z; to[3] = x.w;
+                            } else {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) if (gn + e < p.N) p.C16[(long long)gm * p.ldc16 + gn + e] = __float2bfloat16_rn(o[e]);
-                }
+                                for (int e = 0; e < 4; ++e) if (e < left) to[e] = from[e];
+                            }
+                        };
+                        if (in && p.C32 && p.beta != 0.0f) fetch(cp, prev);
+                        if (in && p.bias) fetch(p.bias + gn, add);
+                        const float4 s = sum_of(at);
+                        if (!in) continue;
+                        float o[4] = {s.x, s.y, s.z, s.w};
+                        if (p.bias) { o[0] += add[0]; o[1] += add[1]; o[2] += add[2]; o[3] += add[3]; }
+                        if (p.C32) {
+                            if (p.beta != 0.0f) { o[0] += p.beta * prev[0]; o[1] += p.beta * prev[1]; o[2] += p.beta * prev[2]; o[3] += p.beta * prev[3]; }
+                            if (vec) *reinterpret_cast<float4*>(cp) = make_float4(o[0], o[1], o[2], o[3]);
+                            else {
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) if (e < left) cp[e] = o[e];
+                            }
+                        }
+                        if (p.C16) {
+                            bf16* c16 = p.C16 + (long long)gm * p.ldc16 + gn;
+                            if (vec) {
+                                __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
+                                *reinterpret_cast<uint2*>(c16) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+                            } else {
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) if (e < left) c16[e] = __float2bfloat16_rn(o[e]);
+                            }
+                        }
+                    }
+                };
+                const bool aligned = (!p.C32 || p.vec32) && (!p.C16 || p.vec16) && (!p.bias || p.bias_vec);
+                if (aligned && p.N % 4 == 0) add_parts(std::true_type{});
+                else add_parts(std::false_type{});
             }
         }
         if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.err, 3); }
@@ -1623,8 +1688,9 @@ static int cluster_room(const DeviceCtx* ctx, int s) {
 }
 
 // Whether the splits of a product are added by clusters: one wave of them, alone on the chip (beside another product the SMs of a
-// cluster may not be free together).  As many splits as with the reduction kernel, so sums are rounded as often.  (Three products of a
-// layer, 1024 rows of 384 : 1152 in float32 pieces 51.0 -> 49.7 us, 8192 of 384 : 2048 in bf16 60.7 -> 60.0.)
+// cluster may not be free together).  As many splits as with the reduction kernel, so sums are rounded as often.  us, reduction kernel :
+// cluster, over 128 products of 16 .. 8192 rows in three operand types 0.64 .. 1.03 of the time, 5 of them above 1.02 (384 x 384 over
+// 2048 rows 7.4 : 7.6): 16 x 384 x 1152 5.8 : 4.7, 700 x 384 x 1024 6.9 : 6.6, 384 x 1152 over 1024 rows 8.7 : 7.6, 384 x 2048 over 8192 18.8 : 18.2.
 static bool cluster_adds(const DeviceCtx* ctx, const GemmArgs& a, int bn, int splits) {
     if (splits < 2 || splits > 8 || bn > 192 || a.batch != 1 || a.c_inner > 1 || a.causal != CAUSAL_NONE || a.max_ctas > 0 || (!a.C32 && !a.C16) ||
         a.residual || a.swapped || getenv("TB_GEMM_NO_CLUSTER_SPLIT") != nullptr)
