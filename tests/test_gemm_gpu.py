@@ -816,3 +816,41 @@ def test_cluster_sums_of_few_rows_and_bf16_outputs(tb, monkeypatch, shape, pad, 
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
     want = 0.75 * (A.double() @ B[:, :N].double()) + bias.double() + (0.5 * C0[:, :N].double() if outputs == "both" else 0.0)
     assert ((got[0][1][:, :N].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2e-5 * want.abs().max()).all()
+
+
+def tile_of(tb, call):
+    """Tile width, splits and shape that a call's product was launched with, from the profile's tags."""
+    tb.profile_begin()
+    call()
+    tags = [t for t in tb.profile_end(torch.cuda.current_stream().cuda_stream) if t.startswith("gemm_")]
+    assert len(tags) == 1, tags
+    _, _, shape, _, s, _, bn = tags[0].split(":")[:7]
+    return int(bn[2:]), int(s[1:]), tuple(int(v) for v in shape.split("x"))
+
+
+@pytest.mark.parametrize("M,N,K,wide", [(384, 1152, 8192, False), (384, 696, 12000, False), (384, 1496, 10000, False), (384, 2048, 5000, False),
+                                        (384, 2048, 14336, True)])
+def test_wide_tiles_of_a_weight_gradient_alone_only_where_they_gain(tb, M, N, K, wide):
+    """Float32 operands read as tf32: 384 columns formed the other way round took 1.1 to 1.5 times as long as the usual tile with few
+    tiles or a short K, and 0.86 at the last of these shapes."""
+    A, B, C = torch.randn(K, M, device="cuda"), torch.randn(K, N, device="cuda"), torch.zeros(M, N, device="cuda")
+    bn, _, shape = tile_of(tb, lambda: tb.gemm_f32(tb.TN, A, B, C, M, N, K, M, N, N, beta=1.0, precision=tb.PREC_TF32))
+    assert (bn == 384) == wide and shape == ((N, M, K) if wide else (M, N, K))
+
+
+@pytest.mark.parametrize("beta", [0.0, 1.0])
+@pytest.mark.parametrize("M,N", [(300, 1994), (260, 2049), (384, 1802)])
+def test_weight_gradient_formed_the_other_way_round(tb, M, N, beta):
+    """C^T = B^T A in 384-column tiles, turned back by the reduction: rows and columns that end inside its 32 x 32 blocks, a leading
+    dimension beyond the columns, against float64.  Operands are exact in tf32, so what differs is the sum: every addition of eight
+    products may lose 2^-23 of the magnitudes."""
+    K = 14000
+    A, B = torch.randn(K, M, device="cuda").bfloat16().float(), torch.randn(K, N, device="cuda").bfloat16().float()
+    C0 = torch.randn(M, N + 5, device="cuda")
+    C = C0.clone()
+    bn, splits, shape = tile_of(tb, lambda: tb.gemm_f32(tb.TN, A, B, C, M, N, K, M, N, N + 5, beta=beta, precision=tb.PREC_TF32))
+    assert bn == 384 and splits > 1 and shape == (N, M, K)
+    want = A.double().T @ B.double() + beta * C0[:, :N].double()
+    bound = (K / 8 + 4) * 2.0 ** -23 * (A.double().abs().T @ B.double().abs() + beta * C0[:, :N].abs())
+    assert bool(((C[:, :N].double() - want).abs() <= bound).all())
+    assert torch.equal(C[:, N:], C0[:, N:])

@@ -1738,6 +1738,10 @@ static int choose_splits(const DeviceCtx* ctx, const GemmArgs& a, int bn) {
 // are 128- and 192-column tiles and 256 x 384 tiles of a CTA pair, these also with the product formed the other way round
 // (C^T = op(B)^T op(A)^T, turned by the reduction) where it is M that fits 384.  Bytes per flop of the three: 1, 0.83, 0.42.
 // The default rule stays where nothing is expected to beat it by a tenth, and no choice makes a split's share of K longer than its.
+// Alone on the chip a slice takes longer than its bytes say: 0.75 us of 384 columns (columns that do not exist take none), 0.50 of 192 in
+// float32.  With more than nine splits of the 384-column tile it is 0.9 - 1.3, so those are left out.  For float32 the figures are near
+// enough to ask for 1.5 % only.  us, default rule : 384 columns, float32: 384 x 1152 over 8192 rows 22.2 : 27.8, 384 x 696 over 12000 21.5 : 33.2,
+// 384 x 2048 over 5000 22.1 : 24.9, over 8192 35.8 : 34.5, over 14336 55.3 : 47.5; bf16: 384 x 1496 over 14336 25.5 : 30.6.
 static bool arranged(const DeviceCtx* ctx, const GemmArgs& a, GemmArgs* out) {
     const int bke = a.tf32 ? BK_TF32 : BK;
     if (a.kind != GEMM_TN || a.bn != 0 || a.swapped || a.batch != 1 || a.causal != CAUSAL_NONE || a.c_inner > 1 || a.bias || a.residual || a.C16 ||
@@ -1745,6 +1749,7 @@ static bool arranged(const DeviceCtx* ctx, const GemmArgs& a, GemmArgs* out) {
         return false;
     const int sms = (a.max_ctas > 0 && a.max_ctas < ctx->sm_count) ? a.max_ctas : ctx->sm_count, kb = (a.K + bke - 1) / bke;
     const int given = a.planned ? 0 : a.splits;
+    const bool alone = a.max_ctas == 0;
     auto turned = [&]() {
         GemmArgs t = a;
         t.A = a.B; t.B = a.A; t.M = a.N; t.N = a.M; t.lda = a.ldb; t.ldb = a.lda; t.swapped = true;
@@ -1760,15 +1765,17 @@ static bool arranged(const DeviceCtx* ctx, const GemmArgs& a, GemmArgs* out) {
         const long long tiles = (long long)((g.M + (pair ? 2 * BM : BM) - 1) / (pair ? 2 * BM : BM)) * ((g.N + bn - 1) / bn) * s;
         const int workers = pair ? sms / 2 : sms;
         const double waves = (double)((tiles + workers - 1) / workers), slab = (double)a.M * a.N * 4e-6;
-        return waves * (per * (bn == 128 ? 32.0 : 40.0) / 94.0 + (pair ? 5.0 : bn == 192 ? 1.8 : 1.2)) +
+        const double slice = alone && pair ? 0.75 * g.N / 384 : alone && a.tf32 && bn == 192 ? 0.50 : (bn == 128 ? 32.0 : 40.0) / 94.0;
+        return waves * (per * slice + (pair ? 5.0 : bn == 192 ? 1.8 : 1.2)) +
                (s == 1 ? 0.0 : cluster_adds(ctx, g, bn, s) ? 1.5 : 2.0 + (s + 1) * slab / 6.0);
     };
     int best_bn = 0;
     const int longest = share_of(a, pick_bn(ctx, a));
-    double least = time_of(a, pick_bn(ctx, a)) * 0.9;
+    const double usual = time_of(a, pick_bn(ctx, a));
+    double least = usual * (alone && a.tf32 ? 0.985 : 0.9);
     auto consider = [&](const GemmArgs& g, int bn) {
         const double t = time_of(g, bn);
-        if (t < least && share_of(g, bn) <= longest) { least = t; *out = g; out->bn = best_bn = bn; }
+        if (t < least && share_of(g, bn) <= longest && !(alone && bn == 384 && kb > 9 * share_of(g, bn))) { least = t; *out = g; out->bn = best_bn = bn; }
     };
     consider(a, 128);
     if (a.N > 128) consider(a, 192);
