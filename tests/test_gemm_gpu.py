@@ -854,3 +854,32 @@ def test_weight_gradient_formed_the_other_way_round(tb, M, N, beta):
     bound = (K / 8 + 4) * 2.0 ** -23 * (A.double().abs().T @ B.double().abs() + beta * C0[:, :N].abs())
     assert bool(((C[:, :N].double() - want).abs() <= bound).all())
     assert torch.equal(C[:, N:], C0[:, N:])
+
+
+def test_products_that_a_cluster_adds_reserve_no_memory_for_their_parts():
+    """The device's scratch memory grows by a device-wide wait and an allocation: not for partial sums that nobody writes."""
+    code = """
+import torch
+from turkce_llm_b200 import lib as tb
+tb.init(0)
+def product(M, N, K, tf32):
+    A, B, C = torch.randn(M, K, device="cuda"), torch.randn(K, N, device="cuda"), torch.zeros(M, N, device="cuda")
+    before = tb.launch_count()
+    if tf32: tb.gemm_f32(tb.NN, A, B, C, M, N, K, K, N, N, precision=tb.PREC_TF32)
+    else: tb.gemm_bf16(tb.NN, A.bfloat16(), B.bfloat16(), M, N, K, K, N, C32=C, ldc32=N, splits=8, tile_n=128)
+    tb.sync_check()
+    assert tb.launch_count() - before == 1
+for tf32 in (False, True):
+    M, N, K = (1408, 256, 1024) if tf32 else (640, 384, 4096)
+    product(128, 128, 512, tf32)          # the kernel's code and a first scratch allocation
+    product(M, N, 64, True)               # torch's own memory (unsplit)
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    product(M, N, K, tf32)
+    torch.cuda.empty_cache()
+    left = torch.cuda.mem_get_info()[0]
+    print("taken", free - left)
+    assert free - left < 4 << 20          # slabs of 7.9 and 8.7 MB, and a quarter
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=ROOT)
+    assert r.returncode == 0, r.stdout + r.stderr

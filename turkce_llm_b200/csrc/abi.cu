@@ -290,9 +290,8 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
         const size_t a_bytes = round_up((size_t)a_stride * batch * 2, 256);
         const size_t b_bytes = round_up((size_t)b_stride * batch * 2, 256);
         g.lda = a_ld; g.ldb = b_ld; g.strideA = a_stride; g.strideB = b_stride;
-        const int splits = planned_splits(ctx, g);
-        g.splits = splits; g.planned = true;
-        const size_t ws_floats = splits > 1 ? (size_t)splits * batch * M * N : 0;
+        size_t ws_floats;
+        g.splits = planned_splits(ctx, g, &ws_floats); g.planned = true;
         TB_TRY(take_scratch(a_bytes + b_bytes + ws_floats * sizeof(float)));
         bf16* pb = reinterpret_cast<bf16*>(scratch);
         bf16* pa = reinterpret_cast<bf16*>(scratch + b_bytes);
@@ -332,9 +331,10 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
     const size_t b_bytes = b_inplace ? 0 : round_up((size_t)b_stride * batch * 4, 256);
     if (split3) g.K = 3 * K;
     g.lda = a_ld; g.ldb = b_ld; g.strideA = a_stride; g.strideB = b_stride;
-    const int splits = planned_splits(ctx, g);
-    g.splits = splits; g.planned = true;
-    const size_t ws_floats = splits > 1 ? (size_t)splits * batch * M * N : 0;
+    if (a_inplace) g.A = A;
+    if (b_inplace) g.B = B;
+    size_t ws_floats;
+    g.splits = planned_splits(ctx, g, &ws_floats); g.planned = true;
     TB_TRY(take_scratch(a_bytes + b_bytes + ws_floats * sizeof(float)));
     float* pb = reinterpret_cast<float*>(scratch);
     float* pa = reinterpret_cast<float*>(scratch + b_bytes);
@@ -350,8 +350,8 @@ static int gemm_f32_impl(int kind, const float* A, const float* B, float* C, int
         if (!b_inplace && !same_b) sides[n++] = {B, pb, b_rows, b_cols, ldb, b_ld, sB, b_stride};
         if (n) TB_TRY(launch_copy_operands(ctx, sides, n, batch, stream));
     }
-    g.A = a_inplace ? static_cast<const void*>(A) : pa;
-    g.B = b_inplace ? static_cast<const void*>(B) : pb;
+    if (!a_inplace) g.A = pa;
+    if (!b_inplace) g.B = pb;
     return launch_gemm_bf16_ws(ctx, g, ws, ws_floats, stream);
 }
 

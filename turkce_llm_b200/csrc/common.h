@@ -183,7 +183,7 @@ bool gemm_norm_pays(const DeviceCtx* ctx, int M, int N, bool tf32);
 // split-K with caller-provided partial-sum storage (needs splits*batch*M*N floats)
 int launch_gemm_bf16_ws(DeviceCtx* ctx, const GemmArgs& a, float* workspace, size_t workspace_floats,
                         cudaStream_t stream);
-int planned_splits(const DeviceCtx* ctx, const GemmArgs& a);
+int planned_splits(const DeviceCtx* ctx, const GemmArgs& a, size_t* slab_floats = nullptr);       // (partial sums in memory that it needs)
 // The product of float32 operands to float32 accuracy in one launch without scratch memory.  The plan says whether it is the faster
 // way, and fills in tile and splits.
 bool plan_gemm_x3(const DeviceCtx* ctx, GemmArgs* a);

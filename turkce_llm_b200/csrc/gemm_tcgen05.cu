@@ -1703,6 +1703,7 @@ static bool cluster_adds(const DeviceCtx* ctx, const GemmArgs& a, int bn, int sp
 static bool output_apart(const GemmArgs& a) {
     const int es = a.tf32 ? 4 : 2;
     auto over = [](const void* x, long long rows, long long cols, long long ld, int size, const void* y, long long yrows, long long ycols, long long yld, int ysize) {
+        if (x == nullptr) return false;          // (an operand that is still to be packed: not the caller's memory)
         const uintptr_t x0 = reinterpret_cast<uintptr_t>(x), x1 = x0 + ((rows - 1) * ld + cols) * size;
         const uintptr_t y0 = reinterpret_cast<uintptr_t>(y), y1 = y0 + ((yrows - 1) * yld + ycols) * ysize;
         return y != nullptr && x0 < y1 && y0 < x1;
@@ -1715,6 +1716,14 @@ static bool output_apart(const GemmArgs& a) {
             return false;
     }
     return true;
+}
+
+static bool added_in_cluster(const DeviceCtx* ctx, const GemmArgs& a, int bn, int splits) {
+    return a.x3 || (cluster_adds(ctx, a, bn, splits) && output_apart(a));
+}
+// partial sums in memory that a product needs
+static size_t slab_floats(const DeviceCtx* ctx, const GemmArgs& a, int bn, int splits) {
+    return splits > 1 && !added_in_cluster(ctx, a, bn, splits) ? (size_t)splits * a.batch * a.M * a.N : 0;
 }
 
 static int choose_splits(const DeviceCtx* ctx, const GemmArgs& a, int bn) {
@@ -1790,11 +1799,14 @@ static bool arranged(const DeviceCtx* ctx, const GemmArgs& a, GemmArgs* out) {
     return best_bn != 0;
 }
 
-int planned_splits(const DeviceCtx* ctx, const GemmArgs& a0) {
+int planned_splits(const DeviceCtx* ctx, const GemmArgs& a0, size_t* slabs) {
+    if (slabs) *slabs = 0;
     if (a0.residual || a0.c_inner > 1) return 1;
     GemmArgs other;
     const GemmArgs& a = arranged(ctx, a0, &other) ? other : a0;
-    return choose_splits(ctx, a, pick_bn(ctx, a));
+    const int bn = pick_bn(ctx, a), splits = choose_splits(ctx, a, bn);
+    if (slabs) *slabs = slab_floats(ctx, a, bn, splits);
+    return splits;
 }
 
 template <int BN, bool TF32, bool PAIR = false, int EPI = EPI_ANY>
@@ -1931,7 +1943,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
     p.a_mn = a_mn; p.b_mn = b_mn; p.causal = (int)a.causal;
     p.dsw = 0; p.wide16 = 0;
     p.err = ctx->d_err;
-    const bool in_cluster = a.x3 || (cluster_adds(ctx, a, bn, splits) && output_apart(a));
+    const bool in_cluster = added_in_cluster(ctx, a, bn, splits);
     p.csplit = in_cluster ? splits : 0;
     if (in_cluster) p.splits = 1;
     if (splits > 1 && !in_cluster) {
@@ -2206,9 +2218,8 @@ int launch_gemm_bf16(DeviceCtx* ctx, const GemmArgs& a0, cudaStream_t stream) {
     int splits = a.splits > 0 ? a.splits : choose_splits(ctx, a, bn);
     TB_TRY(check_splits(a, &splits));
     float* ws = nullptr;
-    if (splits > 1) {
-        const size_t need = (size_t)splits * a.batch * a.M * a.N * sizeof(float);
-        TB_TRY(ensure_scratch(ctx, need));
+    if (const size_t need = slab_floats(ctx, a, bn, splits)) {
+        TB_TRY(ensure_scratch(ctx, need * sizeof(float)));
         ws = static_cast<float*>(ctx->scratch);
     }
     return launch_core(ctx, a, bn, splits, ws, stream);
@@ -2221,8 +2232,7 @@ int launch_gemm_bf16_ws(DeviceCtx* ctx, const GemmArgs& a0, float* workspace, si
     const int bn = pick_bn(ctx, a);
     int splits = a.splits > 0 ? a.splits : choose_splits(ctx, a, bn);
     TB_TRY(check_splits(a, &splits));
-    if (splits > 1) {
-        const size_t need = (size_t)splits * a.batch * a.M * a.N;
+    if (const size_t need = slab_floats(ctx, a, bn, splits)) {
         TB_CHECK(workspace != nullptr && workspace_floats >= need,
                  "split-K workspace too small: need %zu floats, have %zu", need, workspace_floats);
     }
