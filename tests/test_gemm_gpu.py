@@ -622,22 +622,26 @@ def test_splits_added_inside_a_cluster(tb, monkeypatch, kind, shape, precision):
         assert np.array_equal(out[:, N:], C0[:, N:])
         got.append(out)
     if precision == "bf16" and splits:
-        # the same parts in the same order, but bias and previous contents are added to other roundings of alpha times the sum
-        assert np.abs(got[0] - got[1]).max() <= 1e-6 * np.abs(got[1]).max()
+        # the same parts in the same order
+        assert np.array_equal(got[0], got[1])
 
 
-@pytest.mark.parametrize("shape", [(384, 1152, 8192), (1024, 384, 8192), (400, 232, 2608), (384, 1152, 2048), (64, 72, 1100)])
+@pytest.mark.parametrize("shape", [(64, 72, 1100, 4, 64), (200, 72, 1100, 2, 64), (130, 264, 2048, 8, 64), (384, 520, 2048, 4, 128),
+                                   (640, 384, 4096, 8, 128), (640, 376, 2600, 7, 128), (1024, 1152, 1024, 2, 128), (300, 568, 2608, 5, 192),
+                                   (384, 1152, 2048, 6, 192)])
 def test_cluster_sums_round_like_the_reduction_kernel(tb, monkeypatch, shape):
-    """Whoever adds them, the parts of a product are as many and come in the same order: the same bits."""
-    M, N, K = shape
+    """Whoever adds them, the parts of a product are as many and come in the same order: the same bits, in one launch and in two."""
+    M, N, K, splits, bn = shape
     A, B = (torch.randn(r, c, device="cuda").bfloat16() for r, c in ((M, (K + 7) // 8 * 8), (K, N)))
     got = []
     for off in (False, True):
         if off:
             monkeypatch.setenv("TB_GEMM_NO_CLUSTER_SPLIT", "1")
         C = torch.empty(M, N, device="cuda")
-        tb.gemm_bf16(tb.NN, A, B, M, N, K, A.shape[1], N, C32=C, ldc32=N)
+        before = tb.launch_count()
+        tb.gemm_bf16(tb.NN, A, B, M, N, K, A.shape[1], N, C32=C, ldc32=N, splits=splits, tile_n=bn)
         tb.sync_check()
+        assert tb.launch_count() - before == (2 if off else 1)
         got.append(C)
     assert torch.equal(*got)
 
@@ -714,7 +718,7 @@ def test_split_product_over_its_operand(tb, over):
     assert torch.equal(*got)
 
 
-@pytest.mark.parametrize("shape", [(4739, 300, 1190), (7400, 190, 2104), (5000, 1000, 700)])
+@pytest.mark.parametrize("shape", [(4739, 390, 2100), (9601, 190, 2104), (9601, 150, 1190), (8300, 570, 1030), (5000, 1000, 700)])
 @pytest.mark.parametrize("tf32", [False, True], ids=["bf16", "tf32"])
 def test_192_column_tiles_on_cta_pairs(tb, monkeypatch, shape, tf32):
     """B stored [N, K], tiles of 256 x 192: ragged rows, columns and K, previous contents and bias, against float64 and single CTAs.
@@ -736,10 +740,13 @@ def test_192_column_tiles_on_cta_pairs(tb, monkeypatch, shape, tf32):
         if single:
             monkeypatch.setenv("TB_GEMM_NO_PAIR", "1")
         C = C0.clone()
+        tb.profile_begin()
         if tf32:
             tb.gemm_f32(tb.NT, a32, b32, C, M, N, K, ld, ld, N, beta=2.0, precision=tb.PREC_TF32)
         else:
             tb.gemm_bf16(tb.NT, A, B, M, N, K, ld, ld, C32=C, ldc32=N, bias=bias, beta=2.0, tile_n=192)
+        tags = [t for t in tb.profile_end(torch.cuda.current_stream().cuda_stream) if t.startswith("gemm_")]
+        assert len(tags) == 1 and (tags[0].endswith("bn192:pair") != single), tags
         tb.sync_check()
         assert bool(((C.double() - want).abs() <= bound).all())
         got.append(C)

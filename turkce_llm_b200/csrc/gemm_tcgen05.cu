@@ -2081,7 +2081,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
             char tag[128];
             static const char* kn[3] = {"NN", "NT", "TN"};
             snprintf(tag, sizeof(tag), "%s:%s:%dx%dx%d:b%d:s%d:c%d:bn%d%s", a.x3 ? "gemm_x3" : a.tf32 ? "gemm_tf32" : "gemm_bf16",
-                     kn[(int)a.kind], a.M, a.N, a.K, a.batch, splits, (int)a.causal, bn, swiglu ? ":swiglu" : a.rope_qkv ? ":rope" : a.ce_mode == 1 ? ":ce_stats" : a.ce_mode == 2 ? ":ce_grad" : a.norm_w ? ":norm" : "");
+                     kn[(int)a.kind], a.M, a.N, a.K, a.batch, splits, (int)a.causal, bn, swiglu ? ":swiglu" : a.rope_qkv ? ":rope" : a.ce_mode == 1 ? ":ce_stats" : a.ce_mode == 2 ? ":ce_grad" : a.norm_w ? ":norm" : pair && bn == 192 ? ":pair" : "");
             // the second cross-entropy pass repeats pass 1's product: its flops are not algorithmic work
             prof_mark(ctx, prof_intern(tag), a.ce_mode == 2 ? 0.0 : 2.0 * macs, in_bytes + out_bytes, stream);
         }
@@ -2183,8 +2183,8 @@ static int check_splits(const GemmArgs& a, int* splits) {
 //  * several waves, each paying the fixed part again: 8192 x 1152 x 384 52 : 62, 8192 x 2048 x 384 69 : 111, 3000 x 1000 x 1000 42 : 55;
 //  * short K, where little is written out: 64 x 256 x 64 5.6 : 6.0, 256 x 256 x 128 7.1 : 7.5, 240 x 70 x 168 6.7 : 6.8, and with most
 //    SMs taken by unsplit tiles (pair tiles are as fast there) 1024 x 2048 x 384 15.7 : 16.1, 2953 x 492 x 192 12.4 : 12.8.
-// A share of K is at most twice as long as the other way's (two pairs of accumulators): the sums are rounded no more often.
-// 64 x 64 x 8192, one cluster of eight against 148 splits: error 1.0e-6 : 1.6e-6.
+// A share of K is at most twice as long as the other way's (two pairs of accumulators): the sums are rounded no more often.  That keeps
+// products of one tile and a long K (64 x 64 x 8192: 128 splits) on the other way.
 bool plan_gemm_x3(const DeviceCtx* ctx, GemmArgs* a) {
     const int kb = (a->K + BK_TF32 - 1) / BK_TF32;
     if (kb < 6 || a->batch != 1 || a->residual || !a->C32 || getenv("TB_GEMM_NO_X3") != nullptr) return false;
