@@ -801,7 +801,7 @@ for tag in tb.profile_end(torch.cuda.current_stream().cuda_stream):
 
 @pytest.mark.parametrize("outputs", ["C16", "both"])
 @pytest.mark.parametrize("pad", [0, 3], ids=["by_four", "by_one"])
-@pytest.mark.parametrize("shape", [(3, 72, 1024, 8, 64), (16, 136, 1024, 5, 128), (130, 70, 2048, 3, 64), (129, 388, 1024, 2, 192)])
+@pytest.mark.parametrize("shape", [(3, 72, 1024, 8, 64), (16, 136, 1024, 5, 128), (130, 70, 2048, 3, 64), (257, 92, 1024, 2, 128), (129, 388, 1024, 3, 192)])
 def test_cluster_sums_of_few_rows_and_bf16_outputs(tb, monkeypatch, shape, pad, outputs):
     """Fewer rows than CTAs, a last tile of one or two rows, bf16 outputs that can and cannot be written four at a time, with bias and
     previous contents: the bits of the reduction kernel, and nothing written past a row's end."""

@@ -467,7 +467,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             ok = mbar_wait_cluster(&norm_bar[0], 0, abort_flag);
         }
         if (ok) {
-            constexpr int PIECES = BN / 4;                   // 16-byte pieces of a row
+            // 16-byte pieces of a row, those with columns that exist; i / pieces is i * per_piece >> 20 (exact: i < 128 pieces, so i times
+            // what per_piece is rounded up by stays below 2^20 / pieces)
+            const int pieces = (min(BN, p.N - c_first.n0) + 3) >> 2;
+            const uint32_t per_piece = ((1u << 20) + pieces - 1) / pieces;
             const int there = min(BM, p.M - c_first.m0), per = (there + p.csplit - 1) / p.csplit, first = srank * per;       // (rows that exist)
             const int rows = min(there, first + per) - first;
             const uint32_t base = smem_u32(stage_base);
@@ -479,15 +482,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                 for (int k = 0; k < 8; ++k) if (k < p.csplit) { s.x += v[k].x; s.y += v[k].y; s.z += v[k].z; s.w += v[k].w; }
                 return s;
             };
-            // Only rows that exist are shared out, and previous contents and bias are on their way while the parts are (us, with a tile's
+            // Only rows and columns that exist are shared out, and previous contents and bias are on their way while the parts are (us, with a tile's
             // 128 rows shared out and unaligned contents read behind the sum : now; the reduction kernel in brackets): 16 x 384 x 1152 NT
-            // bf16 5.9 : 4.7 [5.8], 64 x 384 x 1024 6.3 : 5.3 [5.9], 303 x 70 over 519 rows, tf32 with beta, 15.2 : 9.0 [11.5].  The code
-            // runs once per launch and its fetches count: outputs that can be addressed by four columns have a loop of their own.
+            // bf16 5.9 : 4.7 [5.8], 64 x 384 x 1024 6.3 : 5.3 [5.9], 7986 x 88 x 1552 12.8 : 10.7 [11.1], 303 x 70 over 519 rows, tf32 with
+            // beta, 15.2 : 8.5 [11.5].  The code runs once per launch and its fetches count: outputs that can be addressed by four
+            // columns have a loop of their own.
             if constexpr (X3) {
                 // (one loop for every output: faster here, 384 x 1152 over 1024 rows 12.8 -> 12.2)
 #pragma unroll 1
-                for (int i = (int)threadIdx.x - 64; i < rows * PIECES; i += EPI_WARPS * 32) {
-                    const int row = first + i / PIECES, c4 = i % PIECES;
+                for (int i = (int)threadIdx.x - 64; i < rows * pieces; i += EPI_WARPS * 32) {
+                    const int r = (int)((uint32_t)i * per_piece >> 20), row = first + r, c4 = i - r * pieces;
                     const uint32_t at = base + (uint32_t)((c4 >> 3) * (BM * ROW_BYTES) + row * ROW_BYTES + (((c4 & 7) ^ (row & 7)) << 4));
                     const int gm = c_first.m0 + row, gn = c_first.n0 + 4 * c4;
                     float* cp = p.C32 + (long long)gm * p.ldc32 + gn;
@@ -524,8 +528,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             } else {
                 auto add_parts = [&](auto by_four) {
 #pragma unroll 1
-                    for (int i = (int)threadIdx.x - 64; i < rows * PIECES; i += EPI_WARPS * 32) {
-                        const int row = first + i / PIECES, c4 = i % PIECES;
+                    for (int i = (int)threadIdx.x - 64; i < rows * pieces; i += EPI_WARPS * 32) {
+                        const int r = (int)((uint32_t)i * per_piece >> 20), row = first + r, c4 = i - r * pieces;
                         const int gm = c_first.m0 + row, gn = c_first.n0 + 4 * c4, left = p.N - gn;
                         constexpr bool vec = decltype(by_four)::value;
                         const bool in = left > 0;
@@ -1691,8 +1695,10 @@ static int cluster_room(const DeviceCtx* ctx, int s) {
 // cluster may not be free together).  As many splits as with the reduction kernel, so sums are rounded as often.  us, reduction kernel :
 // cluster, over 128 products of 16 .. 8192 rows in three operand types 0.64 .. 1.03 of the time, 5 of them above 1.02 (384 x 384 over
 // 2048 rows 7.4 : 7.6): 16 x 384 x 1152 5.8 : 4.7, 700 x 384 x 1024 6.9 : 6.6, 384 x 1152 over 1024 rows 8.7 : 7.6, 384 x 2048 over 8192 18.8 : 18.2.
+// Two CTAs of 192 columns have 64 rows of 48 pieces each to add, twelve steps one after the other, and stay with the kernel: 6200 x 192 x 1104
+// 11.0 : 11.9, 2500 x 576 x 2400 14.6 : 15.2, eight sizes in three layouts 1.01 - 1.09.
 static bool cluster_adds(const DeviceCtx* ctx, const GemmArgs& a, int bn, int splits) {
-    if (splits < 2 || splits > 8 || bn > 192 || a.batch != 1 || a.c_inner > 1 || a.causal != CAUSAL_NONE || a.max_ctas > 0 || (!a.C32 && !a.C16) ||
+    if (splits < 2 || splits > 8 || bn > 192 || (bn == 192 && splits == 2) || a.batch != 1 || a.c_inner > 1 || a.causal != CAUSAL_NONE || a.max_ctas > 0 || (!a.C32 && !a.C16) ||
         a.residual || a.swapped || getenv("TB_GEMM_NO_CLUSTER_SPLIT") != nullptr)
         return false;
     return (long long)((a.M + BM - 1) / BM) * ((a.N + bn - 1) / bn) <= cluster_room(ctx, splits);
@@ -2149,7 +2155,7 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         if (blocks < 1) blocks = 1;
         dim3 grid(blocks, a.batch);
         // (alone on its SMs behind the product it may be launched early whatever its grid; beside another product it would
-        // take that one's thread slots)
+        // take that one's thread slots; a turned reduction has more blocks than that by either kernel's count)
         const bool early = a.max_ctas == 0 || (long long)blocks * a.batch <= kEarlyBlocks;
         prof_mark(ctx, "splitk_reduce", 0.0, (double)(splits + 2) * per * a.batch * 4.0, stream);
         if (a.swapped)
