@@ -1695,10 +1695,13 @@ static int cluster_room(const DeviceCtx* ctx, int s) {
 // cluster may not be free together).  As many splits as with the reduction kernel, so sums are rounded as often.  us, reduction kernel :
 // cluster, over 128 products of 16 .. 8192 rows in three operand types 0.64 .. 1.03 of the time, 5 of them above 1.02 (384 x 384 over
 // 2048 rows 7.4 : 7.6): 16 x 384 x 1152 5.8 : 4.7, 700 x 384 x 1024 6.9 : 6.6, 384 x 1152 over 1024 rows 8.7 : 7.6, 384 x 2048 over 8192 18.8 : 18.2.
-// Two CTAs of 192 columns have 64 rows of 48 pieces each to add, twelve steps one after the other, and stay with the kernel: 6200 x 192 x 1104
-// 11.0 : 11.9, 2500 x 576 x 2400 14.6 : 15.2, eight sizes in three layouts 1.01 - 1.09.
+// Two CTAs have 64 rows each to add, of 128 or 192 columns eight or twelve steps one after the other, and stay with the kernel: 6200 x 192 x 1104
+// 11.0 : 11.9, 2500 x 576 x 2400 14.6 : 15.2, 948 x 968 x 520 8.7 : 9.2, 1024 x 1024 x 1024 8.9 : 9.2, eighteen sizes 1.00 - 1.09.  Not so with
+// previous contents and whole tiles of 128 columns (0.96 - 0.99), nor with fewer columns (7986 x
+// 88 x 1552 11.1 : 10.7), nor where the kernel adds column by column (N no multiple of 4: 0.66 - 0.79).
 static bool cluster_adds(const DeviceCtx* ctx, const GemmArgs& a, int bn, int splits) {
-    if (splits < 2 || splits > 8 || bn > 192 || (bn == 192 && splits == 2) || a.batch != 1 || a.c_inner > 1 || a.causal != CAUSAL_NONE || a.max_ctas > 0 || (!a.C32 && !a.C16) ||
+    if (splits == 2 && std::min(bn, a.N) >= 128 && a.N % 4 == 0 && !(a.C32 && a.beta != 0.0f && bn == 128 && a.N % 128 == 0)) return false;
+    if (splits < 2 || splits > 8 || bn > 192 || a.batch != 1 || a.c_inner > 1 || a.causal != CAUSAL_NONE || a.max_ctas > 0 || (!a.C32 && !a.C16) ||
         a.residual || a.swapped || getenv("TB_GEMM_NO_CLUSTER_SPLIT") != nullptr)
         return false;
     return (long long)((a.M + BM - 1) / BM) * ((a.N + bn - 1) / bn) <= cluster_room(ctx, splits);
