@@ -345,7 +345,7 @@ def test_rmsnorm_is_in_the_epilogues_where_that_is_faster(tb, oracle, monkeypatc
     assert (launches[0] < launches[1]) == fused, launches
 
 
-@pytest.mark.parametrize("T,B", [(31, 9), (32, 9), (34, 8), (45, 7), (64, 6), (777, 2)])
+@pytest.mark.parametrize("T,B", [(13, 9), (24, 9), (31, 9), (32, 9), (33, 8), (34, 8), (45, 7), (64, 6), (777, 2)])
 def test_rotation_tables_by_tma(tb, oracle, monkeypatch, T, B):
     """Cosines and sines that come in by TMA, 32 positions at a time, against those read row by row (64-byte output rows): the same
     bits, also where 32 rows lie in two sequences and where the last rows are missing."""

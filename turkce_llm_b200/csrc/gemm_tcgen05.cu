@@ -2013,10 +2013,11 @@ static int launch_core(DeviceCtx* ctx, const GemmArgs& a, int bn, int splits, fl
         TB_CHECK(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled (QKV output) failed with code %d", (int)r);
         p.tma_mode = 5;
         // The tables come in by TMA where they are one array, the sines behind the cosines (the trainer's and the decoder's are); a
-        // map whose outer stride spans two allocations is not used.  Where most of 32 rows lie in two sequences, a warp's rows go both
-        // ways and the other instantiation is faster (validation loss of 3800 tokens, 12 layers, us, row by row : by TMA: sequences of 31
-        // 854 : 856, 32 836 : 810, 33 852 : 858, 36 847 : 838, 48 809 : 772).
-        if (wide && (a.rope_T >= 34 || a.rope_T == 32) && a.rope_sin == a.rope_cos + (size_t)a.rope_rows * (hd / 2) && a.rope_rows >= a.rope_T && aligned16(a.rope_cos)) {
+        // map whose outer stride spans two allocations is not used.  Where 32 rows lie in two sequences, a warp's rows go both ways, and for
+        // short sequences the other instantiation is faster (validation loss of 3800 and 7800 tokens, 12 layers, us, row by row : by TMA:
+        // sequences of 13 1035 : 1043 and 1683 : 1704, 20 921 : 925 and 1449 : 1445, 24 899 : 894 and 1387 : 1356, 28 863 : 862 and 1336 : 1313,
+        // 32 836 : 810, 33 848 : 853 and 1279 : 1289, 36 847 : 838, 48 809 : 772).
+        if (wide && a.rope_T >= 24 && a.rope_T != 33 && a.rope_sin == a.rope_cos + (size_t)a.rope_rows * (hd / 2) && a.rope_rows >= a.rope_T && aligned16(a.rope_cos)) {
             const cuuint64_t rows = (cuuint64_t)a.rope_rows;
             cuuint64_t tdims[3] = {hd / 2, rows, 2}, tstrides[2] = {hd * 2, rows * hd * 2};
             cuuint32_t tbox[3] = {32u, 32u, 2u};
